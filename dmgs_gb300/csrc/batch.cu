@@ -295,13 +295,16 @@ extern "C" int dmgs_raster_bwd_batched(const DmgsBatch *b, const DmgsGaussians *
   char *st = static_cast<char *>(state);
   BlendBatch bb;
   fill_blend(b, L, same_base(st), bb);
+  ClearViews cv;
   for (int v = 0; v < b->nviews; ++v) {
     bb.v[v].dL_dout = dL_dout_color[v];
-    DMGS_CUDA(cudaMemsetAsync(bb.v[v].gacc, 0, (size_t)g->P * 48, s));
+    const char *geom = st + L.v[v].geom;
+    cv.v[v] = {reinterpret_cast<const uint32_t *>(geom + L.v[v].G.vlist),
+               reinterpret_cast<const uint32_t *>(geom + L.v[v].G.counters), bb.v[v].gacc, (uint32_t)g->P};
   }
   uint32_t *queue = reinterpret_cast<uint32_t *>(st + L.queue) + 1;
   DMGS_CUDA(cudaMemsetAsync(queue, 0, 4, s));
-  RET_IF(launch_blend_batch_bwd(bb, cfg_of(b), queue, s));
+  RET_IF(launch_blend_batch_bwd(bb, cv, ZeroSpans(), cfg_of(b), queue, s));
   BatchViews bv;
   fill_views(b, L, same_base(st), bv);
   for (int v = 0; v < b->nviews; ++v) bv.v[v].dL_dmeans2D = dL_dmeans2D ? dL_dmeans2D[v] : nullptr;

@@ -203,6 +203,7 @@ compact_kernel(const BinViews bv) {
     const int idx = i0 + __ffs(m) - 1;
     B.k0[pos] = __float_as_uint(feat[12 * (size_t)idx + 9]);  // depth: record float 9
     B.v0[pos] = (uint32_t)idx;
+    B.vlist[pos] = (uint32_t)idx;
     ++pos;
   }
 }
@@ -967,6 +968,7 @@ int make_bin_view(const GeomLayout &L, char *geom, uint32_t K_cap, char *bin, ui
   B.blkcnt = reinterpret_cast<uint32_t *>(geom + L.blkcnt);
   B.counters = reinterpret_cast<uint32_t *>(geom + L.counters);
   B.part = reinterpret_cast<uint32_t *>(geom + L.scanpart);
+  B.vlist = reinterpret_cast<uint32_t *>(geom + L.vlist);
   B.k0 = reinterpret_cast<uint32_t *>(geom + L.dkey0);
   B.k1 = reinterpret_cast<uint32_t *>(geom + L.dkey1);
   B.v0 = reinterpret_cast<uint32_t *>(geom + L.dval0);

@@ -568,12 +568,30 @@ __device__ __forceinline__ int slot9(int q) {
 }
 
 
+// The block's share (part of parts) of every span, set to zero.
+__device__ __forceinline__ void zero_spans(const ZeroSpans &z, unsigned part, unsigned parts) {
+  for (int k = 0; k < z.n; ++k) {
+    const size_t n = z.words[k];
+    const size_t chunk = (((n + parts - 1) / parts) + 3) & ~(size_t)3;
+    const size_t a = min(n, chunk * part), e = min(n, a + chunk);
+    float *p = z.p[k];
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {  // a is a multiple of 4 words (or the end)
+      const size_t e4 = a + ((e - a) & ~(size_t)3);
+      for (size_t i = a + 4 * (size_t)threadIdx.x; i < e4; i += 4 * (size_t)blockDim.x)
+        *reinterpret_cast<float4 *>(p + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (size_t i = e4 + threadIdx.x; i < e; i += blockDim.x) p[i] = 0.f;
+    } else {
+      for (size_t i = a + threadIdx.x; i < e; i += blockDim.x) p[i] = 0.f;
+    }
+  }
+}
+
 // F64: the FP64-sum mode — the warp sums are added into double accumulators
 // (V.gacc64), so the result does not depend on the order in which warps and
 // tiles finish to well below float32 resolution.
 template <int PPT, int BATCH, bool F64 = false, int NT = 1>
 __global__ void __launch_bounds__(NT * 256 / PPT, (PPT == 4 ? 10 : (PPT == 2 ? 6 : 4)) / NT)
-blend_bwd_kernel(const BlendBatch bb, uint32_t *queue) {
+blend_bwd_kernel(const BlendBatch bb, const ZeroSpans zero, uint32_t *queue) {
   constexpr int THREADS = 256 / PPT;
   __shared__ float4 S0[NT][BATCH], S1[NT][BATCH], S2[NT][BATCH], S3[NT][BATCH];
   __shared__ uint32_t SM[NT][BATCH];                 // footprint rows
@@ -584,6 +602,7 @@ blend_bwd_kernel(const BlendBatch bb, uint32_t *queue) {
   const int tid = (int)threadIdx.x - h * THREADS;
   const int lane = tid & 31;
   const PixelLayout<PPT> lay(tid);
+  zero_spans(zero, blockIdx.x, gridDim.x);
   int slot_ = 0;
   for (int item = next_item(queue, slot_, &s_item); item < bb.total;
        item = next_item(queue, slot_, &s_item)) {
@@ -707,13 +726,39 @@ int run_fwd(const BlendBatch &bb, uint32_t *queue, cudaStream_t s) {
 }
 
 template <int PPT, int BATCH, bool F64 = false, int NT = 1>
-int run_bwd(const BlendBatch &bb, uint32_t *queue, cudaStream_t s) {
+int run_bwd(const BlendBatch &bb, const ZeroSpans &zero, uint32_t *queue, cudaStream_t s) {
   thread_local int cdev = -1, cslots = 0;  // per kernel instantiation and host thread
   int grid;
   const int r = grid_for(blend_bwd_kernel<PPT, BATCH, F64, NT>, NT * 256 / PPT, bb.total,
                          queue != nullptr, grid, cdev, cslots);
   if (r != DMGS_OK) return r;
-  dmgs_host::note_launch(), blend_bwd_kernel<PPT, BATCH, F64, NT><<<grid, NT * 256 / PPT, 0, s>>>(bb, queue);
+  dmgs_host::note_launch(), blend_bwd_kernel<PPT, BATCH, F64, NT><<<grid, NT * 256 / PPT, 0, s>>>(bb, zero, queue);
+  return DMGS_OK;
+}
+
+// Clears the gradient records of the visible Gaussians, the only ones the
+// adjoints add to or read: 48 B each instead of 48 B for every Gaussian
+// (16 views of 3M Gaussians, 0.14-0.55M visible per view: 0.17 GB written
+// instead of 2.3 GB).
+__global__ void __launch_bounds__(256) clear_gacc_kernel(const ClearViews cv) {
+  const auto &V = cv.v[blockIdx.y];
+  const uint32_t n = min(V.counters[CI_V], V.P);
+  const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (uint32_t s = blockIdx.x * 256 + threadIdx.x; s < n; s += gridDim.x * 256) {
+    const uint32_t id = V.vlist[s];
+    if (id >= V.P) continue;
+    float4 *r = reinterpret_cast<float4 *>(V.gacc + 12 * (size_t)id);
+    r[0] = z; r[1] = z; r[2] = z;
+  }
+}
+
+int launch_clear_gacc(const ClearViews &cv, int nviews, cudaStream_t s) {
+  uint32_t P = 0;
+  for (int v = 0; v < nviews; ++v) P = max(P, cv.v[v].P);
+  if (P == 0) return DMGS_OK;
+  const unsigned grid = min((P + 255) / 256, (unsigned)max(1, 16 * NUM_SMS_HINT / nviews));
+  dmgs_host::note_launch(), clear_gacc_kernel<<<dim3(grid, nviews), 256, 0, s>>>(cv);
+  DMGS_LAUNCH_CHECK("clear_gacc_kernel");
   return DMGS_OK;
 }
 
@@ -725,7 +770,8 @@ __global__ void gacc_round_kernel(const double *__restrict__ g64, float *__restr
 }
 
 template <bool FWD>
-int dispatch(const BlendBatch &bb, const BlendCfg &cfg, uint32_t *queue, cudaStream_t s) {
+int dispatch(const BlendBatch &bb, const ZeroSpans &zero, const BlendCfg &cfg, uint32_t *queue,
+             cudaStream_t s) {
   const bool pair = cfg.sx * cfg.sy == 2;
   if (cfg.sx * cfg.sy > 2 || cfg.sx < 1 || cfg.sy < 1) {
     dmgs_host::set_error("unsupported blend CTA shape: %d x %d tiles", cfg.sx, cfg.sy);
@@ -733,14 +779,14 @@ int dispatch(const BlendBatch &bb, const BlendCfg &cfg, uint32_t *queue, cudaStr
   }
 #define DMGS_BLEND_CASE(P_, B_)                                                     \
   if (!pair && cfg.ppt == P_ && cfg.batch == B_)                                    \
-    return FWD ? run_fwd<P_, B_>(bb, queue, s) : run_bwd<P_, B_>(bb, queue, s);
+    return FWD ? run_fwd<P_, B_>(bb, queue, s) : run_bwd<P_, B_>(bb, zero, queue, s);
   DMGS_BLEND_CASE(1, 128) DMGS_BLEND_CASE(1, 256) DMGS_BLEND_CASE(1, 512)
   DMGS_BLEND_CASE(2, 128) DMGS_BLEND_CASE(2, 256) DMGS_BLEND_CASE(2, 512)
   DMGS_BLEND_CASE(4, 128) DMGS_BLEND_CASE(4, 256) DMGS_BLEND_CASE(4, 512)
 #undef DMGS_BLEND_CASE
 #define DMGS_BLEND_PAIR(P_, B_)                                                     \
   if (pair && cfg.ppt == P_ && cfg.batch == B_)                                     \
-    return FWD ? run_fwd<P_, B_, 2>(bb, queue, s) : run_bwd<P_, B_, false, 2>(bb, queue, s);
+    return FWD ? run_fwd<P_, B_, 2>(bb, queue, s) : run_bwd<P_, B_, false, 2>(bb, zero, queue, s);
   DMGS_BLEND_PAIR(2, 128) DMGS_BLEND_PAIR(2, 256)
   DMGS_BLEND_PAIR(4, 128) DMGS_BLEND_PAIR(4, 256)
 #undef DMGS_BLEND_PAIR
@@ -773,18 +819,19 @@ int launch_blend_batch_fwd(const BlendBatch &bb, const BlendCfg &cfg, uint32_t *
   if (bb.total <= 0) return DMGS_OK;
   int r = DMGS_OK;
   const BlendBatch b = with_shape(bb, cfg);
-  DMGS_TIMED(K_BLEND_FWD, s, r = dispatch<true>(b, cfg, queue, s));
+  DMGS_TIMED(K_BLEND_FWD, s, r = dispatch<true>(b, ZeroSpans(), cfg, queue, s));
   if (r != DMGS_OK) return r;
   DMGS_LAUNCH_CHECK("blend_fwd_kernel");
   return DMGS_OK;
 }
 
-int launch_blend_batch_bwd(const BlendBatch &bb, const BlendCfg &cfg, uint32_t *queue,
-                           cudaStream_t s) {
+int launch_blend_batch_bwd(const BlendBatch &bb, const ClearViews &cv, const ZeroSpans &zero,
+                           const BlendCfg &cfg, uint32_t *queue, cudaStream_t s) {
   if (bb.total <= 0) return DMGS_OK;
-  int r = DMGS_OK;
+  int r = launch_clear_gacc(cv, bb.nviews, s);
+  if (r != DMGS_OK) return r;
   const BlendBatch b = with_shape(bb, cfg);
-  DMGS_TIMED(K_BLEND_BWD, s, r = dispatch<false>(b, cfg, queue, s));
+  DMGS_TIMED(K_BLEND_BWD, s, r = dispatch<false>(b, zero, cfg, queue, s));
   if (r != DMGS_OK) return r;
   DMGS_LAUNCH_CHECK("blend_bwd_kernel");
   return DMGS_OK;
@@ -823,8 +870,7 @@ int launch_blend_fwd(const ViewParams &vp, const GeomLayout &L, const char *geom
 int launch_blend_bwd(const ViewParams &vp, const GeomLayout &L, const char *geom,
                      const BinLayout &B, const char *bin, const ImgLayout &I, const char *img,
                      const float *bg, const float *dL_dout, float *gacc, double *gacc64,
-                     cudaStream_t s) {
-  DMGS_CUDA(cudaMemsetAsync(gacc, 0, (size_t)L.P * 48, s));
+                     const ZeroSpans &zero, cudaStream_t s) {
   BlendBatch bb;
   bb.nviews = 1;
   bb.v[0] = make_blend_view(vp, L, geom, B, bin, I, const_cast<char *>(img), bg);
@@ -832,12 +878,17 @@ int launch_blend_bwd(const ViewParams &vp, const GeomLayout &L, const char *geom
   bb.v[0].gacc = gacc;
   bb.v[0].gacc64 = gacc64;
   bb.total = bb.v[0].T;
-  if (gacc64 == nullptr) return launch_blend_batch_bwd(bb, default_blend_cfg(), nullptr, s);
+  if (gacc64 == nullptr) {
+    ClearViews cv;
+    cv.v[0] = {reinterpret_cast<const uint32_t *>(geom + L.vlist),
+               reinterpret_cast<const uint32_t *>(geom + L.counters), gacc, (uint32_t)L.P};
+    return launch_blend_batch_bwd(bb, cv, zero, default_blend_cfg(), nullptr, s);
+  }
   const size_t n = (size_t)L.P * 12;
   DMGS_CUDA(cudaMemsetAsync(gacc64, 0, n * sizeof(double), s));
   if (bb.total > 0) {
     int r = DMGS_OK;
-    DMGS_TIMED(K_BLEND_BWD, s, r = (run_bwd<4, 128, true>(bb, nullptr, s)));
+    DMGS_TIMED(K_BLEND_BWD, s, r = (run_bwd<4, 128, true>(bb, zero, nullptr, s)));
     if (r != DMGS_OK) return r;
     DMGS_LAUNCH_CHECK("blend_bwd_kernel (FP64 sums)");
   }

@@ -294,9 +294,10 @@ int raster_bwd_impl(const DmgsView *view, const DmgsGaussians *g, const float *d
                                                     bwd_scratch_bytes(g->P))
                        : nullptr;
   const ViewParams vp = make_params(view);
-  RET_IF(launch_blend_bwd(vp, L, geom, B, bin, I, img, view->bg, dL_dout_color, gacc, gacc64, s));
+  const DmgsGrads out = *grads;
+  RET_IF(launch_blend_bwd(vp, L, geom, B, bin, I, img, view->bg, dL_dout_color, gacc, gacc64,
+                          preprocess_bwd_outputs(out, g->P, g->M), s));
   RET_IF(debug_sync(view, s, "blend_bwd"));
-  DmgsGrads out = *grads;
   RET_IF(launch_preprocess_bwd(vp, view->viewmatrix, view->projmatrix, view->campos,
                                make_gptrs(g), L, geom, gacc, out, s));
   RET_IF(debug_sync(view, s, "preprocess_bwd"));

@@ -83,6 +83,7 @@ constexpr int CI_NRC = 9;      // row-count entries = gy * C
 constexpr int CI_WORDS = 16;
 
 // Geometry state of one view.  Binning arrays: per-block visible counts;
+// the visible Gaussians in index order (vlist, kept for the adjoint);
 // (depth bits, index) ping-pong pairs of the radix sort; radix histograms;
 // per depth-sorted position the packed tile rectangle (srect, 8 B); chunk
 // starts; the row counts [gy][C] (Gaussians of chunk c covering tile row r,
@@ -90,7 +91,7 @@ constexpr int CI_WORDS = 16;
 // (instances of tile t from row segment s, scanned in place into list
 // offsets); scan partials; tile ranges; counters.
 struct GeomLayout {
-  size_t feat, flags, blkcnt, dkey0, dkey1, dval0, dval1, rhist, srect, cstart, rcnt, cnt2,
+  size_t feat, flags, blkcnt, vlist, dkey0, dkey1, dval0, dval1, rhist, srect, cstart, rcnt, cnt2,
       scanpart, ranges, counters, total;
   int P, gx, gy;
   int nb_pre, nb_radix;
@@ -118,6 +119,7 @@ __host__ __device__ inline GeomLayout geom_layout(int P, int W, int H) {
   L.feat = o;      o = align_up(o + (size_t)P * 48, 256);
   L.flags = o;     o = align_up(o + (size_t)P, 256);
   L.blkcnt = o;    o = align_up(o + (size_t)L.nb_pre * 4 + 4, 256);
+  L.vlist = o;     o = align_up(o + (size_t)P * 4, 256);
   L.dkey0 = o;     o = align_up(o + (size_t)P * 4, 256);
   L.dkey1 = o;     o = align_up(o + (size_t)P * 4, 256);
   L.dval0 = o;     o = align_up(o + (size_t)P * 4, 256);

@@ -53,7 +53,7 @@ struct BinView {
   uint32_t n_rhist_max, n_rcnt_max;
   const uint8_t *flags;
   const float4 *feat;
-  uint32_t *blkcnt, *counters, *part, *k0, *k1, *v0, *v1, *rhist, *cstart, *rcnt, *cnt2;
+  uint32_t *blkcnt, *counters, *part, *vlist, *k0, *k1, *v0, *v1, *rhist, *cstart, *rcnt, *cnt2;
   uint2 *srect;          // packed tile rectangle per depth-sorted position
   uint2 *ranges;
   uint32_t *point_list;  // emission target (K_alloc entries)
@@ -123,6 +123,28 @@ struct BlendView {
   double *gacc64;       // adjoint in FP64-sum mode: [P][12] double accumulators (else null)
 };
 
+// Each view's visible Gaussians (index-ordered list, the counters holding
+// their number) and gradient records: what the adjoint clears first.
+struct ClearViews {
+  struct {
+    const uint32_t *vlist, *counters;
+    float *gacc;
+    uint32_t P;
+  } v[MAX_BATCH_VIEWS];
+};
+
+// Arrays the blend adjoint sets to zero while it runs (its stores meet an
+// idle DRAM): the outputs of which the preprocess adjoint then writes only
+// the visible Gaussians' rows.
+struct ZeroSpans {
+  int n = 0;
+  float *p[8];
+  size_t words[8];
+  void add(float *q, size_t w) {
+    if (q && w) { p[n] = q; words[n++] = w; }
+  }
+};
+
 struct BlendBatch {
   int nviews, total;    // views, work items (sum of tiles, or of CTA cells)
   int sx = 1, sy = 1;   // tiles per CTA along x and y (set by the launchers)
@@ -143,8 +165,10 @@ inline BlendCfg default_blend_cfg() { return BlendCfg{4, 128, 1, 1}; }  // autot
 // items from *queue (which must be zero at launch).
 int launch_blend_batch_fwd(const BlendBatch &bb, const BlendCfg &cfg, uint32_t *queue,
                            cudaStream_t s);
-int launch_blend_batch_bwd(const BlendBatch &bb, const BlendCfg &cfg, uint32_t *queue,
-                           cudaStream_t s);
+// Clears the visible Gaussians' gradient records (cv) and runs the adjoint,
+// which also sets the arrays of `zero` to zero.
+int launch_blend_batch_bwd(const BlendBatch &bb, const ClearViews &cv, const ZeroSpans &zero,
+                           const BlendCfg &cfg, uint32_t *queue, cudaStream_t s);
 int launch_blend_fwd(const ViewParams &vp, const GeomLayout &L, const char *geom,
                      const BinLayout &B, const char *bin, const ImgLayout &I, char *img,
                      const float *bg, float *out_color, cudaStream_t s);
@@ -153,11 +177,14 @@ int launch_blend_fwd(const ViewParams &vp, const GeomLayout &L, const char *geom
 int launch_blend_bwd(const ViewParams &vp, const GeomLayout &L, const char *geom,
                      const BinLayout &B, const char *bin, const ImgLayout &I, const char *img,
                      const float *bg, const float *dL_dout, float *gacc, double *gacc64,
-                     cudaStream_t s);
+                     const ZeroSpans &zero, cudaStream_t s);
 
 // preprocess_bwd.cu
 int launch_preprocess_bwd_batched(const BatchViews &bv, const GaussianPtrs &g, const DmgsGrads &out,
                                   float *densify_accum, float *densify_count, cudaStream_t s);
+// The outputs of a single-view adjoint, to be zero before launch_preprocess_bwd
+// writes the visible Gaussians' rows.
+ZeroSpans preprocess_bwd_outputs(const DmgsGrads &out, int P, int M);
 int launch_preprocess_bwd(const ViewParams &vp, const float *viewm, const float *projm,
                           const float *campos, const GaussianPtrs &g, const GeomLayout &L,
                           const char *geom, const float *gacc, const DmgsGrads &out,

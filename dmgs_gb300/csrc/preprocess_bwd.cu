@@ -14,10 +14,9 @@
 //   rgb = max(0, SH(dir) + 0.5)      -> dL/dsh, dL/dm through dir = unit(m - campos)
 //   Sigma = (R S)(R S)^T             -> dL/dscale, dL/dquaternion (unnormalised)
 // Culled Gaussians (radius 0, empty rectangle in the geometry state) get
-// zeros in every output.  Results are staged in shared memory and each
-// block stores its contiguous slice of every output array with coalesced
-// writes (most Gaussians are culled: their outputs are zero-filled at full
-// bandwidth instead of by strided per-thread stores).
+// zeros in every output.
+#include <algorithm>
+
 #include "kernels.cuh"
 
 namespace dmgs {
@@ -25,30 +24,6 @@ namespace dmgs {
 namespace {
 
 constexpr int BWD_BLOCK = 128;
-constexpr int SP = BWD_BLOCK + 1;  // shared-memory row pitch of the output slots
-
-// Shared-memory output slots of one block: element k of Gaussian g of a
-// field lives at field[k * SP + g].  Lanes writing element k of different
-// Gaussians hit consecutive banks, and the pitch of BWD_BLOCK + 1 keeps the
-// Gaussian-major reads of the stores (consecutive k of one g) conflict-free.
-struct Slots {
-  float *m2, *col, *op, *m3, *cov, *sc, *rot, *sh;
-};
-
-__host__ __device__ constexpr size_t slot_floats(int M) { return (size_t)(23 + 3 * M) * SP; }
-
-__device__ __forceinline__ Slots make_slots(float *sm) {
-  Slots S;
-  S.m2 = sm;
-  S.col = S.m2 + 3 * SP;
-  S.op = S.col + 3 * SP;
-  S.m3 = S.op + SP;
-  S.cov = S.m3 + 3 * SP;
-  S.sc = S.cov + 6 * SP;
-  S.rot = S.sc + 3 * SP;
-  S.sh = S.rot + 4 * SP;
-  return S;
-}
 
 // Calls term(k, b_k, db_k/dx, db_k/dy, db_k/dz) for every SH basis function
 // of degree <= D at the unit direction (x, y, z) (the real SH basis with the
@@ -85,36 +60,28 @@ __device__ __forceinline__ void for_each_sh_term(int D, float x, float y, float 
   }
 }
 
-// ACC: add into the slots (several views of one Gaussian, possibly from
-// several threads at once: a shared-memory atomic add); else assign.
-template <bool ACC>
-__device__ __forceinline__ void put(float &slot, float v) {
-  if (ACC) atomicAdd(&slot, v);
-  else slot = v;
-}
-
-// SH: also the SH adjoint (dL/dsh and the direction term of dL/dmean);
-// without it the caller handles the SH colour's adjoint.
-template <bool ACC, bool SH = true>
+// Geometric adjoint of one (Gaussian, view) pair: every gradient but the SH
+// colour's, handed to sink (color, opacity, cov, scale, rot: element index
+// and value); the mean's gradient is returned in dm, where the caller adds
+// the SH direction term, and the colour's in drgb.
+template <typename Sink>
 __device__ __forceinline__ void
-preprocess_bwd_one(int idx, int t, const ViewParams &vp, const float *__restrict__ viewm_g,
-                   const float *__restrict__ projm_g, const float *__restrict__ campos_g, int M,
-                   const float *__restrict__ means, const float *__restrict__ shs,
+preprocess_bwd_one(int idx, const ViewParams &vp, const float *__restrict__ viewm_g,
+                   const float *__restrict__ projm_g, const float *__restrict__ means,
                    const float *__restrict__ scales, const float *__restrict__ rots,
-                   const float *__restrict__ cov3D, const uint8_t *__restrict__ flags,
-                   const float *__restrict__ gacc, const DmgsGrads &out, const Slots &S_) {
-  const int nsh = (vp.D + 1) * (vp.D + 1);
+                   const float *__restrict__ cov3D, const float *__restrict__ gacc,
+                   const DmgsGrads &out, const Sink &sink, float (&dm)[3], float (&drgb)[3]) {
   const float4 ga = reinterpret_cast<const float4 *>(gacc)[3 * idx];
   const float4 gb = reinterpret_cast<const float4 *>(gacc)[3 * idx + 1];
   const float gblue = gacc[12 * idx + 8];
   const float dndc_x = ga.x, dndc_y = ga.y;
   const float dca = ga.z, dcb = ga.w, dcc = gb.x;
   const float dop = gb.y;
-  float drgb[3] = {gb.z, gb.w, gblue};
+  drgb[0] = gb.z; drgb[1] = gb.w; drgb[2] = gblue;
 
-  if (out.dL_dmeans2D && !ACC) { S_.m2[t] = dndc_x; S_.m2[SP + t] = dndc_y; S_.m2[2 * SP + t] = 0.f; }
-  if (out.dL_dopacity) put<ACC>(S_.op[t], dop);
-  if (out.dL_dcolors) { put<ACC>(S_.col[t], drgb[0]); put<ACC>(S_.col[SP + t], drgb[1]); put<ACC>(S_.col[2 * SP + t], drgb[2]); }
+  sink.mean2d(dndc_x, dndc_y);
+  if (out.dL_dopacity) sink.opacity(dop);
+  if (out.dL_dcolors) { sink.color(0, drgb[0]); sink.color(1, drgb[1]); sink.color(2, drgb[2]); }
 
   float V[16], Pm[16];
 #pragma unroll
@@ -206,9 +173,8 @@ preprocess_bwd_one(int idx, int t, const ViewParams &vp, const float *__restrict
 #pragma unroll
     for (int j = 0; j < 3; ++j) dS[i * 3 + j] = T[0][i] * GT[0][j] + T[1][i] * GT[1][j];
   if (out.dL_dcov3D) {
-    float *o = S_.cov + t;
-    put<ACC>(o[0], dS[0]); put<ACC>(o[SP], 2.f * dS[1]); put<ACC>(o[2 * SP], 2.f * dS[2]);
-    put<ACC>(o[3 * SP], dS[4]); put<ACC>(o[4 * SP], 2.f * dS[5]); put<ACC>(o[5 * SP], dS[8]);
+    sink.cov(0, dS[0]); sink.cov(1, 2.f * dS[1]); sink.cov(2, 2.f * dS[2]);
+    sink.cov(3, dS[4]); sink.cov(4, 2.f * dS[5]); sink.cov(5, dS[8]);
   }
 
   // dL/dT = 2 Gs T Sigma
@@ -231,7 +197,6 @@ preprocess_bwd_one(int idx, int t, const ViewParams &vp, const float *__restrict
   const float dty = ymul * (-vp.fy * inv2) * dJ12;
   const float dtz = -vp.fx * inv2 * dJ00 - vp.fy * inv2 * dJ11 +
                     2.f * vp.fx * tx * inv3 * dJ02 + 2.f * vp.fy * ty * inv3 * dJ12;
-  float dm[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) dm[k] = V[4 * k] * dtx + V[4 * k + 1] * dty + V[4 * k + 2] * dtz;
 
@@ -248,43 +213,6 @@ preprocess_bwd_one(int idx, int t, const ViewParams &vp, const float *__restrict
       const float jy = Pm[4 * k + 1] * mw - hy * mw2 * Pm[4 * k + 3];
       dm[k] += dndc_x * jx + dndc_y * jy;
     }
-  }
-
-  // --- SH colour ---------------------------------------------------------
-  if (SH && shs != nullptr) {
-    const uint8_t cl = flags[idx];
-    if (cl & 1) drgb[0] = 0.f;
-    if (cl & 2) drgb[1] = 0.f;
-    if (cl & 4) drgb[2] = 0.f;
-    const float vx_ = mx - campos_g[0], vy_ = my - campos_g[1], vz_ = mz - campos_g[2];
-    const float len = sqrtf(vx_ * vx_ + vy_ * vy_ + vz_ * vz_);
-    const float il = 1.f / len;
-    const float x = vx_ * il, y = vy_ * il, z = vz_ * il;
-    const float *sh = shs + (size_t)idx * M * 3;
-    float *dsh = out.dL_dsh ? S_.sh + t : nullptr;
-    // basis value b_k and its partial derivatives (bx, by, bz) w.r.t. the
-    // unnormalised-direction components x, y, z
-    float gdx = 0.f, gdy = 0.f, gdz = 0.f;
-    auto term = [&](int k, float b, float bx, float by, float bz) {
-      const float s0 = sh[3 * k], s1 = sh[3 * k + 1], s2 = sh[3 * k + 2];
-      if (dsh) { put<ACC>(dsh[3 * k * SP], b * drgb[0]); put<ACC>(dsh[(3 * k + 1) * SP], b * drgb[1]); put<ACC>(dsh[(3 * k + 2) * SP], b * drgb[2]); }
-      const float dot = s0 * drgb[0] + s1 * drgb[1] + s2 * drgb[2];
-      gdx += bx * dot; gdy += by * dot; gdz += bz * dot;
-    };
-    for_each_sh_term(vp.D, x, y, z, term);
-    if (dsh)
-      if (!ACC) for (int i = 3 * nsh; i < 3 * M; ++i) dsh[i * SP] = 0.f;
-    // d unit(v)/dv . g = (g - u (u . g)) / |v|
-    const float ug = x * gdx + y * gdy + z * gdz;
-    dm[0] += (gdx - x * ug) * il;
-    dm[1] += (gdy - y * ug) * il;
-    dm[2] += (gdz - z * ug) * il;
-  }
-
-  if (out.dL_dmeans3D) {
-    put<ACC>(S_.m3[t], dm[0]);
-    put<ACC>(S_.m3[SP + t], dm[1]);
-    put<ACC>(S_.m3[2 * SP + t], dm[2]);
   }
 
   // --- scale / rotation --------------------------------------------------
@@ -304,8 +232,7 @@ preprocess_bwd_one(int idx, int t, const ViewParams &vp, const float *__restrict
     if (out.dL_dscales) {
 #pragma unroll
       for (int j = 0; j < 3; ++j)
-        put<ACC>(S_.sc[j * SP + t],
-                 vp.scale_modifier * (dM[j] * R[j] + dM[3 + j] * R[3 + j] + dM[6 + j] * R[6 + j]));
+        sink.scale(j, vp.scale_modifier * (dM[j] * R[j] + dM[3 + j] * R[3 + j] + dM[6 + j] * R[6 + j]));
     }
     if (out.dL_drotations) {
       float G[9];
@@ -321,71 +248,157 @@ preprocess_bwd_one(int idx, int t, const ViewParams &vp, const float *__restrict
                               z * G[7] - 2.f * y * G[8]);
       const float dz = 2.f * (-2.f * z * G[0] - r * G[1] + x * G[2] + r * G[3] - 2.f * z * G[4] +
                               y * G[5] + x * G[6] + y * G[7]);
-      { put<ACC>(S_.rot[t], dr); put<ACC>(S_.rot[SP + t], dx); put<ACC>(S_.rot[2 * SP + t], dy); put<ACC>(S_.rot[3 * SP + t], dz); }
+      sink.rot(dr, dx, dy, dz);
     }
   }
 }
 
 
-// Stores the block's contiguous slice of one output array (n elements per
-// Gaussian): element i of the slice is element i % n of Gaussian i / n;
-// Gaussians culled in every view get zeros (their slots are never written).
-__device__ __forceinline__ void store_slice(float *dst, const float *src, int n, int start,
-                                            int nvalid, const uint32_t *vmask) {
-  if (!dst) return;
-  float *d = dst + (size_t)start * n;
-  const int cnt = nvalid * n;
-  // ceil(2^32 / n) for n >= 2; i / n = umulhi(i, magic) exactly for i, n < 2^16
-  const uint32_t magic = n > 1 ? (uint32_t)(0xffffffffull / (uint32_t)n) + 1u : 0u;
-  auto gauss = [&](int i) { return n > 1 ? (int)__umulhi((uint32_t)i, magic) : i; };
-  auto vis = [&](int g) { return (vmask[g >> 5] >> (g & 31)) & 1u; };
-  if ((n & 3) == 0 && (cnt & 3) == 0 && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {
-    // whole float4s never straddle two Gaussians when n % 4 == 0
-    float4 *d4 = reinterpret_cast<float4 *>(d);
-    for (int i = threadIdx.x; i < (cnt >> 2); i += BWD_BLOCK) {
-      const int g = gauss(i << 2), k = (i << 2) - g * n;
-      const float *s = src + k * SP + g;
-      d4[i] = vis(g) ? make_float4(s[0], s[SP], s[2 * SP], s[3 * SP]) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  } else {
-    for (int i = threadIdx.x; i < cnt; i += BWD_BLOCK) {
-      const int g = gauss(i), k = i - g * n;
-      d[i] = vis(g) ? src[k * SP + g] : 0.f;
-    }
-  }
+// SH adjoint of one view at mean (mx, my, mz): put(j, v) receives element j
+// of dL/dsh (3 per coefficient), sh(j) reads the input's; the direction's
+// term is added to the mean gradient dm.  drgb is the gradient of the colour
+// before its clamp at zero.
+template <typename Read, typename Put>
+__device__ __forceinline__ void sh_bwd(int D, float mx, float my, float mz, const float *cam,
+                                       const float (&drgb)[3], Read &&sh, Put &&put, float (&dm)[3]) {
+  const float vx_ = mx - cam[0], vy_ = my - cam[1], vz_ = mz - cam[2];
+  const float len = sqrtf(vx_ * vx_ + vy_ * vy_ + vz_ * vz_);
+  const float il = 1.f / len;
+  const float x = vx_ * il, y = vy_ * il, z = vz_ * il;
+  float gdx = 0.f, gdy = 0.f, gdz = 0.f;
+  for_each_sh_term(D, x, y, z, [&](int k, float b, float bx, float by, float bz) {
+    const float s0 = sh(3 * k), s1 = sh(3 * k + 1), s2 = sh(3 * k + 2);
+    put(3 * k, b * drgb[0]);  // may overwrite what sh() reads
+    put(3 * k + 1, b * drgb[1]);
+    put(3 * k + 2, b * drgb[2]);
+    const float dot = s0 * drgb[0] + s1 * drgb[1] + s2 * drgb[2];
+    gdx += bx * dot; gdy += by * dot; gdz += bz * dot;
+  });
+  // d unit(v)/dv . g = (g - u (u . g)) / |v|
+  const float ug = x * gdx + y * gdy + z * gdz;
+  dm[0] += (gdx - x * ug) * il;
+  dm[1] += (gdy - y * ug) * il;
+  dm[2] += (gdz - z * ug) * il;
 }
 
-__global__ void __launch_bounds__(BWD_BLOCK)
-preprocess_bwd_kernel(ViewParams vp, const float *__restrict__ viewm_g,
-                      const float *__restrict__ projm_g, const float *__restrict__ campos_g,
-                      int P, int M, const float *__restrict__ means,
-                      const float *__restrict__ shs, const float *__restrict__ scales,
-                      const float *__restrict__ rots, const float *__restrict__ cov3D,
-                      const uint8_t *__restrict__ flags, const float *__restrict__ gacc,
-                      DmgsGrads out) {
+__device__ __forceinline__ void apply_clamp(uint32_t flags, float (&drgb)[3]) {
+  if (flags & 1) drgb[0] = 0.f;
+  if (flags & 2) drgb[1] = 0.f;
+  if (flags & 4) drgb[2] = 0.f;
+}
+
+// Single-view adjoint, one thread per visible Gaussian of the
+// (index-ordered) visible list; the outputs are zero already (the blend adjoint cleared them while
+// it ran).  Only ~5-20% of a large scene's Gaussians are visible in a view,
+// so a thread per Gaussian ran the ~1,500 instructions of the chain in warps
+// of which two lanes in thirty-two had work, and wrote the zeros of the rest
+// itself: 273 us at 3M Gaussians (0.14M visible), bound by issue.  Dense
+// lanes leave the gathers and the rows written (600 B per visible Gaussian).
+// The SH rows are staged per warp in shared memory so that each row's 192
+// bytes go out as whole sectors.
+constexpr int SH_COEFFS_MAX = 124;  // coefficients per Gaussian accepted by the single-view adjoint
+constexpr int SHP = 49;  // staging row pitch in floats: lanes writing element j hit different banks
+
+struct RowSink {
+  float *m2_, *col_, *op_, *cov_, *sc_, *rot_;  // this Gaussian's row of each output (or null)
+  __device__ __forceinline__ void mean2d(float x, float y) const { if (m2_) { m2_[0] = x; m2_[1] = y; } }
+  __device__ __forceinline__ void opacity(float v) const { *op_ = v; }
+  __device__ __forceinline__ void color(int k, float v) const { col_[k] = v; }
+  __device__ __forceinline__ void cov(int k, float v) const { cov_[k] = v; }
+  __device__ __forceinline__ void scale(int k, float v) const { sc_[k] = v; }
+  __device__ __forceinline__ void rot(float r, float x, float y, float z) const {
+    *reinterpret_cast<float4 *>(rot_) = make_float4(r, x, y, z);
+  }
+};
+
+__global__ void __launch_bounds__(BWD_BLOCK, 5)
+preprocess_bwd_list_kernel(ViewParams vp, const float *__restrict__ viewm_g,
+                           const float *__restrict__ projm_g, const float *__restrict__ campos_g,
+                           int P, int M, const float *__restrict__ means,
+                           const float *__restrict__ shs, const float *__restrict__ scales,
+                           const float *__restrict__ rots, const float *__restrict__ cov3D,
+                           const uint8_t *__restrict__ flags, const float *__restrict__ gacc,
+                           const uint32_t *__restrict__ vlist, const uint32_t *__restrict__ counters,
+                           DmgsGrads out) {
   extern __shared__ float sm[];
-  __shared__ uint32_t vmask[BWD_BLOCK / 32];
-  const int B = BWD_BLOCK;
-  const int t = threadIdx.x;
-  const int start = blockIdx.x * B;
-  const int idx = start + t;
-  const Slots S_ = make_slots(sm);
-  const bool vis = idx < P && (flags[idx] & FLAG_VISIBLE);
-  const uint32_t bal = __ballot_sync(0xffffffffu, vis);
-  if ((t & 31) == 0) vmask[t >> 5] = bal;
-  if (vis)
-    preprocess_bwd_one<false>(idx, t, vp, viewm_g, projm_g, campos_g, M, means, shs, scales, rots,
-                              cov3D, flags, gacc, out, S_);
-  __syncthreads();
-  const int nvalid = min(B, P - start);
-  store_slice(out.dL_dmeans2D, S_.m2, 3, start, nvalid, vmask);
-  store_slice(out.dL_dcolors, S_.col, 3, start, nvalid, vmask);
-  store_slice(out.dL_dopacity, S_.op, 1, start, nvalid, vmask);
-  store_slice(out.dL_dmeans3D, S_.m3, 3, start, nvalid, vmask);
-  store_slice(out.dL_dcov3D, S_.cov, 6, start, nvalid, vmask);
-  store_slice(out.dL_dscales, S_.sc, 3, start, nvalid, vmask);
-  store_slice(out.dL_drotations, S_.rot, 4, start, nvalid, vmask);
-  store_slice(out.dL_dsh, S_.sh, 3 * M, start, nvalid, vmask);
+  const int lane = threadIdx.x & 31;
+  float *st = sm + (threadIdx.x >> 5) * (32 * SHP);
+  const uint32_t V = min(counters[CI_V], (uint32_t)P);
+  const int nsh3 = 3 * (vp.D + 1) * (vp.D + 1);
+  const int n4 = (nsh3 + 3) / 4;  // float4s of a staged row
+  const bool want_dsh = shs != nullptr && out.dL_dsh != nullptr;
+  const bool vec_in = (M & 3) == 0 && (reinterpret_cast<uintptr_t>(shs) & 15) == 0;
+  const bool vec_out = (M & 3) == 0 && (reinterpret_cast<uintptr_t>(out.dL_dsh) & 15) == 0;
+  auto row = [](float *base, int n, size_t i) { return base ? base + n * i : nullptr; };
+  for (uint32_t s0 = blockIdx.x * BWD_BLOCK + (threadIdx.x & ~31); s0 < V; s0 += gridDim.x * BWD_BLOCK) {
+    const uint32_t s = s0 + lane;
+    uint32_t id = s < V ? vlist[s] : 0xffffffffu;
+    if (id >= (uint32_t)P) id = 0xffffffffu;
+    if (shs != nullptr) {  // the group's SH rows into the staging rows, whole sectors at a time
+      if (vec_in) {
+        for (int q = lane; q < 32 * n4; q += 32) {
+          const int r = q / n4, c = q - r * n4;
+          const uint32_t rid = __shfl_sync(0xffffffffu, id, r);
+          if (rid == 0xffffffffu) continue;
+          const float4 v = __ldg(reinterpret_cast<const float4 *>(shs + (size_t)rid * M * 3) + c);
+          float *e = st + r * SHP + 4 * c;
+          e[0] = v.x; e[1] = v.y; e[2] = v.z; e[3] = v.w;
+        }
+      } else {
+        for (int q = lane; q < 32 * nsh3; q += 32) {
+          const int r = q / nsh3, c = q - r * nsh3;
+          const uint32_t rid = __shfl_sync(0xffffffffu, id, r);
+          if (rid != 0xffffffffu) st[r * SHP + c] = __ldg(shs + (size_t)rid * M * 3 + c);
+        }
+      }
+    }
+    __syncwarp();
+    if (id != 0xffffffffu) {
+      const size_t i = id;
+      RowSink sink;
+      sink.m2_ = row(out.dL_dmeans2D, 3, i);
+      sink.col_ = row(out.dL_dcolors, 3, i);
+      sink.op_ = row(out.dL_dopacity, 1, i);
+      sink.cov_ = row(out.dL_dcov3D, 6, i);
+      sink.sc_ = row(out.dL_dscales, 3, i);
+      sink.rot_ = row(out.dL_drotations, 4, i);
+      float dm[3], drgb[3];
+      preprocess_bwd_one((int)id, vp, viewm_g, projm_g, means, scales, rots, cov3D, gacc, out, sink, dm, drgb);
+      if (shs != nullptr) {
+        apply_clamp(flags[id], drgb);
+        sh_bwd(vp.D, means[3 * i], means[3 * i + 1], means[3 * i + 2], campos_g, drgb,
+               [&](int j) { return st[lane * SHP + j]; },
+               [&](int j, float v) { st[lane * SHP + j] = v; }, dm);
+      }
+      if (out.dL_dmeans3D) {
+        float *d = out.dL_dmeans3D + 3 * i;
+        d[0] = dm[0]; d[1] = dm[1]; d[2] = dm[2];
+      }
+    }
+    if (!want_dsh) {  // block-uniform
+      __syncwarp();
+      continue;
+    }
+    if (id != 0xffffffffu)
+      for (int j = nsh3; j < 4 * n4; ++j) st[lane * SHP + j] = 0.f;
+    __syncwarp();
+    if (vec_out) {
+      for (int q = lane; q < 32 * n4; q += 32) {
+        const int r = q / n4, c = q - r * n4;
+        const uint32_t rid = __shfl_sync(0xffffffffu, id, r);
+        const float *e = st + r * SHP + 4 * c;
+        if (rid != 0xffffffffu)
+          reinterpret_cast<float4 *>(out.dL_dsh + (size_t)rid * M * 3)[c] = make_float4(e[0], e[1], e[2], e[3]);
+      }
+    } else {
+      for (int q = lane; q < 32 * nsh3; q += 32) {
+        const int r = q / nsh3, c = q - r * nsh3;
+        const uint32_t rid = __shfl_sync(0xffffffffu, id, r);
+        if (rid != 0xffffffffu) out.dL_dsh[(size_t)rid * M * 3 + c] = st[r * SHP + c];
+      }
+    }
+    __syncwarp();  // the staged rows are overwritten by the next group
+  }
 }
 
 // Multi-view adjoint: the gradients of all views of a batch, summed.  A
@@ -406,6 +419,22 @@ preprocess_bwd_kernel(ViewParams vp, const float *__restrict__ viewm_g,
 // 2D gradients are loaded at once (independent loads), then written out,
 // zero where the Gaussian is not visible.
 constexpr int ACC_SLOTS = 14;  // colour 3, opacity 1, mean 3, scale 3 + rotation 4 (or covariance 6)
+constexpr int SP = BWD_BLOCK + 1;  // pitch of a slot's row of the block's Gaussians
+
+// The Gaussian's sums: slot k of Gaussian t at acc[k * SP + t].
+struct SlotSink {
+  float *acc;  // + t
+  __device__ __forceinline__ void mean2d(float, float) const {}
+  __device__ __forceinline__ void color(int k, float v) const { atomicAdd(acc + k * SP, v); }
+  __device__ __forceinline__ void opacity(float v) const { atomicAdd(acc + 3 * SP, v); }
+  __device__ __forceinline__ void mean(int k, float v) const { atomicAdd(acc + (4 + k) * SP, v); }
+  __device__ __forceinline__ void scale(int k, float v) const { atomicAdd(acc + (7 + k) * SP, v); }
+  __device__ __forceinline__ void cov(int k, float v) const { atomicAdd(acc + (7 + k) * SP, v); }
+  __device__ __forceinline__ void rot(float r, float x, float y, float z) const {
+    atomicAdd(acc + 10 * SP, r); atomicAdd(acc + 11 * SP, x);
+    atomicAdd(acc + 12 * SP, y); atomicAdd(acc + 13 * SP, z);
+  }
+};
 
 __global__ void __launch_bounds__(BWD_BLOCK)
 preprocess_bwd_batched_kernel(const BatchViews bv, int P, int M, const float *__restrict__ means,
@@ -420,15 +449,6 @@ preprocess_bwd_batched_kernel(const BatchViews bv, int P, int M, const float *__
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
   const int start = blockIdx.x * B;
   const int idx = start + t;
-  Slots S_;
-  S_.m2 = nullptr;
-  S_.col = acc;
-  S_.op = acc + 3 * SP;
-  S_.m3 = acc + 4 * SP;
-  S_.sc = acc + 7 * SP;
-  S_.rot = acc + 10 * SP;
-  S_.cov = acc + 7 * SP;  // covariance mode has no scale/rotation
-  S_.sh = nullptr;
   for (int i = t; i < ACC_SLOTS * SP; i += B) acc[i] = 0.f;
   // per-view constants in shared memory: the pair loop below reads them
   // with a different view per lane, which from the kernel parameters would
@@ -500,14 +520,20 @@ preprocess_bwd_batched_kernel(const BatchViews bv, int P, int M, const float *__
     const uint32_t pr = pairs[i];
     const int gl = (int)(pr >> 4), v = (int)(pr & 15u);
     const ViewParams vp = s_vp[v];
-    preprocess_bwd_one<true, false>(start + gl, gl, vp, s_mat[v], s_mat[v] + 16, s_mat[v] + 32, M,
-                                    means, shs, scales, rots, cov3D, s_flags[v], s_gacc[v], out, S_);
+    const SlotSink sink{acc + gl};
+    float pm[3], prgb[3];
+    preprocess_bwd_one(start + gl, vp, s_mat[v], s_mat[v] + 16, means, scales, rots, cov3D, s_gacc[v],
+                       out, sink, pm, prgb);
+    if (out.dL_dmeans3D)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) sink.mean(k, pm[k]);
   }
   __syncthreads();
   if (idx >= P) return;
 
   // --- the Gaussian's own thread: SH over its views, then every output ---
-  float dm[3] = {S_.m3[t], S_.m3[SP + t], S_.m3[2 * SP + t]};
+  const float *own = acc + t;
+  float dm[3] = {own[4 * SP], own[5 * SP], own[6 * SP]};
   const bool want_sh = shs != nullptr && (out.dL_dsh != nullptr || out.dL_dmeans3D != nullptr);
   float dsh[48];
 #pragma unroll
@@ -520,47 +546,29 @@ preprocess_bwd_batched_kernel(const BatchViews bv, int P, int M, const float *__
       const int v = __ffs(m) - 1;
       const float *gv = s_gacc[v] + 12 * (size_t)idx;
       float drgb[3] = {gv[6], gv[7], gv[8]};
-      const uint32_t clamp = s_flags[v][idx];
-      if (clamp & 1) drgb[0] = 0.f;
-      if (clamp & 2) drgb[1] = 0.f;
-      if (clamp & 4) drgb[2] = 0.f;
-      const float *cp = s_mat[v] + 32;
-      const float vx_ = mx - cp[0], vy_ = my - cp[1], vz_ = mz - cp[2];
-      const float len = sqrtf(vx_ * vx_ + vy_ * vy_ + vz_ * vz_);
-      const float il = 1.f / len;
-      const float x = vx_ * il, y = vy_ * il, z = vz_ * il;
-      float gdx = 0.f, gdy = 0.f, gdz = 0.f;
-      for_each_sh_term(s_vp[v].D, x, y, z, [&](int k, float b, float bx, float by, float bz) {
-        dsh[3 * k] += b * drgb[0];
-        dsh[3 * k + 1] += b * drgb[1];
-        dsh[3 * k + 2] += b * drgb[2];
-        const float dot = sh[3 * k] * drgb[0] + sh[3 * k + 1] * drgb[1] + sh[3 * k + 2] * drgb[2];
-        gdx += bx * dot; gdy += by * dot; gdz += bz * dot;
-      });
-      const float ug = x * gdx + y * gdy + z * gdz;
-      dm[0] += (gdx - x * ug) * il;
-      dm[1] += (gdy - y * ug) * il;
-      dm[2] += (gdz - z * ug) * il;
+      apply_clamp(s_flags[v][idx], drgb);
+      sh_bwd(s_vp[v].D, mx, my, mz, s_mat[v] + 32, drgb, [&](int j) { return sh[j]; },
+             [&](int j, float x) { dsh[j] += x; }, dm);
     }
   }
   const size_t i3 = 3 * (size_t)idx;
   if (out.dL_dcolors) {
-    out.dL_dcolors[i3] = S_.col[t]; out.dL_dcolors[i3 + 1] = S_.col[SP + t]; out.dL_dcolors[i3 + 2] = S_.col[2 * SP + t];
+    out.dL_dcolors[i3] = own[0]; out.dL_dcolors[i3 + 1] = own[SP]; out.dL_dcolors[i3 + 2] = own[2 * SP];
   }
-  if (out.dL_dopacity) out.dL_dopacity[idx] = S_.op[t];
+  if (out.dL_dopacity) out.dL_dopacity[idx] = own[3 * SP];
   if (out.dL_dmeans3D) {
     out.dL_dmeans3D[i3] = dm[0]; out.dL_dmeans3D[i3 + 1] = dm[1]; out.dL_dmeans3D[i3 + 2] = dm[2];
   }
   if (out.dL_dcov3D) {
 #pragma unroll
-    for (int k = 0; k < 6; ++k) out.dL_dcov3D[6 * (size_t)idx + k] = S_.cov[k * SP + t];
+    for (int k = 0; k < 6; ++k) out.dL_dcov3D[6 * (size_t)idx + k] = own[(7 + k) * SP];
   }
   if (out.dL_dscales) {
-    out.dL_dscales[i3] = S_.sc[t]; out.dL_dscales[i3 + 1] = S_.sc[SP + t]; out.dL_dscales[i3 + 2] = S_.sc[2 * SP + t];
+    out.dL_dscales[i3] = own[7 * SP]; out.dL_dscales[i3 + 1] = own[8 * SP]; out.dL_dscales[i3 + 2] = own[9 * SP];
   }
   if (out.dL_drotations)
     reinterpret_cast<float4 *>(out.dL_drotations)[idx] =
-        make_float4(S_.rot[t], S_.rot[SP + t], S_.rot[2 * SP + t], S_.rot[3 * SP + t]);
+        make_float4(own[10 * SP], own[11 * SP], own[12 * SP], own[13 * SP]);
   if (out.dL_dsh) {
     // the Gaussian's 3M contiguous floats: coefficients above degree 3 (or
     // the active degree) stay zero
@@ -582,21 +590,39 @@ preprocess_bwd_batched_kernel(const BatchViews bv, int P, int M, const float *__
 
 }  // namespace
 
+ZeroSpans preprocess_bwd_outputs(const DmgsGrads &out, int P, int M) {
+  ZeroSpans z;
+  const size_t n = P > 0 ? (size_t)P : 0;
+  z.add(out.dL_dmeans2D, 3 * n);
+  z.add(out.dL_dcolors, 3 * n);
+  z.add(out.dL_dopacity, n);
+  z.add(out.dL_dmeans3D, 3 * n);
+  z.add(out.dL_dcov3D, 6 * n);
+  z.add(out.dL_dscales, 3 * n);
+  z.add(out.dL_drotations, 4 * n);
+  z.add(out.dL_dsh, 3 * (size_t)std::max(M, 0) * n);
+  return z;
+}
+
 int launch_preprocess_bwd(const ViewParams &vp, const float *viewm, const float *projm,
                           const float *campos, const GaussianPtrs &g, const GeomLayout &L,
                           const char *geom, const float *gacc, const DmgsGrads &out,
                           cudaStream_t s) {
   if (g.P <= 0) return DMGS_OK;
-  const size_t smem = slot_floats(g.M) * 4;
-  if (smem > 200 * 1024) {
-    dmgs_host::set_error("preprocess_bwd: %d SH coefficients per Gaussian exceed shared memory", g.M);
+  if (g.M > SH_COEFFS_MAX) {
+    dmgs_host::set_error("preprocess_bwd: %d SH coefficients per Gaussian exceed %d", g.M, SH_COEFFS_MAX);
     return DMGS_ERR_ARG;
   }
-  if (int r = dmgs_host::raise_smem_limit((const void *)preprocess_bwd_kernel, smem)) return r;
-  DMGS_TIMED(K_PREPROCESS_BWD, s, dmgs_host::note_launch(), preprocess_bwd_kernel<<<(g.P + BWD_BLOCK - 1) / BWD_BLOCK, BWD_BLOCK, smem, s>>>(
+  const size_t smem = (size_t)BWD_BLOCK * SHP * 4;
+  // the visible count is known on the device alone: a few waves of blocks
+  // stride over the list
+  const int grid = std::min((g.P + BWD_BLOCK - 1) / BWD_BLOCK, 16 * NUM_SMS_HINT);
+  DMGS_TIMED(K_PREPROCESS_BWD, s, dmgs_host::note_launch(), preprocess_bwd_list_kernel<<<grid, BWD_BLOCK, smem, s>>>(
       vp, viewm, projm, campos, g.P, g.M, g.means3D, g.shs, g.scales, g.rotations, g.cov3D,
-      reinterpret_cast<const uint8_t *>(geom + L.flags), gacc, out));
-  DMGS_LAUNCH_CHECK("preprocess_bwd_kernel");
+      reinterpret_cast<const uint8_t *>(geom + L.flags), gacc,
+      reinterpret_cast<const uint32_t *>(geom + L.vlist),
+      reinterpret_cast<const uint32_t *>(geom + L.counters), out));
+  DMGS_LAUNCH_CHECK("preprocess_bwd_list_kernel");
   return DMGS_OK;
 }
 

@@ -191,7 +191,7 @@ class _RasterizeGaussians(torch.autograd.Function):
         dout = _f32(grad_out_color, device)
         z = lambda *s: torch.empty(*s, dtype=torch.float32, device=device)  # noqa: E731
         d_means2D = z(P, 3)
-        d_colors = z(P, 3)
+        d_colors = z(P, 3) if colors is not None else None
         d_opac = z(P, 1)
         d_means3D = z(P, 3)
         d_cov3D = z(P, 6) if cov3D is not None else None
@@ -212,7 +212,7 @@ class _RasterizeGaussians(torch.autograd.Function):
                 _snapshot("snapshot_bw.dump", [means3D, radii, colors, scales, rotations, cov3D, dout,
                                                sh, rs.viewmatrix, rs.projmatrix, rs.campos])
             raise
-        return (d_means3D, d_means2D, d_sh, d_colors if colors is not None else None,
+        return (d_means3D, d_means2D, d_sh, d_colors,
                 d_opac.view(ctx.opac_shape), d_scales, d_rot, d_cov3D, None)
 
 
