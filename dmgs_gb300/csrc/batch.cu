@@ -204,8 +204,10 @@ void fill_views(const DmgsBatch *b, const BatchLayout &L, char *const *base, Bat
     o.radii = (b->radii && b->radii[v]) ? b->radii[v] : reinterpret_cast<int32_t *>(st + V.radii);
     o.feat = reinterpret_cast<float4 *>(geom + V.G.feat);
     o.flags = reinterpret_cast<uint8_t *>(geom + V.G.flags);
-    o.blkcnt = reinterpret_cast<uint32_t *>(geom + V.G.blkcnt);
     o.counters = reinterpret_cast<uint32_t *>(geom + V.G.counters);
+    o.zero_bytes = V.G.zero_bytes;
+    o.vtile = reinterpret_cast<uint32_t *>(geom + V.G.vtile);
+    o.vgroup = reinterpret_cast<uint32_t *>(geom + V.G.vgroup);
     o.gacc = reinterpret_cast<const float *>(st + V.gacc);
     o.dL_dmeans2D = nullptr;
   }

@@ -37,9 +37,18 @@
 // written once and read once.  The row and segment offsets are small (gy x C
 // and T x S words).
 //
-// Every kernel bins several views at once (blockIdx.y = view, each view with
+// Launches: steps 1-5 are ten kernels (compaction, four sort passes, chunks,
+// counts, scans, ranges).  Every prefix that crosses blocks is formed by
+// decoupled look-back inside the kernel that needs it, so no step has a scan
+// launch of its own and the sort reads its keys once per pass: a view has
+// 10^4-10^6 visible Gaussians, a few us of memory traffic, and its time was
+// launches (41 of them: 0.21 ms per view at 3M Gaussians, 0.14M visible).
+//
+// Every kernel bins several views at once (one grid dimension, each view with
 // its own geometry state and sizes): a batch of views fills the GPU with one
-// launch per stage instead of one small launch per stage and view.
+// launch per stage instead of one small launch per stage and view.  In the
+// look-back kernels the view is the fast grid dimension: the tiles that start
+// together then belong to all views and have few predecessors each.
 #include <algorithm>
 
 #include "kernels.cuh"
@@ -161,88 +170,211 @@ scan_down_kernel(const ScanViews sv) {
   }
 }
 
-// ---- compaction of visible Gaussians (index order) ----------------------
+// ---- decoupled look-back ---------------------------------------------------
+//
+// Blocks take their tile from a ticket counter, so every predecessor of a
+// tile is held by a block that runs already and never waits for a later one.
+// A tile publishes its aggregate, adds up its predecessors' words back to one
+// that holds an inclusive prefix, and publishes its own.  Each word carries
+// its state in its top two bits and is written whole, so relaxed accesses
+// suffice.  The polls are bounded: a tile that gives up (or sees that another
+// has) sets ST_BOUNDS, and every later kernel then leaves the view alone.
 
-// Each block compacts CPT preprocess blocks (PRE_BLOCK x CPT Gaussians, CPT
-// consecutive per thread, their flag bytes read as one word); the scanned
-// per-preprocess-block counts give the block's first output position.
-constexpr int CPT = 4;
+constexpr unsigned long long LB_AGG = 1ull << 62, LB_INC = 2ull << 62, LB_VAL = LB_AGG - 1;
+constexpr uint32_t LB32_AGG = 1u << 30, LB32_INC = 2u << 30, LB32_VAL = LB32_AGG - 1;
+constexpr uint32_t LB_POLLS = 1u << 20;
+
+__device__ __forceinline__ uint32_t ld_relaxed(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed(uint32_t *p, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_relaxed(unsigned long long *p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+constexpr uint32_t ST_STOP = ST_OVERFLOW | ST_BOUNDS;  // a view no later binning kernel touches
+
+__device__ __forceinline__ bool give_up(uint32_t polls, const uint32_t *counters) {
+  return polls > LB_POLLS || ((polls & 255u) == 255u && (ld_relaxed(counters + CI_STATUS) & ST_BOUNDS));
+}
+
+// Exclusive prefix of `agg` at tile t, called by one whole warp; *ok is false
+// when the wait was given up.
+__device__ __forceinline__ unsigned long long lookback(unsigned long long *st, uint32_t t,
+                                                       unsigned long long agg,
+                                                       const uint32_t *counters, bool *ok) {
+  const int lane = threadIdx.x & 31;
+  *ok = true;
+  if (lane == 0) st_relaxed(st + t, (t == 0 ? LB_INC : LB_AGG) | agg);
+  if (t == 0) return 0ull;
+  unsigned long long excl = 0;
+  long long base = (long long)t - 1;
+  for (uint32_t polls = 0;;) {
+    const long long i = base - lane;
+    const unsigned long long w = i >= 0 ? ld_relaxed(st + i) : LB_INC;
+    const uint32_t state = (uint32_t)(w >> 62);
+    const unsigned inc = __ballot_sync(FULL, state == 2u), none = __ballot_sync(FULL, state == 0u);
+    const int last = inc ? __ffs(inc) - 1 : 31;  // words of lanes 0..last are added
+    if (none & (0xffffffffu >> (31 - last))) {
+      if (give_up(++polls, counters)) {
+        *ok = false;
+        return 0ull;
+      }
+      continue;
+    }
+    unsigned long long v = lane <= last ? w & LB_VAL : 0ull;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+    excl += v;
+    if (inc) break;
+    base -= 32;
+  }
+  if (lane == 0) st_relaxed(st + t, LB_INC | (excl + agg));
+  return excl;
+}
+
+// Next tile of this block (the same for all its threads).
+__device__ __forceinline__ uint32_t take_ticket(uint32_t *ticket, uint32_t *slot) {
+  __syncthreads();
+  if (threadIdx.x == 0) *slot = atomicAdd(ticket, 1u);
+  __syncthreads();
+  return *slot;
+}
+
+// Chunks of a view with V visible Gaussians.
+__device__ __forceinline__ uint32_t chunk_count(const BinView &B, uint32_t V) {
+  return min((V + CHUNK_MIN_GAUSS - 1) / CHUNK_MIN_GAUSS, B.cmax);
+}
+
+// rect = (x0 | y0 << 16, x1 | y1 << 16): tiles [x0, x1) x [y0, y1)
+__device__ __forceinline__ void unpack_rect(uint2 r, int &x0, int &y0, int &x1, int &y1) {
+  x0 = (int)(r.x & 0xffffu); y0 = (int)(r.x >> 16); x1 = (int)(r.y & 0xffffu); y1 = (int)(r.y >> 16);
+}
+
+// The work a Gaussian costs the binning kernels: a fixed part, one per 16
+// covered tile rows for the row lists and one per 64 covered tiles for the
+// tile lists.
+__device__ __forceinline__ uint32_t chunk_weight(uint2 r) {
+  int x0, y0, x1, y1;
+  unpack_rect(r, x0, y0, x1, y1);
+  const uint32_t rows = (uint32_t)(y1 - y0), area = rows * (uint32_t)(x1 - x0);
+  return CHUNK_W_GAUSS + (rows + 15u) / 16u + (area + 63u) / 64u;
+}
+
+// ---- steps 1, 2: compaction of the visible Gaussians, radix sort ------------
+
+// One block per RADIX_TILE Gaussians, CPT consecutive per thread (their flag
+// bytes read as one word): the visible ones in index order, as (depth bits,
+// index) for the sort and as the list the adjoint walks, from the position
+// that the preprocess's counts give the tile (the earlier groups' sums and
+// the earlier tiles of its own group).  On the way: the
+// digit histograms of all four sort passes, the total chunk weight, and the
+// zeros of the sort's look-back words (a tile's share; the tiles the sort
+// uses are at most those here).
+constexpr int CPT = RADIX_TILE / PRE_BLOCK;
+static_assert(VGROUP <= 32, "a group's tiles are summed by one warp");
+static_assert(CPT == 8, "the flag bytes of a thread are read as one 8-byte word");
 
 __global__ void __launch_bounds__(PRE_BLOCK)
 compact_kernel(const BinViews bv) {
-  const BinView &B = bv.v[blockIdx.y];
-  const int base = blockIdx.x * PRE_BLOCK * CPT;
-  if (base >= B.P) return;  // block-uniform
-  const int i0 = base + threadIdx.x * CPT;
-  uint32_t f4 = 0u;
-  if (i0 + CPT <= B.P) {
-    f4 = *reinterpret_cast<const uint32_t *>(B.flags + i0);  // i0 % 4 == 0, the array 256-B aligned
-  } else {
+  const BinView &B = bv.v[blockIdx.x];
+  __shared__ uint32_t hist[4 * 256], wsum[PRE_BLOCK / 32], wweight[PRE_BLOCK / 32];
+  __shared__ uint32_t s_excl;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  for (uint32_t tile = blockIdx.y; tile < (uint32_t)B.nb_radix; tile += gridDim.y) {
+#pragma unroll
+    for (int p = 0; p < 4; ++p) hist[p * 256 + tid] = 0u;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) B.stsort[((size_t)p * B.nb_radix + tile) * 256 + tid] = 0u;
+    const int i0 = (int)tile * RADIX_TILE + tid * CPT;
+    uint2 f8 = make_uint2(0u, 0u);
+    if (i0 + CPT <= B.P) {
+      f8 = *reinterpret_cast<const uint2 *>(B.flags + i0);  // i0 % 8 == 0, the array 256-byte aligned
+    } else {
+#pragma unroll
+      for (int k = 0; k < CPT; ++k)
+        if (i0 + k < B.P) (k < 4 ? f8.x : f8.y) |= (uint32_t)B.flags[i0 + k] << (8 * (k & 3));
+    }
+    uint32_t vis = 0u;
 #pragma unroll
     for (int k = 0; k < CPT; ++k)
-      if (i0 + k < B.P) f4 |= (uint32_t)B.flags[i0 + k] << (8 * k);
-  }
-  uint32_t vis = 0u;
+      vis |= (((k < 4 ? f8.x : f8.y) >> (8 * (k & 3))) & FLAG_VISIBLE) ? 1u << k : 0u;
+    const uint32_t c = __popc(vis);
+    uint32_t incl = c;
 #pragma unroll
-  for (int k = 0; k < CPT; ++k) vis |= ((f4 >> (8 * k)) & FLAG_VISIBLE) ? 1u << k : 0u;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int c = __popc(vis);
-  int incl = c;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += u;
-  }
-  __shared__ int wsum[PRE_BLOCK / 32];
-  if (lane == 31) wsum[wid] = incl;
-  __syncthreads();
-  uint32_t pos = B.blkcnt[blockIdx.x * CPT] + (uint32_t)(incl - c);
-  for (int w = 0; w < wid; ++w) pos += (uint32_t)wsum[w];
-  const float *feat = reinterpret_cast<const float *>(B.feat);
-  for (uint32_t m = vis; m; m &= m - 1) {
-    const int idx = i0 + __ffs(m) - 1;
-    B.k0[pos] = __float_as_uint(feat[12 * (size_t)idx + 9]);  // depth: record float 9
-    B.v0[pos] = (uint32_t)idx;
-    B.vlist[pos] = (uint32_t)idx;
-    ++pos;
-  }
-}
-
-// One thread per view: derived sizes from V.
-__global__ void params_kernel(const BinViews bv) {
-  const int vi = threadIdx.x;
-  if (vi >= bv.n) return;
-  const BinView &B = bv.v[vi];
-  uint32_t *counters = B.counters;
-  const uint32_t V = counters[CI_V];
-  const uint32_t nbr = (V + RADIX_TILE - 1) / RADIX_TILE;
-  const uint32_t C = min((V + CHUNK_MIN_GAUSS - 1) / CHUNK_MIN_GAUSS, B.cmax);
-  counters[CI_NBR] = nbr;
-  counters[CI_NRH] = 256u * nbr;
-  counters[CI_C] = C;
-  counters[CI_NRC] = (uint32_t)B.gy * C;
-}
-
-// ---- stable LSD radix sort of (depth_bits, index), 8 bits per pass -------
-
-__global__ void __launch_bounds__(RADIX_BLOCK)
-radix_hist_kernel(const BinViews bv, int pass) {
-  const BinView &B = bv.v[blockIdx.y];
-  const uint32_t *keys = (pass & 1) ? B.k1 : B.k0;
-  const int shift = 8 * pass;
-  const uint32_t V = B.counters[CI_V], nbr = B.counters[CI_NBR];
-  __shared__ uint32_t h[256];
-  for (uint32_t b = blockIdx.x; b < nbr; b += gridDim.x) {  // key tiles of RADIX_TILE
-    h[threadIdx.x] = 0;
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < RADIX_ITEMS; ++i) {
-      const uint32_t k = b * RADIX_TILE + i * RADIX_BLOCK + threadIdx.x;
-      if (k < V) atomicAdd(&h[(keys[k] >> shift) & 255u], 1u);
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += u;
     }
+    if (lane == 31) wsum[wid] = incl;
     __syncthreads();
-    B.rhist[threadIdx.x * nbr + b] = h[threadIdx.x];  // digit-major
+    uint32_t before = incl - c, total = 0u;
+#pragma unroll
+    for (int w = 0; w < PRE_BLOCK / 32; ++w) {
+      before += w < wid ? wsum[w] : 0u;
+      total += wsum[w];
+    }
+    // depth and rectangle of the visible ones (the record's third float4)
+    uint32_t key[CPT], weight = 0u;
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) {
+      key[k] = 0u;
+      if ((vis >> k) & 1u) {
+        const float4 f2 = B.feat[3 * (size_t)(i0 + k) + 2];
+        key[k] = __float_as_uint(f2.y);
+        weight += chunk_weight(make_uint2(__float_as_uint(f2.z), __float_as_uint(f2.w)));
+      }
+    }
+    if (wid == 0) {
+      const uint32_t group = tile / VGROUP;
+      uint32_t e = lane < tile % VGROUP ? B.vtile[group * VGROUP + lane] : 0u;
+      for (uint32_t g = lane; g < group; g += 32) e += B.vgroup[g];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(FULL, e, o);
+      if (lane == 0) {
+        s_excl = e;
+        if (tile == (uint32_t)B.nb_radix - 1) B.counters[CI_V] = e + total;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < CPT; ++k)
+      if ((vis >> k) & 1u)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) atomicAdd(&hist[p * 256 + ((key[k] >> (8 * p)) & 255u)], 1u);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) weight += __shfl_xor_sync(FULL, weight, o);
+    if (lane == 0) wweight[wid] = weight;
     __syncthreads();
+    uint32_t pos = s_excl + before;
+#pragma unroll
+    for (int k = 0; k < CPT; ++k)
+      if ((vis >> k) & 1u) {
+        B.k0[pos] = key[k];
+        B.v0[pos] = (uint32_t)(i0 + k);
+        B.vlist[pos] = (uint32_t)(i0 + k);
+        ++pos;
+      }
+    if (tid == 0) {
+      unsigned long long w = 0;
+#pragma unroll
+      for (int i = 0; i < PRE_BLOCK / 32; ++i) w += wweight[i];
+      if (w) atomicAdd(reinterpret_cast<unsigned long long *>(B.counters + CI_W), w);
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const uint32_t h = hist[p * 256 + tid];
+      if (h) atomicAdd(&B.ghist[p * 256 + tid], h);
+    }
+    __syncthreads();  // hist and the sums are cleared for the next tile
   }
 }
 
@@ -259,71 +391,132 @@ __device__ __forceinline__ unsigned digit_peers(int d) {
   return peers;
 }
 
-// Warp w of block b owns keys [b*2048 + w*256, +256), visited in 8 rounds
-// of 32 (round-major, then lane) — the input order, so the pass is stable.
+// One pass of the stable LSD sort of (depth bits, index) by 8-bit digits:
+// every block counts its tile's digits, thread d looks back over the earlier
+// tiles' counts of digit d (LB_WIDE words at a time: the first wave's tiles
+// all start together, and their chain would otherwise cost one memory
+// latency per tile; four passes over 0.14M keys of one view / 3.5M of 16
+// took 42 / 232 us at 4 words, 50 / 206 at 8, 43 / 284 at 16, and 115 / 280
+// as separate histogram, scan and scatter launches), and the tile is
+// scattered to its final place.  Warp w
+// of a tile owns keys [w*256, +256), visited in 8 rounds of 32 (round-major,
+// then lane) — the input order, so the pass is stable.
+constexpr int LB_WIDE = 4;
+
 __global__ void __launch_bounds__(RADIX_BLOCK)
-radix_scatter_kernel(const BinViews bv, int pass) {
-  const BinView &B = bv.v[blockIdx.y];
+radix_pass_kernel(const BinViews bv, int pass) {
+  const BinView &B = bv.v[blockIdx.x];
   // pass p reads (k0, v0) when p is even and writes (k1, v1), and back
   const uint32_t *kin = (pass & 1) ? B.k1 : B.k0, *vin = (pass & 1) ? B.v1 : B.v0;
   uint32_t *kout = (pass & 1) ? B.k0 : B.k1, *vout = (pass & 1) ? B.v0 : B.v1;
   const int shift = 8 * pass;
-  const uint32_t *rhist_scanned = B.rhist;
-  const uint32_t V = B.counters[CI_V], nbr = B.counters[CI_NBR];
+  const uint32_t V = B.counters[CI_V], ntiles = (V + RADIX_TILE - 1) / RADIX_TILE;
+  if (blockIdx.y >= ntiles || (B.counters[CI_STATUS] & ST_STOP)) return;  // block-uniform
   __shared__ uint32_t wh[RADIX_BLOCK / 32][256];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (uint32_t b = blockIdx.x; b < nbr; b += gridDim.x) {  // key tiles of RADIX_TILE
-    for (int i = threadIdx.x; i < (RADIX_BLOCK / 32) * 256; i += RADIX_BLOCK) (&wh[0][0])[i] = 0u;
+  __shared__ uint32_t slot, wsum[RADIX_BLOCK / 32];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  // digit tid's first position: exclusive scan of the pass's histogram
+  uint32_t dbase;
+  {
+    const uint32_t h = B.ghist[pass * 256 + tid];
+    uint32_t incl = h;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += u;
+    }
+    if (lane == 31) wsum[w] = incl;
+    __syncthreads();
+    dbase = incl - h;
+#pragma unroll
+    for (int i = 0; i < RADIX_BLOCK / 32; ++i) dbase += i < w ? wsum[i] : 0u;
+  }
+  uint32_t *st = B.stsort + (size_t)pass * B.nb_radix * 256 + tid;
+  for (;;) {
+    const uint32_t tile = take_ticket(B.counters + TK_SORT + pass, &slot);
+    if (tile >= ntiles) return;
+    for (int i = tid; i < (RADIX_BLOCK / 32) * 256; i += RADIX_BLOCK) (&wh[0][0])[i] = 0u;
     __syncthreads();
     uint32_t key[RADIX_ITEMS], val[RADIX_ITEMS];
     int dig[RADIX_ITEMS];
     unsigned peers[RADIX_ITEMS];
-    const uint32_t base = b * RADIX_TILE + w * (32 * RADIX_ITEMS);
+    const uint32_t base = tile * RADIX_TILE + w * (32 * RADIX_ITEMS);
 #pragma unroll
     for (int r = 0; r < RADIX_ITEMS; ++r) {
       const uint32_t k = base + r * 32 + lane;
       const bool ok = k < V;
       key[r] = ok ? kin[k] : 0u;
       val[r] = ok ? vin[k] : 0u;
-      dig[r] = ok ? (int)((key[r] >> shift) & 255u) : 256;
+    }
+#pragma unroll
+    for (int r = 0; r < RADIX_ITEMS; ++r) {
+      dig[r] = base + r * 32 + lane < V ? (int)((key[r] >> shift) & 255u) : 256;
       peers[r] = digit_peers(dig[r]);
       if (dig[r] < 256 && lane == __ffs(peers[r]) - 1) wh[w][dig[r]] += __popc(peers[r]);
       __syncwarp();
     }
     __syncthreads();
-    {
-      const int d = threadIdx.x;  // RADIX_BLOCK == 256 digits
-      uint32_t run = rhist_scanned[d * nbr + b];
+    uint32_t count = 0u;
 #pragma unroll
-      for (int w2 = 0; w2 < RADIX_BLOCK / 32; ++w2) {
-        const uint32_t c = wh[w2][d];
-        wh[w2][d] = run;
-        run += c;
+    for (int i = 0; i < RADIX_BLOCK / 32; ++i) count += wh[i][tid];
+    st_relaxed(st + (size_t)tile * 256, (tile == 0 ? LB32_INC : LB32_AGG) | count);
+    uint32_t excl = 0u;
+    bool bad = false;
+    if (tile > 0) {
+      long long t = (long long)tile - 1;
+      bool done = false;
+      for (uint32_t polls = 0; !done;) {
+        uint32_t word[LB_WIDE];
+#pragma unroll
+        for (int j = 0; j < LB_WIDE; ++j) word[j] = t - j >= 0 ? ld_relaxed(st + (t - j) * 256) : LB32_INC;
+        int adv = 0;
+        bool stop = false;
+#pragma unroll
+        for (int j = 0; j < LB_WIDE; ++j) {
+          const uint32_t state = word[j] >> 30;
+          stop = stop || state == 0u;
+          if (!stop) {
+            excl += word[j] & LB32_VAL;
+            ++adv;
+            done = state == 2u;
+            stop = done;
+          }
+        }
+        t -= adv;
+        if (!done && adv == 0 && give_up(++polls, B.counters)) {
+          bad = true;
+          break;
+        }
       }
+      if (!bad) st_relaxed(st + (size_t)tile * 256, LB32_INC | (excl + count));
     }
-    __syncthreads();
+    uint32_t run = dbase + excl;
+#pragma unroll
+    for (int i = 0; i < RADIX_BLOCK / 32; ++i) {
+      const uint32_t x = wh[i][tid];
+      wh[i][tid] = run;
+      run += x;
+    }
+    if (__syncthreads_or(bad)) {
+      if (tid == 0) atomicOr(B.counters + CI_STATUS, ST_BOUNDS);
+      return;
+    }
 #pragma unroll
     for (int r = 0; r < RADIX_ITEMS; ++r) {
-      uint32_t pos = 0;
+      uint32_t pos = V;
       if (dig[r] < 256) pos = wh[w][dig[r]] + __popc(peers[r] & lanemask_lt());
       __syncwarp();
-      if (dig[r] < 256) {
+      if (pos < V) {
         kout[pos] = key[r];
         vout[pos] = val[r];
-        if (lane == __ffs(peers[r]) - 1) wh[w][dig[r]] += __popc(peers[r]);
       }
+      if (dig[r] < 256 && lane == __ffs(peers[r]) - 1) wh[w][dig[r]] += __popc(peers[r]);
       __syncwarp();
     }
-    __syncthreads();  // wh is cleared for the next tile
   }
 }
 
-// ---- packed rectangles and shared helpers ---------------------------------
-
-// rect = (x0 | y0 << 16, x1 | y1 << 16): tiles [x0, x1) x [y0, y1)
-__device__ __forceinline__ void unpack_rect(uint2 r, int &x0, int &y0, int &x1, int &y1) {
-  x0 = (int)(r.x & 0xffffu); y0 = (int)(r.x >> 16); x1 = (int)(r.y & 0xffffu); y1 = (int)(r.y >> 16);
-}
+// ---- shared helpers ----------------------------------------------------------
 
 // Inclusive warp prefix sum.
 __device__ __forceinline__ int warp_incl_scan(int v, int lane) {
@@ -369,61 +562,89 @@ __device__ __forceinline__ uint32_t seg_chunk(int sg, uint32_t C, int S) {
 
 // ---- step 3: equal-work chunks of the depth-sorted list --------------------
 
-// Weight of sorted position s: the work its Gaussian costs the binning
-// kernels (a fixed part, one per 16 covered tile rows for the row lists and
-// one per 64 covered tiles for the tile lists), so that chunks and the row
-// segments built from them carry similar numbers of instances; the packed
-// rectangle is stored in sorted order for every later pass.
+// A tile of RADIX_TILE sorted positions per block, eight consecutive ones per
+// thread: their packed rectangles are stored in sorted order for every later
+// pass, and with p the prefix of the weights (block scan + look-back) and W
+// their total (from the compaction), chunk c = the positions whose prefix
+// lies in [c W / C, (c + 1) W / C).  Prefixes strictly increase, so the chunk
+// of a position never decreases: position s ends the chunks between its own
+// and the one its successor's prefix p + weight lies in.  cstart[C] = V.
 __global__ void __launch_bounds__(256)
-chunk_weight_kernel(const BinViews bv) {
-  const BinView &B = bv.v[blockIdx.y];
-  const uint32_t V = B.counters[CI_V];
-  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < V; s += gridDim.x * blockDim.x) {
-    const float4 f2 = B.feat[3 * B.v0[s] + 2];
-    const uint2 r = make_uint2(__float_as_uint(f2.z), __float_as_uint(f2.w));
-    B.srect[s] = r;
-    int x0, y0, x1, y1;
-    unpack_rect(r, x0, y0, x1, y1);
-    const uint32_t rows = (uint32_t)(y1 - y0), area = rows * (uint32_t)(x1 - x0);
-    B.k1[s] = CHUNK_W_GAUSS + (rows + 15u) / 16u + (area + 63u) / 64u;  // k1 is free: the sorted keys end in k0
+chunk_kernel(const BinViews bv) {
+  const BinView &B = bv.v[blockIdx.x];
+  const uint32_t V = B.counters[CI_V], ntiles = (V + RADIX_TILE - 1) / RADIX_TILE;
+  if (blockIdx.y >= ntiles || (B.counters[CI_STATUS] & ST_STOP)) return;  // block-uniform
+  const uint32_t C = chunk_count(B, V);
+  const unsigned long long W = *reinterpret_cast<const unsigned long long *>(B.counters + CI_W);
+  __shared__ uint32_t slot;
+  __shared__ unsigned long long s_excl;
+  __shared__ int s_ok;
+  const int tid = threadIdx.x;
+  for (;;) {
+    const uint32_t tile = take_ticket(B.counters + TK_CHUNK, &slot);
+    if (tile >= ntiles) return;
+    const uint32_t s0 = tile * RADIX_TILE + tid * CPT;
+    uint32_t id[CPT], wt[CPT];
+    if (s0 + CPT <= V) {  // s0 % 8 == 0, the array 256-byte aligned
+      const uint4 a = *reinterpret_cast<const uint4 *>(B.v0 + s0), b = *reinterpret_cast<const uint4 *>(B.v0 + s0 + 4);
+      id[0] = a.x; id[1] = a.y; id[2] = a.z; id[3] = a.w; id[4] = b.x; id[5] = b.y; id[6] = b.z; id[7] = b.w;
+    } else {
+#pragma unroll
+      for (int k = 0; k < CPT; ++k) id[k] = s0 + k < V ? B.v0[s0 + k] : 0u;
+    }
+    unsigned long long sum = 0;
+    uint2 r[CPT];
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) {
+      r[k] = make_uint2(0u, 0u);
+      if (s0 + k < V) r[k] = reinterpret_cast<const uint2 *>(B.feat + 3 * (size_t)id[k] + 2)[1];
+    }
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) {
+      wt[k] = s0 + k < V ? chunk_weight(r[k]) : 0u;
+      sum += wt[k];
+      if (s0 + k < V) B.srect[s0 + k] = r[k];
+    }
+    unsigned long long total;
+    unsigned long long p = block_exclusive_scan<256>(sum, &total);
+    if (tid < 32) {
+      bool ok;
+      const unsigned long long e = lookback(B.stchunk, tile, total, B.counters, &ok);
+      if (tid == 0) {
+        s_excl = e;
+        s_ok = ok;
+        if (!ok) atomicOr(B.counters + CI_STATUS, ST_BOUNDS);
+      }
+    }
+    __syncthreads();
+    if (!s_ok) return;
+    p += s_excl;
+    uint32_t c0 = (uint32_t)(p * C / W);
+    if (s0 == 0 && V > 0) {
+      B.cstart[0] = 0u;
+      B.counters[CI_C] = C;
+      if (W > 0xffffffffull) atomicOr(B.counters + CI_STATUS, ST_OVERFLOW);
+    }
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) {
+      const uint32_t sp = s0 + k;
+      if (sp >= V) break;
+      p += wt[k];
+      const uint32_t c1 = sp == V - 1 ? C : min((uint32_t)(p * C / W), C);
+      for (uint32_t c = c0 + 1; c <= c1; ++c) B.cstart[c] = sp + 1;
+      c0 = c1;
+    }
   }
 }
 
-// From the exclusive prefix of the weights: chunk c = the positions whose
-// prefix lies in [c W / C, (c + 1) W / C).  Prefixes strictly increase (each
-// weight >= 1), so the chunk of a position never decreases; position s opens
-// the chunks between its predecessor's and its own.  cstart[C] = V.
-__global__ void __launch_bounds__(256)
-chunk_bounds_kernel(const BinViews bv) {
-  const BinView &B = bv.v[blockIdx.y];
-  const uint32_t *prefix = B.k1;
-  uint32_t *cstart = B.cstart;
-  const uint32_t V = B.counters[CI_V], C = B.counters[CI_C];
-  const unsigned long long W = B.counters[CI_W];
-  if (W == 0) return;
-  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < V; s += gridDim.x * blockDim.x) {
-    const uint32_t cs = (uint32_t)((unsigned long long)prefix[s] * C / W);
-    const uint32_t cp = s > 0 ? (uint32_t)((unsigned long long)prefix[s - 1] * C / W) : 0u;
-    for (uint32_t c = (s > 0 ? cp + 1 : 0u); c <= cs; ++c) cstart[c] = s;
-    if (s == V - 1)
-      for (uint32_t c = cs + 1; c <= C; ++c) cstart[c] = V;
-  }
-}
+// ---- steps 4, 5: row counts and segment counts -------------------------------
 
-// ---- step 4: row counts, one warp per chunk ---------------------------------
-
-// Gaussians of chunk c per tile row: +1 at the first row and -1 after the
-// last of every rectangle in a difference array over the rows, then a
-// prefix sum.  Written row-major [gy][C] so that one flat exclusive scan
-// gives every (row, chunk)'s offset in the concatenated row lists.
-__global__ void __launch_bounds__(32)
-row_count_kernel(const BinViews bv) {
-  extern __shared__ int rdiff[];  // gy + 1
-  const BinView &B = bv.v[blockIdx.y];
-  const uint32_t C = B.counters[CI_C];
-  const uint32_t c = blockIdx.x;
-  if (c >= C) return;
-  const int lane = threadIdx.x, gy = B.gy;
+// Row counts of chunk c, one warp: +1 at the first row and -1 after the last
+// of every rectangle in a difference array over the rows, then a prefix sum.
+// Written row-major [gy][C] so that one flat exclusive scan gives every
+// (row, chunk)'s offset in the concatenated row lists.
+__device__ __forceinline__ void row_counts(const BinView &B, uint32_t c, uint32_t C, int *rdiff) {
+  const int lane = threadIdx.x & 31, gy = B.gy;
   for (int i = lane; i <= gy; i += 32) rdiff[i] = 0;
   __syncwarp();
   const uint32_t s0 = B.cstart[c], s1 = B.cstart[c + 1];
@@ -445,8 +666,6 @@ row_count_kernel(const BinViews bv) {
   }
 }
 
-// ---- step 5: segment counts per tile ---------------------------------------
-
 // Instances of every tile of a band of tile rows from row segment sg (the
 // Gaussians of chunks [sg C / S, (sg + 1) C / S)): every rectangle clipped to
 // the band adds +1 / -1 at its four corners in a 2D difference grid of
@@ -454,17 +673,11 @@ row_count_kernel(const BinViews bv) {
 // block); prefix sums along the rows, then the columns, give the counts,
 // written to cnt2[t * S + sg] — tile-major, so one flat exclusive scan gives
 // every (tile, segment)'s list offset.
-__global__ void __launch_bounds__(256)
-seg_count_kernel(const BinViews bv, int S) {
-  extern __shared__ int dg[];
-  const BinView &B = bv.v[blockIdx.y];
-  if ((int)blockIdx.x >= S * B.nb) return;  // block-uniform
-  const int sg = blockIdx.x / B.nb, b = blockIdx.x - sg * B.nb;
+__device__ __forceinline__ void segment_counts(const BinView &B, int sg, int b, uint32_t C, int S, int *dg) {
   const int gx = B.gx, ys = b * B.R, ye = min(B.gy, ys + B.R), R = ye - ys, Wd = gx + 1;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   for (int i = tid; i < (R + 1) * Wd; i += 256) dg[i] = 0;
   __syncthreads();
-  const uint32_t C = B.counters[CI_C];
   uint32_t s0 = 0, s1 = 0;
   if (C > 0) {
     s0 = B.cstart[seg_chunk(sg, C, S)];
@@ -501,6 +714,89 @@ seg_count_kernel(const BinViews bv, int S) {
   }
 }
 
+// Both counts in one launch (each waits on shared memory and on a few loads
+// of its own, so they fill one another's gaps): blocks [0, S nb_max) count a
+// (segment, band) each, the rest nw chunks' rows each, a warp per chunk.
+__global__ void __launch_bounds__(256)
+count_kernel(const BinViews bv, int S, int nb_max, int nw) {
+  extern __shared__ int cnt_smem[];
+  const BinView &B = bv.v[blockIdx.y];
+  if (B.counters[CI_STATUS] & ST_STOP) return;
+  const uint32_t C = chunk_count(B, B.counters[CI_V]);
+  if ((int)blockIdx.x < S * nb_max) {
+    if ((int)blockIdx.x < S * B.nb)  // block-uniform
+      segment_counts(B, (int)blockIdx.x / B.nb, (int)blockIdx.x % B.nb, C, S, cnt_smem);
+    return;
+  }
+  const int w = threadIdx.x >> 5;
+  const uint32_t c = (blockIdx.x - S * nb_max) * nw + w;
+  if (w < nw && c < C) row_counts(B, c, C, cnt_smem + w * (B.gy + 1));
+}
+
+// Exclusive scans in place of the row counts [gy][C] (total: the row-list
+// entries K1) and of the segment counts [T][S] (total: the instances K), in
+// tiles of SCAN_TILE: the row counts' tiles first, then the segment counts',
+// each array with its own chain of look-back words.
+__global__ void __launch_bounds__(SCAN_THREADS)
+list_scan_kernel(const BinViews bv, int S) {
+  const BinView &B = bv.v[blockIdx.x];
+  if (B.counters[CI_STATUS] & ST_STOP) return;
+  const uint32_t C = chunk_count(B, B.counters[CI_V]);
+  const size_t nr = (size_t)B.gy * C, ns = (size_t)B.gx * B.gy * S;
+  const uint32_t tr = (uint32_t)scan_tiles(nr), ts = (uint32_t)scan_tiles(ns);
+  __shared__ uint32_t slot;
+  __shared__ unsigned long long s_excl;
+  __shared__ int s_ok;
+  const int tid = threadIdx.x;
+  if (blockIdx.y >= tr + ts) return;  // block-uniform
+  for (;;) {
+    const uint32_t tile = take_ticket(B.counters + TK_SCAN, &slot);
+    if (tile >= tr + ts) return;
+    const bool rows = tile < tr;
+    uint32_t *data = rows ? B.rcnt : B.cnt2;
+    const size_t n = rows ? nr : ns;
+    const uint32_t t = rows ? tile : tile - tr;
+    unsigned long long *st = B.stscan + (rows ? 0 : scan_tiles((size_t)B.gy * CHUNK_COUNT_MAX));
+    const size_t k0 = (size_t)t * SCAN_TILE + tid * SCAN_ITEMS;
+    static_assert(SCAN_ITEMS == 4, "a thread's items are one 16-byte word");
+    uint4 x = make_uint4(0u, 0u, 0u, 0u);
+    const bool whole = k0 + 4 <= n;  // k0 % 4 == 0, the arrays 256-byte aligned
+    if (whole) {
+      x = *reinterpret_cast<const uint4 *>(data + k0);
+    } else {
+      if (k0 < n) x.x = data[k0];
+      if (k0 + 1 < n) x.y = data[k0 + 1];
+      if (k0 + 2 < n) x.z = data[k0 + 2];
+    }
+    unsigned long long total;
+    unsigned long long run = block_exclusive_scan<SCAN_THREADS>(
+        (unsigned long long)x.x + x.y + x.z + x.w, &total);
+    if (tid < 32) {
+      bool ok;
+      const unsigned long long e = lookback(st, t, total, B.counters, &ok);
+      if (tid == 0) {
+        s_excl = e;
+        s_ok = ok;
+        if (!ok) atomicOr(B.counters + CI_STATUS, ST_BOUNDS);
+        if (ok && t == (rows ? tr : ts) - 1) {
+          B.counters[rows ? CI_K1 : CI_K] = (uint32_t)(e + total);
+          if (e + total > 0xffffffffull) atomicOr(B.counters + CI_STATUS, ST_OVERFLOW);
+        }
+      }
+    }
+    __syncthreads();
+    if (!s_ok) return;
+    const uint32_t r0 = (uint32_t)(run + s_excl), r1 = r0 + x.x, r2 = r1 + x.y, r3 = r2 + x.z;
+    if (whole) {
+      *reinterpret_cast<uint4 *>(data + k0) = make_uint4(r0, r1, r2, r3);
+    } else {
+      if (k0 < n) data[k0] = r0;
+      if (k0 + 1 < n) data[k0 + 1] = r1;
+      if (k0 + 2 < n) data[k0 + 2] = r2;
+    }
+  }
+}
+
 // Tile ranges from the scanned segment counts: tile t starts at its first
 // segment's offset.  When the instances exceed the list capacity
 // (capacity-bounded callers), every range is left empty and the overflow bit
@@ -512,8 +808,9 @@ __global__ void ranges_kernel(const BinViews bv, int S) {
   if (t >= T) return;
   uint32_t *counters = B.counters;
   const uint32_t K = counters[CI_K];
-  const bool over = K > B.K_cap || (counters[CI_STATUS] & ST_OVERFLOW);
-  if (over && t == 0) atomicOr(&counters[CI_STATUS], ST_OVERFLOW);
+  const uint32_t status = counters[CI_STATUS];
+  const bool over = K > B.K_cap || (status & ST_STOP);
+  if (t == 0 && (K > B.K_cap || (status & ST_OVERFLOW))) atomicOr(&counters[CI_STATUS], ST_OVERFLOW);
   uint2 r = make_uint2(0u, 0u);
   if (B.P > 0 && !over) {
     const uint32_t a = B.cnt2[(size_t)t * S];
@@ -538,7 +835,7 @@ row_emit_kernel(const BinViews bv) {
   uint32_t *counters = B.counters;
   const uint32_t C = counters[CI_C];
   const uint32_t c = blockIdx.x;
-  if (c >= C || (counters[CI_STATUS] & ST_OVERFLOW)) return;
+  if (c >= C || (counters[CI_STATUS] & ST_STOP)) return;
   const int lane = threadIdx.x, gy = B.gy, nbits = bits_for(gy);
   for (int r = lane; r < gy; r += 32) rcur[r] = B.rcnt[(size_t)r * C + c];
   __syncwarp();
@@ -627,7 +924,7 @@ tile_emit_kernel(const BinViews bv, int S) {
   if (r >= B.gy) return;  // block-uniform
   uint32_t *counters = B.counters;
   const uint32_t C = counters[CI_C];
-  if (C == 0 || (counters[CI_STATUS] & ST_OVERFLOW)) return;
+  if (C == 0 || (counters[CI_STATUS] & ST_STOP)) return;
   const uint32_t f0 = seg_chunk(sg, C, S), f1 = seg_chunk(sg + 1, C, S);
   if (f0 >= f1) return;
   const uint32_t e0 = B.rcnt[(size_t)r * C + f0];
@@ -924,14 +1221,6 @@ int launch_scan_views(const ScanViews &sv, cudaStream_t s) {
   return DMGS_OK;
 }
 
-template <typename F>
-ScanViews scan_views(const BinViews &bv, F &&f) {
-  ScanViews sv;
-  sv.n = bv.n;
-  for (int v = 0; v < bv.n; ++v) sv.v[v] = f(bv.v[v]);
-  return sv;
-}
-
 constexpr size_t SMEM_LIMIT = 220 * 1024;
 
 }  // namespace
@@ -961,19 +1250,20 @@ int make_bin_view(const GeomLayout &L, char *geom, uint32_t K_cap, char *bin, ui
                          L.gx, L.gy);
     return DMGS_ERR_ARG;
   }
-  B.n_rhist_max = (uint32_t)L.n_rhist_max;
-  B.n_rcnt_max = (uint32_t)L.n_rcnt_max;
   B.flags = reinterpret_cast<const uint8_t *>(geom + L.flags);
   B.feat = reinterpret_cast<const float4 *>(geom + L.feat);
-  B.blkcnt = reinterpret_cast<uint32_t *>(geom + L.blkcnt);
   B.counters = reinterpret_cast<uint32_t *>(geom + L.counters);
-  B.part = reinterpret_cast<uint32_t *>(geom + L.scanpart);
+  B.ghist = reinterpret_cast<uint32_t *>(geom + L.ghist);
+  B.stsort = reinterpret_cast<uint32_t *>(geom + L.stsort);
+  B.vtile = reinterpret_cast<uint32_t *>(geom + L.vtile);
+  B.vgroup = reinterpret_cast<uint32_t *>(geom + L.vgroup);
+  B.stchunk = reinterpret_cast<unsigned long long *>(geom + L.stchunk);
+  B.stscan = reinterpret_cast<unsigned long long *>(geom + L.stscan);
   B.vlist = reinterpret_cast<uint32_t *>(geom + L.vlist);
   B.k0 = reinterpret_cast<uint32_t *>(geom + L.dkey0);
   B.k1 = reinterpret_cast<uint32_t *>(geom + L.dkey1);
   B.v0 = reinterpret_cast<uint32_t *>(geom + L.dval0);
   B.v1 = reinterpret_cast<uint32_t *>(geom + L.dval1);
-  B.rhist = reinterpret_cast<uint32_t *>(geom + L.rhist);
   B.srect = reinterpret_cast<uint2 *>(geom + L.srect);
   B.cstart = reinterpret_cast<uint32_t *>(geom + L.cstart);
   B.rcnt = reinterpret_cast<uint32_t *>(geom + L.rcnt);
@@ -994,12 +1284,11 @@ int make_bin_view(const GeomLayout &L, char *geom, uint32_t K_cap, char *bin, ui
 
 int launch_binning_geometry(const BinViews &bv, cudaStream_t s) {
   if (bv.n < 1) return DMGS_OK;
-  int nb_pre = 0, nb_radix = 0, P = 0, T = 0, gy = 0, nb = 0;
+  int nb_radix = 0, P = 0, T = 0, gy = 0, nb = 0;
   uint32_t cmax = 0;
   size_t seg_smem = 0;
   for (int v = 0; v < bv.n; ++v) {
     const BinView &B = bv.v[v];
-    nb_pre = std::max(nb_pre, B.nb_pre);
     nb_radix = std::max(nb_radix, B.nb_radix);
     P = std::max(P, B.P);
     T = std::max(T, B.gx * B.gy);
@@ -1010,60 +1299,30 @@ int launch_binning_geometry(const BinViews &bv, cudaStream_t s) {
   }
   const int S = seg_plan(bv);
   const int nv = bv.n;
-  // grid-stride kernels over the visible Gaussians (counted on the device)
-  const int rgrid = bounded_blocks((size_t)nb_radix, nv, 8);  // key tiles
-  const int pgrid = bounded_blocks((size_t)nb_pre, nv, 8);    // blocks of 256 positions
-  const size_t rows_smem = (size_t)(gy + 1) * 4;
-  if (int r = dmgs_host::raise_smem_limit((const void *)row_count_kernel, rows_smem)) return r;
-  if (int r = dmgs_host::raise_smem_limit((const void *)seg_count_kernel, seg_smem)) return r;
   if (P > 0) {
-    DMGS_TIMED(K_BIN_COMPACT, s, {
-      int r = launch_scan_views(scan_views(bv, [](const BinView &B) {
-        return ScanView{B.blkcnt, nullptr, (uint32_t)B.nb_pre, B.part, B.counters + CI_V, B.counters};
-      }), s);
-      if (r != DMGS_OK) return r;
-      dmgs_host::note_launch(), compact_kernel<<<dim3((nb_pre + CPT - 1) / CPT, nv), PRE_BLOCK, 0, s>>>(bv);
-    });
+    // tiles of the visible Gaussians, whose number is known on the device
+    const int tgrid = bounded_blocks((size_t)nb_radix, nv, 8);
+    // chunk warps of a counting block: as many rows as 48 KB hold, 1 to 8
+    const size_t row_smem = (size_t)(gy + 1) * 4;
+    const int nw = (int)std::max<size_t>(1, std::min<size_t>(8, 48 * 1024 / row_smem));
+    const size_t cnt_smem = std::max(seg_smem, nw * row_smem);
+    if (int r = dmgs_host::raise_smem_limit((const void *)count_kernel, cnt_smem)) return r;
+    const size_t st_max = scan_tiles((size_t)gy * cmax) + scan_tiles((size_t)T * S);
+    DMGS_TIMED(K_BIN_COMPACT, s,
+               dmgs_host::note_launch(), compact_kernel<<<dim3(nv, std::min(nb_radix, 65535)), PRE_BLOCK, 0, s>>>(bv));
     DMGS_LAUNCH_CHECK("compact_kernel");
-  }
-  dmgs_host::note_launch(), params_kernel<<<1, 32, 0, s>>>(bv);
-  DMGS_LAUNCH_CHECK("params_kernel");
-  if (P > 0) {
     DMGS_TIMED(K_BIN_SORT, s, {
-      const ScanViews hs = scan_views(bv, [](const BinView &B) {
-        return ScanView{B.rhist, B.counters + CI_NRH, B.n_rhist_max, B.part, nullptr, nullptr};
-      });
-      for (int pass = 0; pass < 4; ++pass) {
-        dmgs_host::note_launch(), radix_hist_kernel<<<dim3(rgrid, nv), RADIX_BLOCK, 0, s>>>(bv, pass);
-        int r = launch_scan_views(hs, s);
-        if (r != DMGS_OK) return r;
-        dmgs_host::note_launch(), radix_scatter_kernel<<<dim3(rgrid, nv), RADIX_BLOCK, 0, s>>>(bv, pass);
-      }
+      for (int pass = 0; pass < 4; ++pass)
+        dmgs_host::note_launch(), radix_pass_kernel<<<dim3(nv, tgrid), RADIX_BLOCK, 0, s>>>(bv, pass);
     });  // four passes: the sorted order ends in (k0, v0)
     DMGS_LAUNCH_CHECK("radix_sort");
     DMGS_TIMED(K_BIN_COUNT, s, {
-      dmgs_host::note_launch(), chunk_weight_kernel<<<dim3(pgrid, nv), 256, 0, s>>>(bv);
-      int r = launch_scan_views(scan_views(bv, [](const BinView &B) {
-        return ScanView{B.k1, B.counters + CI_V, (uint32_t)B.P, B.part, B.counters + CI_W, B.counters};
-      }), s);
-      if (r != DMGS_OK) return r;
-      dmgs_host::note_launch(), chunk_bounds_kernel<<<dim3(pgrid, nv), 256, 0, s>>>(bv);
-      dmgs_host::note_launch(), row_count_kernel<<<dim3(cmax, nv), 32, rows_smem, s>>>(bv);
-      dmgs_host::note_launch(), seg_count_kernel<<<dim3(S * nb, nv), 256, seg_smem, s>>>(bv, S);
+      dmgs_host::note_launch(), chunk_kernel<<<dim3(nv, tgrid), 256, 0, s>>>(bv);
+      dmgs_host::note_launch(), count_kernel<<<dim3(S * nb + (cmax + nw - 1) / nw, nv), 256, cnt_smem, s>>>(bv, S, nb, nw);
     });
     DMGS_LAUNCH_CHECK("tile_count");
-    DMGS_TIMED(K_BIN_SCAN, s, {
-      int r = launch_scan_views(scan_views(bv, [](const BinView &B) {
-        return ScanView{B.rcnt, B.counters + CI_NRC, B.n_rcnt_max, B.part, B.counters + CI_K1,
-                        B.counters};
-      }), s);
-      if (r != DMGS_OK) return r;
-      r = launch_scan_views(scan_views(bv, [S](const BinView &B) {
-        return ScanView{B.cnt2, nullptr, (uint32_t)(B.gx * B.gy) * (uint32_t)S, B.part,
-                        B.counters + CI_K, B.counters};
-      }), s);
-      if (r != DMGS_OK) return r;
-    });
+    DMGS_TIMED(K_BIN_SCAN, s,
+               dmgs_host::note_launch(), list_scan_kernel<<<dim3(nv, bounded_blocks(st_max, nv, 2)), SCAN_THREADS, 0, s>>>(bv, S));
     DMGS_LAUNCH_CHECK("binning scans");
   }
   dmgs_host::note_launch(), ranges_kernel<<<dim3((T + 255) / 256, nv), 256, 0, s>>>(bv, S);

@@ -50,16 +50,14 @@ struct ViewParams {
 //   f2 = (b, depth, rect_lo, rect_hi) rect packed as 2 x (u16 | u16 << 16)
 // A culled Gaussian has rect_lo == rect_hi == 0 and radius 0.
 // Per Gaussian also one flags byte: FLAG_VISIBLE | SH clamp bits (r, g, b).
-// Then the binning working set: per-block visible counts, the visible
-// Gaussians' depth keys / indices (two ping-pong copies for the radix sort),
-// the radix block histograms, the per-(tile, chunk) count matrix, scan
-// partials, per-tile ranges and the counters word block.
+// Then the binning working set (GeomLayout below).
 // ---------------------------------------------------------------------------
 constexpr uint8_t FLAG_VISIBLE = 8;      // flags byte: radius > 0, tile rectangle non-empty
 constexpr int PRE_BLOCK = 256;           // preprocess / compaction block
 constexpr int RADIX_BLOCK = 256;         // radix sort block (8 warps)
 constexpr int RADIX_ITEMS = 8;           // keys per thread
 constexpr int RADIX_TILE = RADIX_BLOCK * RADIX_ITEMS;  // 2048 keys per block
+constexpr int VGROUP = 32;               // tiles of RADIX_TILE Gaussians per group of visible counts
 constexpr int CHUNK_MIN_GAUSS = 64;     // visible Gaussians per binning chunk (mean, minimum)
 constexpr int CHUNK_COUNT_MAX = 2048;    // binning chunks per view (maximum)
 constexpr int CHUNK_W_GAUSS = 2;         // chunk weight of a Gaussian: this + ceil(rows / 16)
@@ -75,29 +73,36 @@ constexpr int CI_K = 1;        // instances (u32; K < 2^32 enforced)
 constexpr int CI_K1 = 2;       // row-list entries (visible Gaussian x tile row it covers)
 constexpr int CI_MAXLIST = 3;  // longest tile list
 constexpr int CI_V = 4;        // visible Gaussians
-constexpr int CI_NBR = 5;      // radix blocks in use = ceil(V / RADIX_TILE)
-constexpr int CI_NRH = 6;      // radix histogram entries = 256 * NBR
-constexpr int CI_W = 7;        // total chunk weight of the visible Gaussians
 constexpr int CI_C = 8;        // chunks
-constexpr int CI_NRC = 9;      // row-count entries = gy * C
+constexpr int CI_W = 10;       // total chunk weight of the visible Gaussians (64-bit: words 10, 11)
 constexpr int CI_WORDS = 16;
+// tickets: the words after the counters, from which the blocks of the
+// look-back kernels draw their tiles
+constexpr int TK_SORT = 16, TK_CHUNK = 20, TK_SCAN = 21;
+constexpr int CI_TICKETS_END = 32;
 
-// Geometry state of one view.  Binning arrays: per-block visible counts;
-// the visible Gaussians in index order (vlist, kept for the adjoint);
-// (depth bits, index) ping-pong pairs of the radix sort; radix histograms;
-// per depth-sorted position the packed tile rectangle (srect, 8 B); chunk
-// starts; the row counts [gy][C] (Gaussians of chunk c covering tile row r,
-// scanned in place into row-list offsets); the segment counts [T][S]
-// (instances of tile t from row segment s, scanned in place into list
-// offsets); scan partials; tile ranges; counters.
+// Geometry state of one view.  Binning arrays: the visible Gaussians in index
+// order (vlist, kept for the adjoint); (depth bits, index) ping-pong pairs of
+// the radix sort; per depth-sorted position the packed tile rectangle (srect,
+// 8 B); chunk starts; the row counts [gy][C] (Gaussians of chunk c covering
+// tile row r, scanned in place into row-list offsets); the segment counts
+// [T][S] (instances of tile t from row segment s, scanned in place into list
+// offsets); tile ranges; the radix sort's look-back words (stsort, per pass
+// and key tile one word per digit); and one region that must be zero when a
+// view's preprocess starts: the counters and tickets, the digit histograms
+// of the four passes, the preprocess's visible counts (per tile of RADIX_TILE
+// Gaussians and per group of VGROUP tiles), and the look-back words of the
+// chunk weights and of the row / segment scans.
 struct GeomLayout {
-  size_t feat, flags, blkcnt, vlist, dkey0, dkey1, dval0, dval1, rhist, srect, cstart, rcnt, cnt2,
-      scanpart, ranges, counters, total;
+  size_t feat, flags, vlist, dkey0, dkey1, dval0, dval1, srect, cstart, rcnt, cnt2, ranges, stsort,
+      counters, ghist, vtile, vgroup, stchunk, stscan, total;
+  size_t zero_bytes;     // from counters on
   int P, gx, gy;
-  int nb_pre, nb_radix;
-  size_t n_rhist_max, n_rcnt_max, n_cnt2_max, n_part_max;
+  int nb_pre, nb_radix;  // preprocess blocks; tiles of RADIX_TILE keys (or Gaussians)
   __host__ __device__ int T() const { return gx * gy; }
 };
+
+__host__ __device__ inline size_t scan_tiles(size_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE; }
 
 __host__ __device__ inline GeomLayout geom_layout(int P, int W, int H) {
   GeomLayout L;
@@ -107,31 +112,28 @@ __host__ __device__ inline GeomLayout geom_layout(int P, int W, int H) {
   const size_t T = (size_t)L.gx * L.gy;
   L.nb_pre = (P + PRE_BLOCK - 1) / PRE_BLOCK;
   L.nb_radix = (P + RADIX_TILE - 1) / RADIX_TILE;
-  L.n_rhist_max = (size_t)256 * L.nb_radix;
-  L.n_rcnt_max = (size_t)L.gy * CHUNK_COUNT_MAX;
-  L.n_cnt2_max = T * SEG_MAX;
-  size_t nmax = L.n_rcnt_max > L.n_rhist_max ? L.n_rcnt_max : L.n_rhist_max;
-  if (L.n_cnt2_max > nmax) nmax = L.n_cnt2_max;
-  if ((size_t)L.nb_pre > nmax) nmax = L.nb_pre;
-  if ((size_t)P > nmax) nmax = P;
-  L.n_part_max = (nmax + SCAN_TILE - 1) / SCAN_TILE + 1;
+  const size_t n_rcnt = (size_t)L.gy * CHUNK_COUNT_MAX, n_cnt2 = T * SEG_MAX;
   size_t o = 0;
   L.feat = o;      o = align_up(o + (size_t)P * 48, 256);
   L.flags = o;     o = align_up(o + (size_t)P, 256);
-  L.blkcnt = o;    o = align_up(o + (size_t)L.nb_pre * 4 + 4, 256);
   L.vlist = o;     o = align_up(o + (size_t)P * 4, 256);
   L.dkey0 = o;     o = align_up(o + (size_t)P * 4, 256);
   L.dkey1 = o;     o = align_up(o + (size_t)P * 4, 256);
   L.dval0 = o;     o = align_up(o + (size_t)P * 4, 256);
   L.dval1 = o;     o = align_up(o + (size_t)P * 4, 256);
-  L.rhist = o;     o = align_up(o + L.n_rhist_max * 4 + 4, 256);
   L.srect = o;     o = align_up(o + (size_t)P * 8, 256);
   L.cstart = o;    o = align_up(o + (CHUNK_COUNT_MAX + 1) * 4, 256);
-  L.rcnt = o;      o = align_up(o + L.n_rcnt_max * 4 + 4, 256);
-  L.cnt2 = o;      o = align_up(o + L.n_cnt2_max * 4 + 4, 256);
-  L.scanpart = o;  o = align_up(o + L.n_part_max * 4, 256);
+  L.rcnt = o;      o = align_up(o + n_rcnt * 4, 256);
+  L.cnt2 = o;      o = align_up(o + n_cnt2 * 4, 256);
   L.ranges = o;    o = align_up(o + T * 8, 256);
-  L.counters = o;  o = align_up(o + CI_WORDS * 4, 256);
+  L.stsort = o;    o = align_up(o + (size_t)L.nb_radix * (4 * 256 * 4), 256);
+  L.counters = o;  o = align_up(o + CI_TICKETS_END * 4, 256);
+  L.ghist = o;     o = align_up(o + 4 * 256 * 4, 256);
+  L.vtile = o;     o = align_up(o + (size_t)L.nb_radix * 4, 256);
+  L.vgroup = o;    o = align_up(o + (size_t)(L.nb_radix / VGROUP + 1) * 4, 256);
+  L.stchunk = o;   o = align_up(o + (size_t)L.nb_radix * 8, 256);
+  L.stscan = o;    o = align_up(o + (scan_tiles(n_rcnt) + scan_tiles(n_cnt2)) * 8, 256);
+  L.zero_bytes = o - L.counters;
   L.total = o;
   return L;
 }

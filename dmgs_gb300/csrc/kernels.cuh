@@ -17,8 +17,9 @@ struct BatchView {
   int32_t *radii;                       // [P] or a [P] scratch when the caller passes none
   float4 *feat;                         // geometry state of this view
   uint8_t *flags;
-  uint32_t *blkcnt;
-  uint32_t *counters;
+  uint32_t *counters;                   // start of the geometry state's zeroed region
+  size_t zero_bytes;                    // its size
+  uint32_t *vtile, *vgroup;             // visible counts per tile of Gaussians and per group
   const float *gacc;                    // adjoint: this view's 2D gradient records
   float *dL_dmeans2D;                   // adjoint: optional per-view output [P,3]
 };
@@ -50,10 +51,10 @@ struct BinView {
   int gx, gy;            // tile grid
   int R, nb;             // segment counting: tile rows per band, bands
   int nxs;               // row pieces of at most XSEG tiles
-  uint32_t n_rhist_max, n_rcnt_max;
   const uint8_t *flags;
   const float4 *feat;
-  uint32_t *blkcnt, *counters, *part, *vlist, *k0, *k1, *v0, *v1, *rhist, *cstart, *rcnt, *cnt2;
+  uint32_t *counters, *ghist, *vtile, *vgroup, *stsort, *vlist, *k0, *k1, *v0, *v1, *cstart, *rcnt, *cnt2;
+  unsigned long long *stchunk, *stscan;
   uint2 *srect;          // packed tile rectangle per depth-sorted position
   uint2 *ranges;
   uint32_t *point_list;  // emission target (K_alloc entries)

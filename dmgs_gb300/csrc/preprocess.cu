@@ -8,9 +8,9 @@
 //
 // Design: one thread per Gaussian.  The integer-determining chain (view z,
 // NDC position, 2D covariance, radius, rectangle) uses explicitly rounded
-// IEEE ops so that it is reproducible on the CPU.  Each block also records
-// how many of its Gaussians are visible, for the order-preserving
-// compaction that starts the binning (binning.cu).
+// IEEE ops so that it is reproducible on the CPU.  Each block adds its
+// visible Gaussians to the counts from which the order-preserving compaction
+// that starts the binning (binning.cu) knows every tile's first position.
 #include "kernels.cuh"
 
 namespace dmgs {
@@ -245,6 +245,16 @@ __device__ __forceinline__ void load_gaussian(int idx, float scale_modifier,
   o = __ldg(opac + idx);
 }
 
+// Adds the block's visible Gaussians to its tile's and its group's count.
+__device__ __forceinline__ void count_visible(uint32_t *vtile, uint32_t *vgroup, uint32_t n) {
+  static_assert(RADIX_TILE % PRE_BLOCK == 0, "a preprocess block lies in one tile");
+  const uint32_t tile = blockIdx.x / (RADIX_TILE / PRE_BLOCK);
+  if (n) {
+    atomicAdd(vtile + tile, n);
+    atomicAdd(vgroup + tile / VGROUP, n);
+  }
+}
+
 __global__ void __launch_bounds__(PRE_BLOCK)
 preprocess_kernel(ViewParams vp, const float *__restrict__ viewm_g,
                   const float *__restrict__ projm_g, const float *__restrict__ campos_g,
@@ -253,8 +263,8 @@ preprocess_kernel(ViewParams vp, const float *__restrict__ viewm_g,
                   const float *__restrict__ colors, const float *__restrict__ scales,
                   const float *__restrict__ rots, const float *__restrict__ cov3D,
                   int32_t *__restrict__ radii, float4 *__restrict__ feat,
-                  uint8_t *__restrict__ flags, uint32_t *__restrict__ blkcnt,
-                  uint32_t *__restrict__ counters) {
+                  uint8_t *__restrict__ flags, uint32_t *__restrict__ counters,
+                  uint32_t *__restrict__ vtile, uint32_t *__restrict__ vgroup) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   bool vis = false;
   if (idx < P) {
@@ -266,7 +276,7 @@ preprocess_kernel(ViewParams vp, const float *__restrict__ viewm_g,
     if (vis) color_one(idx, vp, campos_g, M, x, y, z, shs, colors, feat, flags);
   }
   const int nvis = __syncthreads_count(vis);
-  if (threadIdx.x == 0) blkcnt[blockIdx.x] = (uint32_t)nvis;
+  if (threadIdx.x == 0) count_visible(vtile, vgroup, (uint32_t)nvis);
 }
 
 // Lists the block's (Gaussian, view) pairs whose bits are set in the
@@ -312,15 +322,13 @@ __device__ __forceinline__ uint32_t list_pairs(uint32_t m, uint16_t *pairs, uint
 // compactly so that every lane does useful work (a per-lane early exit
 // would leave the warps running the chain for their slowest lane).
 // Phase 3 takes the visible pairs, listed the same way, through the colour
-// (SH evaluation, 48 coefficient loads).  Each view's per-block visible
-// count feeds its compaction.
+// (SH evaluation, 48 coefficient loads).
 __global__ void __launch_bounds__(PRE_BLOCK)
 preprocess_batched_kernel(const BatchViews bv, int P, int M, const float *__restrict__ means,
                           const float *__restrict__ opac, const float *__restrict__ shs,
                           const float *__restrict__ colors, const float *__restrict__ scales,
                           const float *__restrict__ rots, const float *__restrict__ cov3D) {
   constexpr int NW = PRE_BLOCK / 32;
-  __shared__ uint32_t wcnt[NW][MAX_BATCH_VIEWS];
   __shared__ uint32_t wsum[NW];
   __shared__ uint16_t pairs[PRE_BLOCK * MAX_BATCH_VIEWS];
   __shared__ uint32_t s_vm[PRE_BLOCK];
@@ -342,7 +350,8 @@ preprocess_batched_kernel(const BatchViews bv, int P, int M, const float *__rest
   __shared__ uint8_t *s_flags[MAX_BATCH_VIEWS];
   __shared__ int32_t *s_radii[MAX_BATCH_VIEWS];
   __shared__ uint32_t *s_counters[MAX_BATCH_VIEWS];
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  __shared__ uint32_t s_nvis[MAX_BATCH_VIEWS];
+  const int t = threadIdx.x;
   const int nv = bv.nviews;
   if (t < nv) {
     const BatchView &V = bv.v[t];
@@ -354,6 +363,7 @@ preprocess_batched_kernel(const BatchViews bv, int P, int M, const float *__rest
     s_flags[t] = V.flags;
     s_radii[t] = V.radii;
     s_counters[t] = V.counters;
+    s_nvis[t] = 0u;
     // |J|_F^2 z^2 |W|_F^2 bound factor of the pre-test
     float w2 = 0.f;
 #pragma unroll
@@ -445,24 +455,16 @@ preprocess_batched_kernel(const BatchViews bv, int P, int M, const float *__rest
     if (cov3D == nullptr && s_vp[v].scale_modifier != mod0)
       load_gaussian(base + gl, s_vp[v].scale_modifier, means, opac, scales, rots, cov3D, x, y, z, S, o);
     if (geometry_one(base + gl, s_vp[v], s_V[v], s_P[v], x, y, z, S, o, s_radii[v], s_feat[v],
-                     s_flags[v], s_counters[v]))
+                     s_flags[v], s_counters[v])) {
       atomicOr(&s_vm[gl], 1u << v);
+      atomicAdd(&s_nvis[v], 1u);
+    }
   }
   __syncthreads();
 
-  // Phase 3: colour of the visible pairs, and the per-view block counts.
-  const uint32_t vm = s_vm[t];
-  for (int v = 0; v < nv; ++v) {
-    const uint32_t b = __ballot_sync(0xffffffffu, (vm >> v) & 1u);
-    if (lane == 0) wcnt[wid][v] = __popc(b);
-  }
-  const uint32_t total = list_pairs<NW>(vm, pairs, wsum);
-  if (t < nv) {
-    uint32_t n = 0;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) n += wcnt[w][t];
-    bv.v[t].blkcnt[blockIdx.x] = n;
-  }
+  // Phase 3: colour of the visible pairs, and the per-view counts.
+  if (t < nv) count_visible(bv.v[t].vtile, bv.v[t].vgroup, s_nvis[t]);
+  const uint32_t total = list_pairs<NW>(s_vm[t], pairs, wsum);
   for (uint32_t i = t; i < total; i += PRE_BLOCK) {
     const uint32_t pr = pairs[i];
     const int gl = (int)(pr >> 4), v = (int)(pr & 15u);
@@ -490,15 +492,16 @@ int launch_preprocess(const ViewParams &vp, const float *viewm, const float *pro
                       const GeomLayout &L, char *geom, cudaStream_t s) {
   float4 *feat = reinterpret_cast<float4 *>(geom + L.feat);
   uint8_t *flags = reinterpret_cast<uint8_t *>(geom + L.flags);
-  uint32_t *blkcnt = reinterpret_cast<uint32_t *>(geom + L.blkcnt);
   uint32_t *counters = reinterpret_cast<uint32_t *>(geom + L.counters);
-  DMGS_CUDA(cudaMemsetAsync(counters, 0, CI_WORDS * 4, s));
+  DMGS_CUDA(cudaMemsetAsync(counters, 0, L.zero_bytes, s));
   if (g.P > 0) {
     const int blocks = L.nb_pre;
     DMGS_TIMED(K_PREPROCESS, s, dmgs_host::note_launch(), preprocess_kernel<<<blocks, PRE_BLOCK, 0, s>>>(vp, viewm, projm, campos, g.P, g.M, g.means3D,
                                                  g.opacities, g.shs, g.colors, g.scales,
-                                                 g.rotations, g.cov3D, radii, feat, flags, blkcnt,
-                                                 counters));
+                                                 g.rotations, g.cov3D, radii, feat, flags,
+                                                 counters,
+                                                 reinterpret_cast<uint32_t *>(geom + L.vtile),
+                                                 reinterpret_cast<uint32_t *>(geom + L.vgroup)));
     DMGS_LAUNCH_CHECK("preprocess_kernel");
   }
   return DMGS_OK;
@@ -557,9 +560,17 @@ int launch_debug_geometry(const GeomLayout &L, const char *geom, int32_t *rect,
 
 namespace dmgs {
 
+// One launch instead of a memset per view.
+__global__ void __launch_bounds__(256) zero_views_kernel(const BatchViews bv) {
+  const BatchView &V = bv.v[blockIdx.y];
+  uint4 *p = reinterpret_cast<uint4 *>(V.counters);  // 256-byte aligned, a multiple of 256 bytes
+  for (size_t i = blockIdx.x * 256 + threadIdx.x; i < V.zero_bytes / 16; i += gridDim.x * 256)
+    p[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 int launch_preprocess_batched(const BatchViews &bv, const GaussianPtrs &g, cudaStream_t s) {
-  for (int v = 0; v < bv.nviews; ++v)
-    DMGS_CUDA(cudaMemsetAsync(bv.v[v].counters, 0, CI_WORDS * 4, s));
+  dmgs_host::note_launch(), zero_views_kernel<<<dim3(8, bv.nviews), 256, 0, s>>>(bv);
+  DMGS_LAUNCH_CHECK("zero_views_kernel");
   if (g.P <= 0) return DMGS_OK;
   DMGS_TIMED(K_BATCH_PREPROCESS, s,
              dmgs_host::note_launch(), preprocess_batched_kernel<<<(g.P + PRE_BLOCK - 1) / PRE_BLOCK, PRE_BLOCK, 0, s>>>(
