@@ -242,6 +242,19 @@ void fill_blend(const DmgsBatch *b, const BatchLayout &L, char *const *bases, Bl
   bb.total = base;
 }
 
+// The views' work lists.
+BlendWork fill_work(int n, const BatchLayout &L, char *const *bases) {
+  BlendWork w;
+  for (int v = 0; v < n; ++v) {
+    const GeomLayout &G = L.v[v].G;
+    const char *geom = bases[v] + L.v[v].geom;
+    w.v[v] = {reinterpret_cast<const uint32_t *>(geom + G.clsn),
+              reinterpret_cast<const uint32_t *>(geom + G.clslist),
+              reinterpret_cast<const uint32_t *>(geom + G.counters)};
+  }
+  return w;
+}
+
 }  // namespace
 
 extern "C" size_t dmgs_batch_state_bytes(const DmgsBatch *b, int32_t P) {
@@ -275,7 +288,7 @@ extern "C" int dmgs_raster_fwd_batched(const DmgsBatch *b, const DmgsGaussians *
   fill_blend(b, L, same_base(st), bb);
   uint32_t *queue = reinterpret_cast<uint32_t *>(st + L.queue);
   DMGS_CUDA(cudaMemsetAsync(queue, 0, 4, s));
-  RET_IF(launch_blend_batch_fwd(bb, cfg_of(b), queue, s));
+  RET_IF(launch_blend_batch_fwd(bb, fill_work(b->nviews, L, same_base(st)), cfg_of(b), queue, s));
   return DMGS_OK;
 }
 
@@ -305,8 +318,8 @@ extern "C" int dmgs_raster_bwd_batched(const DmgsBatch *b, const DmgsGaussians *
                reinterpret_cast<const uint32_t *>(geom + L.v[v].G.counters), bb.v[v].gacc, (uint32_t)g->P};
   }
   uint32_t *queue = reinterpret_cast<uint32_t *>(st + L.queue) + 1;
-  DMGS_CUDA(cudaMemsetAsync(queue, 0, 4, s));
-  RET_IF(launch_blend_batch_bwd(bb, cv, ZeroSpans(), cfg_of(b), queue, s));
+  RET_IF(launch_blend_batch_bwd(bb, fill_work(b->nviews, L, same_base(st)), cv, ZeroSpans(), cfg_of(b),
+                                queue, s));
   BatchViews bv;
   fill_views(b, L, same_base(st), bv);
   for (int v = 0; v < b->nviews; ++v) bv.v[v].dL_dmeans2D = dL_dmeans2D ? dL_dmeans2D[v] : nullptr;
@@ -431,7 +444,7 @@ extern "C" int dmgs_render_multi(const DmgsBatch *b, const DmgsGaussians *g, voi
   BlendBatch bb;
   fill_blend(b, L, base, bb);
   DMGS_CUDA(cudaMemsetAsync(queue, 0, 4, s));
-  RET_IF(launch_blend_batch_fwd(bb, cfg_of(b), queue, s));
+  RET_IF(launch_blend_batch_fwd(bb, fill_work(b->nviews, L, base), cfg_of(b), queue, s));
   return DMGS_OK;
 }
 

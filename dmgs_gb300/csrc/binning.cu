@@ -819,6 +819,14 @@ __global__ void ranges_kernel(const BinViews bv, int S) {
     atomicMax(&counters[CI_MAXLIST], e - a);
   }
   B.ranges[t] = r;
+  // the tile's class, by half octaves of its length
+  int c = BLEND_CLASSES - 1;
+  if (r.y > r.x) {
+    const uint32_t n = r.y - r.x;
+    const int l = 31 - __clz(n), b = 2 * l + (l > 0 ? (int)((n >> (l - 1)) & 1u) : 0);
+    c = max(0, BLEND_CLASSES - 2 - b);
+  }
+  B.clslist[(size_t)c * T + atomicAdd(&B.clsn[c], 1u)] = (uint32_t)t;
 }
 
 // ---- step 6a: row lists, one warp per chunk --------------------------------
@@ -1255,6 +1263,8 @@ int make_bin_view(const GeomLayout &L, char *geom, uint32_t K_cap, char *bin, ui
   B.counters = reinterpret_cast<uint32_t *>(geom + L.counters);
   B.ghist = reinterpret_cast<uint32_t *>(geom + L.ghist);
   B.stsort = reinterpret_cast<uint32_t *>(geom + L.stsort);
+  B.clsn = reinterpret_cast<uint32_t *>(geom + L.clsn);
+  B.clslist = reinterpret_cast<uint32_t *>(geom + L.clslist);
   B.vtile = reinterpret_cast<uint32_t *>(geom + L.vtile);
   B.vgroup = reinterpret_cast<uint32_t *>(geom + L.vgroup);
   B.stchunk = reinterpret_cast<unsigned long long *>(geom + L.stchunk);

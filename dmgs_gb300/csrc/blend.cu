@@ -42,24 +42,11 @@
 // * the adjoint sums a Gaussian's nine gradient terms over the thread's
 //   pixels, then over the warp with a transposed reduce-scatter (12
 //   shuffles); nine lanes then issue one scalar reduction each.
-#include "kernels.cuh"
+#include "blend_common.cuh"
 
 namespace dmgs {
 
 namespace {
-
-constexpr float ALPHA_MIN = 1.0f / 255.0f;
-constexpr float ALPHA_MAX = 0.99f;
-constexpr float T_EPS = 0.0001f;
-constexpr float LOG2E = 1.4426950408889634f;
-constexpr float LOG2_255 = 7.994353436858858f;
-constexpr unsigned FULL = 0xffffffffu;
-
-__device__ __forceinline__ float ex2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 
 // Staged Gaussian (forward): s0 = (x, y, A, B), s1 = (C, o, thr, r),
 // s2 = (g, b, footprint rows, 0) with exponent2 = A dx^2 + B dx dy + C dy^2
@@ -177,26 +164,6 @@ __device__ __forceinline__ Staged stage(const float4 f0, const float4 f1, const 
   return S;
 }
 
-// Exponent (base 2) of the Gaussian at (dx, dy).  Explicit intrinsics: the
-// adjoint evaluates the identical sequence.
-__device__ __forceinline__ float exponent2(float A, float B, float C, float dx, float dy) {
-  const float ax2 = __fmul_rn(__fmul_rn(A, dx), dx);
-  const float q = __fmul_rn(B, dx);
-  return __fmaf_rn(__fmaf_rn(C, dy, q), dy, ax2);
-}
-
-// The 48-byte record of list entry id; an entry outside the Gaussians (which
-// a correct list never holds) reads as a zero-opacity record, whose
-// footprint is empty, so no read leaves the geometry state.
-__device__ __forceinline__ void load_record(const BlendView &V, uint32_t id, float4 &f0, float4 &f1,
-                                            float4 &f2) {
-  if (id < V.P) {
-    f0 = V.feat[3 * id]; f1 = V.feat[3 * id + 1]; f2 = V.feat[3 * id + 2];
-  } else {
-    f0 = f1 = f2 = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-}
-
 // Work item -> (view, tile).
 __device__ __forceinline__ int find_view(const BlendBatch &bb, int item) {
   int v = 0;
@@ -256,12 +223,6 @@ __device__ __forceinline__ int next_item(uint32_t *queue, int &slot, int *s_item
   if (threadIdx.x == 0) *s_item = (int)atomicAdd(queue, 1u);
   __syncthreads();
   return *s_item;
-}
-
-__device__ __forceinline__ unsigned lanemask_lt() {
-  unsigned m;
-  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-  return m;
 }
 
 // The staged Gaussians (of cnt) whose footprint rows meet this warp's rows,
@@ -461,12 +422,6 @@ struct PixelState {
   uint32_t last_contrib;
 };
 
-__device__ __forceinline__ float rcp_approx(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 __device__ __forceinline__ void init_pixel(PixelState &ps, bool inside, int pix, size_t HW,
                                            const float *__restrict__ final_Ts,
                                            const uint32_t *__restrict__ n_contrib,
@@ -513,79 +468,6 @@ __device__ __forceinline__ void adjoint_pair(PixelState &ps, bool take, float al
   ps.ag = fmaf(at, S, ps.ag);
 }
 
-// From the thread's sums (e[0] = sum Gd, e[1] = sum Gd dy, e[2] = sum Gd dy^2
-// over its pixels; u = o Gd = dL/dpower) to the gradient terms: e0 =
-// dL/dndc_x, e1 = dL/dndc_y, e2..e4 = (sum u dx^2, sum u dx dy, sum u dy^2)
-// for the conic (scaled by -1/2, -1, -1/2 at the atomics), e5 = dL/dopacity.
-__device__ __forceinline__ void adjoint_finish(float dx, float o, const float4 &s2,
-                                               const float4 &s3, float *e) {
-  e[5] = e[0];
-  const float su = o * e[0], suy = o * e[1], suy2 = o * e[2];
-  const float sux = dx * su;
-  e[0] = sux * s2.z + suy * s2.w;
-  e[1] = suy * s3.x + sux * s3.y;
-  e[2] = sux * dx;
-  e[3] = suy * dx;
-  e[4] = suy2;
-}
-
-// Transposed reduce-scatter of the 9 gradient slots over the warp, 12
-// shuffles: each level halves the slots a lane keeps (5 | 4, 3 | 2, 2 | 1,
-// 1 | 1) and adds its partner's copy of them; afterwards the even lane 2q
-// holds the warp sum of slot slot9(q) (q = lane bits 4..1), none when that
-// is >= 9.
-__device__ __forceinline__ float warp_reduce_scatter9(const float (&v)[9], int lane) {
-  float a[5], b[3], c[2];
-  {
-    const bool hi = lane & 16;
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      const float up = i < 4 ? v[5 + i] : 0.f;
-      a[i] = (hi ? up : v[i]) + __shfl_xor_sync(FULL, hi ? v[i] : up, 16);
-    }
-  }
-  {
-    const bool hi = lane & 8;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const float up = i < 2 ? a[3 + i] : 0.f;
-      b[i] = (hi ? up : a[i]) + __shfl_xor_sync(FULL, hi ? a[i] : up, 8);
-    }
-  }
-  {
-    const bool hi = lane & 4;
-    c[0] = (hi ? b[2] : b[0]) + __shfl_xor_sync(FULL, hi ? b[0] : b[2], 4);
-    c[1] = (hi ? 0.f : b[1]) + __shfl_xor_sync(FULL, hi ? b[1] : 0.f, 4);
-  }
-  const bool hi = lane & 2;
-  const float d = (hi ? c[1] : c[0]) + __shfl_xor_sync(FULL, hi ? c[0] : c[1], 2);
-  return d + __shfl_xor_sync(FULL, d, 1);
-}
-
-// slot of the even lane 2q after warp_reduce_scatter9 (15: none)
-__device__ __forceinline__ int slot9(int q) {
-  return (int)((0xFFF8F765FF43F210ull >> (4 * q)) & 15u);
-}
-
-
-// The block's share (part of parts) of every span, set to zero.
-__device__ __forceinline__ void zero_spans(const ZeroSpans &z, unsigned part, unsigned parts) {
-  for (int k = 0; k < z.n; ++k) {
-    const size_t n = z.words[k];
-    const size_t chunk = (((n + parts - 1) / parts) + 3) & ~(size_t)3;
-    const size_t a = min(n, chunk * part), e = min(n, a + chunk);
-    float *p = z.p[k];
-    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {  // a is a multiple of 4 words (or the end)
-      const size_t e4 = a + ((e - a) & ~(size_t)3);
-      for (size_t i = a + 4 * (size_t)threadIdx.x; i < e4; i += 4 * (size_t)blockDim.x)
-        *reinterpret_cast<float4 *>(p + i) = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (size_t i = e4 + threadIdx.x; i < e; i += blockDim.x) p[i] = 0.f;
-    } else {
-      for (size_t i = a + threadIdx.x; i < e; i += blockDim.x) p[i] = 0.f;
-    }
-  }
-}
-
 // F64: the FP64-sum mode — the warp sums are added into double accumulators
 // (V.gacc64), so the result does not depend on the order in which warps and
 // tiles finish to well below float32 resolution.
@@ -602,7 +484,7 @@ blend_bwd_kernel(const BlendBatch bb, const ZeroSpans zero, uint32_t *queue) {
   const int tid = (int)threadIdx.x - h * THREADS;
   const int lane = tid & 31;
   const PixelLayout<PPT> lay(tid);
-  zero_spans(zero, blockIdx.x, gridDim.x);
+  zero_spans(zero, blockIdx.x, gridDim.x, threadIdx.x, blockDim.x);
   int slot_ = 0;
   for (int item = next_item(queue, slot_, &s_item); item < bb.total;
        item = next_item(queue, slot_, &s_item)) {
@@ -740,7 +622,8 @@ int run_bwd(const BlendBatch &bb, const ZeroSpans &zero, uint32_t *queue, cudaSt
 // adjoints add to or read: 48 B each instead of 48 B for every Gaussian
 // (16 views of 3M Gaussians, 0.14-0.55M visible per view: 0.17 GB written
 // instead of 2.3 GB).
-__global__ void __launch_bounds__(256) clear_gacc_kernel(const ClearViews cv) {
+__global__ void __launch_bounds__(256) clear_gacc_kernel(const ClearViews cv, uint32_t *queue) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *queue = 0u;
   const auto &V = cv.v[blockIdx.y];
   const uint32_t n = min(V.counters[CI_V], V.P);
   const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -752,12 +635,11 @@ __global__ void __launch_bounds__(256) clear_gacc_kernel(const ClearViews cv) {
   }
 }
 
-int launch_clear_gacc(const ClearViews &cv, int nviews, cudaStream_t s) {
-  uint32_t P = 0;
+int launch_clear_gacc(const ClearViews &cv, int nviews, uint32_t *queue, cudaStream_t s) {
+  uint32_t P = 1;
   for (int v = 0; v < nviews; ++v) P = max(P, cv.v[v].P);
-  if (P == 0) return DMGS_OK;
   const unsigned grid = min((P + 255) / 256, (unsigned)max(1, 16 * NUM_SMS_HINT / nviews));
-  dmgs_host::note_launch(), clear_gacc_kernel<<<dim3(grid, nviews), 256, 0, s>>>(cv);
+  dmgs_host::note_launch(), clear_gacc_kernel<<<dim3(grid, nviews), 256, 0, s>>>(cv, queue);
   DMGS_LAUNCH_CHECK("clear_gacc_kernel");
   return DMGS_OK;
 }
@@ -814,9 +696,17 @@ BlendBatch with_shape(const BlendBatch &bb, const BlendCfg &cfg) {
 
 }  // namespace
 
-int launch_blend_batch_fwd(const BlendBatch &bb, const BlendCfg &cfg, uint32_t *queue,
-                           cudaStream_t s) {
+namespace {
+bool is_default(const BlendCfg &c) {
+  const BlendCfg d = default_blend_cfg();
+  return c.ppt == d.ppt && c.batch == d.batch && c.sx == d.sx && c.sy == d.sy;
+}
+}  // namespace
+
+int launch_blend_batch_fwd(const BlendBatch &bb, const BlendWork &wk, const BlendCfg &cfg,
+                           uint32_t *queue, cudaStream_t s) {
   if (bb.total <= 0) return DMGS_OK;
+  if (is_default(cfg)) return launch_blend_warp_fwd(bb, wk, queue, s);
   int r = DMGS_OK;
   const BlendBatch b = with_shape(bb, cfg);
   DMGS_TIMED(K_BLEND_FWD, s, r = dispatch<true>(b, ZeroSpans(), cfg, queue, s));
@@ -825,11 +715,13 @@ int launch_blend_batch_fwd(const BlendBatch &bb, const BlendCfg &cfg, uint32_t *
   return DMGS_OK;
 }
 
-int launch_blend_batch_bwd(const BlendBatch &bb, const ClearViews &cv, const ZeroSpans &zero,
-                           const BlendCfg &cfg, uint32_t *queue, cudaStream_t s) {
+int launch_blend_batch_bwd(const BlendBatch &bb, const BlendWork &wk, const ClearViews &cv,
+                           const ZeroSpans &zero, const BlendCfg &cfg, uint32_t *queue,
+                           cudaStream_t s) {
   if (bb.total <= 0) return DMGS_OK;
-  int r = launch_clear_gacc(cv, bb.nviews, s);
+  int r = launch_clear_gacc(cv, bb.nviews, queue, s);
   if (r != DMGS_OK) return r;
+  if (is_default(cfg)) return launch_blend_warp_bwd(bb, wk, zero, queue, s);
   const BlendBatch b = with_shape(bb, cfg);
   DMGS_TIMED(K_BLEND_BWD, s, r = dispatch<false>(b, zero, cfg, queue, s));
   if (r != DMGS_OK) return r;
@@ -856,21 +748,30 @@ BlendView make_blend_view(const ViewParams &vp, const GeomLayout &L, const char 
   return v;
 }
 
+static BlendWork make_work(const GeomLayout &L, const char *geom) {
+  BlendWork w;
+  w.v[0] = {reinterpret_cast<const uint32_t *>(geom + L.clsn),
+            reinterpret_cast<const uint32_t *>(geom + L.clslist),
+            reinterpret_cast<const uint32_t *>(geom + L.counters)};
+  return w;
+}
+
 int launch_blend_fwd(const ViewParams &vp, const GeomLayout &L, const char *geom,
                      const BinLayout &B, const char *bin, const ImgLayout &I, char *img,
-                     const float *bg, float *out_color, cudaStream_t s) {
+                     const float *bg, float *out_color, uint32_t *queue, cudaStream_t s) {
+  DMGS_CUDA(cudaMemsetAsync(queue, 0, 4, s));  // a state may be rendered more than once
   BlendBatch bb;
   bb.nviews = 1;
   bb.v[0] = make_blend_view(vp, L, geom, B, bin, I, img, bg);
   bb.v[0].out_color = out_color;
   bb.total = bb.v[0].T;
-  return launch_blend_batch_fwd(bb, default_blend_cfg(), nullptr, s);
+  return launch_blend_batch_fwd(bb, make_work(L, geom), default_blend_cfg(), queue, s);
 }
 
 int launch_blend_bwd(const ViewParams &vp, const GeomLayout &L, const char *geom,
                      const BinLayout &B, const char *bin, const ImgLayout &I, const char *img,
                      const float *bg, const float *dL_dout, float *gacc, double *gacc64,
-                     const ZeroSpans &zero, cudaStream_t s) {
+                     const ZeroSpans &zero, uint32_t *queue, cudaStream_t s) {
   BlendBatch bb;
   bb.nviews = 1;
   bb.v[0] = make_blend_view(vp, L, geom, B, bin, I, const_cast<char *>(img), bg);
@@ -882,7 +783,7 @@ int launch_blend_bwd(const ViewParams &vp, const GeomLayout &L, const char *geom
     ClearViews cv;
     cv.v[0] = {reinterpret_cast<const uint32_t *>(geom + L.vlist),
                reinterpret_cast<const uint32_t *>(geom + L.counters), gacc, (uint32_t)L.P};
-    return launch_blend_batch_bwd(bb, cv, zero, default_blend_cfg(), nullptr, s);
+    return launch_blend_batch_bwd(bb, make_work(L, geom), cv, zero, default_blend_cfg(), queue, s);
   }
   const size_t n = (size_t)L.P * 12;
   DMGS_CUDA(cudaMemsetAsync(gacc64, 0, n * sizeof(double), s));

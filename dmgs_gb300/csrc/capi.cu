@@ -231,7 +231,8 @@ int dmgs_raster_fwd_render(const DmgsView *view, const DmgsGaussians *g, void *g
   RET_IF(make_bin_view(L, geom, 0xffffffffu, bin + B.point_list, (uint32_t)num_rendered, bv.v[0]));
   RET_IF(launch_emit(bv, s));
   RET_IF(debug_sync(view, s, "emit"));
-  RET_IF(launch_blend_fwd(vp, L, geom, B, bin, I, img, view->bg, out_color, s));
+  RET_IF(launch_blend_fwd(vp, L, geom, B, bin, I, img, view->bg, out_color,
+                          reinterpret_cast<uint32_t *>(geom + L.counters) + TK_BLEND, s));
   RET_IF(debug_sync(view, s, "blend_fwd"));
   if (view->debug) RET_IF(check_status(geom, L, s, nullptr));
   return DMGS_OK;
@@ -296,7 +297,9 @@ int raster_bwd_impl(const DmgsView *view, const DmgsGaussians *g, const float *d
   const ViewParams vp = make_params(view);
   const DmgsGrads out = *grads;
   RET_IF(launch_blend_bwd(vp, L, geom, B, bin, I, img, view->bg, dL_dout_color, gacc, gacc64,
-                          preprocess_bwd_outputs(out, g->P, g->M), s));
+                          preprocess_bwd_outputs(out, g->P, g->M),
+                          reinterpret_cast<uint32_t *>(static_cast<char *>(bwd_scratch) + bwd_queue_offset(g->P)),
+                          s));
   RET_IF(debug_sync(view, s, "blend_bwd"));
   RET_IF(launch_preprocess_bwd(vp, view->viewmatrix, view->projmatrix, view->campos,
                                make_gptrs(g), L, geom, gacc, out, s));

@@ -63,6 +63,7 @@ constexpr int CHUNK_COUNT_MAX = 2048;    // binning chunks per view (maximum)
 constexpr int CHUNK_W_GAUSS = 2;         // chunk weight of a Gaussian: this + ceil(rows / 16)
 constexpr int SEG_MAX = 32;              // row segments (groups of chunks) per view, maximum
 constexpr int XSEG = 512;                // tiles of one row handled by a tile-emission block
+constexpr int BLEND_CLASSES = 32;        // classes of tiles by list length, longest first; the last: empty
 constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;  // 4096 elements per block
@@ -78,7 +79,7 @@ constexpr int CI_W = 10;       // total chunk weight of the visible Gaussians (6
 constexpr int CI_WORDS = 16;
 // tickets: the words after the counters, from which the blocks of the
 // look-back kernels draw their tiles
-constexpr int TK_SORT = 16, TK_CHUNK = 20, TK_SCAN = 21;
+constexpr int TK_SORT = 16, TK_CHUNK = 20, TK_SCAN = 21, TK_BLEND = 22;
 constexpr int CI_TICKETS_END = 32;
 
 // Geometry state of one view.  Binning arrays: the visible Gaussians in index
@@ -87,15 +88,16 @@ constexpr int CI_TICKETS_END = 32;
 // 8 B); chunk starts; the row counts [gy][C] (Gaussians of chunk c covering
 // tile row r, scanned in place into row-list offsets); the segment counts
 // [T][S] (instances of tile t from row segment s, scanned in place into list
-// offsets); tile ranges; the radix sort's look-back words (stsort, per pass
+// offsets); tile ranges; per class of list lengths the tiles in it (clslist
+// [BLEND_CLASSES][T], clsn of them); the radix sort's look-back words (stsort, per pass
 // and key tile one word per digit); and one region that must be zero when a
 // view's preprocess starts: the counters and tickets, the digit histograms
 // of the four passes, the preprocess's visible counts (per tile of RADIX_TILE
 // Gaussians and per group of VGROUP tiles), and the look-back words of the
 // chunk weights and of the row / segment scans.
 struct GeomLayout {
-  size_t feat, flags, vlist, dkey0, dkey1, dval0, dval1, srect, cstart, rcnt, cnt2, ranges, stsort,
-      counters, ghist, vtile, vgroup, stchunk, stscan, total;
+  size_t feat, flags, vlist, dkey0, dkey1, dval0, dval1, srect, cstart, rcnt, cnt2, ranges, clslist, stsort,
+      counters, ghist, vtile, vgroup, clsn, stchunk, stscan, total;
   size_t zero_bytes;     // from counters on
   int P, gx, gy;
   int nb_pre, nb_radix;  // preprocess blocks; tiles of RADIX_TILE keys (or Gaussians)
@@ -126,11 +128,13 @@ __host__ __device__ inline GeomLayout geom_layout(int P, int W, int H) {
   L.rcnt = o;      o = align_up(o + n_rcnt * 4, 256);
   L.cnt2 = o;      o = align_up(o + n_cnt2 * 4, 256);
   L.ranges = o;    o = align_up(o + T * 8, 256);
+  L.clslist = o;   o = align_up(o + T * BLEND_CLASSES * 4, 256);
   L.stsort = o;    o = align_up(o + (size_t)L.nb_radix * (4 * 256 * 4), 256);
   L.counters = o;  o = align_up(o + CI_TICKETS_END * 4, 256);
   L.ghist = o;     o = align_up(o + 4 * 256 * 4, 256);
   L.vtile = o;     o = align_up(o + (size_t)L.nb_radix * 4, 256);
   L.vgroup = o;    o = align_up(o + (size_t)(L.nb_radix / VGROUP + 1) * 4, 256);
+  L.clsn = o;      o = align_up(o + BLEND_CLASSES * 4, 256);
   L.stchunk = o;   o = align_up(o + (size_t)L.nb_radix * 8, 256);
   L.stscan = o;    o = align_up(o + (scan_tiles(n_rcnt) + scan_tiles(n_cnt2)) * 8, 256);
   L.zero_bytes = o - L.counters;
@@ -183,7 +187,9 @@ __host__ __device__ inline ImgLayout img_layout(int W, int H) {
 //   g0 = (dL/dndc_x, dL/dndc_y, dL/dconic_a, dL/dconic_b)
 //   g1 = (dL/dconic_c, dL/dopacity, dL/dr, dL/dg)
 //   g2 = (dL/db, 0, 0, 0)
-inline size_t bwd_scratch_bytes(int P) { return align_up((size_t)P * 48, 256); }
+// then the queue word of the blend adjoint.
+inline size_t bwd_scratch_bytes(int P) { return align_up((size_t)P * 48, 256) + 256; }
+inline size_t bwd_queue_offset(int P) { return align_up((size_t)P * 48, 256); }
 
 __device__ __forceinline__ uint32_t pack_u16x2(int lo, int hi) {
   return (uint32_t)lo | ((uint32_t)hi << 16);

@@ -55,6 +55,7 @@ struct BinView {
   const float4 *feat;
   uint32_t *counters, *ghist, *vtile, *vgroup, *stsort, *vlist, *k0, *k1, *v0, *v1, *cstart, *rcnt, *cnt2;
   unsigned long long *stchunk, *stscan;
+  uint32_t *clsn, *clslist;
   uint2 *srect;          // packed tile rectangle per depth-sorted position
   uint2 *ranges;
   uint32_t *point_list;  // emission target (K_alloc entries)
@@ -134,6 +135,14 @@ struct ClearViews {
   } v[MAX_BATCH_VIEWS];
 };
 
+// Each view's tiles sorted into classes of list length (BLEND_CLASSES), and
+// its counters: the work list of the default blend kernels.
+struct BlendWork {
+  struct {
+    const uint32_t *cls_n, *cls_list, *counters;
+  } v[MAX_BATCH_VIEWS];
+};
+
 // Arrays the blend adjoint sets to zero while it runs (its stores meet an
 // idle DRAM): the outputs of which the preprocess adjoint then writes only
 // the visible Gaussians' rows.
@@ -162,23 +171,29 @@ struct BlendCfg {
 };
 inline BlendCfg default_blend_cfg() { return BlendCfg{4, 128, 1, 1}; }  // autotuned on GB300
 
-// queue == nullptr: one CTA per work item; else a persistent grid pulling
-// items from *queue (which must be zero at launch).
-int launch_blend_batch_fwd(const BlendBatch &bb, const BlendCfg &cfg, uint32_t *queue,
+// Blends the batch's views from the work list wk.  The default configuration
+// runs blend_warp.cu's kernels, any other the CTA-per-tile form with a
+// persistent grid; either pulls its items from *queue, which must be zero at
+// launch (forward) or is cleared here (adjoint).
+int launch_blend_batch_fwd(const BlendBatch &bb, const BlendWork &wk, const BlendCfg &cfg,
+                           uint32_t *queue, cudaStream_t s);
+// Clears the visible Gaussians' gradient records (cv) and *queue and runs the
+// adjoint, which also sets the arrays of `zero` to zero.
+int launch_blend_batch_bwd(const BlendBatch &bb, const BlendWork &wk, const ClearViews &cv,
+                           const ZeroSpans &zero, const BlendCfg &cfg, uint32_t *queue,
                            cudaStream_t s);
-// Clears the visible Gaussians' gradient records (cv) and runs the adjoint,
-// which also sets the arrays of `zero` to zero.
-int launch_blend_batch_bwd(const BlendBatch &bb, const ClearViews &cv, const ZeroSpans &zero,
-                           const BlendCfg &cfg, uint32_t *queue, cudaStream_t s);
+int launch_blend_warp_fwd(const BlendBatch &bb, const BlendWork &wk, uint32_t *queue, cudaStream_t s);
+int launch_blend_warp_bwd(const BlendBatch &bb, const BlendWork &wk, const ZeroSpans &zero,
+                          uint32_t *queue, cudaStream_t s);
 int launch_blend_fwd(const ViewParams &vp, const GeomLayout &L, const char *geom,
                      const BinLayout &B, const char *bin, const ImgLayout &I, char *img,
-                     const float *bg, float *out_color, cudaStream_t s);
+                     const float *bg, float *out_color, uint32_t *queue, cudaStream_t s);
 // gacc64 != nullptr: the FP64-sum mode (gradient terms added into [P][12]
 // doubles, then rounded into gacc for the preprocess adjoint).
 int launch_blend_bwd(const ViewParams &vp, const GeomLayout &L, const char *geom,
                      const BinLayout &B, const char *bin, const ImgLayout &I, const char *img,
                      const float *bg, const float *dL_dout, float *gacc, double *gacc64,
-                     const ZeroSpans &zero, cudaStream_t s);
+                     const ZeroSpans &zero, uint32_t *queue, cudaStream_t s);
 
 // preprocess_bwd.cu
 int launch_preprocess_bwd_batched(const BatchViews &bv, const GaussianPtrs &g, const DmgsGrads &out,

@@ -26,8 +26,10 @@
 namespace {
 
 constexpr size_t kFloatsPerGaussian = 12;  // 48-byte accumulator record
+constexpr size_t kQueueFloats = 64;        // the blend adjoint's queue word, in a line of its own
 static __device__ __align__(256) float g_noalloc_bwd_scratch[(size_t)DMGS_NOALLOC_MAX_GAUSSIANS *
-                                                             kFloatsPerGaussian];
+                                                                 kFloatsPerGaussian +
+                                                             kQueueFloats];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
