@@ -371,51 +371,41 @@ blend_fwd_warp_kernel(const BlendBatch bb, const BlendWork wk, uint32_t *queue) 
 // ---- adjoint --------------------------------------------------------------------
 
 // What the warp's visits leave to be summed over its lanes: per Gaussian nine
-// rows of 32 (with Gd = dL/dopacity's term of a pixel: sums of Gd dx, Gd dy,
-// Gd dx^2, Gd dx dy, Gd dy^2, Gd, and of dL/drgb), RED_N Gaussians at a time.
-// Lane t < 9 RED_N then adds up row t (16-byte loads; the pitch puts eight
-// consecutive rows in different banks), applies the Gaussian's own factors
-// and issues one reduction: 20 instructions a Gaussian, where a shuffle tree
-// per visit took 48 and the factors 10 more.
+// rows of 32 (with Gd = dL/dopacity's term of a pixel: dL/dndc x and y per
+// unit opacity, sums of Gd dx^2, Gd dx dy, Gd dy^2, Gd, and of dL/drgb),
+// RED_N Gaussians at a time.  Lane t < 9 RED_N then adds up row t (16-byte
+// loads; the pitch puts eight consecutive rows in different banks) and issues
+// one reduction: 20 instructions a Gaussian, where a shuffle tree per visit
+// took 48.  The NDC terms a dx + b dy and b dx + c dy are formed per lane:
+// for a needle the two products nearly cancel, and summed apart first their
+// rounding would be that of the whole sums.
 constexpr int RED_N = 3, RED_P = 36;
-constexpr int AUX_WORDS = 6;  // a W / 2, b W / 2, c H / 2, b H / 2, opacity, index
 
 struct alignas(16) Pending {
   float row[9 * RED_N][RED_P];
-  float aux[RED_N][AUX_WORDS];
+  float opacity[RED_N];
+  uint32_t id[RED_N];
 };
 
 __device__ __forceinline__ void flush_pending(Pending &R, int n, float *gacc, int lane) {
   __syncwarp();
-  float sum = 0.f;
   if (lane < 9 * n) {
     const float4 *r = reinterpret_cast<const float4 *>(R.row[lane]);
-    float4 a = r[0];
-#pragma unroll
-    for (int k = 1; k < 8; ++k) {
-      const float4 x = r[k];
-      a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
-    }
-    sum = (a.x + a.y) + (a.z + a.w);
-  }
-  const int which = lane / 9, slot = lane - 9 * which;
-  const float other = __shfl_sync(FULL, sum, slot == 0 ? lane + 1 : lane - 1);  // slots 0 and 1: each other's
-  if (lane < 9 * n) {
-    const float *x = R.aux[which];
-    // dL/dndc = -(W/2) (a Sx + b Sy), -(H/2) (c Sy + b Sx); the conic's terms
-    // are -1/2 Sxx, -Sxy, -1/2 Syy; each S times the opacity (dL/dpower = o Gd)
-    float v = sum;
-    if (slot < 2) v = -(x[2 * slot] * sum + x[slot == 0 ? 1 : 3] * other);
-    if (slot >= 2 && slot < 5) v = (slot == 3 ? -1.f : -0.5f) * sum;
-    if (slot < 5) v *= x[4];
-    atomicAdd(gacc + (size_t)__float_as_uint(x[5]) * 12 + slot, v);
+    // lanes 16, 8, 4, 2, 1 apart in turn: the rounding of a shuffle tree
+    auto add = [](float4 x, float4 y) { return make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w); };
+    const float4 a = add(add(add(r[0], r[4]), add(r[2], r[6])), add(add(r[1], r[5]), add(r[3], r[7])));
+    const int which = lane / 9, slot = lane - 9 * which;
+    float v = (a.x + a.z) + (a.y + a.w);
+    if (slot < 5) v *= R.opacity[which];  // dL/dpower = o Gd
+    if (slot >= 2 && slot < 5) v *= slot == 3 ? -1.f : -0.5f;  // the conic's terms
+    atomicAdd(gacc + (size_t)R.id[which] * 12 + slot, v);
   }
   __syncwarp();
 }
 
 template <int PPT>
-__device__ __forceinline__ void bwd_part(const BlendView &V, int tile, int part, float4 (*S)[32],
-                                         float (*X)[AUX_WORDS], Pending &R, int lane) {
+__device__ __forceinline__ void bwd_part(const BlendView &V, int tile, int part, float4 (*S)[32], float4 *K,
+                                         uint32_t *I, Pending &R, int lane) {
   using P = Px<PPT>;
   using F = typename P::V;
   constexpr int RB = 2 * PPT, N = P::N, G = P::G;
@@ -471,8 +461,8 @@ __device__ __forceinline__ void bwd_part(const BlendView &V, int tile, int part,
       const int s = __popc(bal & lanemask_lt());
       const Entry E{f0.x, f0.y, A, B, C, f1.y, thr, f1.z, f1.w, f2.x, most - 1u - base - lane};
       E.put(S, s);
-      X[s][0] = f0.z * hw; X[s][1] = f0.w * hw; X[s][2] = f1.x * hh; X[s][3] = f0.w * hh;
-      X[s][4] = f1.y; X[s][5] = __uint_as_float(id);
+      K[s] = make_float4(-f0.z * hw, -f0.w * hw, -f1.x * hh, -f0.w * hh);
+      I[s] = id;
     }
     if (base + 32 < most) {
       id = nid;
@@ -537,8 +527,9 @@ __device__ __forceinline__ void bwd_part(const BlendView &V, int tile, int part,
       // the lane's pixels share dx
       const float m0 = P::sum(M[0]), m1 = P::sum(M[1]), mx = dx * m0;
       float(*row)[RED_P] = R.row + 9 * np;
-      row[0][lane] = mx;
-      row[1][lane] = m1;
+      const float4 kk = K[i];
+      row[0][lane] = mx * kk.x + m1 * kk.y;
+      row[1][lane] = m1 * kk.z + mx * kk.w;
       row[2][lane] = mx * dx;
       row[3][lane] = m1 * dx;
       row[4][lane] = P::sum(M[2]);
@@ -546,7 +537,10 @@ __device__ __forceinline__ void bwd_part(const BlendView &V, int tile, int part,
       row[6][lane] = P::sum(M[3]);
       row[7][lane] = P::sum(M[4]);
       row[8][lane] = P::sum(M[5]);
-      if (lane < AUX_WORDS) R.aux[np][lane] = X[i][lane];
+      if (lane == 0) {
+        R.opacity[np] = E.o;
+        R.id[np] = I[i];
+      }
       if (++np == RED_N) {
         flush_pending(R, RED_N, V.gacc, lane);
         np = 0;
@@ -561,7 +555,8 @@ __global__ void __launch_bounds__(32 * BW_WARPS, 10)
 blend_bwd_warp_kernel(const BlendBatch bb, const BlendWork wk, const ZeroSpans zero, uint32_t *queue) {
   __shared__ WorkTable tab;
   __shared__ float4 S[BW_WARPS][3][32];
-  __shared__ float X[BW_WARPS][32][AUX_WORDS];
+  __shared__ float4 K[BW_WARPS][32];
+  __shared__ uint32_t I[BW_WARPS][32];
   __shared__ Pending R[BW_WARPS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   build_table<true>(wk, bb.nviews, tab);
@@ -572,8 +567,8 @@ blend_bwd_warp_kernel(const BlendBatch bb, const BlendWork wk, const ZeroSpans z
     const Item it = find_item(wk, bb, tab, i, lane);
     const BlendView &V = bb.v[it.view];
     zero_spans(zero, i, tab.total, lane, 32u);
-    if (it.fine) bwd_part<1>(V, it.tile, it.part, S[w], X[w], R[w], lane);
-    else bwd_part<4>(V, it.tile, it.part, S[w], X[w], R[w], lane);
+    if (it.fine) bwd_part<1>(V, it.tile, it.part, S[w], K[w], I[w], R[w], lane);
+    else bwd_part<4>(V, it.tile, it.part, S[w], K[w], I[w], R[w], lane);
   }
 }
 
