@@ -183,6 +183,34 @@ def load(path: str | None = None):
         return lib
 
 
+_native = None
+
+
+def native():
+    """The extension with the native autograd nodes (csrc/autograd.cpp).  On a
+    machine with a GPU it must be there; without one its entries would refuse
+    every call, so a package that was not built has None."""
+    global _native
+    if _native is None:
+        if not os.path.exists(os.path.join(_HERE, "_autograd.so")) and not torch.cuda.is_available():
+            return None
+        load()
+        try:
+            from . import _autograd
+        except ImportError as e:
+            raise RuntimeError("dmgs_gb300/_autograd.so is missing or does not load: build it with "
+                               "`python -m dmgs_gb300.build` (or __graft_entry__.build())") from e
+        _native = _autograd
+    return _native
+
+
+def native_call(name, *args):
+    """The result of the native entry `name`, or None when the call needs the
+    general form (see csrc/autograd.cpp)."""
+    n = native()
+    return None if n is None else getattr(n, name)(*args)
+
+
 class DmgsError(RuntimeError):
     def __init__(self, code: int, where: str, msg: str):
         super().__init__(f"{where}: {DMGS_ERRORS.get(code, code)}: {msg}")

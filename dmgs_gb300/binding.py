@@ -96,8 +96,12 @@ def bind_faces(verts, faces, bc, scale_factor, rad_base, spatial_lr_scale, max_s
     per_g = bc.dim() == 3
     G = bc.shape[1] if per_g else bc.shape[0]
     z_scale = float(spatial_lr_scale) * 1e-6
-    return _Bind2.apply(verts, scale_factor, faces, bc.reshape(-1, 3), G, per_g, rad_base,
-                        z_scale, max_scale, adaptive_cov)
+    bc = bc.reshape(-1, 3)
+    out = _lib.native_call("bind2", verts, scale_factor, faces, bc, G, per_g, float(rad_base), z_scale,
+                           float(max_scale), bool(adaptive_cov))
+    if out is not None:
+        return out
+    return _Bind2.apply(verts, scale_factor, faces, bc, G, per_g, rad_base, z_scale, max_scale, adaptive_cov)
 
 
 class _Bind3(torch.autograd.Function):
@@ -140,7 +144,8 @@ class _Bind3(torch.autograd.Function):
 def bind_faces_scale_rot(verts, faces, bc, scaling2d, rotation2d, thin_z):
     """Stage-3 binding.  Returns (xyz, scales, rotations) for the rasteriser's
     scale/rotation input mode."""
-    return _Bind3.apply(verts, scaling2d, rotation2d, faces, bc, thin_z)
+    out = _lib.native_call("bind3", verts, scaling2d, rotation2d, faces, bc, float(thin_z))
+    return _Bind3.apply(verts, scaling2d, rotation2d, faces, bc, thin_z) if out is None else out
 
 
 def frustum_faces(verts, faces, full_proj):

@@ -1,8 +1,10 @@
 """Build recipe for libdmgs_gb300.so (sm_103a only).
 
 Compiles every ``csrc/*.cu`` translation unit in parallel with nvcc and links
-them into ``dmgs_gb300/libdmgs_gb300.so`` (in-tree, git-ignored).  Objects go
-to ``dmgs_gb300/_build/``.  Rebuilds only what changed.
+them into ``dmgs_gb300/libdmgs_gb300.so`` (in-tree, git-ignored); beside them
+the host compiler builds ``csrc/autograd.cpp``, the native autograd nodes, into
+``dmgs_gb300/_autograd.so``.  Objects go to ``dmgs_gb300/_build/``.  Rebuilds
+only what changed.
 """
 from __future__ import annotations
 
@@ -11,11 +13,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libdmgs_gb300.so")
+EXT = os.path.join(HERE, "_autograd.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
@@ -40,6 +44,23 @@ def _headers():
     return hs
 
 
+def _ext_commands():
+    """(compile, link) commands of the autograd extension, its object."""
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    obj = os.path.join(BUILD, "autograd.cpp.o")
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    cxx = os.environ.get("CXX") or shutil.which("g++") or "c++"
+    comp = [cxx, "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-w",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *[a for i in inc for a in ("-isystem", i)], "-c", os.path.join(CSRC, "autograd.cpp"), "-o", obj]
+    link = [cxx, "-shared", "-o", EXT + ".tmp", obj, "-L", os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu",
+            "-ltorch_python", "-lc10", "-lc10_cuda", "-L", HERE, "-l:libdmgs_gb300.so", "-Wl,-rpath,$ORIGIN"]
+    return comp, link, obj
+
+
 def _stale(target: str, deps) -> bool:
     if not os.path.exists(target):
         return True
@@ -61,6 +82,12 @@ def build(verbose: bool = False, force: bool = False, extra_flags=()) -> str:
             cmd = [nvcc, *NVCC_FLAGS, *extra_flags, "-I", INCLUDE, "-c", src, "-o", obj]
             jobs.append(cmd)
 
+    ext_src = os.path.join(CSRC, "autograd.cpp")
+    ext_compile, ext_link, ext_obj = _ext_commands()
+    ext_stale = force or _stale(ext_obj, [ext_src, os.path.join(INCLUDE, "dmgs.h"), __file__])
+    if ext_stale:
+        jobs.insert(0, ext_compile)
+
     def run(cmd):
         r = subprocess.run(cmd, capture_output=True, text=True)
         return cmd, r
@@ -71,7 +98,7 @@ def build(verbose: bool = False, force: bool = False, extra_flags=()) -> str:
                 if verbose or r.returncode != 0:
                     sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
                 if r.returncode != 0:
-                    raise RuntimeError(f"nvcc failed for {cmd[-3]}")
+                    raise RuntimeError(f"{os.path.basename(cmd[0])} failed for {cmd[-3]}")
     if force or jobs or _stale(LIB, objs):
         tmp = LIB + ".tmp"
         cmd = [nvcc, *ARCH, "-shared", "-cudart", "shared", "-o", tmp, *objs,
@@ -82,6 +109,13 @@ def build(verbose: bool = False, force: bool = False, extra_flags=()) -> str:
         if r.returncode != 0:
             raise RuntimeError("link of libdmgs_gb300.so failed")
         os.replace(tmp, LIB)
+    if ext_stale or _stale(EXT, [ext_obj]):
+        r = subprocess.run(ext_link, capture_output=True, text=True)
+        if verbose or r.returncode != 0:
+            sys.stderr.write(" ".join(ext_link) + "\n" + r.stdout + r.stderr)
+        if r.returncode != 0:
+            raise RuntimeError("link of _autograd.so failed")
+        os.replace(EXT + ".tmp", EXT)
     return LIB
 
 

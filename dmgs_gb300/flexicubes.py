@@ -178,11 +178,14 @@ def flexicubes(x_nx3, s_n, res, beta_fx12=None, alpha_fx8=None, gamma_f=None, tr
     nocheck = not de_ambiguity
     W = _fused_weights(beta_fx12, alpha_fx8, gamma_f, Cn)
     if W is not None:  # the three weights are column slices of one tensor: read it in place
-        v, f, L, se = _FlexiCubesFn.apply(x_nx3, s_n.reshape(-1), W, None, None, res,
-                                          bool(training), True, vm, nocheck)
+        weights = (W, None, None)
     else:
-        v, f, L, se = _FlexiCubesFn.apply(x_nx3, s_n.reshape(-1), beta_fx12, alpha_fx8,
-                                          gamma_f, res, bool(training), False, vm, nocheck)
+        weights = (beta_fx12, alpha_fx8, gamma_f)
+    s = s_n.reshape(-1)
+    out = _lib.native_call("flexicubes", x_nx3, s, *weights, vm, *res, bool(training), W is not None, nocheck)
+    if out is None:
+        out = _FlexiCubesFn.apply(x_nx3, s, *weights, res, bool(training), W is not None, vm, nocheck)
+    v, f, L, se = out
     if v.shape[0] == 0 and f.shape[0] == 0 and se.shape[0] == 0:
         return v, f, L, None   # the reference's result for a grid without surface
     return v, f, L, se

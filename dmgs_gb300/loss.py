@@ -35,4 +35,5 @@ class _L1SSIM(torch.autograd.Function):
 def l1_ssim_loss(image, target, lambda_dssim=0.2):
     """(1 - lambda) mean|image - target| + lambda (1 - mean SSIM) for [C,H,W]
     images; differentiable w.r.t. image."""
-    return _L1SSIM.apply(image, target, lambda_dssim)
+    out = _lib.native_call("l1_ssim", image, target, float(lambda_dssim))
+    return _L1SSIM.apply(image, target, lambda_dssim) if out is None else out

@@ -218,6 +218,14 @@ class _RasterizeGaussians(torch.autograd.Function):
 
 def rasterize_gaussians(means3D, means2D, sh, colors_precomp, opacities, scales, rotations,
                         cov3Ds_precomp, raster_settings):
+    rs = raster_settings
+    if not rs.debug:  # the debug snapshots are the general form's
+        out = _lib.native_call("raster", means3D, means2D, sh, colors_precomp, opacities, scales, rotations,
+                               cov3Ds_precomp, rs.bg, rs.viewmatrix, rs.projmatrix, rs.campos,
+                               int(rs.image_height), int(rs.image_width), float(rs.tanfovx), float(rs.tanfovy),
+                               float(rs.scale_modifier), int(rs.sh_degree), bool(rs.prefiltered))
+        if out is not None:
+            return out
     return _RasterizeGaussians.apply(means3D, means2D, sh, colors_precomp, opacities, scales,
                                      rotations, cov3Ds_precomp, raster_settings)
 

@@ -55,4 +55,5 @@ def sh_colors(deg, sh, xyz, campos):
         raise ValueError("sh_colors: sh must be [P, 3, K] with P = xyz.shape[0]")
     if not 0 <= int(deg) <= 3 or sh.shape[2] < (int(deg) + 1) ** 2:
         raise ValueError("sh_colors: degree 0..3 with K >= (deg + 1)^2")
-    return _SHColors.apply(int(deg), sh, xyz, campos)
+    out = _lib.native_call("sh_colors", sh, xyz, campos, int(deg))
+    return _SHColors.apply(int(deg), sh, xyz, campos) if out is None else out

@@ -141,6 +141,7 @@ class MLPTexture3D(torch.nn.Module):
         if getattr(self, "_aabb_src", None) is not a or self._aabb_ver != version:
             self._aabb_cache = torch.as_tensor(a, dtype=torch.float32).detach().cpu().reshape(2, 3).clone()
             self._aabb_src, self._aabb_ver = a, version
+            self._aabb_list = self._aabb_cache.reshape(-1).tolist()
         return self._aabb_cache
 
     def sample_noact(self, texc):
@@ -151,8 +152,11 @@ class MLPTexture3D(torch.nn.Module):
         W1, W2, W3 = self.net.weights()
         keep = torch.is_grad_enabled() and any(
             t.requires_grad for t in (texc, self.encoder.params, W1, W2, W3))
-        out = _TextureFn.apply(texc.reshape(-1, 3), self.encoder.params, W1, W2, W3,
-                               self._aabb_host(), self.per_level_scale, keep)
+        aabb, x = self._aabb_host(), texc.reshape(-1, 3)
+        out = _lib.native_call("texture", x, self.encoder.params, W1, W2, W3, self._aabb_list,
+                               self.per_level_scale, keep)
+        if out is None:
+            out = _TextureFn.apply(x, self.encoder.params, W1, W2, W3, aabb, self.per_level_scale, keep)
         return out.view(*texc.shape[:-1], self.channels)
 
     def sample(self, texc):
