@@ -7,7 +7,7 @@
 // pixels (Wang et al. 2004).  In torch that is five depthwise convolutions
 // forward and their adjoints.  Here two kernels:
 //
-//   1. moments: each 16 x 16 tile of every channel loads x, y with a 5-pixel
+//   1. moments: each 32 x 54 tile of every channel loads x, y with a 5-pixel
 //      halo into shared memory, blurs the five moments (x, y, xx, yy, xy)
 //      separably, and per pixel forms S and the partial derivatives of S
 //      w.r.t. mu_x (A), E[x^2] (B) and E[xy] (D); the block's sums of S and
@@ -16,6 +16,14 @@
 //      adjoint of the blur is the same blur) and forms
 //      dL/dx = (1 - lambda)/N sign(x - y) - lambda/N (wA + 2 x wB + y wD);
 //      the first block also reduces the partials into the loss.
+//
+// Bound by instruction issue: 110 multiply-adds a pixel and channel in the
+// first kernel.  A thread forms four horizontal or seven vertical outputs
+// from values held in registers, so that an output costs 3.5 and 2.4 shared
+// loads per quantity instead of 11 (one output per thread and products kept
+// in shared memory: 178 us for both kernels at 3 x 822 x 1237, against 81).
+// 54 rows + 10 of halo are 64 rows of 8 groups of 4 columns (two rounds of
+// the 256 threads) and 8 groups of 7 rows of 32 columns (one round).
 //
 // With s11 = E[x^2] - mu_x^2, s22 = E[y^2] - mu_y^2, s12 = E[xy] - mu_x mu_y,
 // N1 = 2 mu_x mu_y + C1, N2 = 2 s12 + C2, D1 = mu_x^2 + mu_y^2 + C1,
@@ -30,48 +38,94 @@ namespace dmgs {
 
 namespace {
 
-constexpr int LT = 16;        // output tile
-constexpr int LR = 5;         // window radius
-constexpr int LH = LT + 2 * LR;  // tile with halo (26)
+constexpr int LR = 5;              // window radius
+constexpr int LTAP = 2 * LR + 1;
+constexpr int LW = 32, LHT = 54;   // output tile: columns, rows
+constexpr int LROWS = LHT + 2 * LR;  // 64 rows with the halo
+constexpr int LP = 44;             // pitch of a haloed row (42 columns; rows 16-byte aligned)
+constexpr int LN = 256;            // threads
+constexpr int LV = 7;              // vertical outputs per thread
+constexpr int LHS = LV * (LN / LW) + 2 * LR;  // rows the vertical pass reads (the last two of no output)
+static_assert(LROWS * (LW / 4) == 2 * LN && LW * ((LHT + LV - 1) / LV) == LN, "tile and block sizes");
 
 struct Window {
-  float w[2 * LR + 1];
+  float w[LTAP];
 };
 
-// Separable blur of NQ quantities held in shared memory as [NQ][LH][LH]
-// (halo included): horizontal pass into hs [NQ][LH][LT], vertical pass to
-// the tile's pixel (ty, tx) -> out[NQ].
+// One or two images' haloed tile into shared memory, zero outside the image:
+// a warp per row (columns lane and lane + 32), rows LN / 32 apart, so that a
+// row's bounds are the warp's and no index is divided.
 template <int NQ>
-__device__ __forceinline__ void blur_tile(const float (*in)[LH][LH], float (*hs)[LH][LT],
-                                          const Window &W, float *out) {
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  for (int r = ty; r < LH; r += LT) {
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      float a = 0.f;
-#pragma unroll
-      for (int k = 0; k <= 2 * LR; ++k) a = fmaf(W.w[k], in[q][r][tx + k], a);
-      hs[q][r][tx] = a;
+__device__ __forceinline__ void load_tile(const float *__restrict__ a, const float *__restrict__ b, int H, int Wd,
+                                          int ox, int oy, float (*da)[LP], float (*db)[LP]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int x0 = ox + lane, x1 = x0 + 32;
+  const bool in0 = x0 >= 0 && x0 < Wd, more = lane < LW + 2 * LR - 32, in1 = more && x1 < Wd;
+#pragma unroll 4
+  for (int r = w; r < LROWS; r += LN / 32) {
+    const int gy = oy + r;
+    const bool row = gy >= 0 && gy < H;
+    const size_t o = (size_t)(row ? gy : 0) * Wd;
+    const float a0 = row && in0 ? a[o + x0] : 0.f, a1 = row && in1 ? a[o + x1] : 0.f;
+    float b0 = 0.f, b1 = 0.f;
+    if (NQ == 2) {
+      b0 = row && in0 ? b[o + x0] : 0.f;
+      b1 = row && in1 ? b[o + x1] : 0.f;
+    }
+    da[r][lane] = a0;
+    if (more) da[r][lane + 32] = a1;
+    if (NQ == 2) {
+      db[r][lane] = b0;
+      if (more) db[r][lane + 32] = b1;
     }
   }
-  __syncthreads();
+}
+
+// Row r's 14 values from column 4 g on.
+__device__ __forceinline__ void load_row(const float (*src)[LP], int r, int g, float (&v)[16]) {
+  const float4 *p = reinterpret_cast<const float4 *>(&src[r][4 * g]);
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) {
+  for (int k = 0; k < 4; ++k) {  // the last two of the 16 (of the pitch's padding at most) are not used
+    const float4 x = p[k];
+    v[4 * k] = x.x; v[4 * k + 1] = x.y; v[4 * k + 2] = x.z; v[4 * k + 3] = x.w;
+  }
+}
+
+// Four horizontal outputs of a quantity, taps in ascending order.
+__device__ __forceinline__ float4 blur4(const Window &W, const float (&v)[16]) {
+  float o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
     float a = 0.f;
 #pragma unroll
-    for (int k = 0; k <= 2 * LR; ++k) a = fmaf(W.w[k], hs[q][ty + k][tx], a);
-    out[q] = a;
+    for (int k = 0; k < LTAP; ++k) a = fmaf(W.w[k], v[j + k], a);
+    o[j] = a;
+  }
+  return make_float4(o[0], o[1], o[2], o[3]);
+}
+
+// The thread's LV vertical outputs of a quantity (column c, rows LV gv ..).
+__device__ __forceinline__ void blur_column(const Window &W, const float (*hs)[LW], int c, int gv, float (&o)[LV]) {
+  float v[LV + 2 * LR];
+#pragma unroll
+  for (int k = 0; k < LV + 2 * LR; ++k) v[k] = hs[gv * LV + k][c];
+#pragma unroll
+  for (int j = 0; j < LV; ++j) {
+    float a = 0.f;
+#pragma unroll
+    for (int k = 0; k < LTAP; ++k) a = fmaf(W.w[k], v[j + k], a);
+    o[j] = a;
   }
 }
 
 __device__ __forceinline__ float block_sum(float v, float *red) {
-  const int t = threadIdx.y * LT + threadIdx.x;
+  const int t = threadIdx.x;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   if ((t & 31) == 0) red[t >> 5] = v;
   __syncthreads();
   float s = 0.f;
-  if (t < LT * LT / 32) s = red[t];
+  if (t < LN / 32) s = red[t];
   if (t < 32) {
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -79,108 +133,140 @@ __device__ __forceinline__ float block_sum(float v, float *red) {
   return s;  // valid in thread 0
 }
 
+struct MomentsSmem {
+  float x[LROWS][LP], y[LROWS][LP];
+  float hs[5][LHS][LW];
+  float red[LN / 32];
+};
+
+struct GradSmem {
+  float in[LROWS][LP];
+  float hs[3][LHS][LW];
+  float red[LN / 32];
+};
+
 // Grid: (tiles x, tiles y, channels).  ABD: [3][C][H][W] scratch;
 // part: 2 floats per block (sum S, sum |x - y|).
-__global__ void __launch_bounds__(LT * LT)
+__global__ void __launch_bounds__(LN)
 ssim_moments_kernel(const float *__restrict__ x, const float *__restrict__ y, int H, int Wd,
                     Window W, float *__restrict__ ABD, float *__restrict__ part) {
-  __shared__ float in[5][LH][LH];
-  __shared__ float hs[5][LH][LT];
-  __shared__ float red[LT * LT / 32];
-  const int c = blockIdx.z;
+  extern __shared__ __align__(16) char loss_smem[];
+  MomentsSmem &sm = *reinterpret_cast<MomentsSmem *>(loss_smem);
+  const int c = blockIdx.z, t = threadIdx.x;
   const size_t plane = (size_t)H * Wd;
-  const float *xc = x + c * plane, *yc = y + c * plane;
-  const int ox = blockIdx.x * LT - LR, oy = blockIdx.y * LT - LR;
-  for (int i = threadIdx.y * LT + threadIdx.x; i < LH * LH; i += LT * LT) {
-    const int r = i / LH, q = i - r * LH;
-    const int gy = oy + r, gx = ox + q;
-    float a = 0.f, b = 0.f;
-    if (gy >= 0 && gy < H && gx >= 0 && gx < Wd) {
-      a = xc[(size_t)gy * Wd + gx];
-      b = yc[(size_t)gy * Wd + gx];
-    }
-    in[0][r][q] = a; in[1][r][q] = b;
-    in[2][r][q] = a * a; in[3][r][q] = b * b; in[4][r][q] = a * b;
+  const int ox = blockIdx.x * LW, oy = blockIdx.y * LHT;
+  load_tile<2>(x + c * plane, y + c * plane, H, Wd, ox - LR, oy - LR, sm.x, sm.y);
+  __syncthreads();
+#pragma unroll 1
+  for (int i = t; i < LROWS * (LW / 4); i += LN) {
+    const int r = i >> 3, g = i & 7;
+    float a[16], b[16], p[16];
+    load_row(sm.x, r, g, a);
+    load_row(sm.y, r, g, b);
+    auto put = [&](int q, float4 v) { *reinterpret_cast<float4 *>(&sm.hs[q][r][4 * g]) = v; };
+    put(0, blur4(W, a));
+    put(1, blur4(W, b));
+#pragma unroll
+    for (int k = 0; k < 14; ++k) p[k] = __fmul_rn(a[k], a[k]);
+    put(2, blur4(W, p));
+#pragma unroll
+    for (int k = 0; k < 14; ++k) p[k] = __fmul_rn(b[k], b[k]);
+    put(3, blur4(W, p));
+#pragma unroll
+    for (int k = 0; k < 14; ++k) p[k] = __fmul_rn(a[k], b[k]);
+    put(4, blur4(W, p));
   }
   __syncthreads();
-  float m[5];
-  blur_tile<5>(in, hs, W, m);
-  const int px = blockIdx.x * LT + threadIdx.x, py = blockIdx.y * LT + threadIdx.y;
-  const bool inside = px < Wd && py < H;
-  float S = 0.f, l1 = 0.f;
-  if (inside) {
+  const int col = t & (LW - 1), gv = t / LW;
+  float m[5][LV];
+#pragma unroll
+  for (int q = 0; q < 5; ++q) blur_column(W, sm.hs[q], col, gv, m[q]);
+  float S_sum = 0.f, l1 = 0.f;
+  const int px = ox + col;
+#pragma unroll
+  for (int j = 0; j < LV; ++j) {
+    const int row = gv * LV + j, py = oy + row;
+    if (row >= LHT || px >= Wd || py >= H) continue;
     constexpr float C1 = 0.01f * 0.01f, C2 = 0.03f * 0.03f;
-    const float mx = m[0], my = m[1];
-    const float s11 = m[2] - mx * mx, s22 = m[3] - my * my, s12 = m[4] - mx * my;
+    const float mx = m[0][j], my = m[1][j];
+    const float s11 = m[2][j] - mx * mx, s22 = m[3][j] - my * my, s12 = m[4][j] - mx * my;
     const float N1 = 2.f * mx * my + C1, N2 = 2.f * s12 + C2;
     const float D1 = mx * mx + my * my + C1, D2 = s11 + s22 + C2;
     const float inv = 1.f / (D1 * D2);
-    S = N1 * N2 * inv;
-    const float A = 2.f * my * (N2 - N1) * inv - 2.f * mx * S / D1 + 2.f * mx * S / D2;
-    const float B = -S / D2;
+    const float S = N1 * N2 * inv;
+    const float S1 = S * (D2 * inv), S2 = S * (D1 * inv);  // S / D1, S / D2
+    const float A = 2.f * my * (N2 - N1) * inv - 2.f * mx * S1 + 2.f * mx * S2;
+    const float B = -S2;
     const float Dd = 2.f * N1 * inv;
     const size_t o = c * plane + (size_t)py * Wd + px;
     const size_t all = (size_t)gridDim.z * plane;
     ABD[o] = A;
     ABD[all + o] = B;
     ABD[2 * all + o] = Dd;
-    l1 = fabsf(in[0][threadIdx.y + LR][threadIdx.x + LR] - in[1][threadIdx.y + LR][threadIdx.x + LR]);
+    S_sum += S;
+    l1 += fabsf(sm.x[row + LR][col + LR] - sm.y[row + LR][col + LR]);
   }
-  const float sS = block_sum(S, red);
+  const float sS = block_sum(S_sum, sm.red);
   __syncthreads();
-  const float sL = block_sum(l1, red);
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
+  const float sL = block_sum(l1, sm.red);
+  if (t == 0) {
     const size_t b = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
     part[2 * b] = sS;
     part[2 * b + 1] = sL;
   }
 }
 
-__global__ void __launch_bounds__(LT * LT)
+__global__ void __launch_bounds__(LN)
 ssim_grad_kernel(const float *__restrict__ x, const float *__restrict__ y, int H, int Wd,
                  Window W, const float *__restrict__ ABD, float lambda, float inv_n,
                  float *__restrict__ grad, const float *__restrict__ part, int nparts,
                  float *__restrict__ loss) {
-  __shared__ float in[3][LH][LH];
-  __shared__ float hs[3][LH][LT];
-  __shared__ float red[LT * LT / 32];
-  const int c = blockIdx.z;
+  extern __shared__ __align__(16) char loss_smem[];
+  GradSmem &sm = *reinterpret_cast<GradSmem *>(loss_smem);
+  const int c = blockIdx.z, t = threadIdx.x;
   const size_t plane = (size_t)H * Wd;
   const size_t all = (size_t)gridDim.z * plane;
-  const int ox = blockIdx.x * LT - LR, oy = blockIdx.y * LT - LR;
-  for (int i = threadIdx.y * LT + threadIdx.x; i < LH * LH; i += LT * LT) {
-    const int r = i / LH, q = i - r * LH;
-    const int gy = oy + r, gx = ox + q;
-    const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < Wd;
-    const size_t o = c * plane + (size_t)gy * Wd + gx;
-    in[0][r][q] = ok ? ABD[o] : 0.f;
-    in[1][r][q] = ok ? ABD[all + o] : 0.f;
-    in[2][r][q] = ok ? ABD[2 * all + o] : 0.f;
+  const int ox = blockIdx.x * LW, oy = blockIdx.y * LHT;
+#pragma unroll 1
+  for (int q = 0; q < 3; ++q) {
+    load_tile<1>(ABD + q * all + c * plane, nullptr, H, Wd, ox - LR, oy - LR, sm.in, nullptr);
+    __syncthreads();
+#pragma unroll
+    for (int i = t; i < LROWS * (LW / 4); i += LN) {
+      const int r = i >> 3, g = i & 7;
+      float a[16];
+      load_row(sm.in, r, g, a);
+      *reinterpret_cast<float4 *>(&sm.hs[q][r][4 * g]) = blur4(W, a);
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  float b[3];
-  blur_tile<3>(in, hs, W, b);
-  const int px = blockIdx.x * LT + threadIdx.x, py = blockIdx.y * LT + threadIdx.y;
-  if (px < Wd && py < H) {
+  const int col = t & (LW - 1), gv = t / LW;
+  float b[3][LV];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) blur_column(W, sm.hs[q], col, gv, b[q]);
+  const int px = ox + col;
+#pragma unroll
+  for (int j = 0; j < LV; ++j) {
+    const int row = gv * LV + j, py = oy + row;
+    if (row >= LHT || px >= Wd || py >= H) continue;
     const size_t o = c * plane + (size_t)py * Wd + px;
     const float xv = x[o], yv = y[o], d = xv - yv;
     const float sgn = (d > 0.f) ? 1.f : (d < 0.f ? -1.f : 0.f);
-    const float dS = b[0] + 2.f * xv * b[1] + yv * b[2];
+    const float dS = b[0][j] + 2.f * xv * b[1][j] + yv * b[2][j];
     grad[o] = (1.f - lambda) * inv_n * sgn - lambda * inv_n * dS;
   }
   if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && loss) {
     // the partials of all blocks of the moments kernel (launched before)
     float sS = 0.f, sL = 0.f;
-    for (int i = threadIdx.y * LT + threadIdx.x; i < nparts; i += LT * LT) {
+    for (int i = t; i < nparts; i += LN) {
       sS += part[2 * i];
       sL += part[2 * i + 1];
     }
     __syncthreads();
-    sS = block_sum(sS, red);
+    sS = block_sum(sS, sm.red);
     __syncthreads();
-    sL = block_sum(sL, red);
-    if (threadIdx.x == 0 && threadIdx.y == 0)
-      *loss = (1.f - lambda) * sL * inv_n + lambda * (1.f - sS * inv_n);
+    sL = block_sum(sL, sm.red);
+    if (t == 0) *loss = (1.f - lambda) * sL * inv_n + lambda * (1.f - sS * inv_n);
   }
 }
 
@@ -196,7 +282,7 @@ Window gaussian_window() {
 }
 
 size_t nblocks(int C, int H, int W) {
-  return (size_t)C * ((H + LT - 1) / LT) * ((W + LT - 1) / LT);
+  return (size_t)C * ((H + LHT - 1) / LHT) * ((W + LW - 1) / LW);
 }
 
 }  // namespace
@@ -236,11 +322,14 @@ int launch_l1_ssim(const float *x, const float *y, int C, int H, int W, float la
   const Window win = gaussian_window();
   float *ABD = reinterpret_cast<float *>(scratch);
   float *part = reinterpret_cast<float *>(scratch + align_up((size_t)3 * C * H * W * 4, 256));
-  const dim3 grid((W + LT - 1) / LT, (H + LT - 1) / LT, C), block(LT, LT);
+  const dim3 grid((W + LW - 1) / LW, (H + LHT - 1) / LHT, C);
+  const size_t m_smem = sizeof(MomentsSmem), g_smem = sizeof(GradSmem);
+  if (int r = dmgs_host::raise_smem_limit((const void *)ssim_moments_kernel, m_smem)) return r;
+  if (int r = dmgs_host::raise_smem_limit((const void *)ssim_grad_kernel, g_smem)) return r;
   const float inv_n = 1.f / ((float)C * (float)H * (float)W);
   DMGS_TIMED(K_LOSS, s, {
-    dmgs_host::note_launch(), ssim_moments_kernel<<<grid, block, 0, s>>>(x, y, H, W, win, ABD, part);
-    dmgs_host::note_launch(), ssim_grad_kernel<<<grid, block, 0, s>>>(
+    dmgs_host::note_launch(), ssim_moments_kernel<<<grid, LN, m_smem, s>>>(x, y, H, W, win, ABD, part);
+    dmgs_host::note_launch(), ssim_grad_kernel<<<grid, LN, g_smem, s>>>(
         x, y, H, W, win, ABD, lambda, inv_n, grad, part, (int)nblocks(C, H, W), loss);
   });
   DMGS_LAUNCH_CHECK("ssim kernels");
