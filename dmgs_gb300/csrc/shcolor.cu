@@ -13,6 +13,17 @@
 // 12 B.  The adjoint recomputes the basis, writes dL/dsh (zero for the
 // coefficients above the active degree) and, optionally, dL/dxyz through the
 // direction's normalisation.
+//
+// Bound by memory.  Where every coefficient is active (K = (deg + 1)^2) a
+// block moves its Gaussians' rows, one contiguous range, through shared
+// memory with 16-byte accesses of consecutive addresses: a thread reading its
+// own row makes a warp touch 32 rows 12 K bytes apart, each for 16 bytes at a
+// time, and the lines were evicted between the touches (1M Gaussians, degree
+// 3: 165 us for both directions, against 143; floor 64 us).  With K larger
+// than needed the threads read their rows' leading part themselves: the
+// staged form would move all of it.
+#include <initializer_list>
+
 #include "kernels.cuh"
 
 namespace dmgs {
@@ -101,6 +112,118 @@ __device__ __forceinline__ void unit_dir(const float *xyz, const float *campos, 
   d[0] = dx / len;
   d[1] = dy / len;
   d[2] = dz / len;
+}
+
+// ---- staged form: K = (DEG + 1)^2 -----------------------------------------------
+
+constexpr int SHS_THREADS = 128;  // Gaussians per block
+
+// The block's n floats between global memory (16-byte aligned) and rows of R
+// floats at an odd pitch (lanes at the same column of consecutive rows hit
+// different banks).
+template <int R>
+__device__ __forceinline__ void rows_in(const float *__restrict__ g, int n, float *sm) {
+  constexpr int PITCH = R | 1;
+  for (int i = threadIdx.x; i < n / 4; i += SHS_THREADS) {
+    const float4 v = __ldg(reinterpret_cast<const float4 *>(g) + i);
+    const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sm[(4 * i + k) / R * PITCH + (4 * i + k) % R] = e[k];
+  }
+  for (int i = (n & ~3) + threadIdx.x; i < n; i += SHS_THREADS) sm[i / R * PITCH + i % R] = g[i];
+}
+template <int R>
+__device__ __forceinline__ void rows_out(float *__restrict__ g, int n, const float *sm) {
+  constexpr int PITCH = R | 1;
+  for (int i = threadIdx.x; i < n / 4; i += SHS_THREADS) {
+    float e[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) e[k] = sm[(4 * i + k) / R * PITCH + (4 * i + k) % R];
+    reinterpret_cast<float4 *>(g)[i] = make_float4(e[0], e[1], e[2], e[3]);
+  }
+  for (int i = (n & ~3) + threadIdx.x; i < n; i += SHS_THREADS) g[i] = sm[i / R * PITCH + i % R];
+}
+
+template <int DEG>
+__global__ void __launch_bounds__(SHS_THREADS)
+sh_colors_fwd_staged_kernel(int P, const float *__restrict__ sh, const float *__restrict__ xyz,
+                            const float *__restrict__ campos, float *__restrict__ colors) {
+  constexpr int K = (DEG + 1) * (DEG + 1), R = 3 * K;
+  __shared__ float row[SHS_THREADS * (R | 1)];
+  __shared__ float out[SHS_THREADS * 3];
+  const int p0 = blockIdx.x * SHS_THREADS, n = min(SHS_THREADS, P - p0), t = threadIdx.x;
+  rows_in<R>(sh + (size_t)p0 * R, n * R, row);
+  __syncthreads();
+  if (t < n) {
+    float d[3], len;
+    unit_dir(xyz, campos, p0 + t, d, len);
+    float b[16], G[16][3];
+    sh_basis<false>(d[0], d[1], d[2], DEG, b, G);
+    const float *v = row + t * (R | 1);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      float r = 0.f;
+#pragma unroll
+      for (int k = 0; k < K; ++k) r = fmaf(b[k], v[c * K + k], r);
+      out[3 * t + c] = 1.f / (1.f + expf(-r));
+    }
+  }
+  __syncthreads();
+  rows_out<3>(colors + (size_t)p0 * 3, 3 * n, out);
+}
+
+template <int DEG>
+__global__ void __launch_bounds__(SHS_THREADS)
+sh_colors_bwd_staged_kernel(int P, const float *__restrict__ sh, const float *__restrict__ xyz,
+                            const float *__restrict__ campos, const float *__restrict__ dcolors,
+                            float *__restrict__ dsh, float *__restrict__ dxyz) {
+  constexpr int K = (DEG + 1) * (DEG + 1), R = 3 * K;
+  __shared__ float row[SHS_THREADS * (R | 1)];
+  __shared__ float io[SHS_THREADS * 3];
+  const int p0 = blockIdx.x * SHS_THREADS, n = min(SHS_THREADS, P - p0), t = threadIdx.x;
+  rows_in<R>(sh + (size_t)p0 * R, n * R, row);
+  rows_in<3>(dcolors + (size_t)p0 * 3, 3 * n, io);
+  __syncthreads();
+  if (t < n) {
+    float d[3], len;
+    unit_dir(xyz, campos, p0 + t, d, len);
+    float b[16], G[16][3];
+    sh_basis<true>(d[0], d[1], d[2], DEG, b, G);
+    float *v = row + t * (R | 1);
+    float gd[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      float x[K], r = 0.f;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        x[k] = v[c * K + k];
+        r = fmaf(b[k], x[k], r);
+      }
+      const float sg = 1.f / (1.f + expf(-r));
+      const float dr = io[3 * t + c] * sg * (1.f - sg);
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        v[c * K + k] = dr * b[k];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) gd[a] = fmaf(dr * x[k], G[k][a], gd[a]);
+      }
+    }
+    // through dir = D / |D|: dL/dD = (g - dir (dir . g)) / |D|
+    const float dot = gd[0] * d[0] + gd[1] * d[1] + gd[2] * d[2];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) io[3 * t + a] = (gd[a] - d[a] * dot) / len;
+  }
+  __syncthreads();
+  rows_out<R>(dsh + (size_t)p0 * R, n * R, row);
+  if (dxyz) rows_out<3>(dxyz + (size_t)p0 * 3, 3 * n, io);
+}
+
+// The staged form's rule: every coefficient active (see above) and every row
+// array 16-byte aligned (a block's range starts a multiple of 128 rows on).
+bool staged(int deg, int K, std::initializer_list<const void *> arrays) {
+  uintptr_t bits = 0;
+  for (const void *a : arrays) bits |= reinterpret_cast<uintptr_t>(a);
+  return K == (deg + 1) * (deg + 1) && (bits & 15) == 0;
 }
 
 __global__ void __launch_bounds__(SHC_THREADS)
@@ -197,6 +320,20 @@ int dmgs_sh_colors_fwd(int32_t P, int32_t deg, int32_t K, const float *sh, const
   }
   if (P == 0) return DMGS_OK;
   const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (staged(deg, K, {sh, colors})) {
+    const int grid = (P - 1) / SHS_THREADS + 1;
+    DMGS_TIMED(K_SH_COLORS, s, {
+      dmgs_host::note_launch();
+      switch (deg) {
+        case 0: sh_colors_fwd_staged_kernel<0><<<grid, SHS_THREADS, 0, s>>>(P, sh, xyz, campos, colors); break;
+        case 1: sh_colors_fwd_staged_kernel<1><<<grid, SHS_THREADS, 0, s>>>(P, sh, xyz, campos, colors); break;
+        case 2: sh_colors_fwd_staged_kernel<2><<<grid, SHS_THREADS, 0, s>>>(P, sh, xyz, campos, colors); break;
+        default: sh_colors_fwd_staged_kernel<3><<<grid, SHS_THREADS, 0, s>>>(P, sh, xyz, campos, colors); break;
+      }
+    });
+    DMGS_LAUNCH_CHECK("sh_colors_fwd");
+    return DMGS_OK;
+  }
   DMGS_TIMED(K_SH_COLORS, s,
              dmgs_host::note_launch(), sh_colors_fwd_kernel<<<(P + SHC_THREADS - 1) / SHC_THREADS, SHC_THREADS, 0, s>>>(
                  P, deg, K, sh, xyz, campos, colors));
@@ -214,6 +351,20 @@ int dmgs_sh_colors_bwd(int32_t P, int32_t deg, int32_t K, const float *sh, const
   }
   if (P == 0) return DMGS_OK;
   const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (staged(deg, K, {sh, dL_dcolors, dL_dsh, dL_dxyz})) {
+    const int grid = (P - 1) / SHS_THREADS + 1;
+    DMGS_TIMED(K_SH_COLORS, s, {
+      dmgs_host::note_launch();
+      switch (deg) {
+        case 0: sh_colors_bwd_staged_kernel<0><<<grid, SHS_THREADS, 0, s>>>(P, sh, xyz, campos, dL_dcolors, dL_dsh, dL_dxyz); break;
+        case 1: sh_colors_bwd_staged_kernel<1><<<grid, SHS_THREADS, 0, s>>>(P, sh, xyz, campos, dL_dcolors, dL_dsh, dL_dxyz); break;
+        case 2: sh_colors_bwd_staged_kernel<2><<<grid, SHS_THREADS, 0, s>>>(P, sh, xyz, campos, dL_dcolors, dL_dsh, dL_dxyz); break;
+        default: sh_colors_bwd_staged_kernel<3><<<grid, SHS_THREADS, 0, s>>>(P, sh, xyz, campos, dL_dcolors, dL_dsh, dL_dxyz); break;
+      }
+    });
+    DMGS_LAUNCH_CHECK("sh_colors_bwd");
+    return DMGS_OK;
+  }
   DMGS_TIMED(K_SH_COLORS, s,
              dmgs_host::note_launch(), sh_colors_bwd_kernel<<<(P + SHC_THREADS - 1) / SHC_THREADS, SHC_THREADS, 0, s>>>(
                  P, deg, K, sh, xyz, campos, dL_dcolors, dL_dsh, dL_dxyz));
