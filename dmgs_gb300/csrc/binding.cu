@@ -2,9 +2,17 @@
 //
 // Stage-2 form: scene/gaussian_geo_model_mlp_flex.py:258-335 (renew_gaussian)
 // and :370-385 (get_covariance_dyn), with the frame of geo/mesh_utils.py:43-57.
-// The reference evaluates it as ~40 separate torch ops per step; here one
-// thread handles one face (frame, affine triangle-space covariance, the G
-// Gaussian means) and one thread one face in the adjoint.
+// The reference evaluates it as ~40 separate torch ops per step.
+//
+// The kernels are bound by memory, and a thread per face looping over its
+// Gaussians' rows in global memory touched each array G rows apart per lane:
+// every 32-byte sector moved several times (700k faces, G = 6, stage 3: 206
+// us forward and 195 us adjoint, against 82 and 150; floors 39 and 35).
+// Rows now pass through shared memory, a warp's accesses consecutive.
+// A thread per face walks its Gaussians in order, 64 faces a block, on the
+// block's staged rows.  (A thread per Gaussian, with the faces formed by the
+// block's first 128 / G threads: three warps in four waited at the barriers,
+// 90 and 240 us.)
 //
 // Stage-3 form: scene/gaussian_geo_model_finetune.py:396-421 (renew_gaussian)
 // and :446-483 (get_scaling / get_rotation / get_rot_matrix).  The rotation
@@ -12,6 +20,8 @@
 // trace, R00, R11, R22 to divide by), made sign-unique by a non-negative real
 // part, then normalised — the same function the reference obtains from
 // pytorch3d's matrix_to_quaternion followed by F.normalize.
+#include <algorithm>
+
 #include "kernels.cuh"
 
 namespace dmgs {
@@ -104,74 +114,181 @@ __device__ __forceinline__ float bc_at(const DmgsFaceBinding &b, int f, int g, i
   return b.bc_per_gaussian ? b.bc[((size_t)f * b.G + g) * 3 + k] : b.bc[g * 3 + k];
 }
 
-__global__ void bind_fwd_kernel(DmgsFaceBinding b, float *__restrict__ xyz,
-                                float *__restrict__ cov, float *__restrict__ rot,
-                                float *__restrict__ covL) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= b.F) return;
-  const int64_t i0 = b.faces[3 * (size_t)f], i1 = b.faces[3 * (size_t)f + 1],
-                i2 = b.faces[3 * (size_t)f + 2];
-  if (!face_ok(i0, i1, i2, b.V)) return;
-  const f3 v0 = load_v(b.verts, i0), v1 = load_v(b.verts, i1), v2 = load_v(b.verts, i2);
-  const Frame F = face_frame(v0, v1, v2);
-  float L[9];
-  tri_L(F, b.rad_base, b.z_scale, b.adaptive_cov, L);
-  // no scale factor: the real-scene variant's covariance, L unscaled
-  // (scene/gaussian_geo_model_mlp_flex_colmap.py:494-512)
-  const float k = b.scale_factor ? tanhf(b.scale_factor[0]) * b.max_scale : 1.f;
-  const float R[9] = {F.x.x, F.y.x, F.n.x, F.x.y, F.y.y, F.n.y, F.x.z, F.y.z, F.n.z};
-  float Mf[9];
+// ---- the blocks of the four kernels ---------------------------------------------
+
+constexpr int BB = 64;  // threads, and faces per block
+
+// Rows of a block: the faces it takes and the Gaussians of each that
+// its shared memory holds at a time (all of them, or, with one face, a part).
+struct FaceBlocks {
+  int faces, chunk, blocks;
+  size_t smem;
+};
+
+FaceBlocks face_blocks(int F, int G, int words) {
+  FaceBlocks k;
+  const int fit = 22 * 1024 / 4 / words;  // Gaussians whose rows fit (ten blocks per SM)
+  k.faces = std::max(1, std::min(BB, fit / G));
+  k.chunk = std::min(G, fit);
+  k.blocks = (F + k.faces - 1) / k.faces;
+  k.smem = (size_t)k.faces * k.chunk * words * 4 + 5 * 16;  // each array padded to 16 bytes
+  return k;
+}
+
+// The next of the consecutive arrays in a block's shared memory.
+__device__ __forceinline__ float *take(float *&p, int floats) {
+  float *q = p;
+  p += (floats + 3) & ~3;
+  return q;
+}
+
+// n floats of consecutive rows between global and shared memory.
+__device__ __forceinline__ void rows_in(const float *__restrict__ g, int n, float *sm) {
+  if ((reinterpret_cast<uintptr_t>(g) & 15) == 0) {
+    for (int i = threadIdx.x; i < n / 4; i += BB)
+      reinterpret_cast<float4 *>(sm)[i] = __ldg(reinterpret_cast<const float4 *>(g) + i);
+    for (int i = (n & ~3) + threadIdx.x; i < n; i += BB) sm[i] = __ldg(g + i);
+  } else {
+    for (int i = threadIdx.x; i < n; i += BB) sm[i] = __ldg(g + i);
+  }
+}
+__device__ __forceinline__ void rows_out(float *__restrict__ g, int n, const float *sm) {
+  if ((reinterpret_cast<uintptr_t>(g) & 15) == 0) {
+    for (int i = threadIdx.x; i < n / 4; i += BB)
+      reinterpret_cast<float4 *>(g)[i] = reinterpret_cast<const float4 *>(sm)[i];
+    for (int i = (n & ~3) + threadIdx.x; i < n; i += BB) g[i] = sm[i];
+  } else {
+    for (int i = threadIdx.x; i < n; i += BB) g[i] = sm[i];
+  }
+}
+// A face's triangle; false when an index is out of range.
+struct Tri {
+  int64_t i0, i1, i2;
+  f3 v0, v1, v2;
+};
+__device__ __forceinline__ bool load_tri(const int64_t *__restrict__ faces, const float *__restrict__ verts, int V, int f,
+                                         Tri &T) {
+  T.i0 = faces[3 * (size_t)f]; T.i1 = faces[3 * (size_t)f + 1]; T.i2 = faces[3 * (size_t)f + 2];
+  if (!face_ok(T.i0, T.i1, T.i2, V)) return false;
+  T.v0 = load_v(verts, T.i0); T.v1 = load_v(verts, T.i1); T.v2 = load_v(verts, T.i2);
+  return true;
+}
+
+__device__ __forceinline__ void scatter_vertices(float *__restrict__ dverts, const Tri &T, f3 g0, f3 g1, f3 g2) {
+  atomicAdd(dverts + 3 * T.i0, g0.x); atomicAdd(dverts + 3 * T.i0 + 1, g0.y); atomicAdd(dverts + 3 * T.i0 + 2, g0.z);
+  atomicAdd(dverts + 3 * T.i1, g1.x); atomicAdd(dverts + 3 * T.i1 + 1, g1.y); atomicAdd(dverts + 3 * T.i1 + 2, g1.z);
+  atomicAdd(dverts + 3 * T.i2, g2.x); atomicAdd(dverts + 3 * T.i2 + 1, g2.y); atomicAdd(dverts + 3 * T.i2 + 2, g2.z);
+}
+
+// ----------------------------- stage 2 -----------------------------------
+
+__global__ void __launch_bounds__(BB)
+bind_fwd_kernel(DmgsFaceBinding b, FaceBlocks kb, float *__restrict__ xyz, float *__restrict__ cov,
+                float *__restrict__ rot, float *__restrict__ covL) {
+  extern __shared__ __align__(16) float bind_smem[];
+  const int t = threadIdx.x, f0 = blockIdx.x * kb.faces, nf = min(kb.faces, b.F - f0), f = f0 + t;
+  float *p = bind_smem;
+  float *sx = take(p, 3 * kb.faces * kb.chunk), *sc = take(p, 6 * kb.faces * kb.chunk);
+  Tri T;
+  float c[6];
+  bool good = true;
+  if (t < nf) {
+    good = load_tri(b.faces, b.verts, b.V, f, T);
+    if (good) {
+      const Frame F = face_frame(T.v0, T.v1, T.v2);
+      float L[9];
+      tri_L(F, b.rad_base, b.z_scale, b.adaptive_cov, L);
+      // no scale factor: the real-scene variant's covariance, L unscaled
+      // (scene/gaussian_geo_model_mlp_flex_colmap.py:494-512)
+      const float k = b.scale_factor ? tanhf(b.scale_factor[0]) * b.max_scale : 1.f;
+      const float R[9] = {F.x.x, F.y.x, F.n.x, F.x.y, F.y.y, F.n.y, F.x.z, F.y.z, F.n.z};
+      float Mf[9];
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+      for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int j = 0; j < 3; ++j)
-      Mf[i * 3 + j] = k * (R[i * 3] * L[j] + R[i * 3 + 1] * L[3 + j] + R[i * 3 + 2] * L[6 + j]);
-  auto sig = [&](int i, int j) {
-    return Mf[i * 3] * Mf[j * 3] + Mf[i * 3 + 1] * Mf[j * 3 + 1] + Mf[i * 3 + 2] * Mf[j * 3 + 2];
-  };
-  const float c[6] = {sig(0, 0), sig(0, 1), sig(0, 2), sig(1, 1), sig(1, 2), sig(2, 2)};
-  if (rot)
-    for (int i = 0; i < 9; ++i) rot[(size_t)f * 9 + i] = R[i];
-  if (covL)
-    for (int i = 0; i < 9; ++i) covL[(size_t)f * 9 + i] = L[i];
-  for (int g = 0; g < b.G; ++g) {
-    const float w0 = bc_at(b, f, g, 0), w1 = bc_at(b, f, g, 1), w2 = bc_at(b, f, g, 2);
-    const size_t o = (size_t)f * b.G + g;
-    if (xyz) {
-      xyz[3 * o] = w0 * v0.x + w1 * v1.x + w2 * v2.x;
-      xyz[3 * o + 1] = w0 * v0.y + w1 * v1.y + w2 * v2.y;
-      xyz[3 * o + 2] = w0 * v0.z + w1 * v1.z + w2 * v2.z;
+        for (int j = 0; j < 3; ++j)
+          Mf[i * 3 + j] = k * (R[i * 3] * L[j] + R[i * 3 + 1] * L[3 + j] + R[i * 3 + 2] * L[6 + j]);
+      auto sig = [&](int i, int j) {
+        return Mf[i * 3] * Mf[j * 3] + Mf[i * 3 + 1] * Mf[j * 3 + 1] + Mf[i * 3 + 2] * Mf[j * 3 + 2];
+      };
+      c[0] = sig(0, 0); c[1] = sig(0, 1); c[2] = sig(0, 2); c[3] = sig(1, 1); c[4] = sig(1, 2); c[5] = sig(2, 2);
+      if (rot)
+        for (int i = 0; i < 9; ++i) rot[(size_t)f * 9 + i] = R[i];
+      if (covL)
+        for (int i = 0; i < 9; ++i) covL[(size_t)f * 9 + i] = L[i];
     }
-    if (cov)
-      for (int i = 0; i < 6; ++i) cov[6 * o + i] = c[i];
+  }
+  const bool all_good = __syncthreads_and(good);
+  for (int gs = 0; gs < b.G; gs += kb.chunk) {  // once, unless one face's rows do not fit
+    const int gn = min(kb.chunk, b.G - gs), m = nf * gn;
+    const size_t o0 = (size_t)f0 * b.G + gs;
+    if (good && t < nf) {
+      for (int g = 0; g < gn; ++g) {
+        const int q = t * gn + g;
+        const float w0 = bc_at(b, f, gs + g, 0), w1 = bc_at(b, f, gs + g, 1), w2 = bc_at(b, f, gs + g, 2);
+        const float x = w0 * T.v0.x + w1 * T.v1.x + w2 * T.v2.x, y = w0 * T.v0.y + w1 * T.v1.y + w2 * T.v2.y;
+        const float z = w0 * T.v0.z + w1 * T.v1.z + w2 * T.v2.z;
+        if (all_good) {
+          sx[3 * q] = x; sx[3 * q + 1] = y; sx[3 * q + 2] = z;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) reinterpret_cast<float2 *>(sc)[3 * q + i] = make_float2(c[2 * i], c[2 * i + 1]);
+        } else {  // a skipped face's outputs stay as the caller left them
+          const size_t o = o0 + q;
+          if (xyz) { xyz[3 * o] = x; xyz[3 * o + 1] = y; xyz[3 * o + 2] = z; }
+          if (cov)
+#pragma unroll
+            for (int i = 0; i < 6; ++i) cov[6 * o + i] = c[i];
+        }
+      }
+    }
+    __syncthreads();
+    if (all_good) {
+      if (xyz) rows_out(xyz + 3 * o0, 3 * m, sx);
+      if (cov) rows_out(cov + 6 * o0, 6 * m, sc);
+      __syncthreads();
+    }
   }
 }
 
-__global__ void bind_bwd_kernel(DmgsFaceBinding b, const float *__restrict__ dxyz,
-                                const float *__restrict__ dcov, float *__restrict__ dverts,
-                                float *__restrict__ dsf) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  float dk_local = 0.f;
-  if (f < b.F) {
-    const int64_t i0 = b.faces[3 * (size_t)f], i1 = b.faces[3 * (size_t)f + 1],
-                  i2 = b.faces[3 * (size_t)f + 2];
-    if (face_ok(i0, i1, i2, b.V)) {
-    const f3 v0 = load_v(b.verts, i0), v1 = load_v(b.verts, i1), v2 = load_v(b.verts, i2);
-    f3 g0 = mk(0.f, 0.f, 0.f), g1 = g0, g2 = g0;
-    float gc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int g = 0; g < b.G; ++g) {
-      const size_t o = (size_t)f * b.G + g;
-      if (dxyz) {
-        const f3 d = mk(dxyz[3 * o], dxyz[3 * o + 1], dxyz[3 * o + 2]);
-        g0 = g0 + bc_at(b, f, g, 0) * d;
-        g1 = g1 + bc_at(b, f, g, 1) * d;
-        g2 = g2 + bc_at(b, f, g, 2) * d;
+__global__ void __launch_bounds__(BB)
+bind_bwd_kernel(DmgsFaceBinding b, FaceBlocks kb, const float *__restrict__ dxyz,
+                const float *__restrict__ dcov, float *__restrict__ dverts,
+                float *__restrict__ dsf) {
+  extern __shared__ __align__(16) float bind_smem[];
+  const int t = threadIdx.x, f0 = blockIdx.x * kb.faces, nf = min(kb.faces, b.F - f0), f = f0 + t;
+  float *p = bind_smem;
+  float *sx = take(p, 3 * kb.faces * kb.chunk), *sc = take(p, 6 * kb.faces * kb.chunk);
+  Tri T;
+  bool good = false;
+  f3 g0 = mk(0.f, 0.f, 0.f), g1 = g0, g2 = g0;
+  float gc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int gs = 0; gs < b.G; gs += kb.chunk) {  // once, unless one face's rows do not fit
+    const int gn = min(kb.chunk, b.G - gs), m = nf * gn;
+    const size_t o = (size_t)f0 * b.G + gs;
+    if (dxyz) rows_in(dxyz + 3 * o, 3 * m, sx);
+    if (dcov) rows_in(dcov + 6 * o, 6 * m, sc);
+    if (gs == 0 && t < nf) good = load_tri(b.faces, b.verts, b.V, f, T);
+    __syncthreads();
+    if (good) {
+      for (int g = 0; g < gn; ++g) {
+        const int q = t * gn + g;
+        if (dxyz) {
+          const f3 d = mk(sx[3 * q], sx[3 * q + 1], sx[3 * q + 2]);
+          g0 = g0 + bc_at(b, f, gs + g, 0) * d;
+          g1 = g1 + bc_at(b, f, gs + g, 1) * d;
+          g2 = g2 + bc_at(b, f, gs + g, 2) * d;
+        }
+        if (dcov)
+#pragma unroll
+          for (int i = 0; i < 6; ++i) gc[i] += sc[6 * q + i];
       }
-      if (dcov)
-        for (int i = 0; i < 6; ++i) gc[i] += dcov[6 * o + i];
     }
+    __syncthreads();
+  }
+  float dk_local = 0.f;
+  if (good) {
     if (dcov) {
-      const Frame F = face_frame(v0, v1, v2);
+      const Frame F = face_frame(T.v0, T.v1, T.v2);
       float L[9];
       tri_L(F, b.rad_base, b.z_scale, b.adaptive_cov, L);
       const float th = b.scale_factor ? tanhf(b.scale_factor[0]) : 0.f;
@@ -211,10 +328,7 @@ __global__ void bind_bwd_kernel(DmgsFaceBinding b, const float *__restrict__ dxy
       face_frame_adj(F, gxv, gyv, gnv, h0, h1, h2);
       g0 = g0 + h0; g1 = g1 + h1; g2 = g2 + h2;
     }
-    atomicAdd(dverts + 3 * i0, g0.x); atomicAdd(dverts + 3 * i0 + 1, g0.y); atomicAdd(dverts + 3 * i0 + 2, g0.z);
-    atomicAdd(dverts + 3 * i1, g1.x); atomicAdd(dverts + 3 * i1 + 1, g1.y); atomicAdd(dverts + 3 * i1 + 2, g1.z);
-    atomicAdd(dverts + 3 * i2, g2.x); atomicAdd(dverts + 3 * i2 + 1, g2.y); atomicAdd(dverts + 3 * i2 + 2, g2.z);
-    }
+    scatter_vertices(dverts, T, g0, g1, g2);
   }
   if (dsf) {
     const float s = warp_sum(dk_local);
@@ -224,204 +338,278 @@ __global__ void bind_bwd_kernel(DmgsFaceBinding b, const float *__restrict__ dxy
 
 // ----------------------------- stage 3 -----------------------------------
 
+// 1 / sqrt(x) for positive normal x: the hardware's estimate and one
+// Newton-Raphson step (within an ulp; a root and a division each cost some
+// thirty instructions with their special cases, and a Gaussian needs three).
+__device__ __forceinline__ float inv_sqrt(float x) {
+  const float y = rsqrtf(x);
+  return fmaf(fmaf(-x * y, y, 1.f), 0.5f * y, y);
+}
+
+// 1 / max(sqrt(x), NRM_EPS) for x >= 0 (the guard of torch's normalize).
+__device__ __forceinline__ float inv_norm(float x) {
+  return x > NRM_EPS * NRM_EPS ? inv_sqrt(x) : 1.f / NRM_EPS;
+}
+
 // Unit quaternion (w, x, y, z), w >= 0, of a rotation matrix (row-major),
-// Shepperd's method, plus the unnormalised value and branch for the adjoint.
-struct QuatOut { float q[4]; float raw[4]; int branch; };
+// Shepperd's method: with big the largest component, half the root of its
+// arg, the others are K[big][c] 0.25 / max(big, 0.05), where K[0][c] are the
+// differences and the rest the sums of mirrored entries.  Every choice is a
+// select (a warp's lanes differ in it); the reciprocals are kept for the
+// adjoint.
+struct QuatOut { float q[4]; int br; float sgn, big, d, inv; };
+
+// Component c of the K row of the largest component br (0 for c == br).
+__device__ __forceinline__ float quat_k(const float *R, int br, int c) {
+  const float k01 = R[7] - R[5], k02 = R[2] - R[6], k03 = R[3] - R[1];
+  const float k12 = R[1] + R[3], k13 = R[2] + R[6], k23 = R[5] + R[7];
+  if (c == 0) return br == 1 ? k01 : (br == 2 ? k02 : (br == 3 ? k03 : 0.f));
+  if (c == 1) return br == 0 ? k01 : (br == 2 ? k12 : (br == 3 ? k13 : 0.f));
+  if (c == 2) return br == 0 ? k02 : (br == 1 ? k12 : (br == 3 ? k23 : 0.f));
+  return br == 0 ? k03 : (br == 1 ? k13 : (br == 2 ? k23 : 0.f));
+}
 
 __device__ __forceinline__ QuatOut mat_to_quat(const float *R) {
   QuatOut o;
   const float tr = R[0] + R[4] + R[8];
-  float w, x, y, z;
-  int br;
-  if (tr >= R[0] && tr >= R[4] && tr >= R[8]) {
-    br = 0;
-    w = 0.5f * sqrtf(fmaxf(1.f + tr, 0.f));
-    const float d = 0.25f / fmaxf(w, 0.05f);
-    x = (R[7] - R[5]) * d; y = (R[2] - R[6]) * d; z = (R[3] - R[1]) * d;
-  } else if (R[0] >= R[4] && R[0] >= R[8]) {
-    br = 1;
-    x = 0.5f * sqrtf(fmaxf(1.f + R[0] - R[4] - R[8], 0.f));
-    const float d = 0.25f / fmaxf(x, 0.05f);
-    w = (R[7] - R[5]) * d; y = (R[1] + R[3]) * d; z = (R[2] + R[6]) * d;
-  } else if (R[4] >= R[8]) {
-    br = 2;
-    y = 0.5f * sqrtf(fmaxf(1.f - R[0] + R[4] - R[8], 0.f));
-    const float d = 0.25f / fmaxf(y, 0.05f);
-    w = (R[2] - R[6]) * d; x = (R[1] + R[3]) * d; z = (R[5] + R[7]) * d;
-  } else {
-    br = 3;
-    z = 0.5f * sqrtf(fmaxf(1.f - R[0] - R[4] + R[8], 0.f));
-    const float d = 0.25f / fmaxf(z, 0.05f);
-    w = (R[3] - R[1]) * d; x = (R[2] + R[6]) * d; y = (R[5] + R[7]) * d;
-  }
-  const float sgn = w < 0.f ? -1.f : 1.f;
-  o.raw[0] = sgn * w; o.raw[1] = sgn * x; o.raw[2] = sgn * y; o.raw[3] = sgn * z;
-  const float n = sqrtf(o.raw[0] * o.raw[0] + o.raw[1] * o.raw[1] + o.raw[2] * o.raw[2] + o.raw[3] * o.raw[3]);
-  const float inv = 1.f / fmaxf(n, NRM_EPS);
-  for (int i = 0; i < 4; ++i) o.q[i] = o.raw[i] * inv;
-  o.branch = br | (sgn < 0.f ? 4 : 0);
+  o.br = (tr >= R[0] && tr >= R[4] && tr >= R[8]) ? 0 : (R[0] >= R[4] && R[0] >= R[8]) ? 1 : (R[4] >= R[8]) ? 2 : 3;
+  const float s0 = o.br < 2 ? R[0] : -R[0], s4 = (o.br & 1) ? -R[4] : R[4], s8 = (o.br == 0 || o.br == 3) ? R[8] : -R[8];
+  const float arg = fmaxf(o.br == 0 ? 1.f + tr : 1.f + s0 + s4 + s8, 0.f);
+  const float ia = inv_sqrt(fmaxf(arg, 1e-30f));
+  o.big = 0.5f * (arg * ia);
+  o.d = o.big < 0.05f ? 0.25f / 0.05f : 0.5f * ia;  // 0.25 / max(big, 0.05)
+  float raw[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) raw[c] = c == o.br ? o.big : quat_k(R, o.br, c) * o.d;
+  o.sgn = raw[0] < 0.f ? -1.f : 1.f;
+  o.inv = inv_norm(raw[0] * raw[0] + raw[1] * raw[1] + raw[2] * raw[2] + raw[3] * raw[3]);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) o.q[c] = o.sgn * raw[c] * o.inv;
   return o;
 }
 
 // Adjoint of mat_to_quat: dq (w.r.t. the normalised output) -> dR.
 __device__ __forceinline__ void mat_to_quat_adj(const float *R, const QuatOut &o, const float *dq,
                                                 float *dR) {
-  const float n = sqrtf(o.raw[0] * o.raw[0] + o.raw[1] * o.raw[1] + o.raw[2] * o.raw[2] + o.raw[3] * o.raw[3]);
   float dr[4];
   const float qd = o.q[0] * dq[0] + o.q[1] * dq[1] + o.q[2] * dq[2] + o.q[3] * dq[3];
-  for (int i = 0; i < 4; ++i) dr[i] = n > NRM_EPS ? (dq[i] - o.q[i] * qd) / n : dq[i] / NRM_EPS;
-  const float sgn = (o.branch & 4) ? -1.f : 1.f;
-  for (int i = 0; i < 4; ++i) dr[i] *= sgn;  // gradient w.r.t. the pre-sign (w, x, y, z)
-  for (int i = 0; i < 9; ++i) dR[i] = 0.f;
-  const int br = o.branch & 3;
-  // big = 0.5 sqrt(arg); the other three = (R[a] +/- R[b]) * 0.25 / max(big, 0.05)
-  float big;
-  int bi;
-  float arg;
-  float sgnd[9];
-  for (int i = 0; i < 9; ++i) sgnd[i] = 0.f;
-  if (br == 0) { arg = 1.f + R[0] + R[4] + R[8]; sgnd[0] = sgnd[4] = sgnd[8] = 1.f; bi = 0; }
-  else if (br == 1) { arg = 1.f + R[0] - R[4] - R[8]; sgnd[0] = 1.f; sgnd[4] = sgnd[8] = -1.f; bi = 1; }
-  else if (br == 2) { arg = 1.f - R[0] + R[4] - R[8]; sgnd[4] = 1.f; sgnd[0] = sgnd[8] = -1.f; bi = 2; }
-  else { arg = 1.f - R[0] - R[4] + R[8]; sgnd[8] = 1.f; sgnd[0] = sgnd[4] = -1.f; bi = 3; }
-  big = 0.5f * sqrtf(fmaxf(arg, 0.f));
-  const bool clampd = big < 0.05f;
-  const float den = fmaxf(big, 0.05f);
-  const float d = 0.25f / den;
-  // the three linear components: value_c = lin_c * d, lin_c = R[a] +/- R[b]
-  int ia[3], ib[3], oc[3];
-  float sb[3];
-  if (br == 0) { oc[0] = 1; ia[0] = 7; ib[0] = 5; sb[0] = -1.f; oc[1] = 2; ia[1] = 2; ib[1] = 6; sb[1] = -1.f; oc[2] = 3; ia[2] = 3; ib[2] = 1; sb[2] = -1.f; }
-  else if (br == 1) { oc[0] = 0; ia[0] = 7; ib[0] = 5; sb[0] = -1.f; oc[1] = 2; ia[1] = 1; ib[1] = 3; sb[1] = 1.f; oc[2] = 3; ia[2] = 2; ib[2] = 6; sb[2] = 1.f; }
-  else if (br == 2) { oc[0] = 0; ia[0] = 2; ib[0] = 6; sb[0] = -1.f; oc[1] = 1; ia[1] = 1; ib[1] = 3; sb[1] = 1.f; oc[2] = 3; ia[2] = 5; ib[2] = 7; sb[2] = 1.f; }
-  else { oc[0] = 0; ia[0] = 3; ib[0] = 1; sb[0] = -1.f; oc[1] = 1; ia[1] = 2; ib[1] = 6; sb[1] = 1.f; oc[2] = 2; ia[2] = 5; ib[2] = 7; sb[2] = 1.f; }
-  float dd = 0.f;  // gradient w.r.t. d
-  for (int c = 0; c < 3; ++c) {
-    const float lin = R[ia[c]] + sb[c] * R[ib[c]];
-    dR[ia[c]] += dr[oc[c]] * d;
-    dR[ib[c]] += dr[oc[c]] * d * sb[c];
-    dd += dr[oc[c]] * lin;
+#pragma unroll
+  for (int c = 0; c < 4; ++c)  // w.r.t. the pre-sign (w, x, y, z)
+    dr[c] = o.sgn * ((o.inv < 1.f / NRM_EPS ? dq[c] - o.q[c] * qd : dq[c]) * o.inv);
+  float dd = 0.f, dk[4], dbig = 0.f;  // gradients w.r.t. d and the K row
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const bool own = c == o.br;
+    dd += own ? 0.f : dr[c] * quat_k(R, o.br, c);
+    dk[c] = own ? 0.f : dr[c] * o.d;
+    dbig = own ? dr[c] : dbig;
   }
-  float dbig = dr[bi];
-  if (!clampd) dbig += dd * (-0.25f / (den * den));
-  // big = 0.5 sqrt(arg)  ->  dbig/darg = 0.25 / sqrt(arg) = 0.125 / big
-  if (big > 0.f) {
-    const float darg = dbig * 0.125f / big;
-    for (int i = 0; i < 9; ++i) dR[i] += darg * sgnd[i];
+  // d = 0.25 / big -> -0.25 / big^2 = -4 d^2; big = 0.5 sqrt(arg) -> 0.125 / big
+  float darg;
+  if (!(o.big < 0.05f)) {
+    dbig += dd * (-4.f * o.d * o.d);
+    darg = dbig * (0.5f * o.d);
+  } else {  // d is clamped
+    darg = o.big > 0.f ? dbig * 0.125f / o.big : 0.f;
   }
+  const float e01 = o.br == 0 ? dk[1] : (o.br == 1 ? dk[0] : 0.f), e02 = o.br == 0 ? dk[2] : (o.br == 2 ? dk[0] : 0.f);
+  const float e03 = o.br == 0 ? dk[3] : (o.br == 3 ? dk[0] : 0.f), e12 = o.br == 1 ? dk[2] : (o.br == 2 ? dk[1] : 0.f);
+  const float e13 = o.br == 1 ? dk[3] : (o.br == 3 ? dk[1] : 0.f), e23 = o.br == 2 ? dk[3] : (o.br == 3 ? dk[2] : 0.f);
+  dR[0] = o.br < 2 ? darg : -darg;
+  dR[4] = (o.br & 1) ? -darg : darg;
+  dR[8] = (o.br == 0 || o.br == 3) ? darg : -darg;
+  dR[7] = e01 + e23; dR[5] = e23 - e01;
+  dR[2] = e02 + e13; dR[6] = e13 - e02;
+  dR[3] = e03 + e12; dR[1] = e12 - e03;
 }
 
-__global__ void bind3_fwd_kernel(DmgsFaceBinding3 b, float *__restrict__ xyz,
-                                 float *__restrict__ scales, float *__restrict__ rots) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= b.F) return;
-  const int64_t i0 = b.faces[3 * (size_t)f], i1 = b.faces[3 * (size_t)f + 1],
-                i2 = b.faces[3 * (size_t)f + 2];
-  if (!face_ok(i0, i1, i2, b.V)) return;
-  const f3 v0 = load_v(b.verts, i0), v1 = load_v(b.verts, i1), v2 = load_v(b.verts, i2);
-  const Frame F = face_frame(v0, v1, v2);
-  const float Rw[9] = {F.x.x, F.y.x, F.n.x, F.x.y, F.y.y, F.n.y, F.x.z, F.y.z, F.n.z};
-  for (int g = 0; g < b.G; ++g) {
-    const size_t o = (size_t)f * b.G + g;
-    const float w0 = b.bc[g * 3], w1 = b.bc[g * 3 + 1], w2 = b.bc[g * 3 + 2];
-    if (xyz) {
-      xyz[3 * o] = w0 * v0.x + w1 * v1.x + w2 * v2.x;
-      xyz[3 * o + 1] = w0 * v0.y + w1 * v1.y + w2 * v2.y;
-      xyz[3 * o + 2] = w0 * v0.z + w1 * v1.z + w2 * v2.z;
-    }
-    if (scales) {
-      scales[3 * o] = expf(b.scaling2d[2 * o]);
-      scales[3 * o + 1] = expf(b.scaling2d[2 * o + 1]);
-      scales[3 * o + 2] = b.thin_z;
-    }
-    if (rots) {
-      const float ra = b.rotation2d[2 * o], rb = b.rotation2d[2 * o + 1];
-      const float cn = 1.f / fmaxf(sqrtf(ra * ra + rb * rb), NRM_EPS);
-      const float a = ra * cn, s = rb * cn;
-      // R = Rw * [[a,-s,0],[s,a,0],[0,0,1]]
-      float R[9];
-      for (int i = 0; i < 3; ++i) {
-        R[i * 3 + 0] = Rw[i * 3] * a + Rw[i * 3 + 1] * s;
-        R[i * 3 + 1] = -Rw[i * 3] * s + Rw[i * 3 + 1] * a;
-        R[i * 3 + 2] = Rw[i * 3 + 2];
+__global__ void __launch_bounds__(BB, 10)
+bind3_fwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, float *__restrict__ xyz,
+                 float *__restrict__ scales, float *__restrict__ rots) {
+  extern __shared__ __align__(16) float bind_smem[];
+  const int t = threadIdx.x, f0 = blockIdx.x * kb.faces, nf = min(kb.faces, b.F - f0), cap = kb.faces * kb.chunk;
+  float *p = bind_smem;
+  float *sq = take(p, 4 * cap), *sx = take(p, 3 * cap), *ss = take(p, 3 * cap), *s2 = take(p, 2 * cap), *r2 = take(p, 2 * cap);
+  Tri T;
+  float Rw[9];
+  bool good = true;
+  for (int gs = 0; gs < b.G; gs += kb.chunk) {  // once, unless one face's rows do not fit
+    const int gn = min(kb.chunk, b.G - gs), m = nf * gn;
+    const size_t o0 = (size_t)f0 * b.G + gs;
+    if (scales) rows_in(b.scaling2d + 2 * o0, 2 * m, s2);
+    if (rots) rows_in(b.rotation2d + 2 * o0, 2 * m, r2);
+    if (gs == 0 && t < nf) {
+      good = load_tri(b.faces, b.verts, b.V, f0 + t, T);
+      if (good) {
+        const Frame F = face_frame(T.v0, T.v1, T.v2);
+        const float R[9] = {F.x.x, F.y.x, F.n.x, F.x.y, F.y.y, F.n.y, F.x.z, F.y.z, F.n.z};
+#pragma unroll
+        for (int i = 0; i < 9; ++i) Rw[i] = R[i];
       }
-      const QuatOut q = mat_to_quat(R);
-      for (int i = 0; i < 4; ++i) rots[4 * o + i] = q.q[i];
+    }
+    const bool all_good = __syncthreads_and(good);
+    if (good && t < nf) {
+      for (int g = 0; g < gn; ++g) {
+        const int q = t * gn + g;
+        const float *w = b.bc + 3 * (gs + g);
+        const float w0 = w[0], w1 = w[1], w2 = w[2];
+        const float x = w0 * T.v0.x + w1 * T.v1.x + w2 * T.v2.x, y = w0 * T.v0.y + w1 * T.v1.y + w2 * T.v2.y;
+        const float z = w0 * T.v0.z + w1 * T.v1.z + w2 * T.v2.z;
+        float e0 = 0.f, e1 = 0.f;
+        if (scales) {
+          e0 = expf(s2[2 * q]);
+          e1 = expf(s2[2 * q + 1]);
+        }
+        float4 quat = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (rots) {
+          const float ra = r2[2 * q], rb = r2[2 * q + 1];
+          const float cn = inv_norm(ra * ra + rb * rb);
+          const float a = ra * cn, s = rb * cn;
+          // R = Rw * [[a,-s,0],[s,a,0],[0,0,1]]
+          float R[9];
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            R[i * 3 + 0] = Rw[i * 3] * a + Rw[i * 3 + 1] * s;
+            R[i * 3 + 1] = -Rw[i * 3] * s + Rw[i * 3 + 1] * a;
+            R[i * 3 + 2] = Rw[i * 3 + 2];
+          }
+          const QuatOut o = mat_to_quat(R);
+          quat = make_float4(o.q[0], o.q[1], o.q[2], o.q[3]);
+        }
+        if (all_good) {
+          sx[3 * q] = x; sx[3 * q + 1] = y; sx[3 * q + 2] = z;
+          ss[3 * q] = e0; ss[3 * q + 1] = e1; ss[3 * q + 2] = b.thin_z;
+          reinterpret_cast<float4 *>(sq)[q] = quat;
+        } else {  // a skipped face's outputs stay as the caller left them
+          const size_t o = o0 + q;
+          if (xyz) { xyz[3 * o] = x; xyz[3 * o + 1] = y; xyz[3 * o + 2] = z; }
+          if (scales) { scales[3 * o] = e0; scales[3 * o + 1] = e1; scales[3 * o + 2] = b.thin_z; }
+          if (rots) { rots[4 * o] = quat.x; rots[4 * o + 1] = quat.y; rots[4 * o + 2] = quat.z; rots[4 * o + 3] = quat.w; }
+        }
+      }
+    }
+    __syncthreads();
+    if (all_good) {
+      if (xyz) rows_out(xyz + 3 * o0, 3 * m, sx);
+      if (scales) rows_out(scales + 3 * o0, 3 * m, ss);
+      if (rots) rows_out(rots + 4 * o0, 4 * m, sq);
+      __syncthreads();
     }
   }
 }
 
-__global__ void bind3_bwd_kernel(DmgsFaceBinding3 b, const float *__restrict__ dxyz,
-                                 const float *__restrict__ dscales,
-                                 const float *__restrict__ drots, float *__restrict__ dverts,
-                                 float *__restrict__ dscaling, float *__restrict__ drot2d) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= b.F) return;
-  const int64_t i0 = b.faces[3 * (size_t)f], i1 = b.faces[3 * (size_t)f + 1],
-                i2 = b.faces[3 * (size_t)f + 2];
-  if (!face_ok(i0, i1, i2, b.V)) return;
-  const f3 v0 = load_v(b.verts, i0), v1 = load_v(b.verts, i1), v2 = load_v(b.verts, i2);
-  const Frame F = face_frame(v0, v1, v2);
-  const float Rw[9] = {F.x.x, F.y.x, F.n.x, F.x.y, F.y.y, F.n.y, F.x.z, F.y.z, F.n.z};
+__global__ void __launch_bounds__(BB, 10)
+bind3_bwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, const float *__restrict__ dxyz,
+                 const float *__restrict__ dscales, const float *__restrict__ drots,
+                 float *__restrict__ dverts, float *__restrict__ dscaling, float *__restrict__ drot2d) {
+  extern __shared__ __align__(16) float bind_smem[];
+  const int t = threadIdx.x, f0 = blockIdx.x * kb.faces, nf = min(kb.faces, b.F - f0), cap = kb.faces * kb.chunk;
+  float *p = bind_smem;
+  float *sq = take(p, 4 * cap), *sx = take(p, 3 * cap), *ss = take(p, 3 * cap), *s2 = take(p, 2 * cap), *r2 = take(p, 2 * cap);
+  Tri T;
+  bool good = true;
+  float Rw[9];
   f3 g0 = mk(0.f, 0.f, 0.f), g1 = g0, g2 = g0;
   float dRw[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int g = 0; g < b.G; ++g) {
-    const size_t o = (size_t)f * b.G + g;
-    if (dxyz) {
-      const f3 d = mk(dxyz[3 * o], dxyz[3 * o + 1], dxyz[3 * o + 2]);
-      g0 = g0 + b.bc[g * 3] * d;
-      g1 = g1 + b.bc[g * 3 + 1] * d;
-      g2 = g2 + b.bc[g * 3 + 2] * d;
+  for (int gs = 0; gs < b.G; gs += kb.chunk) {  // once, unless one face's rows do not fit
+    const int gn = min(kb.chunk, b.G - gs), m = nf * gn;
+    const size_t o0 = (size_t)f0 * b.G + gs;
+    if (dxyz) rows_in(dxyz + 3 * o0, 3 * m, sx);
+    if (dscales && dscaling) {
+      rows_in(dscales + 3 * o0, 3 * m, ss);
+      rows_in(b.scaling2d + 2 * o0, 2 * m, s2);
     }
-    if (dscaling) {
-      dscaling[2 * o] = dscales ? dscales[3 * o] * expf(b.scaling2d[2 * o]) : 0.f;
-      dscaling[2 * o + 1] = dscales ? dscales[3 * o + 1] * expf(b.scaling2d[2 * o + 1]) : 0.f;
-    }
-    float dra = 0.f, drb = 0.f;
     if (drots) {
-      const float ra = b.rotation2d[2 * o], rb = b.rotation2d[2 * o + 1];
-      const float clen = sqrtf(ra * ra + rb * rb);
-      const float cn = 1.f / fmaxf(clen, NRM_EPS);
-      const float a = ra * cn, s = rb * cn;
-      float R[9];
-      for (int i = 0; i < 3; ++i) {
-        R[i * 3 + 0] = Rw[i * 3] * a + Rw[i * 3 + 1] * s;
-        R[i * 3 + 1] = -Rw[i * 3] * s + Rw[i * 3 + 1] * a;
-        R[i * 3 + 2] = Rw[i * 3 + 2];
-      }
-      const QuatOut q = mat_to_quat(R);
-      const float dq[4] = {drots[4 * o], drots[4 * o + 1], drots[4 * o + 2], drots[4 * o + 3]};
-      float dR[9];
-      mat_to_quat_adj(R, q, dq, dR);
-      float da = 0.f, ds = 0.f;
-      for (int i = 0; i < 3; ++i) {
-        dRw[i * 3] += dR[i * 3] * a - dR[i * 3 + 1] * s;
-        dRw[i * 3 + 1] += dR[i * 3] * s + dR[i * 3 + 1] * a;
-        dRw[i * 3 + 2] += dR[i * 3 + 2];
-        da += dR[i * 3] * Rw[i * 3] + dR[i * 3 + 1] * Rw[i * 3 + 1];
-        ds += dR[i * 3] * Rw[i * 3 + 1] - dR[i * 3 + 1] * Rw[i * 3];
-      }
-      // (a, s) = unit(ra, rb)
-      if (clen > NRM_EPS) {
-        const float dot_ = a * da + s * ds;
-        dra = (da - a * dot_) / clen;
-        drb = (ds - s * dot_) / clen;
-      } else {
-        dra = da / NRM_EPS;
-        drb = ds / NRM_EPS;
+      rows_in(drots + 4 * o0, 4 * m, sq);
+      rows_in(b.rotation2d + 2 * o0, 2 * m, r2);
+    }
+    if (gs == 0 && t < nf) {
+      good = load_tri(b.faces, b.verts, b.V, f0 + t, T);
+      if (good) {
+        const Frame F = face_frame(T.v0, T.v1, T.v2);
+        const float R[9] = {F.x.x, F.y.x, F.n.x, F.x.y, F.y.y, F.n.y, F.x.z, F.y.z, F.n.z};
+#pragma unroll
+        for (int i = 0; i < 9; ++i) Rw[i] = R[i];
       }
     }
-    if (drot2d) { drot2d[2 * o] = dra; drot2d[2 * o + 1] = drb; }
+    const bool all_good = __syncthreads_and(good);
+    if (good && t < nf) {
+      for (int g = 0; g < gn; ++g) {
+        const int q = t * gn + g;
+        if (dxyz) {
+          const float *w = b.bc + 3 * (gs + g);
+          const f3 d = mk(sx[3 * q], sx[3 * q + 1], sx[3 * q + 2]);
+          g0 = g0 + w[0] * d;
+          g1 = g1 + w[1] * d;
+          g2 = g2 + w[2] * d;
+        }
+        float ds0 = 0.f, ds1 = 0.f, dra = 0.f, drb = 0.f;
+        if (dscales && dscaling) {
+          ds0 = ss[3 * q] * expf(s2[2 * q]);
+          ds1 = ss[3 * q + 1] * expf(s2[2 * q + 1]);
+        }
+        if (drots) {
+          const float ra = r2[2 * q], rb = r2[2 * q + 1];
+          const float cn = inv_norm(ra * ra + rb * rb);
+          const float a = ra * cn, s = rb * cn;
+          float R[9];
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            R[i * 3 + 0] = Rw[i * 3] * a + Rw[i * 3 + 1] * s;
+            R[i * 3 + 1] = -Rw[i * 3] * s + Rw[i * 3 + 1] * a;
+            R[i * 3 + 2] = Rw[i * 3 + 2];
+          }
+          const QuatOut qq = mat_to_quat(R);
+          const float4 v = reinterpret_cast<const float4 *>(sq)[q];
+          const float dq[4] = {v.x, v.y, v.z, v.w};
+          float dR[9];
+          mat_to_quat_adj(R, qq, dq, dR);
+          float da = 0.f, ds = 0.f;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            dRw[i * 3] += dR[i * 3] * a - dR[i * 3 + 1] * s;
+            dRw[i * 3 + 1] += dR[i * 3] * s + dR[i * 3 + 1] * a;
+            dRw[i * 3 + 2] += dR[i * 3 + 2];
+            da += dR[i * 3] * Rw[i * 3] + dR[i * 3 + 1] * Rw[i * 3 + 1];
+            ds += dR[i * 3] * Rw[i * 3 + 1] - dR[i * 3 + 1] * Rw[i * 3];
+          }
+          // (a, s) = unit(ra, rb)
+          if (cn < 1.f / NRM_EPS) {
+            const float dot_ = a * da + s * ds;
+            dra = (da - a * dot_) * cn;
+            drb = (ds - s * dot_) * cn;
+          } else {
+            dra = da / NRM_EPS;
+            drb = ds / NRM_EPS;
+          }
+        }
+        if (all_good) {  // back into the rows' own places
+          s2[2 * q] = ds0; s2[2 * q + 1] = ds1;
+          r2[2 * q] = dra; r2[2 * q + 1] = drb;
+        } else {  // a skipped face's outputs stay as the caller left them
+          const size_t o = o0 + q;
+          if (dscaling) { dscaling[2 * o] = ds0; dscaling[2 * o + 1] = ds1; }
+          if (drot2d) { drot2d[2 * o] = dra; drot2d[2 * o + 1] = drb; }
+        }
+      }
+    }
+    __syncthreads();
+    if (all_good) {
+      if (dscaling) rows_out(dscaling + 2 * o0, 2 * m, s2);
+      if (drot2d) rows_out(drot2d + 2 * o0, 2 * m, r2);
+      __syncthreads();
+    }
   }
-  if (drots) {
-    f3 h0, h1, h2;
-    face_frame_adj(F, mk(dRw[0], dRw[3], dRw[6]), mk(dRw[1], dRw[4], dRw[7]),
-                   mk(dRw[2], dRw[5], dRw[8]), h0, h1, h2);
-    g0 = g0 + h0; g1 = g1 + h1; g2 = g2 + h2;
+  if (good && t < nf) {
+    if (drots) {
+      const Frame F = face_frame(T.v0, T.v1, T.v2);
+      f3 h0, h1, h2;
+      face_frame_adj(F, mk(dRw[0], dRw[3], dRw[6]), mk(dRw[1], dRw[4], dRw[7]),
+                     mk(dRw[2], dRw[5], dRw[8]), h0, h1, h2);
+      g0 = g0 + h0; g1 = g1 + h1; g2 = g2 + h2;
+    }
+    scatter_vertices(dverts, T, g0, g1, g2);
   }
-  atomicAdd(dverts + 3 * i0, g0.x); atomicAdd(dverts + 3 * i0 + 1, g0.y); atomicAdd(dverts + 3 * i0 + 2, g0.z);
-  atomicAdd(dverts + 3 * i1, g1.x); atomicAdd(dverts + 3 * i1 + 1, g1.y); atomicAdd(dverts + 3 * i1 + 2, g1.z);
-  atomicAdd(dverts + 3 * i2, g2.x); atomicAdd(dverts + 3 * i2 + 1, g2.y); atomicAdd(dverts + 3 * i2 + 2, g2.z);
 }
 
 }  // namespace
@@ -429,7 +617,8 @@ __global__ void bind3_bwd_kernel(DmgsFaceBinding3 b, const float *__restrict__ d
 int launch_bind_fwd(const DmgsFaceBinding &b, float *xyz, float *cov, float *rot, float *covL,
                     cudaStream_t s) {
   if (b.F <= 0) return DMGS_OK;
-  DMGS_TIMED(K_BIND_FWD, s, dmgs_host::note_launch(), bind_fwd_kernel<<<(b.F + 255) / 256, 256, 0, s>>>(b, xyz, cov, rot, covL));
+  const FaceBlocks kb = face_blocks(b.F, b.G, 9);
+  DMGS_TIMED(K_BIND_FWD, s, dmgs_host::note_launch(), bind_fwd_kernel<<<kb.blocks, BB, kb.smem, s>>>(b, kb, xyz, cov, rot, covL));
   DMGS_LAUNCH_CHECK("bind_fwd_kernel");
   return DMGS_OK;
 }
@@ -439,7 +628,8 @@ int launch_bind_bwd(const DmgsFaceBinding &b, const float *dxyz, const float *dc
   DMGS_CUDA(cudaMemsetAsync(dverts, 0, (size_t)b.V * 3 * 4, s));
   if (dsf) DMGS_CUDA(cudaMemsetAsync(dsf, 0, 4, s));
   if (b.F <= 0) return DMGS_OK;
-  DMGS_TIMED(K_BIND_BWD, s, dmgs_host::note_launch(), bind_bwd_kernel<<<(b.F + 255) / 256, 256, 0, s>>>(b, dxyz, dcov, dverts, dsf));
+  const FaceBlocks kb = face_blocks(b.F, b.G, 9);
+  DMGS_TIMED(K_BIND_BWD, s, dmgs_host::note_launch(), bind_bwd_kernel<<<kb.blocks, BB, kb.smem, s>>>(b, kb, dxyz, dcov, dverts, dsf));
   DMGS_LAUNCH_CHECK("bind_bwd_kernel");
   return DMGS_OK;
 }
@@ -447,7 +637,8 @@ int launch_bind_bwd(const DmgsFaceBinding &b, const float *dxyz, const float *dc
 int launch_bind3_fwd(const DmgsFaceBinding3 &b, float *xyz, float *scales, float *rots,
                      cudaStream_t s) {
   if (b.F <= 0) return DMGS_OK;
-  DMGS_TIMED(K_BIND3_FWD, s, dmgs_host::note_launch(), bind3_fwd_kernel<<<(b.F + 255) / 256, 256, 0, s>>>(b, xyz, scales, rots));
+  const FaceBlocks kb = face_blocks(b.F, b.G, 14);
+  DMGS_TIMED(K_BIND3_FWD, s, dmgs_host::note_launch(), bind3_fwd_kernel<<<kb.blocks, BB, kb.smem, s>>>(b, kb, xyz, scales, rots));
   DMGS_LAUNCH_CHECK("bind3_fwd_kernel");
   return DMGS_OK;
 }
@@ -457,7 +648,8 @@ int launch_bind3_bwd(const DmgsFaceBinding3 &b, const float *dxyz, const float *
                      cudaStream_t s) {
   DMGS_CUDA(cudaMemsetAsync(dverts, 0, (size_t)b.V * 3 * 4, s));
   if (b.F <= 0) return DMGS_OK;
-  DMGS_TIMED(K_BIND3_BWD, s, dmgs_host::note_launch(), bind3_bwd_kernel<<<(b.F + 255) / 256, 256, 0, s>>>(b, dxyz, dscales, drots, dverts, dscaling,
+  const FaceBlocks kb = face_blocks(b.F, b.G, 14);
+  DMGS_TIMED(K_BIND3_BWD, s, dmgs_host::note_launch(), bind3_bwd_kernel<<<kb.blocks, BB, kb.smem, s>>>(b, kb, dxyz, dscales, drots, dverts, dscaling,
                                                      drot2d));
   DMGS_LAUNCH_CHECK("bind3_bwd_kernel");
   return DMGS_OK;
