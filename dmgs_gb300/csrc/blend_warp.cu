@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "blend_common.cuh"
+#include "f32x2.cuh"
 
 namespace dmgs {
 
@@ -26,39 +27,6 @@ namespace {
 constexpr int BW_WARPS = 2;  // warps per CTA (independent of one another)
 
 // ---- one or two floats per operand, rounded to nearest each ----------------
-
-struct F2 {
-  unsigned long long v;
-};
-__device__ __forceinline__ F2 f2_make(float a, float b) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float vget(F2 x, int i) {
-  float a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
-  return i == 0 ? a : b;
-}
-__device__ __forceinline__ float vget(float x, int) { return x; }
-__device__ __forceinline__ F2 vfma(F2 a, F2 b, F2 c) {
-  F2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return r;
-}
-__device__ __forceinline__ F2 vmul(F2 a, F2 b) {
-  F2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 vadd(F2 a, F2 b) {
-  F2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
 
 // A lane's PPT pixels: G groups of N.
 template <int PPT>

@@ -16,23 +16,24 @@
 // table (size r^3 rounded up to 8, capped at 2^19), else the spatial hash
 // x * 1 ^ y * 2654435761 ^ z * 805459861 (32-bit), modulo the table size.
 //
-// Two kernels, one thread per point, persistent grids:
-//   forward   hash gathers (the 50 MB table is L2-resident), the 32-32-32-C
-//             MLP from shared-memory weights (warp-broadcast reads), outputs
-//             staged per warp in shared memory for coalesced row stores;
-//   adjoint   recomputes the forward, runs the MLP adjoint, accumulates the
-//             three weight gradients as 128-point outer-product GEMMs staged
-//             in shared memory (each thread owns a fixed 3x4 / 2x4 sub-block
-//             in registers across all its tiles; one atomic per entry per
-//             block at the end) and writes each point's dL/denc; then a
-//             light kernel reduces the table gradient (float2 atomics, one
-//             per run of consecutive points in a cell) and forms the position
-//             gradient from the interpolation weights' derivatives.
+// Kernels:
+//   forward   blocks of 128 points: a thread encodes a point (hash gathers
+//             from the 50 MB table, L2-resident) into shared memory, then the
+//             32-32-32-C MLP runs as register-tiled products over the block;
+//   adjoint   recomputes the hidden layers from the forward's encoding, forms
+//             the three weight gradients as outer-product GEMMs over the
+//             block's points (each thread's entries stay in registers across
+//             its tiles; one atomic per entry per block at the end) and each
+//             point's dL/denc;
+//   scatter   reduces the table gradient (float2 atomics, one per run of
+//             consecutive points in a cell) and forms the position gradient
+//             from the interpolation weights' derivatives.
 // The reference's gradient hooks (geo/texture.py:72-73 with _MLP's
 // loss_scale): the table receives 128x its true gradient, the positions
 // their true gradient.
 #include <cmath>
 
+#include "f32x2.cuh"
 #include "kernels.cuh"
 
 namespace dmgs {
@@ -41,7 +42,6 @@ namespace {
 
 constexpr int TEX_LEVELS = 16;
 constexpr int TEX_FEAT = TEX_LEVELS * 2;  // encoding width
-constexpr int TEX_MAXC = 48;              // channels (SH degree 3: 3 x 16)
 constexpr int TEX_THREADS = 128;
 constexpr uint32_t TEX_LOG2_HASHMAP = 19;
 constexpr uint32_t TEX_BASE_RES = 16;
@@ -85,16 +85,19 @@ struct TexArgs {
   int64_t n;
 };
 
-__device__ __forceinline__ uint32_t corner_index(const TexLevels &L, int l, uint32_t cx, uint32_t cy,
-                                                 uint32_t cz) {
-  uint32_t idx;
-  if ((L.hashed >> l) & 1u) {
-    idx = cx ^ (cy * 2654435761u) ^ (cz * 805459861u);
+// Entry of the corner (cx, cy, cz) of a level: the index is below twice the
+// table's size on dense levels, whose tables hold every corner (the last
+// plane wraps), and the hashed tables' size is a power of two.
+__device__ __forceinline__ uint32_t level_entry(uint32_t cx, uint32_t cy, uint32_t cz, uint32_t res,
+                                                uint32_t size, uint32_t offset, bool hashed) {
+  uint32_t i;
+  if (hashed) {
+    i = (cx ^ (cy * 2654435761u) ^ (cz * 805459861u)) & (size - 1u);
   } else {
-    const uint32_t r = L.res[l];
-    idx = cx + cy * r + cz * r * r;
+    i = cx + (cy + cz * res) * res;
+    i = i < size ? i : i % size;
   }
-  return L.offset[l] + idx % L.size[l];
+  return offset + i;
 }
 
 // Normalised, clamped texture coordinate (and whether the clamp passes the
@@ -133,267 +136,354 @@ __device__ __forceinline__ float corner_weight(const LevelPos &q, int corner) {
   return __fmul_rn(__fmul_rn(w0, w1), w2);
 }
 
-__device__ __forceinline__ void encode(const TexArgs &A, const TexLevels &L, const float (&t)[3],
-                                       float (&enc)[TEX_FEAT]) {
+// ---- the block's 128 points: rows [feature][point] in shared memory -------
+//
+// A thread owns 8 points x TJ features of every product (points 4 pg .. + 3
+// of each half of the tile, pairs of points in f32x2): per feature of the
+// reduction it reads two float4 of the points' row and TJ weights for 8 TJ
+// multiply-adds, where a thread per point read a weight per multiply-add and
+// the kernels stood on the delivery of those broadcasts.  Every sum runs over
+// the same terms in the same order as a thread per point's did.
+constexpr int XP = TEX_THREADS + 4;  // row pitch: float4 rows, 8 rows start in 8 different bank groups
+constexpr int WP = 36;               // weight row pitch (likewise)
+
+struct Mine {
+  int pg, jg;  // point group 0..15, feature group 0..7
+  __device__ Mine() : pg(((threadIdx.x >> 6) << 3) | (threadIdx.x & 7)), jg((threadIdx.x >> 3) & 7) {}
+};
+
+// [rows][32] weights into rows of pitch WP.
+__device__ __forceinline__ void load_weights(const float *__restrict__ W, int rows, float *sW) {
+  for (int i = threadIdx.x; i < rows * 32; i += TEX_THREADS) sW[(i >> 5) * WP + (i & 31)] = W[i];
+}
+
+// The points' [n][C] rows of a tile to and from X[feature][point]: a warp
+// takes 8 features of 4 points (whole 32-byte sectors; the 32 shared-memory
+// words lie in 32 banks).  Points beyond n read as zero.
+template <int C>
+__device__ __forceinline__ void load_rows(const float *src, int64_t p0, int64_t n, float *X) {
+  const int j0 = threadIdx.x & 7, q0 = threadIdx.x >> 3;
 #pragma unroll
+  for (int jb = 0; jb < (C + 7) / 8; ++jb)
+#pragma unroll
+    for (int qb = 0; qb < TEX_THREADS / 16; ++qb) {
+      const int j = 8 * jb + j0, q = 16 * qb + q0;
+      if (j < C) X[j * XP + q] = p0 + q < n ? src[(p0 + q) * C + j] : 0.f;
+    }
+}
+template <int C, int POINTS, int PITCH>
+__device__ __forceinline__ void store_rows(float *dst, int64_t p0, int64_t n, const float *X) {
+  const int j0 = threadIdx.x & 7, q0 = threadIdx.x >> 3;
+#pragma unroll
+  for (int jb = 0; jb < (C + 7) / 8; ++jb)
+#pragma unroll
+    for (int qb = 0; qb < POINTS / 16; ++qb) {
+      const int j = 8 * jb + j0, q = 16 * qb + q0;
+      if (j < C && p0 + q < n) dst[(p0 + q) * C + j] = X[j * PITCH + q];
+    }
+}
+
+// The encoding of the thread's point into its column of X.
+__device__ __forceinline__ void encode_tile(const TexArgs &A, const TexLevels &L, const float *__restrict__ xyz,
+                                            int64_t p, float *X) {
+  const bool valid = p < A.n;
+  float t[3] = {0.f, 0.f, 0.f};
+  bool pass[3];
+  if (valid) tex_coord(A, xyz, p, t, pass);
+#pragma unroll 2
   for (int l = 0; l < TEX_LEVELS; ++l) {
-    const LevelPos q = level_pos(L, l, t);
-    float a0 = 0.f, a1 = 0.f;
+    F2 a = f2_make(0.f, 0.f);
+    if (valid) {
+      const LevelPos q = level_pos(L, l, t);
+      const bool hashed = (L.hashed >> l) & 1u;
+      const uint32_t res = L.res[l], size = L.size[l], offset = L.offset[l];
+      float2 v[8];
 #pragma unroll
-    for (int corner = 0; corner < 8; ++corner) {
-      const float w = corner_weight(q, corner);
-      const float2 v = __ldg(A.table + corner_index(L, l, q.c[0] + (corner & 1), q.c[1] + ((corner >> 1) & 1),
-                                                    q.c[2] + ((corner >> 2) & 1)));
-      a0 = __fadd_rn(a0, __fmul_rn(w, v.x));
-      a1 = __fadd_rn(a1, __fmul_rn(w, v.y));
+      for (int c = 0; c < 8; ++c)
+        v[c] = __ldg(A.table + level_entry(q.c[0] + (c & 1), q.c[1] + ((c >> 1) & 1), q.c[2] + (c >> 2), res, size,
+                                           offset, hashed));
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float w = corner_weight(q, c);
+        a = vadd(a, vmul(f2_make(w, w), f2_make(v[c].x, v[c].y)));
+      }
     }
-    enc[2 * l] = a0;
-    enc[2 * l + 1] = a1;
+    X[(2 * l) * XP + threadIdx.x] = vget(a, 0);
+    X[(2 * l + 1) * XP + threadIdx.x] = vget(a, 1);
   }
 }
 
-// y = W x for a row-major [R][32] weight matrix in shared memory (rows read
-// as float4, the same address across the warp: broadcasts).
-template <int R>
-__device__ __forceinline__ void matvec(const float *__restrict__ W, const float (&x)[32], float (&y)[R]) {
+// acc[i][.] += W[j][k] X[k][points], j = jg + 8 i (rows at and beyond J are not the caller's).
+template <int TJ, int J>
+__device__ __forceinline__ void layer(const float *__restrict__ X, const float *__restrict__ W, const Mine &m,
+                                      F2 (&acc)[TJ][4]) {
 #pragma unroll
-  for (int j = 0; j < R; ++j) {
-    const float4 *w = reinterpret_cast<const float4 *>(W + j * 32);
-    float acc = 0.f;
+  for (int i = 0; i < TJ; ++i)
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float4 v = w[k];
-      acc = fmaf(v.x, x[4 * k], acc);
-      acc = fmaf(v.y, x[4 * k + 1], acc);
-      acc = fmaf(v.z, x[4 * k + 2], acc);
-      acc = fmaf(v.w, x[4 * k + 3], acc);
-    }
-    y[j] = acc;
-  }
-}
-
-// x = W^T y for a row-major [R][32] matrix.
-template <int R>
-__device__ __forceinline__ void matvec_t(const float *__restrict__ W, const float (&y)[R], float (&x)[32]) {
+    for (int q = 0; q < 4; ++q) acc[i][q] = f2_make(0.f, 0.f);
+  const float *x = X + 4 * m.pg;
+  const float *w[TJ];
 #pragma unroll
-  for (int k = 0; k < 32; ++k) x[k] = 0.f;
+  for (int i = 0; i < TJ; ++i) w[i] = W + (J % 8 == 0 || m.jg + 8 * i < J ? m.jg + 8 * i : J - 1) * WP;
+#pragma unroll 2
+  for (int k = 0; k < 32; k += 4) {
+    float4 wk[TJ];
 #pragma unroll
-  for (int j = 0; j < R; ++j) {
-    const float4 *w = reinterpret_cast<const float4 *>(W + j * 32);
+    for (int i = 0; i < TJ; ++i) wk[i] = *reinterpret_cast<const float4 *>(w[i] + k);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float4 v = w[k];
-      x[4 * k] = fmaf(v.x, y[j], x[4 * k]);
-      x[4 * k + 1] = fmaf(v.y, y[j], x[4 * k + 1]);
-      x[4 * k + 2] = fmaf(v.z, y[j], x[4 * k + 2]);
-      x[4 * k + 3] = fmaf(v.w, y[j], x[4 * k + 3]);
+    for (int kk = 0; kk < 4; ++kk) {
+      const ulonglong2 lo = *reinterpret_cast<const ulonglong2 *>(x + (k + kk) * XP);
+      const ulonglong2 hi = *reinterpret_cast<const ulonglong2 *>(x + (k + kk) * XP + TEX_THREADS / 2);
+#pragma unroll
+      for (int i = 0; i < TJ; ++i) {
+        const float ws = kk == 0 ? wk[i].x : kk == 1 ? wk[i].y : kk == 2 ? wk[i].z : wk[i].w;
+        const F2 ww = f2_make(ws, ws);
+        acc[i][0] = vfma(ww, F2{lo.x}, acc[i][0]);
+        acc[i][1] = vfma(ww, F2{lo.y}, acc[i][1]);
+        acc[i][2] = vfma(ww, F2{hi.x}, acc[i][2]);
+        acc[i][3] = vfma(ww, F2{hi.y}, acc[i][3]);
+      }
     }
   }
 }
 
+__device__ __forceinline__ float4 f4_of(F2 a, F2 b) {
+  return make_float4(vget(a, 0), vget(a, 1), vget(b, 0), vget(b, 1));
+}
+
+// The hidden layer's rows: relu(acc) at j = jg + 8 i.
+__device__ __forceinline__ void store_relu(const F2 (&acc)[4][4], const Mine &m, float *X) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float4 v = f4_of(acc[i][2 * h], acc[i][2 * h + 1]);
+      v.x = fmaxf(v.x, 0.f), v.y = fmaxf(v.y, 0.f), v.z = fmaxf(v.z, 0.f), v.w = fmaxf(v.w, 0.f);
+      *reinterpret_cast<float4 *>(X + (m.jg + 8 * i) * XP + h * (TEX_THREADS / 2) + 4 * m.pg) = v;
+    }
+}
+
+// Forward.  The encoding's gathers (the table is L2-resident) want warps in
+// flight, the layers shared-memory bandwidth; blocks in different phases
+// cover for each other.  271,824 points, 48 channels, float32: 160 us with a
+// thread per point, 119 us so (130 at five blocks an SM and 197 at six: the
+// shared memory they take is L1 that the gathers lose).
 template <int C>
-__device__ __forceinline__ void load_weights(const TexArgs &A, float *sW1, float *sW2, float *sW3) {
-  for (int i = threadIdx.x; i < 32 * 32; i += blockDim.x) {
-    sW1[i] = A.W1[i];
-    sW2[i] = A.W2[i];
-  }
-  for (int i = threadIdx.x; i < C * 32; i += blockDim.x) sW3[i] = A.W3[i];
-  __syncthreads();
-}
-
-template <int C>
-__global__ void __launch_bounds__(TEX_THREADS)
+__global__ void __launch_bounds__(TEX_THREADS, 4)
 tex_fwd_kernel(const TexArgs A, const TexLevels L, const float *__restrict__ xyz, float *__restrict__ out,
                float *__restrict__ enc_out) {
-  __shared__ __align__(16) float sW1[32 * 32], sW2[32 * 32], sW3[C * 32];
-  constexpr int SC = C | 1;  // odd row stride: conflict-free per-lane row writes
-  __shared__ float stage[TEX_THREADS / 32][32 * SC];
-  load_weights<C>(A, sW1, sW2, sW3);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  constexpr int TJ = (C + 7) / 8, SP = TEX_THREADS / 2 + 4;
+  __shared__ __align__(16) float sW[(64 + C) * WP];
+  __shared__ __align__(16) float X[32 * XP];  // a layer's input rows; at the end half a tile's outputs
+  static_assert(8 * TJ * SP <= 32 * XP, "staged outputs fit");
+  __shared__ TexLevels sL;
+  float *sW1 = sW, *sW2 = sW + 32 * WP, *sW3 = sW + 64 * WP;
+  if (threadIdx.x == 0) sL = L;
+  load_weights(A.W1, 32, sW1);
+  load_weights(A.W2, 32, sW2);
+  load_weights(A.W3, C, sW3);
+  const Mine m;
   const int64_t ntiles = (A.n + TEX_THREADS - 1) / TEX_THREADS;
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int64_t p = tile * TEX_THREADS + threadIdx.x;
-    float o[C];
-    if (p < A.n) {
-      float t[3];
-      bool pass[3];
-      tex_coord(A, xyz, p, t, pass);
-      float enc[TEX_FEAT], h[32], g[32];
-      encode(A, L, t, enc);
-      if (enc_out) {  // kept for the adjoint: [n][32] rows, 16-byte aligned
-        float4 *row = reinterpret_cast<float4 *>(enc_out + 32 * p);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) row[k] = make_float4(enc[4 * k], enc[4 * k + 1], enc[4 * k + 2], enc[4 * k + 3]);
-      }
-      matvec<32>(sW1, enc, h);
-#pragma unroll
-      for (int k = 0; k < 32; ++k) h[k] = fmaxf(h[k], 0.f);
-      matvec<32>(sW2, h, g);
-#pragma unroll
-      for (int k = 0; k < 32; ++k) g[k] = fmaxf(g[k], 0.f);
-      matvec<C>(sW3, g, o);
+    const int64_t p0 = tile * TEX_THREADS;
+    __syncthreads();  // the weights are in; the last tile's outputs are out
+    encode_tile(A, sL, xyz, p0 + threadIdx.x, X);
+    __syncthreads();
+    if (enc_out) store_rows<32, TEX_THREADS, XP>(enc_out, p0, A.n, X);  // kept for the adjoint
+    {
+      F2 acc[4][4];
+      layer<4, 32>(X, sW1, m, acc);
+      __syncthreads();
+      store_relu(acc, m, X);
+      __syncthreads();
+      layer<4, 32>(X, sW2, m, acc);
+      __syncthreads();
+      store_relu(acc, m, X);
+      __syncthreads();
     }
-    // rows of the warp's 32 points are contiguous in out: stage and store
-    float *st = stage[wid];
-    if (p < A.n)
+    F2 acc[TJ][4];
+    layer<TJ, C>(X, sW3, m, acc);
 #pragma unroll
-      for (int j = 0; j < C; ++j) st[lane * SC + j] = o[j];
-    __syncwarp();
-    const int64_t p0 = tile * TEX_THREADS + wid * 32;
-    const int64_t nrow = A.n - p0 < 32 ? A.n - p0 : 32;
-    for (int i = lane; i < nrow * C; i += 32) out[p0 * C + i] = st[(i / C) * SC + i % C];
-    __syncwarp();
+    for (int h = 0; h < 2; ++h) {
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < TJ; ++i)
+        *reinterpret_cast<float4 *>(X + (m.jg + 8 * i) * SP + 4 * m.pg) = f4_of(acc[i][2 * h], acc[i][2 * h + 1]);
+      __syncthreads();
+      store_rows<C, TEX_THREADS / 2, SP>(out, p0 + h * (TEX_THREADS / 2), A.n, X);
+    }
   }
 }
 
-// Adjoint.  Shared memory per block (rows = the block's 128 points): the
-// weights; R0 [128][SA] (dL/dout, then dh2, then dh1: the left operands of
-// the outer-product GEMMs); R1 [128][SB] (h2, then each thread's dL/denc);
-// H1 and E [128][SB] (h1 and enc, kept from the recomputation: right
-// operands of the layer-2 and layer-1 GEMMs and the ReLU masks).
-constexpr int SA = TEX_MAXC + 1, SB = 33;
-
-// acc[r][c] += sum over the block's points q of a[q][row r] b[q][col c]
-template <int R, int SAx>
-__device__ __forceinline__ void outer_gemm(const float *__restrict__ a, int row0, int nrows,
-                                           const float *__restrict__ b, int col0, float (&acc)[R][4]) {
-  for (int q = 0; q < TEX_THREADS; ++q) {
-    float bv[4];
+// acc[i][.] = sum over j of W[j][k] Y[j][points], k = 4 jg + i.
+template <int J>
+__device__ __forceinline__ void layer_adjoint(const float *__restrict__ Y, const float *__restrict__ W, const Mine &m,
+                                              F2 (&acc)[4][4]) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) bv[c] = b[q * SB + col0 + c];
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const float av = row0 + r < nrows ? a[q * SAx + row0 + r] : 0.f;
+    for (int q = 0; q < 4; ++q) acc[i][q] = f2_make(0.f, 0.f);
+  const float *y = Y + 4 * m.pg, *w = W + 4 * m.jg;
+#pragma unroll 4
+  for (int j = 0; j < J; ++j) {
+    const float4 wk = *reinterpret_cast<const float4 *>(w + j * WP);
+    const ulonglong2 lo = *reinterpret_cast<const ulonglong2 *>(y + j * XP);
+    const ulonglong2 hi = *reinterpret_cast<const ulonglong2 *>(y + j * XP + TEX_THREADS / 2);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av, bv[c], acc[r][c]);
+    for (int i = 0; i < 4; ++i) {
+      const float ws = i == 0 ? wk.x : i == 1 ? wk.y : i == 2 ? wk.z : wk.w;
+      const F2 ww = f2_make(ws, ws);
+      acc[i][0] = vfma(ww, F2{lo.x}, acc[i][0]);
+      acc[i][1] = vfma(ww, F2{lo.y}, acc[i][1]);
+      acc[i][2] = vfma(ww, F2{hi.x}, acc[i][2]);
+      acc[i][3] = vfma(ww, F2{hi.y}, acc[i][3]);
     }
   }
+}
+
+// The rows k = 4 jg + i of H: acc where H > 0 (the layer's ReLU), else 0.
+__device__ __forceinline__ void store_masked(const F2 (&acc)[4][4], const Mine &m, float *H) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float4 *e = reinterpret_cast<float4 *>(H + (4 * m.jg + i) * XP + h * (TEX_THREADS / 2) + 4 * m.pg);
+      const float4 o = *e, d = f4_of(acc[i][2 * h], acc[i][2 * h + 1]);
+      *e = make_float4(o.x > 0.f ? d.x : 0.f, o.y > 0.f ? d.y : 0.f, o.z > 0.f ? d.z : 0.f, o.w > 0.f ? d.w : 0.f);
+    }
+}
+
+// A weight gradient's entries (row rg + 8 r, column cg + 8 c) over the
+// points of the thread's half of the block: acc += sum over them of
+// Y[row][q] X[column][q].  Rows at and beyond J are not the caller's.
+template <int R, int J>
+__device__ __forceinline__ void outer(const float *__restrict__ Y, const float *__restrict__ X, float (&acc)[R][4]) {
+  const int half = threadIdx.x >> 6, rg = (threadIdx.x >> 3) & 7, cg = threadIdx.x & 7;
+  const float *y[R], *x = X + cg * XP + half * (TEX_THREADS / 2);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    y[r] = Y + (J % 8 == 0 || rg + 8 * r < J ? rg + 8 * r : J - 1) * XP + half * (TEX_THREADS / 2);
+#pragma unroll 2
+  for (int q = 0; q < TEX_THREADS / 2; q += 4) {
+    float4 xv[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) xv[c] = *reinterpret_cast<const float4 *>(x + 8 * c * XP + q);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float4 yv = *reinterpret_cast<const float4 *>(y[r] + q);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        acc[r][c] = fmaf(yv.x, xv[c].x, acc[r][c]);
+        acc[r][c] = fmaf(yv.y, xv[c].y, acc[r][c]);
+        acc[r][c] = fmaf(yv.z, xv[c].z, acc[r][c]);
+        acc[r][c] = fmaf(yv.w, xv[c].w, acc[r][c]);
+      }
+    }
+  }
+}
+
+// The block's sum of a weight gradient: the second half's entries through
+// shared memory, one reduction per entry.
+template <int R, int J>
+__device__ __forceinline__ void reduce_outer(const float (&acc)[R][4], float *S, float *dW) {
+  const int half = threadIdx.x >> 6, t = threadIdx.x & 63, rg = (threadIdx.x >> 3) & 7, cg = threadIdx.x & 7;
+  __syncthreads();
+  if (half)
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) S[(4 * r + c) * 64 + t] = acc[r][c];
+  __syncthreads();
+  if (!half)
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (J % 8 == 0 || rg + 8 * r < J)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) atomicAdd(dW + (rg + 8 * r) * 32 + cg + 8 * c, acc[r][c] + S[(4 * r + c) * 64 + t]);
+}
+
+// Adjoint: recomputes the hidden layers, then per layer the weight gradient
+// (each thread keeps its entries in registers over all its tiles) and the
+// input's gradient.  Shared memory: the weights, D (the encoding, then
+// dL/dout, then the encoding again), H1 and H2 (the hidden layers, each
+// replaced by its own gradient).  Bound by shared-memory bandwidth; 75 KB, so
+// three blocks an SM.  271,824 points, 48 channels, float32: 269 us with a
+// thread per point, 150 us so.
+constexpr size_t tex_bwd_smem(int C) {
+  return (size_t)((64 + C) * WP + (C > 32 ? C : 32) * XP + 2 * 32 * XP) * sizeof(float);
 }
 
 template <int C>
-__global__ void __launch_bounds__(TEX_THREADS)
-tex_bwd_kernel(const TexArgs A, const TexLevels L, const float *__restrict__ xyz,
-               const float *__restrict__ enc_in, const float *__restrict__ dout, float *__restrict__ denc,
-               float *__restrict__ dW1, float *__restrict__ dW2, float *__restrict__ dW3) {
+__global__ void __launch_bounds__(TEX_THREADS, 3)
+tex_bwd_kernel(const TexArgs A, const TexLevels L, const float *__restrict__ xyz, const float *enc_in,
+               const float *__restrict__ dout, float *denc, float *__restrict__ dW1, float *__restrict__ dW2,
+               float *__restrict__ dW3) {
   extern __shared__ __align__(16) float smem[];
-  float *sW1 = smem, *sW2 = sW1 + 32 * 32, *sW3 = sW2 + 32 * 32;
-  float *R0 = sW3 + TEX_MAXC * 32;
-  float *R1 = R0 + TEX_THREADS * SA;
-  float *H1 = R1 + TEX_THREADS * SB;
-  float *E = H1 + TEX_THREADS * SB;
-  load_weights<C>(A, sW1, sW2, sW3);
-  const int tid = threadIdx.x;
-  // owned sub-blocks: dW3 rows R3 (t/8) .., cols 4 (t%8) .. +3; dW2 / dW1
-  // rows 2 (t/8) .. +1
-  const int cg = (tid & 7) * 4, rg = tid >> 3;
-  constexpr int R3 = (C + 15) / 16;
-  float acc3[R3][4], acc2[2][4], acc1[2][4];
+  __shared__ TexLevels sL;
+  float *sW1 = smem, *sW2 = sW1 + 32 * WP, *sW3 = sW2 + 32 * WP;
+  float *H1 = sW3 + C * WP, *H2 = H1 + 32 * XP, *D = H2 + 32 * XP;
+  if (threadIdx.x == 0) sL = L;
+  load_weights(A.W1, 32, sW1);
+  load_weights(A.W2, 32, sW2);
+  load_weights(A.W3, C, sW3);
+  const Mine m;
+  constexpr int R3 = (C + 7) / 8;
+  float acc3[R3][4], acc2[4][4], acc1[4][4];
 #pragma unroll
-  for (int r = 0; r < R3; ++r)
+  for (int c = 0; c < 4; ++c) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) acc3[r][c] = 0.f;
+    for (int r = 0; r < R3; ++r) acc3[r][c] = 0.f;
 #pragma unroll
-  for (int r = 0; r < 2; ++r)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc2[r][c] = acc1[r][c] = 0.f;
-  float *e_row = E + tid * SB, *h1_row = H1 + tid * SB;
-
+    for (int r = 0; r < 4; ++r) acc2[r][c] = acc1[r][c] = 0.f;
+  }
+  const float *enc = enc_in ? enc_in : denc;  // without the forward's: formed here, kept in denc's rows
   const int64_t ntiles = (A.n + TEX_THREADS - 1) / TEX_THREADS;
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int64_t p = tile * TEX_THREADS + tid;
-    const bool valid = p < A.n;
-    float t[3] = {0.f, 0.f, 0.f};
-    bool pass[3] = {false, false, false};
-    float h2[32];
-    {
-      float enc[TEX_FEAT], h1[32];
-#pragma unroll
-      for (int k = 0; k < 32; ++k) enc[k] = h1[k] = h2[k] = 0.f;
-      if (valid) {
-        if (enc_in) {  // the forward's encoding (the same arithmetic, so the same values)
-          const float4 *row = reinterpret_cast<const float4 *>(enc_in + 32 * p);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const float4 v = __ldg(row + k);
-            enc[4 * k] = v.x; enc[4 * k + 1] = v.y; enc[4 * k + 2] = v.z; enc[4 * k + 3] = v.w;
-          }
-        } else {
-          tex_coord(A, xyz, p, t, pass);
-          encode(A, L, t, enc);
-        }
-        matvec<32>(sW1, enc, h1);
-#pragma unroll
-        for (int k = 0; k < 32; ++k) h1[k] = fmaxf(h1[k], 0.f);
-        matvec<32>(sW2, h1, h2);
-#pragma unroll
-        for (int k = 0; k < 32; ++k) h2[k] = fmaxf(h2[k], 0.f);
-      }
-#pragma unroll
-      for (int k = 0; k < 32; ++k) {
-        e_row[k] = enc[k];
-        h1_row[k] = h1[k];
-        R1[tid * SB + k] = h2[k];
-      }
+    const int64_t p0 = tile * TEX_THREADS;
+    F2 g[4][4];
+    __syncthreads();  // the weights are in; the last tile's reads are done
+    if (enc_in) {
+      load_rows<32>(enc, p0, A.n, D);
+    } else {
+      encode_tile(A, sL, xyz, p0 + threadIdx.x, D);
     }
-    // dL/dout rows of the block into R0 (coalesced); invalid rows zero
-    {
-      const int64_t p0 = tile * TEX_THREADS;
-      const int nrow = (int)(A.n - p0 < TEX_THREADS ? A.n - p0 : TEX_THREADS);
-      for (int i = tid; i < nrow * C; i += TEX_THREADS) R0[(i / C) * SA + i % C] = dout[p0 * C + i];
-      if (!valid)
-#pragma unroll
-        for (int j = 0; j < C; ++j) R0[tid * SA + j] = 0.f;
-    }
+    __syncthreads();
+    if (!enc_in) store_rows<32, TEX_THREADS, XP>(denc, p0, A.n, D);
+    layer<4, 32>(D, sW1, m, g);
+    store_relu(g, m, H1);
+    __syncthreads();
+    load_rows<C>(dout, p0, A.n, D);
+    layer<4, 32>(H1, sW2, m, g);
+    store_relu(g, m, H2);
     __syncthreads();
     // layer 3: dW3 += dy h2^T;  dh2 = relu'(h2) (W3^T dy)
-    outer_gemm<R3, SA>(R0, R3 * rg, C, R1, cg, acc3);
-    float d[32];
-    {
-      float dy[C];
-#pragma unroll
-      for (int j = 0; j < C; ++j) dy[j] = R0[tid * SA + j];
-      matvec_t<C>(sW3, dy, d);
-    }
-#pragma unroll
-    for (int k = 0; k < 32; ++k) d[k] = h2[k] > 0.f ? d[k] : 0.f;
+    outer<R3, C>(D, H2, acc3);
+    layer_adjoint<C>(D, sW3, m, g);
+    __syncthreads();
+    store_masked(g, m, H2);
+    load_rows<32>(enc, p0, A.n, D);
     __syncthreads();
     // layer 2: dW2 += dh2 h1^T;  dh1 = relu'(h1) (W2^T dh2)
-#pragma unroll
-    for (int k = 0; k < 32; ++k) R0[tid * SA + k] = d[k];
+    outer<4, 32>(H2, H1, acc2);
+    layer_adjoint<32>(H2, sW2, m, g);
     __syncthreads();
-    outer_gemm<2, SA>(R0, 2 * rg, 32, H1, cg, acc2);
-    float g[32];
-    matvec_t<32>(sW2, d, g);
-#pragma unroll
-    for (int k = 0; k < 32; ++k) g[k] = h1_row[k] > 0.f ? g[k] : 0.f;
+    store_masked(g, m, H1);
     __syncthreads();
     // layer 1: dW1 += dh1 enc^T;  dL/denc = W1^T dh1
+    outer<4, 32>(H1, D, acc1);
+    layer_adjoint<32>(H1, sW1, m, g);
 #pragma unroll
-    for (int k = 0; k < 32; ++k) R0[tid * SA + k] = g[k];
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<float4 *>(H2 + (4 * m.jg + i) * XP + h * (TEX_THREADS / 2) + 4 * m.pg) =
+            f4_of(g[i][2 * h], g[i][2 * h + 1]);
     __syncthreads();
-    outer_gemm<2, SA>(R0, 2 * rg, 32, E, cg, acc1);
-    matvec_t<32>(sW1, g, d);
-    __syncthreads();  // every GEMM read done before the next tile's staging
-    if (!valid) continue;
-    float4 *row = reinterpret_cast<float4 *>(denc + 32 * p);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) row[k] = make_float4(d[4 * k], d[4 * k + 1], d[4 * k + 2], d[4 * k + 3]);
+    store_rows<32, TEX_THREADS, XP>(denc, p0, A.n, H2);
   }
-  // block partials of the weight gradients
-#pragma unroll
-  for (int r = 0; r < R3; ++r) {
-    const int row = R3 * rg + r;
-    if (row < C)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) atomicAdd(dW3 + row * 32 + cg + c, acc3[r][c]);
-  }
-#pragma unroll
-  for (int r = 0; r < 2; ++r)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      atomicAdd(dW2 + (2 * rg + r) * 32 + cg + c, acc2[r][c]);
-      atomicAdd(dW1 + (2 * rg + r) * 32 + cg + c, acc1[r][c]);
-    }
+  reduce_outer<R3, C>(acc3, D, dW3);
+  reduce_outer<4, 32>(acc2, D, dW2);
+  reduce_outer<4, 32>(acc1, D, dW1);
 }
 
 // Table (128 x the true gradient) and position gradients from each point's
@@ -416,21 +506,6 @@ struct ScatterSmem {
   uint2 cell[32];      // x, y
   uint32_t cellz[32];
 };
-
-// Entry of the corner (cx, cy, cz) of a level: the index is below twice the
-// table's size on dense levels, whose tables hold every corner (the last
-// plane wraps), and the hashed tables' size is a power of two.
-__device__ __forceinline__ uint32_t level_entry(uint32_t cx, uint32_t cy, uint32_t cz, uint32_t res,
-                                                uint32_t size, uint32_t offset, bool hashed) {
-  uint32_t i;
-  if (hashed) {
-    i = (cx ^ (cy * 2654435761u) ^ (cz * 805459861u)) & (size - 1u);
-  } else {
-    i = cx + (cy + cz * res) * res;
-    i = i < size ? i : i % size;
-  }
-  return offset + i;
-}
 
 __global__ void __launch_bounds__(32 * SC_WARPS)
 tex_scatter_kernel(const TexArgs A, const TexLevels L, const float *__restrict__ xyz,
@@ -515,10 +590,6 @@ tex_scatter_kernel(const TexArgs A, const TexLevels L, const float *__restrict__
     for (int dd = 0; dd < 3; ++dd) dxyz[3 * p + dd] = pass[dd] ? gt[dd] / A.ext[dd] : 0.f;
 }
 
-constexpr size_t tex_bwd_smem() {
-  return (size_t)(32 * 32 * 2 + TEX_MAXC * 32 + TEX_THREADS * (SA + 3 * SB)) * sizeof(float);
-}
-
 bool tex_ok(const DmgsTexture *tx) {
   if (!tx || !tx->table || !tx->W1 || !tx->W2 || !tx->W3) return false;
   if (tx->channels != 3 && tx->channels != 12 && tx->channels != 27 && tx->channels != 48) return false;
@@ -572,12 +643,12 @@ template <int C>
 int run_bwd(const TexArgs &A, const TexLevels &L, const float *xyz, const float *enc,
             const float *dout, float *dxyz, float *dtable, float *dW1, float *dW2, float *dW3,
             float *denc, cudaStream_t s) {
-  if (int r = dmgs_host::raise_smem_limit((const void *)tex_bwd_kernel<C>, tex_bwd_smem())) return r;
+  if (int r = dmgs_host::raise_smem_limit((const void *)tex_bwd_kernel<C>, tex_bwd_smem(C))) return r;
   int grid;
-  if (int r = persistent_grid(tex_bwd_kernel<C>, tex_bwd_smem(), A.n, grid)) return r;
+  if (int r = persistent_grid(tex_bwd_kernel<C>, tex_bwd_smem(C), A.n, grid)) return r;
   // timed apart: the MLP adjoint (weight-gradient GEMMs) and the scatter of
   // the encoding gradients into the table and the positions
-  DMGS_TIMED(K_TEX_BWD, s, dmgs_host::note_launch(), tex_bwd_kernel<C><<<grid, TEX_THREADS, tex_bwd_smem(), s>>>(
+  DMGS_TIMED(K_TEX_BWD, s, dmgs_host::note_launch(), tex_bwd_kernel<C><<<grid, TEX_THREADS, tex_bwd_smem(C), s>>>(
       A, L, xyz, enc, dout, denc, dW1, dW2, dW3));
   if (dxyz || dtable)
     DMGS_TIMED(K_TEX_SCATTER, s, dmgs_host::note_launch(),
