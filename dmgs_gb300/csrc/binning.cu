@@ -892,12 +892,13 @@ row_emit_kernel(const BinViews bv) {
 constexpr int TE_WARPS = 8;
 constexpr int TE_THREADS = 32 * TE_WARPS;
 constexpr int STAGE_CAP = 8192;    // staged instances per sub-pass
+constexpr int TE_COPY = 8;         // lanes copying a tile's staged run
 constexpr int TE_PER = 4;          // row-list entries per thread considered for a sub-pass
 constexpr int TE_ENTRIES = TE_THREADS * TE_PER;
 
 __host__ __device__ inline size_t tile_emit_smem_words(int nx) {
   return (size_t)nx + (nx + 1) + (size_t)TE_WARPS * (nx + 1) + STAGE_CAP + TE_WARPS +
-         (TE_WARPS + 1) + (size_t)TE_WARPS * (2 * (size_t)nx + 32);
+         (TE_WARPS + 1) + (size_t)TE_WARPS * ((size_t)nx + 32);
 }
 
 __device__ __forceinline__ int block_sum_te(int v, int *red) {
@@ -923,6 +924,10 @@ __device__ __forceinline__ int block_sum_te(int v, int *red) {
 // every tile it covers (tile x always by lane x % 32, so no two lanes share
 // a cursor and no ranks are needed); (D) each tile's staged run copied to
 // the tile's list at its running position (coalesced).
+// Bound by issue (73% of the slots): the block's fixed work and the XOR scans.
+// 16 views of 3M Gaussians (176M instances): 707 us with a scan each for the
+// begun and the ended entries, 64-bit slice cuts and a warp per copied run,
+// 608 us so; four views of 500k 82 -> 53 us, one of 3M 74 -> 66 us.
 __global__ void __launch_bounds__(TE_THREADS)
 tile_emit_kernel(const BinViews bv, int S) {
   extern __shared__ uint32_t te[];
@@ -939,20 +944,19 @@ tile_emit_kernel(const BinViews bv, int S) {
   const uint32_t e1 = f1 < C ? B.rcnt[(size_t)r * C + f1]
                              : (r + 1 < B.gy ? B.rcnt[(size_t)(r + 1) * C] : counters[CI_K1]);
   if (e0 >= e1) return;
-  const int xa = xs * XSEG, nx = min(B.gx - xa, XSEG), nbits = bits_for(nx);
+  const int xa = xs * XSEG, nx = min(B.gx - xa, XSEG);
   uint32_t *tcur = te;                                   // [nx] running list positions
   uint32_t *soff = tcur + nx;                            // [nx + 1] staging offsets
   int *wc = reinterpret_cast<int *>(soff + nx + 1);      // [TE_WARPS][nx + 1] counts / cursors
   uint32_t *stage = reinterpret_cast<uint32_t *>(wc + TE_WARPS * (nx + 1));  // [STAGE_CAP]
   int *red = reinterpret_cast<int *>(stage + STAGE_CAP);  // [TE_WARPS]
   uint32_t *bnd = reinterpret_cast<uint32_t *>(red + TE_WARPS);  // [TE_WARPS + 1] slice starts
-  // per warp: start / end bit masks per tile [nx] each (zero between
+  // per warp: the entries whose cover changes at a tile [nx] (zero between
   // groups) and the Gaussian indices of the current group of 32 entries
   uint32_t *smask = bnd + TE_WARPS + 1;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  uint32_t *sbeg = smask + (size_t)w * (2 * nx + 32), *send = sbeg + nx, *gids = send + nx;
-  for (int i = tid; i < TE_WARPS * (2 * nx + 32); i += TE_THREADS) smask[i] = 0u;
-  const unsigned lt = lanemask_lt();
+  uint32_t *tog = smask + (size_t)w * (nx + 32), *gids = tog + nx;
+  for (int i = tid; i < TE_WARPS * (nx + 32); i += TE_THREADS) smask[i] = 0u;
   const uint2 *__restrict__ rl = B.rowlist;
   uint32_t *__restrict__ out = B.point_list;
   const uint32_t cap = B.K_alloc;
@@ -1005,24 +1009,20 @@ tile_emit_kernel(const BinViews bv, int S) {
       for (int k = 0; k < TE_PER; ++k) {
         const uint32_t i = (uint32_t)tid * TE_PER + k;
         if (i < En && I > 0) {
-          const int wi = (int)((long long)ex * TE_WARPS / I);
+          // ex <= STAGE_CAP here: the product stays below 2^32
+          const int wi = (int)((uint32_t)ex * TE_WARPS / (uint32_t)I);
           atomicMin(&bnd[min(wi, TE_WARPS - 1)], i);
         }
         ex += wd[k];
       }
     }
     __syncthreads();
-    if (tid == 0) {  // slice starts: first entry whose instances begin in the warp's share
-      uint32_t m = En;
-      bnd[TE_WARPS] = En;
-      for (int i = TE_WARPS - 1; i >= 1; --i) {
-        m = min(m, bnd[i]);
-        bnd[i] = m;
-      }
-      bnd[0] = 0;
-    }
-    __syncthreads();
-    const uint32_t sa = e + bnd[w], sb = e + bnd[w + 1];
+    // slice starts: first entry whose instances begin in the warp's share
+    // (a slice without one starts where the next does)
+    uint32_t bm = lane > 0 && lane < TE_WARPS ? bnd[lane] : (lane == 0 ? 0u : En);
+#pragma unroll
+    for (int o = 1; o < TE_WARPS; o <<= 1) bm = min(bm, __shfl_down_sync(FULL, bm, o));
+    const uint32_t sa = e + __shfl_sync(FULL, bm, w), sb = e + __shfl_sync(FULL, bm, w + 1);
     // (A) this warp's counts per tile
     for (int i = lane; i <= nx; i += 32) wcw[i] = 0;
     __syncwarp();
@@ -1069,19 +1069,14 @@ tile_emit_kernel(const BinViews bv, int S) {
       if (lane == 0) soff[nx] = carry;
     }
     __syncthreads();
-    for (int x = tid; x < nx; x += TE_THREADS) {  // absolute staging cursors of every warp
-      const int o = (int)soff[x];
-#pragma unroll
-      for (int w2 = 0; w2 < TE_WARPS; ++w2) wc[w2 * (nx + 1) + x] += o;
-    }
-    __syncthreads();
+    for (int x = lane; x < nx; x += 32) wcw[x] += (int)soff[x];  // the warp's absolute staging cursors
+    __syncwarp();
     // (C) stage the slice's instances, 32 entries (depth order) at a time:
-    // lane j sets bit j at its entry's first tile a_j in sbeg and at its end
-    // b_j in send; inclusive OR-prefixes over the tiles give the entries
-    // begun at or before tile x and those ended at or before it, so tile x
-    // is covered by M_x = begun & ~ended, which the lane owning x (x % 32)
-    // appends in bit (entry) order at its cursor — so a tile's cursor is
-    // only ever touched by one lane and entries land in the order they come.
+    // lane j flips bit j at its entry's first tile a_j and at its end b_j;
+    // the inclusive XOR-prefix over the tiles is the set of entries that
+    // cover a tile, which the lane owning tile x (x % 32) appends in bit
+    // (entry) order at its cursor — so a tile's cursor is only ever touched
+    // by one lane and entries land in the order they come.
     for (uint32_t g0 = sa; g0 < sb; g0 += 32) {
       const uint32_t i = g0 + lane;
       const uint2 en = i < sb ? rl[i] : make_uint2(0u, 0u);
@@ -1090,30 +1085,26 @@ tile_emit_kernel(const BinViews bv, int S) {
       const bool has = a < b;
       gids[lane] = en.x;
       if (has) {
-        atomicOr(&sbeg[a], 1u << lane);
-        if (b < nx) atomicOr(&send[b], 1u << lane);  // an end at nx is never read
+        atomicXor(&tog[a], 1u << lane);
+        if (b < nx) atomicXor(&tog[b], 1u << lane);  // an end at nx is never read
       }
       const int lo = (int)__reduce_min_sync(FULL, has ? (unsigned)a : 0xffffffffu);
       const int hi = (int)__reduce_max_sync(FULL, has ? (unsigned)b : 0u);
       __syncwarp();
-      if (lo < hi) {  // warp-uniform; chunks up to the one holding hi (clears send[hi])
-        uint32_t cb = 0u, ce = 0u;  // carries of the two OR-prefixes
+      if (lo < hi) {  // warp-uniform; chunks up to the one holding hi (clears tog[hi])
+        uint32_t carry = 0u;
         for (int xb = lo & ~31; xb <= hi && xb < nx; xb += 32) {
           const int x = xb + lane;
-          uint32_t vb = x < nx ? sbeg[x] : 0u, ve = x < nx ? send[x] : 0u;
+          uint32_t mm = x < nx ? tog[x] : 0u;
 #pragma unroll
           for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t ub = __shfl_up_sync(FULL, vb, o), ue = __shfl_up_sync(FULL, ve, o);
-            if (lane >= o) { vb |= ub; ve |= ue; }
+            const uint32_t u = __shfl_up_sync(FULL, mm, o);
+            if (lane >= o) mm ^= u;
           }
-          vb |= cb;
-          ve |= ce;
-          cb = __shfl_sync(FULL, vb, 31);
-          ce = __shfl_sync(FULL, ve, 31);
+          mm ^= carry;
+          carry = __shfl_sync(FULL, mm, 31);
           if (x < nx) {
-            sbeg[x] = 0u;
-            send[x] = 0u;
-            uint32_t mm = vb & ~ve;
+            tog[x] = 0u;
             if (mm) {
               uint32_t p = (uint32_t)wcw[x];
               do {
@@ -1130,16 +1121,16 @@ tile_emit_kernel(const BinViews bv, int S) {
       __syncwarp();
     }
     __syncthreads();
-    // (D) copy each tile's staged run to its list
-    for (int x = w; x < nx; x += TE_WARPS) {
+    // (D) copy each tile's staged run to its list, TE_COPY lanes a tile
+    // (runs are some ten to a hundred instances long)
+    for (int x = w * (32 / TE_COPY) + lane / TE_COPY; x < nx; x += TE_WARPS * (32 / TE_COPY)) {
       const uint32_t a = soff[x], n = soff[x + 1] - a, dst = tcur[x];
-      for (uint32_t j = lane; j < n; j += 32) {
+      for (uint32_t j = lane % TE_COPY; j < n; j += TE_COPY) {
         if (dst + j < cap) out[dst + j] = stage[a + j]; else bad = true;
       }
-      __syncwarp();
-      if (lane == 0) tcur[x] = dst + n;
     }
     __syncthreads();
+    for (int x = tid; x < nx; x += TE_THREADS) tcur[x] += soff[x + 1] - soff[x];
     e += En;
   }
   if (bad) atomicOr(&counters[CI_STATUS], ST_BOUNDS);
@@ -1186,15 +1177,22 @@ int device_sms() {
   return cached_sms;
 }
 
-// Row segments per view for a launch: enough (row, piece, segment) blocks
-// for about five waves of the tile emission (short blocks balance uneven
-// rows).  A pure function of the views'
-// grids and the device, so the geometry and the emission launches of one
-// set of views agree.
+// Row segments per view for a launch: enough (row, piece, segment) blocks for
+// several waves of the tile emission (short blocks balance uneven rows), but
+// not so many that a block's fixed work (sub-pass cut, cursors, run copies)
+// outweighs its instances.  Emission at 16 | 24 | 32 | 48 blocks an SM, us: four
+// views of 500k Gaussians 53 | 60 | 70 | 76, sixteen of 3M 710 | 642 | 623 |
+// 608 (and the counting kernel 202 | 172 | 164 | 152); a single view is at
+// SEG_MAX on most grids.  A pure function of the views' grids and sizes and
+// the device, so the geometry and the emission launches of one set of views
+// agree.
 int seg_plan(const BinViews &bv) {
-  long rows = 0;
-  for (int v = 0; v < bv.n; ++v) rows += (long)bv.v[v].gy * bv.v[v].nxs;
-  const long target = 32L * device_sms();
+  long rows = 0, gaussians = 0;
+  for (int v = 0; v < bv.n; ++v) {
+    rows += (long)bv.v[v].gy * bv.v[v].nxs;
+    gaussians += bv.v[v].P;
+  }
+  const long target = (gaussians < (16l << 20) ? 16L : 48L) * device_sms();
   const long S = rows > 0 ? (target + rows - 1) / rows : 1;
   return (int)std::max(1L, std::min((long)SEG_MAX, S));
 }
