@@ -436,7 +436,14 @@ struct SlotSink {
   }
 };
 
-__global__ void __launch_bounds__(BWD_BLOCK)
+// Bound by latency (SH rows, per-pair gathers).  VEC: the SH rows start on 16
+// bytes (a multiple of four coefficients) and are read as float4.  16 views of
+// 3M Gaussians: 951 us with a load per float and four blocks an SM; with float4
+// 967 | 839 | 824 | 815 | 843 us at 4 | 5 | 6 | 7 | 8 blocks (spills from 6 on).
+// Rows staged through shared memory both ways took 937 to 988 us: the staging
+// takes the L1 that the pairs' gathers hit.
+template <bool VEC>
+__global__ void __launch_bounds__(BWD_BLOCK, 7)
 preprocess_bwd_batched_kernel(const BatchViews bv, int P, int M, const float *__restrict__ means,
                               const float *__restrict__ shs, const float *__restrict__ scales,
                               const float *__restrict__ rots, const float *__restrict__ cov3D,
@@ -547,7 +554,20 @@ preprocess_bwd_batched_kernel(const BatchViews bv, int P, int M, const float *__
       const float *gv = s_gacc[v] + 12 * (size_t)idx;
       float drgb[3] = {gv[6], gv[7], gv[8]};
       apply_clamp(s_flags[v][idx], drgb);
-      sh_bwd(s_vp[v].D, mx, my, mz, s_mat[v] + 32, drgb, [&](int j) { return sh[j]; },
+      // four coefficients' twelve floats as three float4 where rows start on
+      // 16 bytes: lanes read different rows, a wavefront a lane and load
+      float4 q0, q1, q2;
+      sh_bwd(s_vp[v].D, mx, my, mz, s_mat[v] + 32, drgb,
+             [&](int j) {
+               if (!VEC) return sh[j];
+               if (j % 12 == 0) {
+                 q0 = __ldg(reinterpret_cast<const float4 *>(sh + j));
+                 q1 = __ldg(reinterpret_cast<const float4 *>(sh + j) + 1);
+                 q2 = __ldg(reinterpret_cast<const float4 *>(sh + j) + 2);
+               }
+               const float4 q = j % 12 < 4 ? q0 : j % 12 < 8 ? q1 : q2;
+               return j % 4 == 0 ? q.x : j % 4 == 1 ? q.y : j % 4 == 2 ? q.z : q.w;
+             },
              [&](int j, float x) { dsh[j] += x; }, dm);
     }
   }
@@ -635,10 +655,12 @@ int launch_preprocess_bwd_batched(const BatchViews &bv, const GaussianPtrs &g, c
   if (g.P <= 0) return DMGS_OK;
   int want_xy = densify_accum != nullptr;
   for (int v = 0; v < bv.nviews; ++v) want_xy |= bv.v[v].dL_dmeans2D != nullptr;
-  DMGS_TIMED(K_BATCH_PREPROCESS_BWD, s,
-             dmgs_host::note_launch(), preprocess_bwd_batched_kernel<<<(g.P + BWD_BLOCK - 1) / BWD_BLOCK, BWD_BLOCK, 0, s>>>(
-                 bv, g.P, g.M, g.means3D, g.shs, g.scales, g.rotations, g.cov3D, out, want_xy,
-                 densify_accum, densify_count));
+  const bool vec = (g.M & 3) == 0 && (reinterpret_cast<uintptr_t>(g.shs) & 15) == 0;
+  const auto kernel = vec ? preprocess_bwd_batched_kernel<true> : preprocess_bwd_batched_kernel<false>;
+  DMGS_TIMED(K_BATCH_PREPROCESS_BWD, s, dmgs_host::note_launch(),
+             kernel<<<(g.P + BWD_BLOCK - 1) / BWD_BLOCK, BWD_BLOCK, 0, s>>>(
+                 bv, g.P, g.M, g.means3D, g.shs, g.scales, g.rotations, g.cov3D, out, want_xy, densify_accum,
+                 densify_count));
   DMGS_LAUNCH_CHECK("preprocess_bwd_batched_kernel");
   return DMGS_OK;
 }
