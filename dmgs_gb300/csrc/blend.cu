@@ -1,4 +1,6 @@
-// blend.cu — per-tile front-to-back alpha blending (forward) and its adjoint.
+// blend.cu — per-tile front-to-back alpha blending (forward) and its adjoint,
+// a CTA per tile: the tunable shapes and the FP64-sum adjoint.  The default
+// shape (16x16, 4 pixels per thread, batches of 128) runs blend_warp.cu.
 //
 // Semantics (3DGS tile renderer, reached from gaussian_renderer/__init__.py:86-94):
 //   power = -1/2 (a dx^2 + c dy^2) - b dx dy, d = mean2D - pixel

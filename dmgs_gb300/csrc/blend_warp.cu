@@ -26,8 +26,6 @@ namespace {
 
 constexpr int BW_WARPS = 2;  // warps per CTA (independent of one another)
 
-// ---- one or two floats per operand, rounded to nearest each ----------------
-
 // A lane's PPT pixels: G groups of N.
 template <int PPT>
 struct Px;

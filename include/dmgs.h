@@ -164,7 +164,7 @@ int dmgs_raster_bwd_f64sum(const DmgsView *view, const DmgsGaussians *g,
  * that owns the device's memory pool, or a real-time loop that must not call
  * cudaMalloc/cudaFree between frames, cannot hand dmgs_raster_bwd its
  * scratch buffer; this variant keeps that scratch in a static device array
- * of the library instead (DMGS_NOALLOC_MAX_GAUSSIANS x 48 bytes = 12 MiB,
+ * of the library instead (DMGS_NOALLOC_MAX_GAUSSIANS x 48 bytes and a work queue, 12 MiB,
  * held by every GPU that loads the library until exit) and allocates
  * nothing.  Arguments and results are those of dmgs_raster_bwd without the
  * scratch pair; g->P above the limit returns DMGS_ERR_ARG.  The first call on
