@@ -133,15 +133,19 @@ class MLPTexture3D(torch.nn.Module):
         self.net = _MLP(N_LEVELS * N_FEATURES, internal_dims, hidden, channels, device)
 
     def _aabb_host(self):
-        """The AABB as a host float32 [2, 3] tensor for the kernel arguments,
-        copied again only when ``self.AABB`` is replaced or modified in place
-        (a device AABB would otherwise cost a device->host sync per call)."""
+        """The AABB as a host float32 [2, 3] tensor for the kernel arguments
+        (and its six values as ``_aabb_list``), copied again only when
+        ``self.AABB`` is replaced or modified in place (a device AABB would
+        otherwise cost a device->host sync per call).  A module restored from
+        an earlier version has no list."""
         a = self.AABB
         version = getattr(a, "_version", None)
-        if getattr(self, "_aabb_src", None) is not a or self._aabb_ver != version:
-            self._aabb_cache = torch.as_tensor(a, dtype=torch.float32).detach().cpu().reshape(2, 3).clone()
+        if (getattr(self, "_aabb_src", None) is not a or self._aabb_ver != version
+                or "_aabb_list" not in self.__dict__):
+            host = torch.as_tensor(a, dtype=torch.float32).detach().cpu().reshape(2, 3).clone()
+            values = host.reshape(-1).tolist()
+            self._aabb_cache, self._aabb_list = host, values
             self._aabb_src, self._aabb_ver = a, version
-            self._aabb_list = self._aabb_cache.reshape(-1).tolist()
         return self._aabb_cache
 
     def sample_noact(self, texc):

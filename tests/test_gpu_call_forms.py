@@ -1,13 +1,15 @@
 """Forms in which a program calls the differentiable entry points: traced,
-checkpointed, from several streams and threads, out of memory, and under the
-transforms that they refuse."""
+checkpointed, from several streams and threads, from a restored module, out of
+memory, and under the transforms that they refuse."""
+import copy
 import threading
 
 import pytest
 import torch
 from torch.utils.checkpoint import checkpoint
 
-from test_gpu_native_nodes import D, OPS, _run, _same
+from dmgs_gb300.texture import MLPTexture3D
+from test_gpu_native_nodes import D, OPS, _gen, _run, _same
 
 pytestmark = pytest.mark.gpu
 
@@ -70,7 +72,7 @@ def test_streams_and_threads(op):
         _same(r, want)
 
 
-@pytest.mark.parametrize("op", ["loss", "sh", "bind2", "bind3", "raster-sh", "flexicubes-none"])
+@pytest.mark.parametrize("op", ["loss", "sh", "bind2", "bind3", "texture", "raster-sh", "flexicubes-none"])
 def test_transforms_are_refused(op):
     tensors, fn = OPS[op]()
     name = next(iter(tensors))
@@ -103,3 +105,19 @@ def test_out_of_memory_keeps_its_type():
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert bool(torch.isfinite(l1_ssim_loss(x, y)))
+
+
+def test_restored_texture_module():
+    """A module whose host copy of the box was made by an earlier version (or
+    is not there) is used like a new one."""
+    m = MLPTexture3D(torch.tensor([[-1.0] * 3, [1.0] * 3]), channels=3, device=D)
+    x = 2 * torch.rand(50, 3, device=D, generator=_gen(3)) - 1
+    want = m.sample_noact(x)
+    assert "_aabb_cache" in m.__dict__
+    r = copy.deepcopy(m)
+    for k in [k for k in r.__dict__ if k.startswith("_aabb") and k not in ("_aabb_src", "_aabb_ver", "_aabb_cache")]:
+        del r.__dict__[k]
+    r._aabb_src, r._aabb_ver = r.AABB, r.AABB._version  # as a whole-module pickle restores them
+    assert torch.equal(r.sample_noact(x), want)
+    r.AABB = torch.tensor([[-2.0] * 3, [2.0] * 3])
+    assert not torch.equal(r.sample_noact(x), want)
