@@ -469,7 +469,7 @@ __device__ __forceinline__ void bwd_part(const BlendView &V, int tile, int part,
           const float a = fminf(ALPHA_MAX, __fmul_rn(E.o, ex));
           const bool take = ok[k] && !(a < ALPHA_MIN);
           al[j] = take ? a : 0.f;
-          G_[j] = take ? ex : 0.f;
+          G_[j] = ex;
           iv[j] = take ? rcp_approx(1.f - a) : 1.f;  // T stays as it is
         }
         const F inv = P::make(iv), at = P::make(al);
@@ -477,7 +477,13 @@ __device__ __forceinline__ void bwd_part(const BlendView &V, int tile, int part,
         const F cdg = vfma(P::splat(E.b), g2[g], vfma(P::splat(E.g), g1[g], vmul(P::splat(E.r), g0[g])));
         const F Sd = vfma(ag[g], minus, cdg);  // (c - acc) . dL/dpixel
         const F dLa = vfma(Sd, Tn, vmul(nTfb[g], inv));
-        const F Gd = vmul(P::make(G_), dLa);   // dL/dopacity term
+        // dL/dopacity term, selected and not scaled by 0: where dL/dpixel is
+        // not finite, only the Gaussians blended there are to see it
+        const F Gx = vmul(P::make(G_), dLa);
+        float gd[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) gd[j] = al[j] > 0.f ? vget(Gx, j) : 0.f;
+        const F Gd = P::make(gd);
         const F wt = vmul(at, Tn);             // dL/drgb weight
         const F gy = vmul(Gd, dy[g]);
         T[g] = Tn;

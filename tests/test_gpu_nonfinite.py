@@ -1,0 +1,64 @@
+"""Values that are not finite stay where they arise: what does not depend on
+them keeps its value."""
+import pytest
+import torch
+
+import dmgs_gb300
+
+pytestmark = pytest.mark.gpu
+D = "cuda"
+
+
+def _gen(seed):
+    return torch.Generator(device=D).manual_seed(seed)
+
+
+def _pixel_settings(w, h):
+    """A camera at the origin looking along +z: the point (x, y, z) of pixel (i, j)
+    at depth 1 is ((2 i + 1) / w - 1, (2 j + 1) / h - 1, 1)."""
+    n, f = 0.01, 100.0
+    proj = torch.zeros(4, 4, device=D)
+    proj[0, 0] = proj[1, 1] = 1.0
+    proj[2, 2], proj[2, 3], proj[3, 2] = f / (f - n), -f * n / (f - n), 1.0
+    return dmgs_gb300.GaussianRasterizationSettings(
+        image_height=h, image_width=w, tanfovx=1.0, tanfovy=1.0, bg=torch.tensor([0.2, 0.3, 0.4], device=D), scale_modifier=1.0,
+        viewmatrix=torch.eye(4, device=D), projmatrix=proj.T.contiguous(), sh_degree=0, campos=torch.zeros(3, device=D),
+        prefiltered=False, debug=False)
+
+
+@pytest.mark.parametrize("others", [0, 40_000])  # a short work list's strips, a long one's halves
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_pixel_gradient_that_is_not_finite_stays_with_its_gaussians(others, bad):
+    """Two Gaussians a warp visits together, one of them at a pixel whose
+    gradient is not finite: the other one's mean, covariance and opacity
+    gradients are those without that pixel."""
+    w = h = 256
+    rs = _pixel_settings(w, h)
+    g = _gen(7)
+    px = torch.tensor([[3.0, 1.0], [12.0, 1.0]], device=D)
+    if others:
+        px = torch.cat([px, 32 + 220 * torch.rand(others, 2, device=D, generator=g)])
+    P = px.shape[0]
+    means = torch.cat([(2 * px + 1) / w - 1, torch.ones(P, 1, device=D)], 1)
+    means[:, 2] += 0.001 * torch.rand(P, device=D, generator=g)
+    sigma = 0.6 * 2 / w
+    cov = torch.tensor([sigma ** 2, 0, 0, sigma ** 2, 0, sigma ** 2], device=D).repeat(P, 1)
+    t = dict(means3D=means, opacities=torch.full((P, 1), 0.1 if others else 0.8, device=D), colors_precomp=torch.rand(P, 3, device=D, generator=g),
+             cov3D_precomp=cov, means2D=torch.zeros(P, 3, device=D))
+    t["opacities"][:2] = 0.8
+    for x in t.values():
+        x.requires_grad_(True)
+    dimg = torch.randn(3, h, w, device=D, generator=g)
+
+    def grads(value):
+        d = dimg.clone()
+        d[:, 1, 3] = value
+        img, radii = dmgs_gb300.GaussianRasterizer(rs)(**t)
+        assert int(radii[:2].min()) > 0
+        return dict(zip(t, torch.autograd.grad(img, list(t.values()), d)))
+    want, got = grads(0.0), grads(bad)
+    for k in ("means3D", "opacities", "cov3D_precomp", "means2D"):
+        assert bool(torch.isfinite(want[k][1]).all()) and float(want[k][1].abs().max()) > 0
+        assert not bool(torch.isfinite(got[k][0]).all())  # the Gaussian of the pixel itself
+        # one Gaussian, few pixels: the same terms (the warp's sum adds zeros)
+        assert torch.allclose(got[k][1], want[k][1], rtol=1e-5, atol=0), k
