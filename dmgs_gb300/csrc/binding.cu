@@ -346,9 +346,11 @@ __device__ __forceinline__ float inv_sqrt(float x) {
   return fmaf(fmaf(-x * y, y, 1.f), 0.5f * y, y);
 }
 
-// 1 / max(sqrt(x), NRM_EPS) for x >= 0 (the guard of torch's normalize).
+// 1 / max(sqrt(x), NRM_EPS) for x >= 0 (the guard of torch's normalize); 0
+// where x, a sum of squares, has overflowed (the step would give inf * 0).
 __device__ __forceinline__ float inv_norm(float x) {
-  return x > NRM_EPS * NRM_EPS ? inv_sqrt(x) : 1.f / NRM_EPS;
+  if (!(x > NRM_EPS * NRM_EPS)) return 1.f / NRM_EPS;
+  return x < __int_as_float(0x7f800000) ? inv_sqrt(x) : 0.f;
 }
 
 // Unit quaternion (w, x, y, z), w >= 0, of a rotation matrix (row-major),

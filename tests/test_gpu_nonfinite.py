@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import dmgs_gb300
+from dmgs_gb300.binding import barycentric_table, bind_faces_scale_rot
 
 pytestmark = pytest.mark.gpu
 D = "cuda"
@@ -11,6 +12,37 @@ D = "cuda"
 
 def _gen(seed):
     return torch.Generator(device=D).manual_seed(seed)
+
+
+def _bind3(r2, drots):
+    v = torch.randn(40, 3, device=D, generator=_gen(1)).requires_grad_(True)
+    f = torch.stack([torch.randperm(40, device=D, generator=_gen(2 + i))[:3] for i in range(30)])
+    bc, _ = barycentric_table(3, D)
+    s2 = 0.1 * torch.randn(90, 2, device=D, generator=_gen(50))
+    r2 = r2.clone().requires_grad_(True)
+    _, _, q = bind_faces_scale_rot(v, f, bc, s2, r2, 1e-5)
+    return (q.detach(), *torch.autograd.grad(q, [v, r2], drots))
+
+
+@pytest.mark.parametrize("big", [1e19, 2e19, 1e30])
+def test_2d_rotation_whose_square_overflows(big):
+    """|r|^2 beyond float32's range: r / |r| is 0 there (r / infinity), as for
+    a zero row, and the row's own gradient is 0."""
+    drots = torch.randn(90, 4, device=D, generator=_gen(60))
+    r2 = torch.randn(90, 2, device=D, generator=_gen(61))
+    r2[17] = 0.0
+    want = _bind3(r2, drots)
+    r2[17] = torch.tensor([big, -0.5 * big])
+    got = _bind3(r2, drots)
+    if big * big * 1.25 < 3.4e38:  # the square still fits: a plain rotation
+        want = _bind3(torch.where(torch.arange(90, device=D)[:, None] == 17, r2 / big, r2), drots)
+        assert torch.allclose(got[0], want[0], rtol=1e-5, atol=1e-6)
+        return
+    assert all(bool(torch.isfinite(t).all()) for t in got)
+    assert torch.equal(got[0], want[0])
+    assert torch.equal(got[2][17], torch.zeros(2, device=D))
+    keep = torch.arange(90, device=D) != 17
+    assert torch.equal(got[2][keep], want[2][keep])
 
 
 def _pixel_settings(w, h):
