@@ -194,7 +194,8 @@ ssim_moments_kernel(const float *__restrict__ x, const float *__restrict__ y, in
     const float D1 = mx * mx + my * my + C1, D2 = s11 + s22 + C2;
     const float inv = 1.f / (D1 * D2);
     const float S = N1 * N2 * inv;
-    const float S1 = S * (D2 * inv), S2 = S * (D1 * inv);  // S / D1, S / D2
+    // S / D1, S / D2; S is 0 where D1 or D2 has overflowed (inv is 0), and inf * 0 would be NaN
+    const float S1 = S == 0.f ? 0.f : S * (D2 * inv), S2 = S == 0.f ? 0.f : S * (D1 * inv);
     const float A = 2.f * my * (N2 - N1) * inv - 2.f * mx * S1 + 2.f * mx * S2;
     const float B = -S2;
     const float Dd = 2.f * N1 * inv;

@@ -1,5 +1,7 @@
 """Values that are not finite stay where they arise: what does not depend on
 them keeps its value."""
+import math
+
 import pytest
 import torch
 
@@ -94,3 +96,17 @@ def test_pixel_gradient_that_is_not_finite_stays_with_its_gaussians(others, bad)
         assert not bool(torch.isfinite(got[k][0]).all())  # the Gaussian of the pixel itself
         # one Gaussian, few pixels: the same terms (the warp's sum adds zeros)
         assert torch.allclose(got[k][1], want[k][1], rtol=1e-5, atol=0), k
+
+
+def test_loss_gradient_where_a_square_overflows():
+    """A pixel whose square overflows: E[x^2] is infinite in its window, SSIM
+    and its derivatives 0 there, and every gradient stays finite."""
+    from dmgs_gb300.loss import l1_ssim_loss
+    x = torch.rand(1, 40, 40, device=D, generator=_gen(70))
+    y = torch.rand(1, 40, 40, device=D, generator=_gen(71))
+    x[0, 20, 20] = 2.5e19
+    x.requires_grad_(True)
+    (g,) = torch.autograd.grad(l1_ssim_loss(x, y, 0.2), [x])
+    assert bool(torch.isfinite(g).all())
+    # in the pixel's own window only the L1 term is left
+    assert math.isclose(float(g[0, 20, 20]), 0.8 / 1600, rel_tol=1e-5)
