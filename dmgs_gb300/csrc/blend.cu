@@ -760,8 +760,11 @@ static BlendWork make_work(const GeomLayout &L, const char *geom) {
 
 int launch_blend_fwd(const ViewParams &vp, const GeomLayout &L, const char *geom,
                      const BinLayout &B, const char *bin, const ImgLayout &I, char *img,
-                     const float *bg, float *out_color, uint32_t *queue, cudaStream_t s) {
-  DMGS_CUDA(cudaMemsetAsync(queue, 0, 4, s));  // a state may be rendered more than once
+                     const float *bg, float *out_color, cudaStream_t s) {
+  // the queue word belongs to this render, as its image state does: several
+  // streams may render one geometry state at a time
+  uint32_t *queue = reinterpret_cast<uint32_t *>(img + I.queue);
+  DMGS_CUDA(cudaMemsetAsync(queue, 0, 4, s));
   BlendBatch bb;
   bb.nviews = 1;
   bb.v[0] = make_blend_view(vp, L, geom, B, bin, I, img, bg);

@@ -231,8 +231,7 @@ int dmgs_raster_fwd_render(const DmgsView *view, const DmgsGaussians *g, void *g
   RET_IF(make_bin_view(L, geom, 0xffffffffu, bin + B.point_list, (uint32_t)num_rendered, bv.v[0]));
   RET_IF(launch_emit(bv, s));
   RET_IF(debug_sync(view, s, "emit"));
-  RET_IF(launch_blend_fwd(vp, L, geom, B, bin, I, img, view->bg, out_color,
-                          reinterpret_cast<uint32_t *>(geom + L.counters) + TK_BLEND, s));
+  RET_IF(launch_blend_fwd(vp, L, geom, B, bin, I, img, view->bg, out_color, s));
   RET_IF(debug_sync(view, s, "blend_fwd"));
   if (view->debug) RET_IF(check_status(geom, L, s, nullptr));
   return DMGS_OK;

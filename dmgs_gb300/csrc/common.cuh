@@ -79,7 +79,7 @@ constexpr int CI_W = 10;       // total chunk weight of the visible Gaussians (6
 constexpr int CI_WORDS = 16;
 // tickets: the words after the counters, from which the blocks of the
 // look-back kernels draw their tiles
-constexpr int TK_SORT = 16, TK_CHUNK = 20, TK_SCAN = 21, TK_BLEND = 22;
+constexpr int TK_SORT = 16, TK_CHUNK = 20, TK_SCAN = 21;
 constexpr int CI_TICKETS_END = 32;
 
 // Geometry state of one view.  Binning arrays: the visible Gaussians in index
@@ -170,7 +170,7 @@ __host__ __device__ inline BinLayout bin_layout(int64_t K, int W, int H, int64_t
 }
 
 struct ImgLayout {
-  size_t final_T, n_contrib, total;
+  size_t final_T, n_contrib, queue, total;
 };
 
 __host__ __device__ inline ImgLayout img_layout(int W, int H) {
@@ -179,6 +179,7 @@ __host__ __device__ inline ImgLayout img_layout(int W, int H) {
   size_t o = 0;
   L.final_T = o;   o = align_up(o + n * 4, 256);
   L.n_contrib = o; o = align_up(o + n * 4, 256);
+  L.queue = o;     o = align_up(o + 4, 256);
   L.total = o;
   return L;
 }

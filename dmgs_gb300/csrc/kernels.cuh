@@ -187,7 +187,7 @@ int launch_blend_warp_bwd(const BlendBatch &bb, const BlendWork &wk, const ZeroS
                           uint32_t *queue, cudaStream_t s);
 int launch_blend_fwd(const ViewParams &vp, const GeomLayout &L, const char *geom,
                      const BinLayout &B, const char *bin, const ImgLayout &I, char *img,
-                     const float *bg, float *out_color, uint32_t *queue, cudaStream_t s);
+                     const float *bg, float *out_color, cudaStream_t s);
 // gacc64 != nullptr: the FP64-sum mode (gradient terms added into [P][12]
 // doubles, then rounded into gacc for the preprocess adjoint).
 int launch_blend_bwd(const ViewParams &vp, const GeomLayout &L, const char *geom,

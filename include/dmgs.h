@@ -113,7 +113,10 @@ int dmgs_raster_fwd_geometry(const DmgsView *view, const DmgsGaussians *g,
 
 /* Forward, phase 2 (replaces the binning + blend half of
  * `rasterize_gaussians`): emits the instances, sorts every tile's list by
- * (depth, index), writes tile ranges and blends out_color [3,H,W] (device). */
+ * (depth, index), writes tile ranges and blends out_color [3,H,W] (device).
+ * Reads the geometry state (and sets its status word on an error): several
+ * renders of one geometry, each with its own binning and image state, may run
+ * at the same time. */
 int dmgs_raster_fwd_render(const DmgsView *view, const DmgsGaussians *g,
                            void *geom_state, size_t geom_bytes,
                            void *binning_state, size_t binning_bytes,
