@@ -286,6 +286,11 @@ int raster_bwd_impl(const DmgsView *view, const DmgsGaussians *g, const float *d
     set_error("dL_drotations must be 16-byte aligned");
     return DMGS_ERR_ARG;
   }
+  // here and not at the preprocess adjoint: the blend adjoint clears the outputs
+  if (g->P > 0 && g->M > SH_COEFFS_MAX) {
+    set_error("preprocess_bwd: %d SH coefficients per Gaussian exceed %d", g->M, SH_COEFFS_MAX);
+    return DMGS_ERR_ARG;
+  }
   const char *geom = static_cast<const char *>(geom_state);
   const char *bin = static_cast<const char *>(binning_state);
   const char *img = static_cast<const char *>(image_state);

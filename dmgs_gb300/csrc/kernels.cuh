@@ -196,6 +196,7 @@ int launch_blend_bwd(const ViewParams &vp, const GeomLayout &L, const char *geom
                      const ZeroSpans &zero, uint32_t *queue, cudaStream_t s);
 
 // preprocess_bwd.cu
+constexpr int SH_COEFFS_MAX = 124;  // coefficients per Gaussian that the single-view adjoint takes
 int launch_preprocess_bwd_batched(const BatchViews &bv, const GaussianPtrs &g, const DmgsGrads &out,
                                   float *densify_accum, float *densify_count, cudaStream_t s);
 // The outputs of a single-view adjoint, to be zero before launch_preprocess_bwd

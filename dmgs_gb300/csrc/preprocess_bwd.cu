@@ -296,7 +296,6 @@ __device__ __forceinline__ void apply_clamp(uint32_t flags, float (&drgb)[3]) {
 // lanes leave the gathers and the rows written (600 B per visible Gaussian).
 // The SH rows are staged per warp in shared memory so that each row's 192
 // bytes go out as whole sectors.
-constexpr int SH_COEFFS_MAX = 124;  // coefficients per Gaussian accepted by the single-view adjoint
 constexpr int SHP = 49;  // staging row pitch in floats: lanes writing element j hit different banks
 
 struct RowSink {
@@ -629,10 +628,6 @@ int launch_preprocess_bwd(const ViewParams &vp, const float *viewm, const float 
                           const char *geom, const float *gacc, const DmgsGrads &out,
                           cudaStream_t s) {
   if (g.P <= 0) return DMGS_OK;
-  if (g.M > SH_COEFFS_MAX) {
-    dmgs_host::set_error("preprocess_bwd: %d SH coefficients per Gaussian exceed %d", g.M, SH_COEFFS_MAX);
-    return DMGS_ERR_ARG;
-  }
   const size_t smem = (size_t)BWD_BLOCK * SHP * 4;
   // the visible count is known on the device alone: a few waves of blocks
   // stride over the list
