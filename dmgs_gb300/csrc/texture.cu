@@ -613,9 +613,10 @@ TexArgs make_args(const DmgsTexture *tx, int64_t n) {
   return A;
 }
 
+// Resident blocks of a kernel, looked up once per device into the caller's
+// cached_dev and cached_slots, or fewer where the points do not fill them.
 template <typename K>
-int persistent_grid(K kernel, size_t smem, int64_t n, int &grid) {
-  thread_local int cached_dev = -1, cached_slots = 0;  // per kernel instantiation and host thread
+int persistent_grid(K kernel, size_t smem, int64_t n, int &cached_dev, int &cached_slots, int &grid) {
   int dev = 0;
   DMGS_CUDA(cudaGetDevice(&dev));
   if (dev != cached_dev) {
@@ -633,8 +634,9 @@ int persistent_grid(K kernel, size_t smem, int64_t n, int &grid) {
 template <int C>
 int run_fwd(const TexArgs &A, const TexLevels &L, const float *xyz, float *out, float *enc,
             cudaStream_t s) {
+  thread_local int dev = -1, slots = 0;  // per channel count and host thread
   int grid;
-  if (int r = persistent_grid(tex_fwd_kernel<C>, 0, A.n, grid)) return r;
+  if (int r = persistent_grid(tex_fwd_kernel<C>, 0, A.n, dev, slots, grid)) return r;
   dmgs_host::note_launch(), tex_fwd_kernel<C><<<grid, TEX_THREADS, 0, s>>>(A, L, xyz, out, enc);
   return DMGS_OK;
 }
@@ -644,8 +646,9 @@ int run_bwd(const TexArgs &A, const TexLevels &L, const float *xyz, const float 
             const float *dout, float *dxyz, float *dtable, float *dW1, float *dW2, float *dW3,
             float *denc, cudaStream_t s) {
   if (int r = dmgs_host::raise_smem_limit((const void *)tex_bwd_kernel<C>, tex_bwd_smem(C))) return r;
+  thread_local int dev = -1, slots = 0;  // per channel count and host thread
   int grid;
-  if (int r = persistent_grid(tex_bwd_kernel<C>, tex_bwd_smem(C), A.n, grid)) return r;
+  if (int r = persistent_grid(tex_bwd_kernel<C>, tex_bwd_smem(C), A.n, dev, slots, grid)) return r;
   // timed apart: the MLP adjoint (weight-gradient GEMMs) and the scatter of
   // the encoding gradients into the table and the positions
   DMGS_TIMED(K_TEX_BWD, s, dmgs_host::note_launch(), tex_bwd_kernel<C><<<grid, TEX_THREADS, tex_bwd_smem(C), s>>>(
