@@ -5,6 +5,10 @@ them into ``dmgs_gb300/libdmgs_gb300.so`` (in-tree, git-ignored); beside them
 the host compiler builds ``csrc/autograd.cpp``, the native autograd nodes, into
 ``dmgs_gb300/_autograd.so``.  Objects go to ``dmgs_gb300/_build/``.  Rebuilds
 only what changed.
+
+The library needs nvcc alone and is linked whatever becomes of the extension.
+The extension needs the headers of a CUDA torch; without one it is not built,
+and a program that uses the library through its C interface does not miss it.
 """
 from __future__ import annotations
 
@@ -45,8 +49,14 @@ def _headers():
 
 
 def _ext_commands():
-    """(compile, link) commands of the autograd extension, its object."""
-    import torch
+    """(compile command, link command, object) of the autograd extension; None
+    without a CUDA torch."""
+    try:
+        import torch
+    except ImportError:
+        return None
+    if torch.version.cuda is None:
+        return None
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     obj = os.path.join(BUILD, "autograd.cpp.o")
@@ -82,39 +92,46 @@ def build(verbose: bool = False, force: bool = False, extra_flags=()) -> str:
             cmd = [nvcc, *NVCC_FLAGS, *extra_flags, "-I", INCLUDE, "-c", src, "-o", obj]
             jobs.append(cmd)
 
-    ext_src = os.path.join(CSRC, "autograd.cpp")
-    ext_compile, ext_link, ext_obj = _ext_commands()
-    ext_stale = force or _stale(ext_obj, [ext_src, os.path.join(INCLUDE, "dmgs.h"), __file__])
-    if ext_stale:
-        jobs.insert(0, ext_compile)
+    ext = _ext_commands()
+    ext_stale = False
+    if ext is None:
+        sys.stderr.write("no torch with CUDA: _autograd.so is not built\n")
+    else:
+        comp, link, ext_obj = ext
+        ext_src = os.path.join(CSRC, "autograd.cpp")
+        ext_stale = (force or _stale(ext_obj, [ext_src, os.path.join(INCLUDE, "dmgs.h"), __file__])
+                     or not os.path.exists(EXT))
+        if ext_stale:
+            jobs.insert(0, comp)
 
     def run(cmd):
         r = subprocess.run(cmd, capture_output=True, text=True)
-        return cmd, r
+        if verbose or r.returncode != 0:
+            sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+        return r.returncode == 0
 
+    ext_failed = False
     if jobs:
         with cf.ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as ex:
-            for cmd, r in ex.map(run, jobs):
-                if verbose or r.returncode != 0:
-                    sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
-                if r.returncode != 0:
+            for cmd, ok in zip(jobs, ex.map(run, jobs)):
+                if ok:
+                    continue
+                if ext_stale and cmd is comp:
+                    ext_failed = True
+                else:
                     raise RuntimeError(f"{os.path.basename(cmd[0])} failed for {cmd[-3]}")
     if force or jobs or _stale(LIB, objs):
         tmp = LIB + ".tmp"
         cmd = [nvcc, *ARCH, "-shared", "-cudart", "shared", "-o", tmp, *objs,
                "-Xlinker", "-rpath,/usr/local/cuda/lib64"]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if verbose or r.returncode != 0:
-            sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
-        if r.returncode != 0:
+        if not run(cmd):
             raise RuntimeError("link of libdmgs_gb300.so failed")
         os.replace(tmp, LIB)
-    if ext_stale or _stale(EXT, [ext_obj]):
-        r = subprocess.run(ext_link, capture_output=True, text=True)
-        if verbose or r.returncode != 0:
-            sys.stderr.write(" ".join(ext_link) + "\n" + r.stdout + r.stderr)
-        if r.returncode != 0:
-            raise RuntimeError("link of _autograd.so failed")
+    if ext_stale:
+        if ext_failed:
+            raise RuntimeError(f"{os.path.basename(comp[0])} failed for {comp[-3]} (libdmgs_gb300.so is built)")
+        if not run(link):
+            raise RuntimeError("link of _autograd.so failed (libdmgs_gb300.so is built)")
         os.replace(EXT + ".tmp", EXT)
     return LIB
 

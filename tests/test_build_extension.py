@@ -1,0 +1,53 @@
+"""The build of the library and of the autograd extension beside it (a small
+source tree; a stand-in compiler for the extension)."""
+import os
+import stat
+import sys
+
+import pytest
+import torch
+
+from dmgs_gb300 import build as B
+
+
+@pytest.fixture
+def tree(tmp_path, monkeypatch):
+    """build.py on a tree of one kernel source, the extension's compiler a
+    script that writes its output and counts its calls."""
+    csrc = tmp_path / "csrc"
+    csrc.mkdir()
+    (csrc / "one.cu").write_text('extern "C" int one() { return 1; }\n')
+    (csrc / "autograd.cpp").write_text("// stands for the nodes\n")
+    cxx = tmp_path / "cxx"
+    cxx.write_text("#!/bin/sh\n"
+                   f"echo x >> {tmp_path}/calls\n"
+                   f"[ -e {tmp_path}/broken ] && exit 1\n"
+                   "while [ $# -gt 0 ]; do [ \"$1\" = -o ] && echo x > \"$2\"; shift; done\n")
+    cxx.chmod(cxx.stat().st_mode | stat.S_IXUSR)
+    monkeypatch.setenv("CXX", str(cxx))
+    for name, path in (("CSRC", csrc), ("BUILD", tmp_path / "_build"), ("LIB", tmp_path / "lib.so"), ("EXT", tmp_path / "ext.so")):
+        monkeypatch.setattr(B, name, str(path))
+    monkeypatch.calls = lambda: len((tmp_path / "calls").read_text().split()) if (tmp_path / "calls").exists() else 0
+    return tmp_path, monkeypatch
+
+
+def test_the_library_does_not_wait_for_the_extension(tree):
+    path, patch = tree
+    (path / "broken").write_text("")
+    with pytest.raises(RuntimeError):
+        B.build()
+    assert os.path.exists(B.LIB) and not os.path.exists(B.EXT)
+    os.remove(path / "broken")
+    B.build()
+    assert os.path.exists(B.EXT)
+
+
+@pytest.mark.parametrize("torch_is", ["missing", "without CUDA"])
+def test_the_library_without_a_cuda_torch(tree, torch_is):
+    path, patch = tree
+    if torch_is == "missing":
+        patch.setitem(sys.modules, "torch", None)
+    else:
+        patch.setattr(torch.version, "cuda", None)
+    assert B.build() == B.LIB
+    assert os.path.exists(B.LIB) and patch.calls() == 0
