@@ -7,8 +7,10 @@ the host compiler builds ``csrc/autograd.cpp``, the native autograd nodes, into
 only what changed.
 
 The library needs nvcc alone and is linked whatever becomes of the extension.
-The extension needs the headers of a CUDA torch; without one it is not built,
-and a program that uses the library through its C interface does not miss it.
+The extension needs the headers of a CUDA torch and is tied to the torch and
+Python it was built with (recorded in ``_build/autograd.tag``); without a CUDA
+torch it is not built, and a program that uses the library through its C
+interface does not miss it.
 """
 from __future__ import annotations
 
@@ -24,6 +26,7 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libdmgs_gb300.so")
 EXT = os.path.join(HERE, "_autograd.so")
+TAG = os.path.join(BUILD, "autograd.tag")  # what EXT was built with
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
@@ -49,7 +52,8 @@ def _headers():
 
 
 def _ext_commands():
-    """(compile command, link command, object) of the autograd extension; None
+    """(compile command, link command, object, tag) of the autograd extension,
+    the tag naming all that its build depends on besides the sources; None
     without a CUDA torch."""
     try:
         import torch
@@ -68,7 +72,7 @@ def _ext_commands():
             *[a for i in inc for a in ("-isystem", i)], "-c", os.path.join(CSRC, "autograd.cpp"), "-o", obj]
     link = [cxx, "-shared", "-o", EXT + ".tmp", obj, "-L", os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu",
             "-ltorch_python", "-lc10", "-lc10_cuda", "-L", HERE, "-l:libdmgs_gb300.so", "-Wl,-rpath,$ORIGIN"]
-    return comp, link, obj
+    return comp, link, obj, "\n".join([torch.__version__, sys.version, *comp, *link])
 
 
 def _stale(target: str, deps) -> bool:
@@ -76,6 +80,14 @@ def _stale(target: str, deps) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _read(path: str):
+    try:
+        with open(path) as f:
+            return f.read()
+    except OSError:
+        return None
 
 
 def build(verbose: bool = False, force: bool = False, extra_flags=()) -> str:
@@ -97,10 +109,10 @@ def build(verbose: bool = False, force: bool = False, extra_flags=()) -> str:
     if ext is None:
         sys.stderr.write("no torch with CUDA: _autograd.so is not built\n")
     else:
-        comp, link, ext_obj = ext
+        comp, link, ext_obj, tag = ext
         ext_src = os.path.join(CSRC, "autograd.cpp")
         ext_stale = (force or _stale(ext_obj, [ext_src, os.path.join(INCLUDE, "dmgs.h"), __file__])
-                     or not os.path.exists(EXT))
+                     or not os.path.exists(EXT) or _read(TAG) != tag)
         if ext_stale:
             jobs.insert(0, comp)
 
@@ -133,6 +145,8 @@ def build(verbose: bool = False, force: bool = False, extra_flags=()) -> str:
         if not run(link):
             raise RuntimeError("link of _autograd.so failed (libdmgs_gb300.so is built)")
         os.replace(EXT + ".tmp", EXT)
+        with open(TAG, "w") as f:
+            f.write(tag)
     return LIB
 
 

@@ -25,7 +25,8 @@ def tree(tmp_path, monkeypatch):
                    "while [ $# -gt 0 ]; do [ \"$1\" = -o ] && echo x > \"$2\"; shift; done\n")
     cxx.chmod(cxx.stat().st_mode | stat.S_IXUSR)
     monkeypatch.setenv("CXX", str(cxx))
-    for name, path in (("CSRC", csrc), ("BUILD", tmp_path / "_build"), ("LIB", tmp_path / "lib.so"), ("EXT", tmp_path / "ext.so")):
+    for name, path in (("CSRC", csrc), ("BUILD", tmp_path / "_build"), ("LIB", tmp_path / "lib.so"), ("EXT", tmp_path / "ext.so"),
+                       ("TAG", tmp_path / "_build" / "autograd.tag")):
         monkeypatch.setattr(B, name, str(path))
     monkeypatch.calls = lambda: len((tmp_path / "calls").read_text().split()) if (tmp_path / "calls").exists() else 0
     return tmp_path, monkeypatch
@@ -51,3 +52,17 @@ def test_the_library_without_a_cuda_torch(tree, torch_is):
         patch.setattr(torch.version, "cuda", None)
     assert B.build() == B.LIB
     assert os.path.exists(B.LIB) and patch.calls() == 0
+
+
+def test_the_extension_follows_the_torch_it_is_built_with(tree):
+    path, patch = tree
+    B.build()
+    n = patch.calls()
+    assert n == 2  # compiled and linked
+    B.build()
+    assert patch.calls() == n
+    patch.setattr(torch, "__version__", "0.0.1")
+    B.build()
+    assert patch.calls() == 2 * n
+    B.build()
+    assert patch.calls() == 2 * n
