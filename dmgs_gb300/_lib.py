@@ -157,12 +157,13 @@ SIGNATURES = [
 ]
 
 _lib = None
+_loaded = None  # its path
 _lock = threading.Lock()
 
 
 def load(path: str | None = None):
     """Load the library (once) and declare every signature."""
-    global _lib
+    global _lib, _loaded
     with _lock:
         if _lib is not None:
             return _lib
@@ -179,7 +180,7 @@ def load(path: str | None = None):
         if lib.dmgs_abi_version() != ABI_VERSION:
             raise RuntimeError(f"{p} has ABI version {lib.dmgs_abi_version()}, this package expects "
                                f"{ABI_VERSION}: rebuild it with `python -m dmgs_gb300.build`")
-        _lib = lib
+        _lib, _loaded = lib, p
         return lib
 
 
@@ -189,9 +190,13 @@ _native = None
 def native():
     """The extension with the native autograd nodes (csrc/autograd.cpp).  On a
     machine with a GPU it must be there; without one its entries would refuse
-    every call, so a package that was not built has None."""
+    every call, so a package that was not built has None.  It is linked with
+    the in-tree library: a program that loaded another one has None too, so
+    that all its calls, error texts and counters are that library's."""
     global _native
     if _native is None:
+        if _loaded is not None and not (os.path.exists(LIB_PATH) and os.path.samefile(_loaded, LIB_PATH)):
+            return None
         if not os.path.exists(os.path.join(_HERE, "_autograd.so")) and not torch.cuda.is_available():
             return None
         load()

@@ -1,7 +1,10 @@
 """The build of the library and of the autograd extension beside it (a small
-source tree; a stand-in compiler for the extension)."""
+source tree; a stand-in compiler for the extension), and which library the
+extension goes with."""
 import os
+import shutil
 import stat
+import subprocess
 import sys
 
 import pytest
@@ -66,3 +69,16 @@ def test_the_extension_follows_the_torch_it_is_built_with(tree):
     assert patch.calls() == 2 * n
     B.build()
     assert patch.calls() == 2 * n
+
+
+def test_the_extension_goes_with_the_in_tree_library(tmp_path):
+    """A program that loaded another library runs the general forms on it."""
+    B.build()
+    other = tmp_path / "libother.so"
+    shutil.copy(B.LIB, other)
+    code = ("import sys; sys.path.insert(0, sys.argv[2]); from dmgs_gb300 import _lib; _lib.load(sys.argv[1] or None); "
+            "print(_lib.native() is not None, _lib.native_call('l1_ssim', None, None, 0.2))")
+    for path, want in ((str(other), "False None"), (B.LIB, "True None"), ("", "True None")):
+        r = subprocess.run([sys.executable, "-c", code, path, os.path.dirname(B.HERE)], capture_output=True, text=True)
+        assert r.returncode == 0, r.stderr
+        assert r.stdout.strip() == want
