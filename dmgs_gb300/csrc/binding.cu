@@ -10,9 +10,13 @@
 // us forward and 195 us adjoint, against 82 and 150; floors 39 and 35).
 // Rows now pass through shared memory, a warp's accesses consecutive.
 // A thread per face walks its Gaussians in order, 64 faces a block, on the
-// block's staged rows.  (A thread per Gaussian, with the faces formed by the
-// block's first 128 / G threads: three warps in four waited at the barriers,
-// 90 and 240 us.)
+// block's staged rows.  Where fewer faces fit, the stage-3 kernels, whose
+// arithmetic is per Gaussian, share a face's Gaussians among the threads left
+// over (2M Gaussians, both directions, at 24 | 64 | 128 | 512 per face: 404 |
+// 405 | 807 | 3307 us with a thread per face on global rows, 273 | 581 | 1019 |
+// 2632 us with one on staged rows, 125 | 141 | 139 | 199 us so).  (A thread
+// per Gaussian, with the faces formed by the block's first 128 / G threads:
+// three warps in four waited at the barriers, 90 and 240 us.)
 //
 // Stage-3 form: scene/gaussian_geo_model_finetune.py:396-421 (renew_gaussian)
 // and :446-483 (get_scaling / get_rotation / get_rot_matrix).  The rotation
@@ -36,6 +40,9 @@ __device__ __forceinline__ f3 operator*(float s, f3 a) { return {s * a.x, s * a.
 __device__ __forceinline__ float dot(f3 a, f3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ f3 cross(f3 a, f3 b) {
   return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+}
+__device__ __forceinline__ f3 shfl_xor(f3 a, int o) {
+  return {__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o), __shfl_xor_sync(0xffffffffu, a.z, o)};
 }
 __device__ __forceinline__ float norm(f3 a) { return sqrtf(dot(a, a)); }
 
@@ -119,9 +126,11 @@ __device__ __forceinline__ float bc_at(const DmgsFaceBinding &b, int f, int g, i
 constexpr int BB = 64;  // threads, and faces per block
 
 // Rows of a block: the faces it takes and the Gaussians of each that
-// its shared memory holds at a time (all of them, or, with one face, a part).
+// its shared memory holds at a time (all of them, or, with one face, a part),
+// and the threads that share a face's Gaussians (stage 3: a power of two, lanes
+// of one warp).
 struct FaceBlocks {
-  int faces, chunk, blocks;
+  int faces, chunk, blocks, share;
   size_t smem;
 };
 
@@ -131,6 +140,8 @@ FaceBlocks face_blocks(int F, int G, int words) {
   k.faces = std::max(1, std::min(BB, fit / G));
   k.chunk = std::min(G, fit);
   k.blocks = (F + k.faces - 1) / k.faces;
+  k.share = 1;
+  while (2 * k.share * k.faces <= BB && k.share < 32) k.share *= 2;
   k.smem = (size_t)k.faces * k.chunk * words * 4 + 5 * 16;  // each array padded to 16 bytes
   return k;
 }
@@ -429,7 +440,9 @@ __global__ void __launch_bounds__(BB, 10)
 bind3_fwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, float *__restrict__ xyz,
                  float *__restrict__ scales, float *__restrict__ rots) {
   extern __shared__ __align__(16) float bind_smem[];
-  const int t = threadIdx.x, f0 = blockIdx.x * kb.faces, nf = min(kb.faces, b.F - f0), cap = kb.faces * kb.chunk;
+  // thread t: face t / share of the block, its Gaussians sub, sub + share, ...
+  const int t = threadIdx.x / kb.share, sub = threadIdx.x % kb.share;
+  const int f0 = blockIdx.x * kb.faces, nf = min(kb.faces, b.F - f0), cap = kb.faces * kb.chunk;
   float *p = bind_smem;
   float *sq = take(p, 4 * cap), *sx = take(p, 3 * cap), *ss = take(p, 3 * cap), *s2 = take(p, 2 * cap), *r2 = take(p, 2 * cap);
   Tri T;
@@ -451,7 +464,7 @@ bind3_fwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, float *__restrict__ xyz,
     }
     const bool all_good = __syncthreads_and(good);
     if (good && t < nf) {
-      for (int g = 0; g < gn; ++g) {
+      for (int g = sub; g < gn; g += kb.share) {
         const int q = t * gn + g;
         const float *w = b.bc + 3 * (gs + g);
         const float w0 = w[0], w1 = w[1], w2 = w[2];
@@ -505,7 +518,9 @@ bind3_bwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, const float *__restrict__ dx
                  const float *__restrict__ dscales, const float *__restrict__ drots,
                  float *__restrict__ dverts, float *__restrict__ dscaling, float *__restrict__ drot2d) {
   extern __shared__ __align__(16) float bind_smem[];
-  const int t = threadIdx.x, f0 = blockIdx.x * kb.faces, nf = min(kb.faces, b.F - f0), cap = kb.faces * kb.chunk;
+  // thread t: face t / share of the block, its Gaussians sub, sub + share, ...
+  const int t = threadIdx.x / kb.share, sub = threadIdx.x % kb.share;
+  const int f0 = blockIdx.x * kb.faces, nf = min(kb.faces, b.F - f0), cap = kb.faces * kb.chunk;
   float *p = bind_smem;
   float *sq = take(p, 4 * cap), *sx = take(p, 3 * cap), *ss = take(p, 3 * cap), *s2 = take(p, 2 * cap), *r2 = take(p, 2 * cap);
   Tri T;
@@ -536,7 +551,7 @@ bind3_bwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, const float *__restrict__ dx
     }
     const bool all_good = __syncthreads_and(good);
     if (good && t < nf) {
-      for (int g = 0; g < gn; ++g) {
+      for (int g = sub; g < gn; g += kb.share) {
         const int q = t * gn + g;
         if (dxyz) {
           const float *w = b.bc + 3 * (gs + g);
@@ -602,7 +617,13 @@ bind3_bwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, const float *__restrict__ dx
       __syncthreads();
     }
   }
-  if (good && t < nf) {
+  // the face's sums over its threads
+  for (int o = kb.share / 2; o > 0; o >>= 1) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) dRw[i] += __shfl_xor_sync(0xffffffffu, dRw[i], o);
+    g0 = g0 + shfl_xor(g0, o); g1 = g1 + shfl_xor(g1, o); g2 = g2 + shfl_xor(g2, o);
+  }
+  if (good && t < nf && sub == 0) {
     if (drots) {
       const Frame F = face_frame(T.v0, T.v1, T.v2);
       f3 h0, h1, h2;
