@@ -436,7 +436,17 @@ __device__ __forceinline__ void mat_to_quat_adj(const float *R, const QuatOut &o
   dR[3] = e03 + e12; dR[1] = e12 - e03;
 }
 
-__global__ void __launch_bounds__(BB, 10)
+// STAGED: the rows through shared memory, as above.  With up to three Gaussians
+// per face a thread's rows in global memory are short enough for neighbouring
+// lanes to share their sectors, and more blocks an SM count for more: 2M
+// Gaussians, both directions, staged | direct, 264 | 156 us at one per face,
+// 178 | 119 at two, 143 | 133 at three, 138 | 152 at four; 60,000: 20.5 | 18.5,
+// 21.3 | 18.5, 24.6 | 22.6, 23.6 | 23.6.  Blocks an SM of the direct form, at
+// one per face: 189 | 174 | 154 | 162 us at 10 | 12 | 16 | 20.
+constexpr int DIRECT_MAX = 3;
+
+template <bool STAGED>
+__global__ void __launch_bounds__(BB, STAGED ? 10 : 16)
 bind3_fwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, float *__restrict__ xyz,
                  float *__restrict__ scales, float *__restrict__ rots) {
   extern __shared__ __align__(16) float bind_smem[];
@@ -451,8 +461,11 @@ bind3_fwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, float *__restrict__ xyz,
   for (int gs = 0; gs < b.G; gs += kb.chunk) {  // once, unless one face's rows do not fit
     const int gn = min(kb.chunk, b.G - gs), m = nf * gn;
     const size_t o0 = (size_t)f0 * b.G + gs;
-    if (scales) rows_in(b.scaling2d + 2 * o0, 2 * m, s2);
-    if (rots) rows_in(b.rotation2d + 2 * o0, 2 * m, r2);
+    const float *in_s2 = STAGED ? s2 : b.scaling2d + 2 * o0, *in_r2 = STAGED ? r2 : b.rotation2d + 2 * o0;
+    if (STAGED) {
+      if (scales) rows_in(b.scaling2d + 2 * o0, 2 * m, s2);
+      if (rots) rows_in(b.rotation2d + 2 * o0, 2 * m, r2);
+    }
     if (gs == 0 && t < nf) {
       good = load_tri(b.faces, b.verts, b.V, f0 + t, T);
       if (good) {
@@ -462,7 +475,7 @@ bind3_fwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, float *__restrict__ xyz,
         for (int i = 0; i < 9; ++i) Rw[i] = R[i];
       }
     }
-    const bool all_good = __syncthreads_and(good);
+    const bool all_good = STAGED && __syncthreads_and(good);
     if (good && t < nf) {
       for (int g = sub; g < gn; g += kb.share) {
         const int q = t * gn + g;
@@ -472,12 +485,12 @@ bind3_fwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, float *__restrict__ xyz,
         const float z = w0 * T.v0.z + w1 * T.v1.z + w2 * T.v2.z;
         float e0 = 0.f, e1 = 0.f;
         if (scales) {
-          e0 = expf(s2[2 * q]);
-          e1 = expf(s2[2 * q + 1]);
+          e0 = expf(in_s2[2 * q]);
+          e1 = expf(in_s2[2 * q + 1]);
         }
         float4 quat = make_float4(0.f, 0.f, 0.f, 0.f);
         if (rots) {
-          const float ra = r2[2 * q], rb = r2[2 * q + 1];
+          const float ra = in_r2[2 * q], rb = in_r2[2 * q + 1];
           const float cn = inv_norm(ra * ra + rb * rb);
           const float a = ra * cn, s = rb * cn;
           // R = Rw * [[a,-s,0],[s,a,0],[0,0,1]]
@@ -503,7 +516,7 @@ bind3_fwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, float *__restrict__ xyz,
         }
       }
     }
-    __syncthreads();
+    if (STAGED) __syncthreads();
     if (all_good) {
       if (xyz) rows_out(xyz + 3 * o0, 3 * m, sx);
       if (scales) rows_out(scales + 3 * o0, 3 * m, ss);
@@ -513,7 +526,8 @@ bind3_fwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, float *__restrict__ xyz,
   }
 }
 
-__global__ void __launch_bounds__(BB, 10)
+template <bool STAGED>
+__global__ void __launch_bounds__(BB, STAGED ? 10 : 16)
 bind3_bwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, const float *__restrict__ dxyz,
                  const float *__restrict__ dscales, const float *__restrict__ drots,
                  float *__restrict__ dverts, float *__restrict__ dscaling, float *__restrict__ drot2d) {
@@ -531,14 +545,18 @@ bind3_bwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, const float *__restrict__ dx
   for (int gs = 0; gs < b.G; gs += kb.chunk) {  // once, unless one face's rows do not fit
     const int gn = min(kb.chunk, b.G - gs), m = nf * gn;
     const size_t o0 = (size_t)f0 * b.G + gs;
-    if (dxyz) rows_in(dxyz + 3 * o0, 3 * m, sx);
-    if (dscales && dscaling) {
-      rows_in(dscales + 3 * o0, 3 * m, ss);
-      rows_in(b.scaling2d + 2 * o0, 2 * m, s2);
-    }
-    if (drots) {
-      rows_in(drots + 4 * o0, 4 * m, sq);
-      rows_in(b.rotation2d + 2 * o0, 2 * m, r2);
+    const float *in_x = STAGED ? sx : dxyz + 3 * o0, *in_s = STAGED ? ss : dscales + 3 * o0, *in_q = STAGED ? sq : drots + 4 * o0;
+    const float *in_s2 = STAGED ? s2 : b.scaling2d + 2 * o0, *in_r2 = STAGED ? r2 : b.rotation2d + 2 * o0;
+    if (STAGED) {
+      if (dxyz) rows_in(dxyz + 3 * o0, 3 * m, sx);
+      if (dscales && dscaling) {
+        rows_in(dscales + 3 * o0, 3 * m, ss);
+        rows_in(b.scaling2d + 2 * o0, 2 * m, s2);
+      }
+      if (drots) {
+        rows_in(drots + 4 * o0, 4 * m, sq);
+        rows_in(b.rotation2d + 2 * o0, 2 * m, r2);
+      }
     }
     if (gs == 0 && t < nf) {
       good = load_tri(b.faces, b.verts, b.V, f0 + t, T);
@@ -549,24 +567,24 @@ bind3_bwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, const float *__restrict__ dx
         for (int i = 0; i < 9; ++i) Rw[i] = R[i];
       }
     }
-    const bool all_good = __syncthreads_and(good);
+    const bool all_good = STAGED && __syncthreads_and(good);
     if (good && t < nf) {
       for (int g = sub; g < gn; g += kb.share) {
         const int q = t * gn + g;
         if (dxyz) {
           const float *w = b.bc + 3 * (gs + g);
-          const f3 d = mk(sx[3 * q], sx[3 * q + 1], sx[3 * q + 2]);
+          const f3 d = mk(in_x[3 * q], in_x[3 * q + 1], in_x[3 * q + 2]);
           g0 = g0 + w[0] * d;
           g1 = g1 + w[1] * d;
           g2 = g2 + w[2] * d;
         }
         float ds0 = 0.f, ds1 = 0.f, dra = 0.f, drb = 0.f;
         if (dscales && dscaling) {
-          ds0 = ss[3 * q] * expf(s2[2 * q]);
-          ds1 = ss[3 * q + 1] * expf(s2[2 * q + 1]);
+          ds0 = in_s[3 * q] * expf(in_s2[2 * q]);
+          ds1 = in_s[3 * q + 1] * expf(in_s2[2 * q + 1]);
         }
         if (drots) {
-          const float ra = r2[2 * q], rb = r2[2 * q + 1];
+          const float ra = in_r2[2 * q], rb = in_r2[2 * q + 1];
           const float cn = inv_norm(ra * ra + rb * rb);
           const float a = ra * cn, s = rb * cn;
           float R[9];
@@ -577,8 +595,14 @@ bind3_bwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, const float *__restrict__ dx
             R[i * 3 + 2] = Rw[i * 3 + 2];
           }
           const QuatOut qq = mat_to_quat(R);
-          const float4 v = reinterpret_cast<const float4 *>(sq)[q];
-          const float dq[4] = {v.x, v.y, v.z, v.w};
+          float dq[4];
+          if (STAGED) {
+            const float4 v = reinterpret_cast<const float4 *>(sq)[q];
+            dq[0] = v.x; dq[1] = v.y; dq[2] = v.z; dq[3] = v.w;
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dq[i] = in_q[4 * q + i];
+          }
           float dR[9];
           mat_to_quat_adj(R, qq, dq, dR);
           float da = 0.f, ds = 0.f;
@@ -610,7 +634,7 @@ bind3_bwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, const float *__restrict__ dx
         }
       }
     }
-    __syncthreads();
+    if (STAGED) __syncthreads();
     if (all_good) {
       if (dscaling) rows_out(dscaling + 2 * o0, 2 * m, s2);
       if (drot2d) rows_out(drot2d + 2 * o0, 2 * m, r2);
@@ -660,8 +684,9 @@ int launch_bind_bwd(const DmgsFaceBinding &b, const float *dxyz, const float *dc
 int launch_bind3_fwd(const DmgsFaceBinding3 &b, float *xyz, float *scales, float *rots,
                      cudaStream_t s) {
   if (b.F <= 0) return DMGS_OK;
-  const FaceBlocks kb = face_blocks(b.F, b.G, 14);
-  DMGS_TIMED(K_BIND3_FWD, s, dmgs_host::note_launch(), bind3_fwd_kernel<<<kb.blocks, BB, kb.smem, s>>>(b, kb, xyz, scales, rots));
+  const bool staged = b.G > DIRECT_MAX;
+  const FaceBlocks kb = staged ? face_blocks(b.F, b.G, 14) : FaceBlocks{BB, b.G, (b.F - 1) / BB + 1, 1, 0};
+  DMGS_TIMED(K_BIND3_FWD, s, dmgs_host::note_launch(), (staged ? bind3_fwd_kernel<true> : bind3_fwd_kernel<false>)<<<kb.blocks, BB, kb.smem, s>>>(b, kb, xyz, scales, rots));
   DMGS_LAUNCH_CHECK("bind3_fwd_kernel");
   return DMGS_OK;
 }
@@ -671,8 +696,9 @@ int launch_bind3_bwd(const DmgsFaceBinding3 &b, const float *dxyz, const float *
                      cudaStream_t s) {
   DMGS_CUDA(cudaMemsetAsync(dverts, 0, (size_t)b.V * 3 * 4, s));
   if (b.F <= 0) return DMGS_OK;
-  const FaceBlocks kb = face_blocks(b.F, b.G, 14);
-  DMGS_TIMED(K_BIND3_BWD, s, dmgs_host::note_launch(), bind3_bwd_kernel<<<kb.blocks, BB, kb.smem, s>>>(b, kb, dxyz, dscales, drots, dverts, dscaling,
+  const bool staged = b.G > DIRECT_MAX;
+  const FaceBlocks kb = staged ? face_blocks(b.F, b.G, 14) : FaceBlocks{BB, b.G, (b.F - 1) / BB + 1, 1, 0};
+  DMGS_TIMED(K_BIND3_BWD, s, dmgs_host::note_launch(), (staged ? bind3_bwd_kernel<true> : bind3_bwd_kernel<false>)<<<kb.blocks, BB, kb.smem, s>>>(b, kb, dxyz, dscales, drots, dverts, dscaling,
                                                      drot2d));
   DMGS_LAUNCH_CHECK("bind3_bwd_kernel");
   return DMGS_OK;

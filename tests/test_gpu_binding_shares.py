@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 # 402 Gaussians' rows fit a block: faces per block, and threads per face, at 12 | 13 | 25 | 26 | 51 | ... per face
 @pytest.mark.parametrize("G,F", [(12, 70), (13, 61), (25, 33), (26, 31), (50, 17), (51, 15), (100, 9), (101, 7), (201, 5), (202, 3),
-                                 (402, 2), (403, 3), (1000, 2), (1, 1), (1, 257), (2, 130)])
+                                 (402, 2), (403, 3), (1000, 2), (1, 1), (1, 257), (2, 130), (3, 65), (3, 128), (4, 63)])
 @pytest.mark.parametrize("off", [0, 1])
 @pytest.mark.parametrize("bad", [False, True])
 def test_stage3_at_every_share(G, F, off, bad):
