@@ -23,7 +23,8 @@
 // loads per quantity instead of 11 (one output per thread and products kept
 // in shared memory: 178 us for both kernels at 3 x 822 x 1237, against 81).
 // 54 rows + 10 of halo are 64 rows of 8 groups of 4 columns (two rounds of
-// the 256 threads) and 8 groups of 7 rows of 32 columns (one round).
+// the 256 threads) and 8 groups of 7 rows of 32 columns (one round); an image
+// with few such tiles takes tiles of 16 rows, two vertical outputs a thread.
 //
 // With s11 = E[x^2] - mu_x^2, s22 = E[y^2] - mu_y^2, s12 = E[xy] - mu_x mu_y,
 // N1 = 2 mu_x mu_y + C1, N2 = 2 s12 + C2, D1 = mu_x^2 + mu_y^2 + C1,
@@ -40,13 +41,18 @@ namespace {
 
 constexpr int LR = 5;              // window radius
 constexpr int LTAP = 2 * LR + 1;
-constexpr int LW = 32, LHT = 54;   // output tile: columns, rows
-constexpr int LROWS = LHT + 2 * LR;  // 64 rows with the halo
+constexpr int LW = 32;             // columns of an output tile
 constexpr int LP = 44;             // pitch of a haloed row (42 columns; rows 16-byte aligned)
 constexpr int LN = 256;            // threads
-constexpr int LV = 7;              // vertical outputs per thread
-constexpr int LHS = LV * (LN / LW) + 2 * LR;  // rows the vertical pass reads (the last two of no output)
-static_assert(LROWS * (LW / 4) == 2 * LN && LW * ((LHT + LV - 1) / LV) == LN, "tile and block sizes");
+
+// A tile whose threads form LV vertical outputs each.
+template <int LV>
+struct Tile {
+  static constexpr int LHT = LV == 7 ? 54 : LV * (LN / LW);  // output rows
+  static constexpr int LROWS = LHT + 2 * LR;                 // rows with the halo
+  static constexpr int LHS = LV * (LN / LW) + 2 * LR;        // rows the vertical pass reads (of 7: the last two of no output)
+};
+static_assert(Tile<7>::LROWS * (LW / 4) == 2 * LN && LW * ((Tile<7>::LHT + 6) / 7) == LN, "tile and block sizes");
 
 struct Window {
   float w[LTAP];
@@ -55,7 +61,7 @@ struct Window {
 // One or two images' haloed tile into shared memory, zero outside the image:
 // a warp per row (columns lane and lane + 32), rows LN / 32 apart, so that a
 // row's bounds are the warp's and no index is divided.
-template <int NQ>
+template <int LROWS, int NQ>
 __device__ __forceinline__ void load_tile(const float *__restrict__ a, const float *__restrict__ b, int H, int Wd,
                                           int ox, int oy, float (*da)[LP], float (*db)[LP]) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -105,6 +111,7 @@ __device__ __forceinline__ float4 blur4(const Window &W, const float (&v)[16]) {
 }
 
 // The thread's LV vertical outputs of a quantity (column c, rows LV gv ..).
+template <int LV>
 __device__ __forceinline__ void blur_column(const Window &W, const float (*hs)[LW], int c, int gv, float (&o)[LV]) {
   float v[LV + 2 * LR];
 #pragma unroll
@@ -133,29 +140,33 @@ __device__ __forceinline__ float block_sum(float v, float *red) {
   return s;  // valid in thread 0
 }
 
+template <int LV>
 struct MomentsSmem {
-  float x[LROWS][LP], y[LROWS][LP];
-  float hs[5][LHS][LW];
+  float x[Tile<LV>::LROWS][LP], y[Tile<LV>::LROWS][LP];
+  float hs[5][Tile<LV>::LHS][LW];
   float red[LN / 32];
 };
 
+template <int LV>
 struct GradSmem {
-  float in[LROWS][LP];
-  float hs[3][LHS][LW];
+  float in[Tile<LV>::LROWS][LP];
+  float hs[3][Tile<LV>::LHS][LW];
   float red[LN / 32];
 };
 
 // Grid: (tiles x, tiles y, channels).  ABD: [3][C][H][W] scratch;
 // part: 2 floats per block (sum S, sum |x - y|).
+template <int LV>
 __global__ void __launch_bounds__(LN)
 ssim_moments_kernel(const float *__restrict__ x, const float *__restrict__ y, int H, int Wd,
                     Window W, float *__restrict__ ABD, float *__restrict__ part) {
   extern __shared__ __align__(16) char loss_smem[];
-  MomentsSmem &sm = *reinterpret_cast<MomentsSmem *>(loss_smem);
+  constexpr int LHT = Tile<LV>::LHT, LROWS = Tile<LV>::LROWS;
+  MomentsSmem<LV> &sm = *reinterpret_cast<MomentsSmem<LV> *>(loss_smem);
   const int c = blockIdx.z, t = threadIdx.x;
   const size_t plane = (size_t)H * Wd;
   const int ox = blockIdx.x * LW, oy = blockIdx.y * LHT;
-  load_tile<2>(x + c * plane, y + c * plane, H, Wd, ox - LR, oy - LR, sm.x, sm.y);
+  load_tile<LROWS, 2>(x + c * plane, y + c * plane, H, Wd, ox - LR, oy - LR, sm.x, sm.y);
   __syncthreads();
 #pragma unroll 1
   for (int i = t; i < LROWS * (LW / 4); i += LN) {
@@ -180,7 +191,7 @@ ssim_moments_kernel(const float *__restrict__ x, const float *__restrict__ y, in
   const int col = t & (LW - 1), gv = t / LW;
   float m[5][LV];
 #pragma unroll
-  for (int q = 0; q < 5; ++q) blur_column(W, sm.hs[q], col, gv, m[q]);
+  for (int q = 0; q < 5; ++q) blur_column<LV>(W, sm.hs[q], col, gv, m[q]);
   float S_sum = 0.f, l1 = 0.f;
   const int px = ox + col;
 #pragma unroll
@@ -217,20 +228,22 @@ ssim_moments_kernel(const float *__restrict__ x, const float *__restrict__ y, in
   }
 }
 
+template <int LV>
 __global__ void __launch_bounds__(LN)
 ssim_grad_kernel(const float *__restrict__ x, const float *__restrict__ y, int H, int Wd,
                  Window W, const float *__restrict__ ABD, float lambda, float inv_n,
                  float *__restrict__ grad, const float *__restrict__ part, int nparts,
                  float *__restrict__ loss) {
   extern __shared__ __align__(16) char loss_smem[];
-  GradSmem &sm = *reinterpret_cast<GradSmem *>(loss_smem);
+  constexpr int LHT = Tile<LV>::LHT, LROWS = Tile<LV>::LROWS;
+  GradSmem<LV> &sm = *reinterpret_cast<GradSmem<LV> *>(loss_smem);
   const int c = blockIdx.z, t = threadIdx.x;
   const size_t plane = (size_t)H * Wd;
   const size_t all = (size_t)gridDim.z * plane;
   const int ox = blockIdx.x * LW, oy = blockIdx.y * LHT;
 #pragma unroll 1
   for (int q = 0; q < 3; ++q) {
-    load_tile<1>(ABD + q * all + c * plane, nullptr, H, Wd, ox - LR, oy - LR, sm.in, nullptr);
+    load_tile<LROWS, 1>(ABD + q * all + c * plane, nullptr, H, Wd, ox - LR, oy - LR, sm.in, nullptr);
     __syncthreads();
 #pragma unroll
     for (int i = t; i < LROWS * (LW / 4); i += LN) {
@@ -244,7 +257,7 @@ ssim_grad_kernel(const float *__restrict__ x, const float *__restrict__ y, int H
   const int col = t & (LW - 1), gv = t / LW;
   float b[3][LV];
 #pragma unroll
-  for (int q = 0; q < 3; ++q) blur_column(W, sm.hs[q], col, gv, b[q]);
+  for (int q = 0; q < 3; ++q) blur_column<LV>(W, sm.hs[q], col, gv, b[q]);
   const int px = ox + col;
 #pragma unroll
   for (int j = 0; j < LV; ++j) {
@@ -282,8 +295,39 @@ Window gaussian_window() {
   return W;
 }
 
+size_t tiles(int C, int H, int W, int rows) {
+  return (size_t)C * ((H + rows - 1) / rows) * ((W + LW - 1) / LW);
+}
+
+// The small tile (LV = 2, 16 rows) where there are fewer than two large ones per
+// SM: the large one has too few blocks there, and a thread forms its seven
+// outputs one after the other.  Both kernels, 3 channels, large | small tile:
+// 128 x 128 20.6 | 18.4 us, 256 x 256 20.5 | 20.6, 320 x 320 24.7 | 22.6,
+// 400 x 400 28.7 | 28.7, 512 x 512 35.0 | 36.6 (LV = 1: 18.5, 23.2, 26.8, 35.0,
+// 48.2; LV = 4: 20.5, 21.8, 23.0, 28.7, 36.3).
+constexpr int LSMALL = 2;
+bool small_tiles(int C, int H, int W) { return tiles(C, H, W, Tile<7>::LHT) < 2 * (size_t)NUM_SMS_HINT; }
+
 size_t nblocks(int C, int H, int W) {
-  return (size_t)C * ((H + LHT - 1) / LHT) * ((W + LW - 1) / LW);
+  return tiles(C, H, W, small_tiles(C, H, W) ? Tile<LSMALL>::LHT : Tile<7>::LHT);
+}
+
+template <int LV>
+int run(const float *x, const float *y, int C, int H, int W, float lambda, float *loss, float *grad, float *ABD, float *part,
+        cudaStream_t s) {
+  const Window win = gaussian_window();
+  const dim3 grid((W + LW - 1) / LW, (H + Tile<LV>::LHT - 1) / Tile<LV>::LHT, C);
+  const size_t m_smem = sizeof(MomentsSmem<LV>), g_smem = sizeof(GradSmem<LV>);
+  if (int r = dmgs_host::raise_smem_limit((const void *)ssim_moments_kernel<LV>, m_smem)) return r;
+  if (int r = dmgs_host::raise_smem_limit((const void *)ssim_grad_kernel<LV>, g_smem)) return r;
+  const float inv_n = 1.f / ((float)C * (float)H * (float)W);
+  DMGS_TIMED(K_LOSS, s, {
+    dmgs_host::note_launch(), ssim_moments_kernel<LV><<<grid, LN, m_smem, s>>>(x, y, H, W, win, ABD, part);
+    dmgs_host::note_launch(), ssim_grad_kernel<LV><<<grid, LN, g_smem, s>>>(
+        x, y, H, W, win, ABD, lambda, inv_n, grad, part, (int)(grid.x * grid.y * grid.z), loss);
+  });
+  DMGS_LAUNCH_CHECK("ssim kernels");
+  return DMGS_OK;
 }
 
 }  // namespace
@@ -320,21 +364,10 @@ size_t l1_ssim_scratch_bytes(int C, int H, int W) {
 
 int launch_l1_ssim(const float *x, const float *y, int C, int H, int W, float lambda,
                    float *loss, float *grad, char *scratch, cudaStream_t s) {
-  const Window win = gaussian_window();
   float *ABD = reinterpret_cast<float *>(scratch);
   float *part = reinterpret_cast<float *>(scratch + align_up((size_t)3 * C * H * W * 4, 256));
-  const dim3 grid((W + LW - 1) / LW, (H + LHT - 1) / LHT, C);
-  const size_t m_smem = sizeof(MomentsSmem), g_smem = sizeof(GradSmem);
-  if (int r = dmgs_host::raise_smem_limit((const void *)ssim_moments_kernel, m_smem)) return r;
-  if (int r = dmgs_host::raise_smem_limit((const void *)ssim_grad_kernel, g_smem)) return r;
-  const float inv_n = 1.f / ((float)C * (float)H * (float)W);
-  DMGS_TIMED(K_LOSS, s, {
-    dmgs_host::note_launch(), ssim_moments_kernel<<<grid, LN, m_smem, s>>>(x, y, H, W, win, ABD, part);
-    dmgs_host::note_launch(), ssim_grad_kernel<<<grid, LN, g_smem, s>>>(
-        x, y, H, W, win, ABD, lambda, inv_n, grad, part, (int)nblocks(C, H, W), loss);
-  });
-  DMGS_LAUNCH_CHECK("ssim kernels");
-  return DMGS_OK;
+  return small_tiles(C, H, W) ? run<LSMALL>(x, y, C, H, W, lambda, loss, grad, ABD, part, s)
+                              : run<7>(x, y, C, H, W, lambda, loss, grad, ABD, part, s);
 }
 
 }  // namespace dmgs
