@@ -50,6 +50,7 @@
 // look-back kernels the view is the fast grid dimension: the tiles that start
 // together then belong to all views and have few predecessors each.
 #include <algorithm>
+#include <cmath>
 
 #include "kernels.cuh"
 
@@ -1180,25 +1181,28 @@ int device_sms() {
 // Row segments per view for a launch: enough (row, piece, segment) blocks for
 // several waves of the tile emission (short blocks balance uneven rows), but
 // not so many that a block's fixed work (sub-pass cut, cursors, run copies)
-// outweighs its instances.  Emission at 16 | 24 | 32 | 48 blocks an SM, us: four
-// views of 500k Gaussians 53 | 60 | 70 | 76, sixteen of 3M 710 | 642 | 623 |
-// 608 (and the counting kernel 202 | 172 | 164 | 152); a single view is at
-// SEG_MAX on most grids.  A pure function of the views' grids and sizes and
-// the device, so the geometry and the emission launches of one set of views
-// agree.
+// outweighs its instances.  Where the two meet moves with the work: the best
+// count grows about as the root of the Gaussians x views.  Counts, scans and
+// emission together, us, at 16 | 24 | 32 | 48 blocks an SM and (this rule's):
+//   4 views of 0.25M, 0.5M, 1M, 2M   73 | 81 | 90 | 111 (16), 96 | 97 | 105 | 124 (16), 146 | 136 | 138 | 153 (22), 253 | 228 | 220 | 229 (31)
+//   8 views of the same              92 | 95 | 105 | 125 (16), 140 | 135 | 136 | 150 (22), 229 | 208 | 200 | 206 (31), 410 | 363 | 342 | 334 (44)
+//   16 views of the same             120 | 123 | 126 | 147 (22), 193 | 182 | 182 | 196 (31), 347 | 315 | 311 | 313 (44), 637 | 579 | 560 | 545 (48)
+// at 1237 x 822, and at 400 x 300, 200 x 200 and 3000 x 2000 with 0.1M and 1M
+// the same order.  A single view is at SEG_MAX on most grids.  A pure function
+// of the views' grids and sizes and the device, so the geometry and the
+// emission launches of one set of views agree.
 int seg_plan(const BinViews &bv) {
   long rows = 0, gaussians = 0;
   for (int v = 0; v < bv.n; ++v) {
     rows += (long)bv.v[v].gy * bv.v[v].nxs;
     gaussians += bv.v[v].P;
   }
-  const long target = (gaussians < (16l << 20) ? 16L : 48L) * device_sms();
+  const double per_sm = std::min(48.0, std::max(16.0, 16.0 * std::sqrt((double)gaussians / (double)(1 << 21))));
+  const long target = (long)per_sm * device_sms();
   const long S = rows > 0 ? (target + rows - 1) / rows : 1;
   return (int)std::max(1L, std::min((long)SEG_MAX, S));
 }
 
-// Scan of one array per view: host bound n_max (the launch size), device
-// length *n_dev when given.
 // Blocks per view for a grid-stride launch over at most `units` work units
 // whose actual count is only known on the device: about two resident waves
 // of `per_sm` blocks per SM shared by the views, so that a launch sized for
