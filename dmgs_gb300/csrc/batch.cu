@@ -350,7 +350,8 @@ extern "C" int dmgs_batch_status(const DmgsBatch *b, int32_t P, const void *stat
       set_error("batch: view %d: a point failed the frustum test although prefiltered is set", v);
       rc = DMGS_ERR_PREFILTER;
     } else if ((h[v][CI_STATUS] & ST_BOUNDS) && rc == DMGS_OK) {
-      set_error("batch: view %d: a kernel index left its buffer", v);
+      set_error((h[v][CI_STATUS] & ST_WAIT) ? "batch: view %d: a kernel's wait for another block ran out"
+                                            : "batch: view %d: a kernel index left its buffer", v);
       rc = DMGS_ERR_DEVICE;
     }
   }

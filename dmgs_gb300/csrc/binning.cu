@@ -179,11 +179,16 @@ scan_down_kernel(const ScanViews sv) {
 // that holds an inclusive prefix, and publishes its own.  Each word carries
 // its state in its top two bits and is written whole, so relaxed accesses
 // suffice.  The polls are bounded: a tile that gives up (or sees that another
-// has) sets ST_BOUNDS, and every later kernel then leaves the view alone.
+// has) sets ST_BOUNDS and ST_WAIT, and every later kernel then leaves the view
+// alone.
 
 constexpr unsigned long long LB_AGG = 1ull << 62, LB_INC = 2ull << 62, LB_VAL = LB_AGG - 1;
 constexpr uint32_t LB32_AGG = 1u << 30, LB32_INC = 2u << 30, LB32_VAL = LB32_AGG - 1;
-constexpr uint32_t LB_POLLS = 1u << 20;
+#ifndef DMGS_LB_POLLS
+#define DMGS_LB_POLLS (1u << 20)  // about a second
+#endif
+constexpr uint32_t LB_POLLS = DMGS_LB_POLLS;
+constexpr uint32_t ST_GAVE_UP = ST_BOUNDS | ST_WAIT;
 
 __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t *p) {
   uint32_t v;
@@ -226,7 +231,8 @@ __device__ __forceinline__ unsigned long long lookback(unsigned long long *st, u
     const unsigned inc = __ballot_sync(FULL, state == 2u), none = __ballot_sync(FULL, state == 0u);
     const int last = inc ? __ffs(inc) - 1 : 31;  // words of lanes 0..last are added
     if (none & (0xffffffffu >> (31 - last))) {
-      if (give_up(++polls, counters)) {
+      // one decision for the warp: its lanes' loads of the status may differ
+      if (__any_sync(FULL, give_up(++polls, counters))) {
         *ok = false;
         return 0ull;
       }
@@ -241,6 +247,12 @@ __device__ __forceinline__ unsigned long long lookback(unsigned long long *st, u
   }
   if (lane == 0) st_relaxed(st + t, LB_INC | (excl + agg));
   return excl;
+}
+
+// Whether the view is one to leave alone: the same answer for all threads of
+// the block, also while another block of this launch sets the bit.
+__device__ __forceinline__ bool stopped(const BinView &B) {
+  return __syncthreads_or((B.counters[CI_STATUS] & ST_STOP) != 0u);
 }
 
 // Next tile of this block (the same for all its threads).
@@ -412,7 +424,7 @@ radix_pass_kernel(const BinViews bv, int pass) {
   uint32_t *kout = (pass & 1) ? B.k0 : B.k1, *vout = (pass & 1) ? B.v0 : B.v1;
   const int shift = 8 * pass;
   const uint32_t V = B.counters[CI_V], ntiles = (V + RADIX_TILE - 1) / RADIX_TILE;
-  if (blockIdx.y >= ntiles || (B.counters[CI_STATUS] & ST_STOP)) return;  // block-uniform
+  if (blockIdx.y >= ntiles || stopped(B)) return;
   __shared__ uint32_t wh[RADIX_BLOCK / 32][256];
   __shared__ uint32_t slot, wsum[RADIX_BLOCK / 32];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -499,7 +511,7 @@ radix_pass_kernel(const BinViews bv, int pass) {
       run += x;
     }
     if (__syncthreads_or(bad)) {
-      if (tid == 0) atomicOr(B.counters + CI_STATUS, ST_BOUNDS);
+      if (tid == 0) atomicOr(B.counters + CI_STATUS, ST_GAVE_UP);
       return;
     }
 #pragma unroll
@@ -574,7 +586,7 @@ __global__ void __launch_bounds__(256)
 chunk_kernel(const BinViews bv) {
   const BinView &B = bv.v[blockIdx.x];
   const uint32_t V = B.counters[CI_V], ntiles = (V + RADIX_TILE - 1) / RADIX_TILE;
-  if (blockIdx.y >= ntiles || (B.counters[CI_STATUS] & ST_STOP)) return;  // block-uniform
+  if (blockIdx.y >= ntiles || stopped(B)) return;
   const uint32_t C = chunk_count(B, V);
   const unsigned long long W = *reinterpret_cast<const unsigned long long *>(B.counters + CI_W);
   __shared__ uint32_t slot;
@@ -614,7 +626,7 @@ chunk_kernel(const BinViews bv) {
       if (tid == 0) {
         s_excl = e;
         s_ok = ok;
-        if (!ok) atomicOr(B.counters + CI_STATUS, ST_BOUNDS);
+        if (!ok) atomicOr(B.counters + CI_STATUS, ST_GAVE_UP);
       }
     }
     __syncthreads();
@@ -722,7 +734,7 @@ __global__ void __launch_bounds__(256)
 count_kernel(const BinViews bv, int S, int nb_max, int nw) {
   extern __shared__ int cnt_smem[];
   const BinView &B = bv.v[blockIdx.y];
-  if (B.counters[CI_STATUS] & ST_STOP) return;
+  if (B.counters[CI_STATUS] & ST_STOP) return;  // block-uniform: no block of this launch sets a bit
   const uint32_t C = chunk_count(B, B.counters[CI_V]);
   if ((int)blockIdx.x < S * nb_max) {
     if ((int)blockIdx.x < S * B.nb)  // block-uniform
@@ -741,7 +753,7 @@ count_kernel(const BinViews bv, int S, int nb_max, int nw) {
 __global__ void __launch_bounds__(SCAN_THREADS)
 list_scan_kernel(const BinViews bv, int S) {
   const BinView &B = bv.v[blockIdx.x];
-  if (B.counters[CI_STATUS] & ST_STOP) return;
+  if (stopped(B)) return;
   const uint32_t C = chunk_count(B, B.counters[CI_V]);
   const size_t nr = (size_t)B.gy * C, ns = (size_t)B.gx * B.gy * S;
   const uint32_t tr = (uint32_t)scan_tiles(nr), ts = (uint32_t)scan_tiles(ns);
@@ -778,7 +790,7 @@ list_scan_kernel(const BinViews bv, int S) {
       if (tid == 0) {
         s_excl = e;
         s_ok = ok;
-        if (!ok) atomicOr(B.counters + CI_STATUS, ST_BOUNDS);
+        if (!ok) atomicOr(B.counters + CI_STATUS, ST_GAVE_UP);
         if (ok && t == (rows ? tr : ts) - 1) {
           B.counters[rows ? CI_K1 : CI_K] = (uint32_t)(e + total);
           if (e + total > 0xffffffffull) atomicOr(B.counters + CI_STATUS, ST_OVERFLOW);
@@ -844,7 +856,7 @@ row_emit_kernel(const BinViews bv) {
   uint32_t *counters = B.counters;
   const uint32_t C = counters[CI_C];
   const uint32_t c = blockIdx.x;
-  if (c >= C || (counters[CI_STATUS] & ST_STOP)) return;
+  if (c >= C || __any_sync(FULL, (counters[CI_STATUS] & ST_STOP) != 0u)) return;  // one warp a block
   const int lane = threadIdx.x, gy = B.gy, nbits = bits_for(gy);
   for (int r = lane; r < gy; r += 32) rcur[r] = B.rcnt[(size_t)r * C + c];
   __syncwarp();
@@ -938,7 +950,7 @@ tile_emit_kernel(const BinViews bv, int S) {
   if (r >= B.gy) return;  // block-uniform
   uint32_t *counters = B.counters;
   const uint32_t C = counters[CI_C];
-  if (C == 0 || (counters[CI_STATUS] & ST_STOP)) return;
+  if (C == 0 || stopped(B)) return;
   const uint32_t f0 = seg_chunk(sg, C, S), f1 = seg_chunk(sg + 1, C, S);
   if (f0 >= f1) return;
   const uint32_t e0 = B.rcnt[(size_t)r * C + f0];

@@ -145,6 +145,7 @@ int check_status(const char *geom, const GeomLayout &L, cudaStream_t s, uint32_t
     return DMGS_ERR_PREFILTER;
   }
   if (h[0] & ST_OVERFLOW) { set_error("instance buffer overflow"); return DMGS_ERR_OVERFLOW; }
+  if (h[0] & ST_WAIT) { set_error("a kernel's wait for another block ran out"); return DMGS_ERR_DEVICE; }
   if (h[0] & ST_BOUNDS) { set_error("a kernel index left its buffer"); return DMGS_ERR_DEVICE; }
   return DMGS_OK;
 }

@@ -19,6 +19,7 @@ constexpr int NUM_SMS_HINT = 152;             // GB300: 2 dies x 76 SMs
 constexpr uint32_t ST_PREFILTER = 1u;   // prefiltered point failed the z test
 constexpr uint32_t ST_OVERFLOW = 2u;    // instance slots exhausted
 constexpr uint32_t ST_BOUNDS = 4u;      // an index left its buffer
+constexpr uint32_t ST_WAIT = 8u;        // beside ST_BOUNDS: a bounded wait ran out
 
 __host__ __device__ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 

@@ -265,7 +265,8 @@ int dmgs_render_multi(const DmgsBatch *b, const DmgsGaussians *g, void *const *s
  * to stay asynchronous); read them once the stream has passed this point.
  * Status bits: 1 prefiltered point culled, 2 capacity overflow (the view
  * rendered background; the count is the capacity it needs), 4 index out of
- * its buffer. */
+ * its buffer, 8 beside 4 a wait between blocks that ran out (the view rendered
+ * background). */
 int dmgs_multi_status_async(const DmgsBatch *b, const DmgsGaussians *g,
                             void *const *state, const size_t *state_bytes,
                             uint32_t *host_words, dmgs_stream_t stream);
