@@ -839,7 +839,7 @@ __global__ void ranges_kernel(const BinViews bv, int S) {
     const int l = 31 - __clz(n), b = 2 * l + (l > 0 ? (int)((n >> (l - 1)) & 1u) : 0);
     c = max(0, BLEND_CLASSES - 2 - b);
   }
-  B.clslist[(size_t)c * T + atomicAdd(&B.clsn[c], 1u)] = (uint32_t)t;
+  B.clslist[class_slot(c, atomicAdd(&B.clsn[c], 1u), T)] = (uint32_t)t;
 }
 
 // ---- step 6a: row lists, one warp per chunk --------------------------------

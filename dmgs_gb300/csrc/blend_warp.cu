@@ -184,7 +184,7 @@ __device__ __forceinline__ Item find_item(const BlendWork &wk, const BlendBatch 
   it.fine = class_floor(c) >= tab.fine_floor;
   const uint32_t k = i - tab.first[e], parts = it.fine ? PARTS_FINE : PARTS_COARSE;
   it.part = (int)(k % parts);
-  it.tile = (int)wk.v[it.view].cls_list[(size_t)c * bb.v[it.view].T + k / parts];
+  it.tile = (int)wk.v[it.view].cls_list[class_slot(c, k / parts, bb.v[it.view].T)];
   return it;
 }
 

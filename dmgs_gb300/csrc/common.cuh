@@ -89,8 +89,9 @@ constexpr int CI_TICKETS_END = 32;
 // 8 B); chunk starts; the row counts [gy][C] (Gaussians of chunk c covering
 // tile row r, scanned in place into row-list offsets); the segment counts
 // [T][S] (instances of tile t from row segment s, scanned in place into list
-// offsets); tile ranges; per class of list lengths the tiles in it (clslist
-// [BLEND_CLASSES][T], clsn of them); the radix sort's look-back words (stsort, per pass
+// offsets); tile ranges; per class of list lengths the tiles in it (clsn of
+// them; two classes to a row of clslist [BLEND_CLASSES / 2][T], from its two
+// ends: class_slot); the radix sort's look-back words (stsort, per pass
 // and key tile one word per digit); and one region that must be zero when a
 // view's preprocess starts: the counters and tickets, the digit histograms
 // of the four passes, the preprocess's visible counts (per tile of RADIX_TILE
@@ -104,6 +105,11 @@ struct GeomLayout {
   int nb_pre, nb_radix;  // preprocess blocks; tiles of RADIX_TILE keys (or Gaussians)
   __host__ __device__ int T() const { return gx * gy; }
 };
+
+// Place in clslist of tile k of class c, of a view of T tiles.
+__host__ __device__ inline size_t class_slot(int c, uint32_t k, int T) {
+  return (size_t)(c >> 1) * T + ((c & 1) ? (uint32_t)T - 1u - k : k);
+}
 
 __host__ __device__ inline size_t scan_tiles(size_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE; }
 
@@ -121,15 +127,15 @@ __host__ __device__ inline GeomLayout geom_layout(int P, int W, int H) {
   L.flags = o;     o = align_up(o + (size_t)P, 256);
   L.vlist = o;     o = align_up(o + (size_t)P * 4, 256);
   L.dkey0 = o;     o = align_up(o + (size_t)P * 4, 256);
-  L.dkey1 = o;     o = align_up(o + (size_t)P * 4, 256);
   L.dval0 = o;     o = align_up(o + (size_t)P * 4, 256);
+  L.srect = o;  // the sort's second copy ends with its last pass, before the first srect
+  L.dkey1 = o;     o = align_up(o + (size_t)P * 4, 256);
   L.dval1 = o;     o = align_up(o + (size_t)P * 4, 256);
-  L.srect = o;     o = align_up(o + (size_t)P * 8, 256);
   L.cstart = o;    o = align_up(o + (CHUNK_COUNT_MAX + 1) * 4, 256);
   L.rcnt = o;      o = align_up(o + n_rcnt * 4, 256);
   L.cnt2 = o;      o = align_up(o + n_cnt2 * 4, 256);
   L.ranges = o;    o = align_up(o + T * 8, 256);
-  L.clslist = o;   o = align_up(o + T * BLEND_CLASSES * 4, 256);
+  L.clslist = o;   o = align_up(o + T * (BLEND_CLASSES / 2) * 4, 256);
   L.stsort = o;    o = align_up(o + (size_t)L.nb_radix * (4 * 256 * 4), 256);
   L.counters = o;  o = align_up(o + CI_TICKETS_END * 4, 256);
   L.ghist = o;     o = align_up(o + 4 * 256 * 4, 256);
