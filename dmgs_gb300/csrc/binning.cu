@@ -1104,7 +1104,9 @@ tile_emit_kernel(const BinViews bv, int S) {
       const int lo = (int)__reduce_min_sync(FULL, has ? (unsigned)a : 0xffffffffu);
       const int hi = (int)__reduce_max_sync(FULL, has ? (unsigned)b : 0u);
       __syncwarp();
-      if (lo < hi) {  // warp-uniform; chunks up to the one holding hi (clears tog[hi])
+      // none of the group's entries may lie in this piece of a row of more than
+      // XSEG tiles: hi is 0 then, and lo no tile
+      if (hi > 0) {  // warp-uniform; chunks up to the one holding hi (clears tog[hi])
         uint32_t carry = 0u;
         for (int xb = lo & ~31; xb <= hi && xb < nx; xb += 32) {
           const int x = xb + lane;
