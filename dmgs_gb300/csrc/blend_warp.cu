@@ -121,18 +121,19 @@ constexpr int PARTS_FINE = 8, PARTS_COARSE = 2;
 struct WorkTable {
   uint32_t first[MAX_BATCH_VIEWS * BLEND_CLASSES];  // exclusive prefix of the items, view-major
   uint32_t total;
+  uint32_t shares;      // parts in which the adjoint clears its spans
   uint32_t fine_floor;  // lists of classes whose floor is at least this are split into strips
 };
 
-// Built once per CTA (all threads).
+// Built once per CTA (all threads); ctas: those that the tiles can feed.
 template <bool SKIP_EMPTY>
-__device__ __forceinline__ void build_table(const BlendWork &wk, int nviews, WorkTable &tab) {
+__device__ __forceinline__ void build_table(const BlendWork &wk, int nviews, unsigned ctas, WorkTable &tab) {
   const int tid = threadIdx.x, n = nviews * BLEND_CLASSES;
   if (tid < 32) {
     float k = tid < nviews ? (float)wk.v[tid].counters[CI_K] : 0.f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) k += __shfl_xor_sync(FULL, k, o);
-    const float share = FINE_SHARE * k * PARTS_COARSE / (float)(gridDim.x * BW_WARPS);
+    const float share = FINE_SHARE * k * PARTS_COARSE / (float)(ctas * BW_WARPS);
     if (tid == 0) tab.fine_floor = (uint32_t)fminf(fmaxf(share, 1.f), 4e9f);
   }
   __syncthreads();
@@ -325,7 +326,7 @@ blend_fwd_warp_kernel(const BlendBatch bb, const BlendWork wk, uint32_t *queue) 
   __shared__ WorkTable tab;
   __shared__ float4 S[BW_WARPS][3][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  build_table<false>(wk, bb.nviews, tab);
+  build_table<false>(wk, bb.nviews, gridDim.x, tab);
   for (uint32_t i = take_item(queue, lane); i < tab.total; i = take_item(queue, lane)) {
     const Item it = find_item(wk, bb, tab, i, lane);
     const BlendView &V = bb.v[it.view];
@@ -534,21 +535,27 @@ __device__ __forceinline__ bool bwd_part(const BlendView &V, int tile, int part,
 }
 
 __global__ void __launch_bounds__(32 * BW_WARPS, 10)
-blend_bwd_warp_kernel(const BlendBatch bb, const BlendWork wk, const ZeroSpans zero, uint32_t *queue) {
+blend_bwd_warp_kernel(const BlendBatch bb, const BlendWork wk, const ZeroSpans zero, unsigned ctas, uint32_t *queue) {
   __shared__ WorkTable tab;
   __shared__ float4 S[BW_WARPS][3][32];
   __shared__ float4 K[BW_WARPS][32];
   __shared__ uint32_t I[BW_WARPS][32];
   __shared__ Pending R[BW_WARPS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  build_table<true>(wk, bb.nviews, tab);
-  // the spans are cleared a share per item, spread over the launch (all at
-  // its start they took as long as alone: 0.11 ms for 744 MB)
-  if (tab.total == 0u) zero_spans(zero, blockIdx.x, gridDim.x, threadIdx.x, blockDim.x);
-  for (uint32_t i = take_item(queue, lane); i < tab.total; i = take_item(queue, lane)) {
+  build_table<true>(wk, bb.nviews, ctas, tab);
+  // The spans are cleared a share per item, spread over the launch (all at its
+  // start they took as long as alone: 0.11 ms for 744 MB); where there are
+  // fewer items than warps, a share per warp, the last ones by warps that no
+  // item is left for: 3M Gaussians in a view of one tile took 7.5 ms with a
+  // share to each of eight items, 1.8 ms so.  (The number of shares is kept in
+  // shared memory: a register more through the loop cost 5%.)
+  if (threadIdx.x == 0) tab.shares = max(tab.total, gridDim.x * BW_WARPS);
+  __syncthreads();
+  uint32_t i = take_item(queue, lane);
+  for (; i < tab.total; i = take_item(queue, lane)) {
     const Item it = find_item(wk, bb, tab, i, lane);
     const BlendView &V = bb.v[it.view];
-    zero_spans(zero, i, tab.total, lane, 32u);
+    zero_spans(zero, i, tab.shares, lane, 32u);
     const bool done = it.fine ? bwd_part<1, false>(V, it.tile, it.part, S[w], K[w], I[w], R[w], lane)
                               : bwd_part<4, false>(V, it.tile, it.part, S[w], K[w], I[w], R[w], lane);
     if (!done) {  // rare: strips alone, a half being four of them
@@ -557,6 +564,8 @@ blend_bwd_warp_kernel(const BlendBatch bb, const BlendWork wk, const ZeroSpans z
       for (int p = 0; p < n; ++p) bwd_part<1, true>(V, it.tile, n * it.part + p, S[w], K[w], I[w], R[w], lane);
     }
   }
+  if (zero.n == 0) return;
+  for (; i < tab.shares; i = take_item(queue, lane)) zero_spans(zero, i, tab.shares, lane, 32u);
 }
 
 // Resident CTAs of a kernel (looked up once per device and host thread), at
@@ -590,9 +599,13 @@ int launch_blend_warp_fwd(const BlendBatch &bb, const BlendWork &wk, uint32_t *q
 int launch_blend_warp_bwd(const BlendBatch &bb, const BlendWork &wk, const ZeroSpans &zero, uint32_t *queue,
                           cudaStream_t s) {
   thread_local int dev = -1, slots = 0;
-  int grid;
-  if (int r = resident_grid(blend_bwd_warp_kernel, bb.total, dev, slots, grid)) return r;
-  DMGS_TIMED(K_BLEND_BWD, s, dmgs_host::note_launch(), blend_bwd_warp_kernel<<<grid, 32 * BW_WARPS, 0, s>>>(bb, wk, zero, queue));
+  int ctas;
+  if (int r = resident_grid(blend_bwd_warp_kernel, bb.total, dev, slots, ctas)) return r;
+  // more CTAs than the tiles feed where there is enough to clear: 16 KB a warp
+  size_t words = 0;
+  for (int k = 0; k < zero.n; ++k) words += zero.words[k];
+  const int grid = std::max(ctas, (int)std::min<size_t>(slots, words / (4096 * BW_WARPS) + 1));
+  DMGS_TIMED(K_BLEND_BWD, s, dmgs_host::note_launch(), blend_bwd_warp_kernel<<<grid, 32 * BW_WARPS, 0, s>>>(bb, wk, zero, ctas, queue));
   DMGS_LAUNCH_CHECK("blend_bwd_warp_kernel");
   return DMGS_OK;
 }
