@@ -136,7 +136,8 @@ struct FaceBlocks {
 
 FaceBlocks face_blocks(int F, int G, int words) {
   FaceBlocks k;
-  const int fit = 22 * 1024 / 4 / words;  // Gaussians whose rows fit (ten blocks per SM)
+  // Gaussians whose rows fit (64 faces of six: ten blocks share an SM)
+  const int fit = 22 * 1024 / 4 / words;
   k.faces = std::max(1, std::min(BB, fit / G));
   k.chunk = std::min(G, fit);
   k.blocks = (F + k.faces - 1) / k.faces;
@@ -847,7 +848,7 @@ int launch_face_cull(const float *verts, int V, const int64_t *faces, int F,
   uint32_t *part = reinterpret_cast<uint32_t *>(scratch + align_up((size_t)nb * 4 + 4, 256));
   DMGS_TIMED(K_FACE_CULL, s, {
     dmgs_host::note_launch(), face_cull_test_kernel<<<nb, CULL_BLOCK, 0, s>>>(verts, V, faces, F, full_proj, face_mask, blkcnt);
-    int r = launch_scan1(blkcnt, nb, part, reinterpret_cast<uint32_t *>(num_kept), nullptr, s);
+    int r = launch_scan1(blkcnt, nb, part, reinterpret_cast<uint32_t *>(num_kept), s);
     if (r != DMGS_OK) return r;
     dmgs_host::note_launch(), face_cull_compact_kernel<<<nb, CULL_BLOCK, 0, s>>>(verts, V, faces, F, full_proj, blkcnt, kept);
   });

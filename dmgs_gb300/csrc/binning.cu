@@ -37,8 +37,8 @@
 // written once and read once.  The row and segment offsets are small (gy x C
 // and T x S words).
 //
-// Launches: steps 1-5 are ten kernels (compaction, four sort passes, chunks,
-// counts, scans, ranges).  Every prefix that crosses blocks is formed by
+// Launches: steps 1-5 are nine kernels (compaction, four sort passes, chunks,
+// counts, scans, ranges), step 6 two.  Every prefix that crosses blocks is formed by
 // decoupled look-back inside the kernel that needs it, so no step has a scan
 // launch of its own and the sort reads its keys once per pass: a view has
 // 10^4-10^6 visible Gaussians, a few us of memory traffic, and its time was
@@ -96,41 +96,28 @@ __device__ __forceinline__ unsigned long long block_exclusive_scan(unsigned long
   return before;
 }
 
-// ---- generic exclusive scan (u32, in place), three phases, per view -----
-
-__device__ __forceinline__ uint32_t scan_len(const ScanView &v) {
-  return v.n_dev ? min(*v.n_dev, v.n_max) : v.n_max;
-}
+// ---- generic exclusive scan (u32, in place), three phases ------------------
 
 __global__ void __launch_bounds__(SCAN_THREADS)
-scan_reduce_kernel(const ScanViews sv) {
-  const ScanView &v = sv.v[blockIdx.y];
-  const uint32_t n = scan_len(v);
+scan_reduce_kernel(const uint32_t *__restrict__ data, uint32_t n, uint32_t *__restrict__ part) {
   for (uint32_t tile = blockIdx.x; tile * (uint32_t)SCAN_TILE < n; tile += gridDim.x) {
     const uint32_t base = tile * SCAN_TILE;
     unsigned long long s = 0;
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; ++i) {
       const uint32_t k = base + i * SCAN_THREADS + threadIdx.x;
-      if (k < n) s += v.data[k];
+      if (k < n) s += data[k];
     }
     unsigned long long tot;
     block_exclusive_scan<SCAN_THREADS>(s, &tot);
-    if (threadIdx.x == 0) v.part[tile] = (uint32_t)tot;
+    if (threadIdx.x == 0) part[tile] = (uint32_t)tot;
   }
 }
 
-// One block per view: exclusive scan of the per-block partials (or of the
-// whole array when it fits one block); total to *total_out, overflow flagged.
+// One block: exclusive scan of the per-block partials (or of the whole array
+// when it fits one block); total to *total_out.
 __global__ void __launch_bounds__(SCAN_THREADS)
-scan_single_kernel(const ScanViews sv, int partials_of_tiles) {
-  const ScanView &v = sv.v[blockIdx.y];
-  uint32_t n = scan_len(v);
-  uint32_t *data = v.data;
-  if (partials_of_tiles) {
-    n = (n + SCAN_TILE - 1) / SCAN_TILE;
-    data = v.part;
-  }
+scan_single_kernel(uint32_t *__restrict__ data, uint32_t n, uint32_t *__restrict__ total_out) {
   const uint32_t per = (n + SCAN_THREADS - 1) / SCAN_THREADS;
   const uint32_t beg = min(n, threadIdx.x * per), end = min(n, beg + per);
   unsigned long long s = 0;
@@ -142,16 +129,11 @@ scan_single_kernel(const ScanViews sv, int partials_of_tiles) {
     data[k] = (uint32_t)run;
     run += x;
   }
-  if (threadIdx.x == 0) {
-    if (v.total_out) *v.total_out = (uint32_t)tot;
-    if (tot > 0xffffffffull && v.status) atomicOr(v.status, ST_OVERFLOW);
-  }
+  if (threadIdx.x == 0 && total_out) *total_out = (uint32_t)tot;
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS)
-scan_down_kernel(const ScanViews sv) {
-  const ScanView &v = sv.v[blockIdx.y];
-  const uint32_t n = scan_len(v);
+scan_down_kernel(uint32_t *__restrict__ data, uint32_t n, const uint32_t *__restrict__ part) {
   for (uint32_t tile = blockIdx.x; tile * (uint32_t)SCAN_TILE < n; tile += gridDim.x) {
     // blocked: thread i owns elements base + i*ITEMS .. +ITEMS-1
     uint32_t x[SCAN_ITEMS];
@@ -159,13 +141,13 @@ scan_down_kernel(const ScanViews sv) {
     const uint32_t k0 = tile * SCAN_TILE + threadIdx.x * SCAN_ITEMS;
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; ++i) {
-      x[i] = (k0 + i < n) ? v.data[k0 + i] : 0u;
+      x[i] = (k0 + i < n) ? data[k0 + i] : 0u;
       s += x[i];
     }
-    unsigned long long run = block_exclusive_scan<SCAN_THREADS>(s, nullptr) + v.part[tile];
+    unsigned long long run = block_exclusive_scan<SCAN_THREADS>(s, nullptr) + part[tile];
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; ++i) {
-      if (k0 + i < n) v.data[k0 + i] = (uint32_t)run;
+      if (k0 + i < n) data[k0 + i] = (uint32_t)run;
       run += x[i];
     }
   }
@@ -1226,35 +1208,25 @@ int bounded_blocks(size_t units, int nviews, int per_sm) {
   return (int)std::max<size_t>(1, std::min(units, cap));
 }
 
-int launch_scan_views(const ScanViews &sv, cudaStream_t s) {
-  uint32_t n_max = 0;
-  for (int v = 0; v < sv.n; ++v) n_max = std::max(n_max, sv.v[v].n_max);
-  const dim3 one(1, sv.n);
-  if (n_max <= (uint32_t)SCAN_TILE * 4) {
-    dmgs_host::note_launch(), scan_single_kernel<<<one, SCAN_THREADS, 0, s>>>(sv, 0);
-    DMGS_LAUNCH_CHECK("scan_single_kernel");
-    return DMGS_OK;
-  }
-  const dim3 grid(bounded_blocks((n_max + SCAN_TILE - 1) / SCAN_TILE, sv.n, 2), sv.n);
-  dmgs_host::note_launch(), scan_reduce_kernel<<<grid, SCAN_THREADS, 0, s>>>(sv);
-  DMGS_LAUNCH_CHECK("scan_reduce_kernel");
-  dmgs_host::note_launch(), scan_single_kernel<<<one, SCAN_THREADS, 0, s>>>(sv, 1);
-  DMGS_LAUNCH_CHECK("scan_single_kernel");
-  dmgs_host::note_launch(), scan_down_kernel<<<grid, SCAN_THREADS, 0, s>>>(sv);
-  DMGS_LAUNCH_CHECK("scan_down_kernel");
-  return DMGS_OK;
-}
-
 constexpr size_t SMEM_LIMIT = 220 * 1024;
 
 }  // namespace
 
-int launch_scan1(uint32_t *data, uint32_t n, uint32_t *part, uint32_t *total_out,
-                 uint32_t *status, cudaStream_t s) {
-  ScanViews sv;
-  sv.n = 1;
-  sv.v[0] = ScanView{data, nullptr, n, part, total_out, status};
-  return launch_scan_views(sv, s);
+int launch_scan1(uint32_t *data, uint32_t n, uint32_t *part, uint32_t *total_out, cudaStream_t s) {
+  if (n <= (uint32_t)SCAN_TILE * 4) {
+    dmgs_host::note_launch(), scan_single_kernel<<<1, SCAN_THREADS, 0, s>>>(data, n, total_out);
+    DMGS_LAUNCH_CHECK("scan_single_kernel");
+    return DMGS_OK;
+  }
+  const uint32_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
+  const int grid = bounded_blocks(tiles, 1, 2);
+  dmgs_host::note_launch(), scan_reduce_kernel<<<grid, SCAN_THREADS, 0, s>>>(data, n, part);
+  DMGS_LAUNCH_CHECK("scan_reduce_kernel");
+  dmgs_host::note_launch(), scan_single_kernel<<<1, SCAN_THREADS, 0, s>>>(part, tiles, total_out);
+  DMGS_LAUNCH_CHECK("scan_single_kernel");
+  dmgs_host::note_launch(), scan_down_kernel<<<grid, SCAN_THREADS, 0, s>>>(data, n, part);
+  DMGS_LAUNCH_CHECK("scan_down_kernel");
+  return DMGS_OK;
 }
 
 size_t scan_part_words(uint32_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE + 1; }
@@ -1262,7 +1234,6 @@ size_t scan_part_words(uint32_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE + 1;
 int make_bin_view(const GeomLayout &L, char *geom, uint32_t K_cap, char *bin, uint32_t K_alloc,
                   BinView &B) {
   B.P = L.P;
-  B.nb_pre = L.nb_pre;
   B.nb_radix = L.nb_radix;
   B.gx = L.gx;
   B.gy = L.gy;

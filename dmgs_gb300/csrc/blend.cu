@@ -166,6 +166,14 @@ __device__ __forceinline__ Staged stage(const float4 f0, const float4 f1, const 
   return S;
 }
 
+// Exponent (base 2) of the Gaussian at (dx, dy).  Explicit intrinsics: the
+// adjoint evaluates the identical sequence.
+__device__ __forceinline__ float exponent2(float A, float B, float C, float dx, float dy) {
+  const float ax2 = __fmul_rn(__fmul_rn(A, dx), dx);
+  const float q = __fmul_rn(B, dx);
+  return __fmaf_rn(__fmaf_rn(C, dy, q), dy, ax2);
+}
+
 // Work item -> (view, tile).
 __device__ __forceinline__ int find_view(const BlendBatch &bb, int item) {
   int v = 0;
@@ -470,6 +478,60 @@ __device__ __forceinline__ void adjoint_pair(PixelState &ps, bool take, float al
   ps.ag = fmaf(at, S, ps.ag);
 }
 
+// From the thread's sums (e[0] = sum Gd, e[1] = sum Gd dy, e[2] = sum Gd dy^2
+// over its pixels; u = o Gd = dL/dpower) to the gradient terms: e0 =
+// dL/dndc_x, e1 = dL/dndc_y, e2..e4 = (sum u dx^2, sum u dx dy, sum u dy^2)
+// for the conic (scaled by -1/2, -1, -1/2 at the atomics), e5 = dL/dopacity.
+__device__ __forceinline__ void adjoint_finish(float dx, float o, const float4 &s2,
+                                               const float4 &s3, float *e) {
+  e[5] = e[0];
+  const float su = o * e[0], suy = o * e[1], suy2 = o * e[2];
+  const float sux = dx * su;
+  e[0] = sux * s2.z + suy * s2.w;
+  e[1] = suy * s3.x + sux * s3.y;
+  e[2] = sux * dx;
+  e[3] = suy * dx;
+  e[4] = suy2;
+}
+
+// Transposed reduce-scatter of the 9 gradient slots over the warp, 12
+// shuffles: each level halves the slots a lane keeps (5 | 4, 3 | 2, 2 | 1,
+// 1 | 1) and adds its partner's copy of them; afterwards the even lane 2q
+// holds the warp sum of slot slot9(q) (q = lane bits 4..1), none when that
+// is >= 9.
+__device__ __forceinline__ float warp_reduce_scatter9(const float (&v)[9], int lane) {
+  float a[5], b[3], c[2];
+  {
+    const bool hi = lane & 16;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const float up = i < 4 ? v[5 + i] : 0.f;
+      a[i] = (hi ? up : v[i]) + __shfl_xor_sync(FULL, hi ? v[i] : up, 16);
+    }
+  }
+  {
+    const bool hi = lane & 8;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const float up = i < 2 ? a[3 + i] : 0.f;
+      b[i] = (hi ? up : a[i]) + __shfl_xor_sync(FULL, hi ? a[i] : up, 8);
+    }
+  }
+  {
+    const bool hi = lane & 4;
+    c[0] = (hi ? b[2] : b[0]) + __shfl_xor_sync(FULL, hi ? b[0] : b[2], 4);
+    c[1] = (hi ? 0.f : b[1]) + __shfl_xor_sync(FULL, hi ? b[1] : 0.f, 4);
+  }
+  const bool hi = lane & 2;
+  const float d = (hi ? c[1] : c[0]) + __shfl_xor_sync(FULL, hi ? c[0] : c[1], 2);
+  return d + __shfl_xor_sync(FULL, d, 1);
+}
+
+// slot of the even lane 2q after warp_reduce_scatter9 (15: none)
+__device__ __forceinline__ int slot9(int q) {
+  return (int)((0xFFF8F765FF43F210ull >> (4 * q)) & 15u);
+}
+
 // F64: the FP64-sum mode — the warp sums are added into double accumulators
 // (V.gacc64), so the result does not depend on the order in which warps and
 // tiles finish to well below float32 resolution.
@@ -666,7 +728,7 @@ int dispatch(const BlendBatch &bb, const ZeroSpans &zero, const BlendCfg &cfg, u
     return FWD ? run_fwd<P_, B_>(bb, queue, s) : run_bwd<P_, B_>(bb, zero, queue, s);
   DMGS_BLEND_CASE(1, 128) DMGS_BLEND_CASE(1, 256) DMGS_BLEND_CASE(1, 512)
   DMGS_BLEND_CASE(2, 128) DMGS_BLEND_CASE(2, 256) DMGS_BLEND_CASE(2, 512)
-  DMGS_BLEND_CASE(4, 128) DMGS_BLEND_CASE(4, 256) DMGS_BLEND_CASE(4, 512)
+  DMGS_BLEND_CASE(4, 256) DMGS_BLEND_CASE(4, 512)  // (4, 128): blend_warp.cu, before this dispatch
 #undef DMGS_BLEND_CASE
 #define DMGS_BLEND_PAIR(P_, B_)                                                     \
   if (pair && cfg.ppt == P_ && cfg.batch == B_)                                     \

@@ -21,14 +21,6 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
-// Exponent (base 2) of the Gaussian at (dx, dy).  Explicit intrinsics: the
-// adjoint evaluates the identical sequence.
-__device__ __forceinline__ float exponent2(float A, float B, float C, float dx, float dy) {
-  const float ax2 = __fmul_rn(__fmul_rn(A, dx), dx);
-  const float q = __fmul_rn(B, dx);
-  return __fmaf_rn(__fmaf_rn(C, dy, q), dy, ax2);
-}
-
 // The 48-byte record of list entry id; an entry outside the Gaussians (which
 // a correct list never holds) reads as a zero-opacity record, whose
 // footprint is empty, so no read leaves the geometry state.
@@ -52,61 +44,6 @@ __device__ __forceinline__ float rcp_approx(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-
-// From the thread's sums (e[0] = sum Gd, e[1] = sum Gd dy, e[2] = sum Gd dy^2
-// over its pixels; u = o Gd = dL/dpower) to the gradient terms: e0 =
-// dL/dndc_x, e1 = dL/dndc_y, e2..e4 = (sum u dx^2, sum u dx dy, sum u dy^2)
-// for the conic (scaled by -1/2, -1, -1/2 at the atomics), e5 = dL/dopacity.
-__device__ __forceinline__ void adjoint_finish(float dx, float o, const float4 &s2,
-                                               const float4 &s3, float *e) {
-  e[5] = e[0];
-  const float su = o * e[0], suy = o * e[1], suy2 = o * e[2];
-  const float sux = dx * su;
-  e[0] = sux * s2.z + suy * s2.w;
-  e[1] = suy * s3.x + sux * s3.y;
-  e[2] = sux * dx;
-  e[3] = suy * dx;
-  e[4] = suy2;
-}
-
-// Transposed reduce-scatter of the 9 gradient slots over the warp, 12
-// shuffles: each level halves the slots a lane keeps (5 | 4, 3 | 2, 2 | 1,
-// 1 | 1) and adds its partner's copy of them; afterwards the even lane 2q
-// holds the warp sum of slot slot9(q) (q = lane bits 4..1), none when that
-// is >= 9.
-__device__ __forceinline__ float warp_reduce_scatter9(const float (&v)[9], int lane) {
-  float a[5], b[3], c[2];
-  {
-    const bool hi = lane & 16;
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      const float up = i < 4 ? v[5 + i] : 0.f;
-      a[i] = (hi ? up : v[i]) + __shfl_xor_sync(FULL, hi ? v[i] : up, 16);
-    }
-  }
-  {
-    const bool hi = lane & 8;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const float up = i < 2 ? a[3 + i] : 0.f;
-      b[i] = (hi ? up : a[i]) + __shfl_xor_sync(FULL, hi ? a[i] : up, 8);
-    }
-  }
-  {
-    const bool hi = lane & 4;
-    c[0] = (hi ? b[2] : b[0]) + __shfl_xor_sync(FULL, hi ? b[0] : b[2], 4);
-    c[1] = (hi ? 0.f : b[1]) + __shfl_xor_sync(FULL, hi ? b[1] : 0.f, 4);
-  }
-  const bool hi = lane & 2;
-  const float d = (hi ? c[1] : c[0]) + __shfl_xor_sync(FULL, hi ? c[0] : c[1], 2);
-  return d + __shfl_xor_sync(FULL, d, 1);
-}
-
-// slot of the even lane 2q after warp_reduce_scatter9 (15: none)
-__device__ __forceinline__ int slot9(int q) {
-  return (int)((0xFFF8F765FF43F210ull >> (4 * q)) & 15u);
-}
-
 
 // A group's share (part of parts) of every span, set to zero by its `width`
 // threads.

@@ -61,7 +61,7 @@ constexpr int RADIX_TILE = RADIX_BLOCK * RADIX_ITEMS;  // 2048 keys per block
 constexpr int VGROUP = 32;               // tiles of RADIX_TILE Gaussians per group of visible counts
 constexpr int CHUNK_MIN_GAUSS = 64;     // visible Gaussians per binning chunk (mean, minimum)
 constexpr int CHUNK_COUNT_MAX = 2048;    // binning chunks per view (maximum)
-constexpr int CHUNK_W_GAUSS = 2;         // chunk weight of a Gaussian: this + ceil(rows / 16)
+constexpr int CHUNK_W_GAUSS = 2;         // chunk weight of a Gaussian: this + ceil(rows / 16) + ceil(tiles / 64)
 constexpr int SEG_MAX = 32;              // row segments (groups of chunks) per view, maximum
 constexpr int XSEG = 512;                // tiles of one row handled by a tile-emission block
 constexpr int BLEND_CLASSES = 32;        // classes of tiles by list length, longest first; the last: empty
@@ -201,11 +201,6 @@ inline size_t bwd_queue_offset(int P) { return align_up((size_t)P * 48, 256); }
 
 __device__ __forceinline__ uint32_t pack_u16x2(int lo, int hi) {
   return (uint32_t)lo | ((uint32_t)hi << 16);
-}
-
-__device__ __forceinline__ void red_add_v4(float *addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
-               :: "l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

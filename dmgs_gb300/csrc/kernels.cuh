@@ -47,7 +47,7 @@ constexpr int MAX_BIN_VIEWS = 16;
 
 // One view's binning: its geometry-state arrays and sizes.
 struct BinView {
-  int P, nb_pre, nb_radix;
+  int P, nb_radix;
   int gx, gy;            // tile grid
   int R, nb;             // segment counting: tile rows per band, bands
   int nxs;               // row pieces of at most XSEG tiles
@@ -71,21 +71,6 @@ struct BinViews {
   BinView v[MAX_BIN_VIEWS];
 };
 
-// One array per view for the generic scan.
-struct ScanView {
-  uint32_t *data;
-  const uint32_t *n_dev;  // device length (nullptr: n_max)
-  uint32_t n_max;
-  uint32_t *part;
-  uint32_t *total_out;
-  uint32_t *status;
-};
-
-struct ScanViews {
-  int n;
-  ScanView v[MAX_BIN_VIEWS];
-};
-
 // Fill one view's binning record from its geometry state; point_list /
 // K_alloc may be set later (after the instance count is known).
 // bin: the binning state (point list, then row lists: bin_layout(K_alloc)),
@@ -94,9 +79,8 @@ int make_bin_view(const GeomLayout &L, char *geom, uint32_t K_cap, char *bin, ui
                   BinView &B);
 int launch_binning_geometry(const BinViews &bv, cudaStream_t s);
 // Exclusive scan of one u32 array of n entries in place (part: scan_part_words(n)
-// words of scratch; total to *total_out, overflow bit into *status when given).
-int launch_scan1(uint32_t *data, uint32_t n, uint32_t *part, uint32_t *total_out,
-                 uint32_t *status, cudaStream_t s);
+// words of scratch; total to *total_out).
+int launch_scan1(uint32_t *data, uint32_t n, uint32_t *part, uint32_t *total_out, cudaStream_t s);
 size_t scan_part_words(uint32_t n);
 int launch_emit(const BinViews &bv, cudaStream_t s);
 int launch_debug_keys(const GeomLayout &L, const char *geom, const BinLayout &B, const char *bin,
