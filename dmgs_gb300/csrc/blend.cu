@@ -537,7 +537,7 @@ __device__ __forceinline__ int slot9(int q) {
 // tiles finish to well below float32 resolution.
 template <int PPT, int BATCH, bool F64 = false, int NT = 1>
 __global__ void __launch_bounds__(NT * 256 / PPT, (PPT == 4 ? 10 : (PPT == 2 ? 6 : 4)) / NT)
-blend_bwd_kernel(const BlendBatch bb, const ZeroSpans zero, uint32_t *queue) {
+blend_bwd_kernel(const BlendBatch bb, uint32_t *queue) {
   constexpr int THREADS = 256 / PPT;
   __shared__ float4 S0[NT][BATCH], S1[NT][BATCH], S2[NT][BATCH], S3[NT][BATCH];
   __shared__ uint32_t SM[NT][BATCH];                 // footprint rows
@@ -548,7 +548,6 @@ blend_bwd_kernel(const BlendBatch bb, const ZeroSpans zero, uint32_t *queue) {
   const int tid = (int)threadIdx.x - h * THREADS;
   const int lane = tid & 31;
   const PixelLayout<PPT> lay(tid);
-  zero_spans(zero, blockIdx.x, gridDim.x, threadIdx.x, blockDim.x);
   int slot_ = 0;
   for (int item = next_item(queue, slot_, &s_item); item < bb.total;
        item = next_item(queue, slot_, &s_item)) {
@@ -672,13 +671,13 @@ int run_fwd(const BlendBatch &bb, uint32_t *queue, cudaStream_t s) {
 }
 
 template <int PPT, int BATCH, bool F64 = false, int NT = 1>
-int run_bwd(const BlendBatch &bb, const ZeroSpans &zero, uint32_t *queue, cudaStream_t s) {
+int run_bwd(const BlendBatch &bb, uint32_t *queue, cudaStream_t s) {
   thread_local int cdev = -1, cslots = 0;  // per kernel instantiation and host thread
   int grid;
   const int r = grid_for(blend_bwd_kernel<PPT, BATCH, F64, NT>, NT * 256 / PPT, bb.total,
                          queue != nullptr, grid, cdev, cslots);
   if (r != DMGS_OK) return r;
-  dmgs_host::note_launch(), blend_bwd_kernel<PPT, BATCH, F64, NT><<<grid, NT * 256 / PPT, 0, s>>>(bb, zero, queue);
+  dmgs_host::note_launch(), blend_bwd_kernel<PPT, BATCH, F64, NT><<<grid, NT * 256 / PPT, 0, s>>>(bb, queue);
   return DMGS_OK;
 }
 
@@ -699,6 +698,13 @@ __global__ void __launch_bounds__(256) clear_gacc_kernel(const ClearViews cv, ui
   }
 }
 
+// The arrays of `zero` set to zero before an adjoint that does not do it while
+// it runs: a CTA per tile may be one CTA (3M Gaussians in a view of one tile).
+int clear_spans(const ZeroSpans &zero, cudaStream_t s) {
+  for (int k = 0; k < zero.n; ++k) DMGS_CUDA(cudaMemsetAsync(zero.p[k], 0, zero.words[k] * 4, s));
+  return DMGS_OK;
+}
+
 int launch_clear_gacc(const ClearViews &cv, int nviews, uint32_t *queue, cudaStream_t s) {
   uint32_t P = 1;
   for (int v = 0; v < nviews; ++v) P = max(P, cv.v[v].P);
@@ -716,8 +722,7 @@ __global__ void gacc_round_kernel(const double *__restrict__ g64, float *__restr
 }
 
 template <bool FWD>
-int dispatch(const BlendBatch &bb, const ZeroSpans &zero, const BlendCfg &cfg, uint32_t *queue,
-             cudaStream_t s) {
+int dispatch(const BlendBatch &bb, const BlendCfg &cfg, uint32_t *queue, cudaStream_t s) {
   const bool pair = cfg.sx * cfg.sy == 2;
   if (cfg.sx * cfg.sy > 2 || cfg.sx < 1 || cfg.sy < 1) {
     dmgs_host::set_error("unsupported blend CTA shape: %d x %d tiles", cfg.sx, cfg.sy);
@@ -725,14 +730,14 @@ int dispatch(const BlendBatch &bb, const ZeroSpans &zero, const BlendCfg &cfg, u
   }
 #define DMGS_BLEND_CASE(P_, B_)                                                     \
   if (!pair && cfg.ppt == P_ && cfg.batch == B_)                                    \
-    return FWD ? run_fwd<P_, B_>(bb, queue, s) : run_bwd<P_, B_>(bb, zero, queue, s);
+    return FWD ? run_fwd<P_, B_>(bb, queue, s) : run_bwd<P_, B_>(bb, queue, s);
   DMGS_BLEND_CASE(1, 128) DMGS_BLEND_CASE(1, 256) DMGS_BLEND_CASE(1, 512)
   DMGS_BLEND_CASE(2, 128) DMGS_BLEND_CASE(2, 256) DMGS_BLEND_CASE(2, 512)
   DMGS_BLEND_CASE(4, 256) DMGS_BLEND_CASE(4, 512)  // (4, 128): blend_warp.cu, before this dispatch
 #undef DMGS_BLEND_CASE
 #define DMGS_BLEND_PAIR(P_, B_)                                                     \
   if (pair && cfg.ppt == P_ && cfg.batch == B_)                                     \
-    return FWD ? run_fwd<P_, B_, 2>(bb, queue, s) : run_bwd<P_, B_, false, 2>(bb, zero, queue, s);
+    return FWD ? run_fwd<P_, B_, 2>(bb, queue, s) : run_bwd<P_, B_, false, 2>(bb, queue, s);
   DMGS_BLEND_PAIR(2, 128) DMGS_BLEND_PAIR(2, 256)
   DMGS_BLEND_PAIR(4, 128) DMGS_BLEND_PAIR(4, 256)
 #undef DMGS_BLEND_PAIR
@@ -773,7 +778,7 @@ int launch_blend_batch_fwd(const BlendBatch &bb, const BlendWork &wk, const Blen
   if (is_default(cfg)) return launch_blend_warp_fwd(bb, wk, queue, s);
   int r = DMGS_OK;
   const BlendBatch b = with_shape(bb, cfg);
-  DMGS_TIMED(K_BLEND_FWD, s, r = dispatch<true>(b, ZeroSpans(), cfg, queue, s));
+  DMGS_TIMED(K_BLEND_FWD, s, r = dispatch<true>(b, cfg, queue, s));
   if (r != DMGS_OK) return r;
   DMGS_LAUNCH_CHECK("blend_fwd_kernel");
   return DMGS_OK;
@@ -786,8 +791,9 @@ int launch_blend_batch_bwd(const BlendBatch &bb, const BlendWork &wk, const Clea
   int r = launch_clear_gacc(cv, bb.nviews, queue, s);
   if (r != DMGS_OK) return r;
   if (is_default(cfg)) return launch_blend_warp_bwd(bb, wk, zero, queue, s);
+  if (int z = clear_spans(zero, s)) return z;
   const BlendBatch b = with_shape(bb, cfg);
-  DMGS_TIMED(K_BLEND_BWD, s, r = dispatch<false>(b, zero, cfg, queue, s));
+  DMGS_TIMED(K_BLEND_BWD, s, r = dispatch<false>(b, cfg, queue, s));
   if (r != DMGS_OK) return r;
   DMGS_LAUNCH_CHECK("blend_bwd_kernel");
   return DMGS_OK;
@@ -856,7 +862,8 @@ int launch_blend_bwd(const ViewParams &vp, const GeomLayout &L, const char *geom
   DMGS_CUDA(cudaMemsetAsync(gacc64, 0, n * sizeof(double), s));
   if (bb.total > 0) {
     int r = DMGS_OK;
-    DMGS_TIMED(K_BLEND_BWD, s, r = (run_bwd<4, 128, true>(bb, zero, nullptr, s)));
+    if (int z = clear_spans(zero, s)) return z;
+    DMGS_TIMED(K_BLEND_BWD, s, r = (run_bwd<4, 128, true>(bb, nullptr, s)));
     if (r != DMGS_OK) return r;
     DMGS_LAUNCH_CHECK("blend_bwd_kernel (FP64 sums)");
   }
