@@ -358,11 +358,16 @@ __device__ __forceinline__ float inv_sqrt(float x) {
   return fmaf(fmaf(-x * y, y, 1.f), 0.5f * y, y);
 }
 
-// 1 / max(sqrt(x), NRM_EPS) for x >= 0 (the guard of torch's normalize); 0
-// where x, a sum of squares, has overflowed (the step would give inf * 0).
+// 1 / max(sqrt(x), NRM_EPS) for finite x >= 0 (the guard of torch's normalize).
 __device__ __forceinline__ float inv_norm(float x) {
-  if (!(x > NRM_EPS * NRM_EPS)) return 1.f / NRM_EPS;
-  return x < __int_as_float(0x7f800000) ? inv_sqrt(x) : 0.f;
+  return x > NRM_EPS * NRM_EPS ? inv_sqrt(x) : 1.f / NRM_EPS;
+}
+
+// The same of a caller's pair, whose squares may overflow: 0 then (the
+// Newton-Raphson step would give inf * 0).
+__device__ __forceinline__ float inv_norm2(float a, float b) {
+  const float x = a * a + b * b, r = inv_norm(x);
+  return x < __int_as_float(0x7f800000) || x != x ? r : 0.f;
 }
 
 // Unit quaternion (w, x, y, z), w >= 0, of a rotation matrix (row-major),
@@ -492,7 +497,7 @@ bind3_fwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, float *__restrict__ xyz,
         float4 quat = make_float4(0.f, 0.f, 0.f, 0.f);
         if (rots) {
           const float ra = in_r2[2 * q], rb = in_r2[2 * q + 1];
-          const float cn = inv_norm(ra * ra + rb * rb);
+          const float cn = inv_norm2(ra, rb);
           const float a = ra * cn, s = rb * cn;
           // R = Rw * [[a,-s,0],[s,a,0],[0,0,1]]
           float R[9];
@@ -586,7 +591,7 @@ bind3_bwd_kernel(DmgsFaceBinding3 b, FaceBlocks kb, const float *__restrict__ dx
         }
         if (drots) {
           const float ra = in_r2[2 * q], rb = in_r2[2 * q + 1];
-          const float cn = inv_norm(ra * ra + rb * rb);
+          const float cn = inv_norm2(ra, rb);
           const float a = ra * cn, s = rb * cn;
           float R[9];
 #pragma unroll
