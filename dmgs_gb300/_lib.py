@@ -211,11 +211,7 @@ def native():
 
 def native_call(name, *args):
     """The result of the native entry `name`, or None when the call needs the
-    general form (see csrc/autograd.cpp).  A call under torch.jit.trace does:
-    the tracer records Python autograd functions, and would keep a native
-    node's outputs as constants."""
-    if torch.jit.is_tracing():
-        return None
+    general form (see csrc/autograd.cpp)."""
     n = native()
     return None if n is None else getattr(n, name)(*args)
 

@@ -10,6 +10,7 @@
 // marshalling, tensor bookkeeping and the engine thread's wait for the
 // interpreter lock), more than most of these kernels run.
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <c10/cuda/CUDAStream.h>
 #include <pybind11/pybind11.h>
 #include <torch/csrc/Exceptions.h>
@@ -67,6 +68,10 @@ Tensor grad_of(const Tensor &g, at::IntArrayRef sizes, const Tensor &like) {
   if (!g.defined()) return at::zeros(sizes, like.options().dtype(at::kFloat));
   return g.to(like.device(), at::kFloat).contiguous();
 }
+
+// Under torch.jit.trace the tracer records Python autograd functions, and would
+// keep a native node's outputs as constants: such a call takes the general form.
+bool traced() { return at::tracer::impl::is_dispatch_enabled(); }
 
 // The tensor of a Python argument: false unless it is None (undefined) or a
 // tensor.
@@ -192,6 +197,7 @@ py::object raster(py::handle means_, py::handle means2D_, py::handle sh_, py::ha
                   py::handle scales_, py::handle rots_, py::handle cov_, py::handle bg_, py::handle view_,
                   py::handle proj_, py::handle campos_, int64_t H, int64_t W, double tanx, double tany,
                   double modifier, int64_t degree, bool prefiltered) {
+  if (traced()) return py::none();
   Tensor means, means2D, sh, colors, opac, scales, rots, cov;
   RasterSettings rs;
   if (!unpack(means_, means) || !unpack(means2D_, means2D) || !unpack(sh_, sh) || !unpack(colors_, colors) ||
@@ -245,6 +251,7 @@ struct Loss : public Function<Loss> {
 };
 
 py::object l1_ssim(py::handle x_, py::handle y_, double lambda) {
+  if (traced()) return py::none();
   Tensor x, y;
   if (!unpack(x_, x) || !unpack(y_, y) || !x.defined() || !plain(x, x.device()) || !plain(y, x.device()) ||
       x.dim() != 3 || x.sizes() != y.sizes() || x.numel() > INT32_MAX)
@@ -284,6 +291,7 @@ struct ShColors : public Function<ShColors> {
 };
 
 py::object sh_colors(py::handle sh_, py::handle xyz_, py::handle campos_, int64_t deg) {
+  if (traced()) return py::none();
   Tensor sh, xyz, cam;
   if (!unpack(sh_, sh) || !unpack(xyz_, xyz) || !unpack(campos_, cam) || !xyz.defined()) return py::none();
   const at::Device d = xyz.device();
@@ -348,6 +356,7 @@ struct Bind2 : public Function<Bind2> {
 
 py::object bind2(py::handle v_, py::handle sf_, py::handle f_, py::handle bc_, int64_t G, bool per_g, double rad_base,
                  double z_scale, double max_scale, bool adaptive) {
+  if (traced()) return py::none();
   Tensor v, sf, f, bc;
   if (!unpack(v_, v) || !unpack(sf_, sf) || !unpack(f_, f) || !unpack(bc_, bc) || !v.defined()) return py::none();
   const at::Device d = v.device();
@@ -399,6 +408,7 @@ struct Bind3 : public Function<Bind3> {
 };
 
 py::object bind3(py::handle v_, py::handle s2_, py::handle r2_, py::handle f_, py::handle bc_, double thin_z) {
+  if (traced()) return py::none();
   Tensor v, s2, r2, f, bc;
   if (!unpack(v_, v) || !unpack(s2_, s2) || !unpack(r2_, r2) || !unpack(f_, f) || !unpack(bc_, bc) || !v.defined())
     return py::none();
@@ -478,6 +488,7 @@ struct Texture : public Function<Texture> {
 
 py::object texture(py::handle x_, py::handle t_, py::handle w1_, py::handle w2_, py::handle w3_, py::sequence aabb,
                    double pls, bool keep_enc) {
+  if (traced()) return py::none();
   Tensor x, t, w1, w2, w3;
   if (!unpack(x_, x) || !unpack(t_, t) || !unpack(w1_, w1) || !unpack(w2_, w2) || !unpack(w3_, w3) || !x.defined())
     return py::none();
@@ -586,6 +597,7 @@ struct FlexiCubes : public Function<FlexiCubes> {
 
 py::object flexicubes(py::handle x_, py::handle s_, py::handle beta_, py::handle alpha_, py::handle gamma_,
                       py::handle vmask_, int64_t rx, int64_t ry, int64_t rz, bool training, bool fused, bool nocheck) {
+  if (traced()) return py::none();
   Tensor x, s, beta, alpha, gamma, vmask;
   if (!unpack(x_, x) || !unpack(s_, s) || !unpack(beta_, beta) || !unpack(alpha_, alpha) || !unpack(gamma_, gamma) ||
       !unpack(vmask_, vmask) || !x.defined())
