@@ -152,10 +152,17 @@ struct Mine {
   __device__ Mine() : pg(((threadIdx.x >> 6) << 3) | (threadIdx.x & 7)), jg((threadIdx.x >> 3) & 7) {}
 };
 
-// [rows][32] weights into rows of pitch WP.
+// [rows][32] weights into rows of pitch WP, in flight while the block's first
+// points are encoded: weights_in() before the barrier after which they are read.
+// (Waited for at once they made a block of one tile slower than a thread per
+// point: forward alone, 1,000 points at 48 channels, 20.5 us with a thread per
+// point, 22.5 waited for, 18.5 so; 271,824 points 131, 108 and 100 us.)
 __device__ __forceinline__ void load_weights(const float *__restrict__ W, int rows, float *sW) {
-  for (int i = threadIdx.x; i < rows * 32; i += TEX_THREADS) sW[(i >> 5) * WP + (i & 31)] = W[i];
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(sW);
+  for (int i = threadIdx.x; i < rows * 32; i += TEX_THREADS)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s + 4u * ((i >> 5) * WP + (i & 31))), "l"(W + i) : "memory");
 }
+__device__ __forceinline__ void weights_in() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // The points' [n][C] rows of a tile to and from X[feature][point]: a warp
 // takes 8 features of 4 points (whole 32-byte sectors; the 32 shared-memory
@@ -265,9 +272,9 @@ __device__ __forceinline__ void store_relu(const F2 (&acc)[4][4], const Mine &m,
 
 // Forward.  The encoding's gathers (the table is L2-resident) want warps in
 // flight, the layers shared-memory bandwidth; blocks in different phases
-// cover for each other.  271,824 points, 48 channels, float32: 160 us with a
-// thread per point, 119 us so (130 at five blocks an SM and 197 at six: the
-// shared memory they take is L1 that the gathers lose).
+// cover for each other.  271,824 points, 48 channels, float32, the encoding
+// kept: 160 us with a thread per point, 119 us so (130 at five blocks an SM and
+// 197 at six: the shared memory they take is L1 that the gathers lose).
 template <int C>
 __global__ void __launch_bounds__(TEX_THREADS, 4)
 tex_fwd_kernel(const TexArgs A, const TexLevels L, const float *__restrict__ xyz, float *__restrict__ out,
@@ -286,8 +293,9 @@ tex_fwd_kernel(const TexArgs A, const TexLevels L, const float *__restrict__ xyz
   const int64_t ntiles = (A.n + TEX_THREADS - 1) / TEX_THREADS;
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int64_t p0 = tile * TEX_THREADS;
-    __syncthreads();  // the weights are in; the last tile's outputs are out
+    __syncthreads();  // the levels are in; the last tile's outputs are out
     encode_tile(A, sL, xyz, p0 + threadIdx.x, X);
+    weights_in();
     __syncthreads();
     if (enc_out) store_rows<32, TEX_THREADS, XP>(enc_out, p0, A.n, X);  // kept for the adjoint
     {
@@ -441,12 +449,13 @@ tex_bwd_kernel(const TexArgs A, const TexLevels L, const float *__restrict__ xyz
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int64_t p0 = tile * TEX_THREADS;
     F2 g[4][4];
-    __syncthreads();  // the weights are in; the last tile's reads are done
+    __syncthreads();  // the levels are in; the last tile's reads are done
     if (enc_in) {
       load_rows<32>(enc, p0, A.n, D);
     } else {
       encode_tile(A, sL, xyz, p0 + threadIdx.x, D);
     }
+    weights_in();
     __syncthreads();
     if (!enc_in) store_rows<32, TEX_THREADS, XP>(denc, p0, A.n, D);
     layer<4, 32>(D, sW1, m, g);
