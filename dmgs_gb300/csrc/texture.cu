@@ -416,7 +416,7 @@ __device__ __forceinline__ void reduce_outer(const float (&acc)[R][4], float *S,
 // dL/dout, then the encoding again), H1 and H2 (the hidden layers, each
 // replaced by its own gradient).  Bound by shared-memory bandwidth; 75 KB, so
 // three blocks an SM.  271,824 points, 48 channels, float32: 269 us with a
-// thread per point, 150 us so.
+// thread per point, 150 us so (142 with the weights in flight).
 constexpr size_t tex_bwd_smem(int C) {
   return (size_t)((64 + C) * WP + (C > 32 ? C : 32) * XP + 2 * 32 * XP) * sizeof(float);
 }
